@@ -38,8 +38,8 @@ struct Workspace {
     float *x = nullptr, *nx = nullptr, *qkv = nullptr, *att = nullptr, *act = nullptr, *gate = nullptr, *up = nullptr;
     float *logits = nullptr, *logits_local = nullptr, *last_x = nullptr, *part = nullptr, *ids = nullptr;
     // bf16 hi/lo split of the activations the next tensor-core product reads (written by the kernel that finishes the
-    // previous product): [M, max(H, I_l)] each
-    __nv_bfloat16 *p_hi = nullptr, *p_lo = nullptr;
+    // previous product): the normed rows [M, H], and the SwiGLU rows [M, I_l] (the product that writes them still reads the former)
+    __nv_bfloat16 *p_hi = nullptr, *p_lo = nullptr, *g_hi = nullptr, *g_lo = nullptr;
     size_t part_bytes = 0;
     float *h_ids = nullptr;     // pinned
     float *h_logits = nullptr;  // pinned
@@ -115,14 +115,15 @@ int ensure_workspace(lumen_llama *m, size_t M) {
     size_t o_x = take(M * m->H), o_nx = take(M * m->H), o_qkv = take(M * qkvd), o_att = take(M * m->qd_l);
     // gate and up are adjacent: the fused step runs them as one product into [M, 2 * I_l]
     size_t o_act = take(M * m->inter_l), o_gate = take(2 * M * m->inter_l);
-    const size_t pair_floats = (M * std::max(m->H, m->inter_l) + 1) / 2 + 8;
-    size_t o_phi = take(pair_floats), o_plo = take(pair_floats);
+    auto half = [](size_t n) { return (n + 1) / 2 + 8; };
+    size_t o_phi = take(half(M * m->H)), o_plo = take(half(M * m->H)), o_ghi = take(half(M * m->inter_l)), o_glo = take(half(M * m->inter_l));
     size_t o_logits = take(M * m->V), o_ll = take(T > 1 ? T * M * m->vocab_l : 0), o_last = take(M * m->H);
     size_t o_part = take(w.part_bytes / sizeof(float)), o_ids = take(M);
     LUMEN_CUDA(ctx, cudaMalloc(&w.base, off));
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w.base + o); };
     w.x = at(o_x); w.nx = at(o_nx); w.qkv = at(o_qkv); w.att = at(o_att); w.act = at(o_act); w.gate = at(o_gate);
     w.up = w.gate + M * m->inter_l; w.p_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_phi)); w.p_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_plo));
+    w.g_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_ghi)); w.g_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_glo));
     w.logits = at(o_logits); w.logits_local = at(o_ll); w.last_x = at(o_last); w.part = at(o_part);
     w.ids = at(o_ids);
     LUMEN_CUDA(ctx, cudaMallocHost(&w.h_ids, std::max<size_t>(M, 1) * sizeof(float)));
@@ -188,7 +189,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     const float *res_x = (!tp || ctx->tp_rank == 0) ? w.x : nullptr;
 
     // Fused step (tiled products only): every product's finishing kernel writes what the next product reads, as the bf16
-    // hi/lo pair in w.p_hi / w.p_lo, and gate and up run as one product over their adjacent weights.  Per block:
+    // hi/lo pair in w.p_hi / w.p_lo (SwiGLU: w.g_hi / w.g_lo), and gate and up run as one product over their adjacent weights.  Per block:
     // qkv product + split-K sum, attention, o_proj (split + product + finisher), gate/up (product + finisher),
     // down (product + finisher) = 11 launches instead of 20.
     static const bool no_fuse = [] {
@@ -227,11 +228,11 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         return launch_bump_len(ctx, c->d_len, (int)p.S, s);
     };
     // Row-parallel product of the fused step: x = x + a . W^T summed over the ranks, and the split of RMSNorm(x) * norm_w
-    // for the next product (norm_w null after the last block).  `a` null: the activations are the pair already.
+    // for the next product (norm_w null after the last block).  `a` null: the activations are the SwiGLU pair.
     auto row_parallel = [&](const float *a, const void *wmat, size_t K, const float *norm_w) -> int {
         GemmFuse f;
         use_weight_split(m, wmat, f);
-        if (!a) { f.a_hi = w.p_hi; f.a_lo = w.p_lo; }
+        if (!a) { f.a_hi = w.g_hi; f.a_lo = w.g_lo; }
         if (!tp) {
             f.post = GemmFuse::kPostNorm; f.norm_w = norm_w; f.eps = eps; f.next_hi = w.p_hi; f.next_lo = w.p_lo;
             return launch_gemm_tc(ctx, a, wmat, wdt, w.x, M, K, H, res_x, s, nullptr, &f);
@@ -263,7 +264,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
             LUMEN_TRY(attend(lw, c));
             LUMEN_TRY(row_parallel(w.att, lw.wo, m->qd_l, lw.norm2));
             GemmFuse fg;
-            fg.a_hi = w.p_hi; fg.a_lo = w.p_lo; fg.post = GemmFuse::kPostSwiglu; fg.next_hi = w.p_hi; fg.next_lo = w.p_lo;
+            fg.a_hi = w.p_hi; fg.a_lo = w.p_lo; fg.post = GemmFuse::kPostSwiglu; fg.next_hi = w.g_hi; fg.next_lo = w.g_lo;
             use_weight_split(m, lw.wgate, fg);
             LUMEN_TRY(launch_gemm_tc(ctx, nullptr, lw.wgate, wdt, w.gate, M, H, 2 * m->inter_l, nullptr, s, nullptr, &fg));
             nx_ready = l + 1 < m->L;

@@ -26,12 +26,6 @@ __global__ void __launch_bounds__(256) sum_norm_split_kernel(const float *__rest
     }
 }
 
-// SiLU::forward — src/layers/activation.rs:143-146
-__device__ __forceinline__ float silu_mul1(float g, float u) {
-    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
-    return __fmul_rn(__fmul_rn(g, sig), u);
-}
-
 // part: [splits][rows][2 * inter]; thread = 4 adjacent columns of one row
 __global__ void __launch_bounds__(256) sum_swiglu_split_kernel(const float *__restrict__ part, int splits, size_t rows, size_t inter,
                                                                __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {

@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "decoder_kernels.cuh"
+#include "gemm_pair.cuh"
 #include "tc_common.cuh"
 
 namespace lumen {
@@ -389,9 +390,15 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
         return e && e[0] == '1';
     }();
     const bool swap = M <= 64 && !no_swap;
+    // More than one row of 128-row tiles: pairs of SMs (gemm_pair.cu).
+    const bool pair = M > (size_t)kBM && N >= 128;
+    const bool glu = pair && fuse && fuse->post == GemmFuse::kPostSwiglu && !tp && N % 16 == 0 && fuse->next_hi != hi && fuse->next_lo != lo;
+    // (slices of K are added by the kernel that reads the product anyway)
+    const GemmPairPlan plan = pair ? plan_gemm_pair(M, K, N, wsplit ? 3 : 2, glu, tp || (fuse && fuse->post == GemmFuse::kPostNorm), ctx->num_sms) : GemmPairPlan();
     CUtensorMap map_hi, map_lo, map_b, map_blo;  // 128-row side (hi, lo), BN-row side (hi, lo)
     const int bn = swap ? 64 : pick_bn(M, N, ctx->num_sms);
-    if (!swap) {
+    if (pair) {
+    } else if (!swap) {
         if (rc == LUMEN_OK) rc = make_map(ctx, &map_hi, hi, M, K, kBM);
         if (rc == LUMEN_OK) rc = make_map(ctx, &map_lo, lo, M, K, kBM);
         if (rc == LUMEN_OK) rc = make_map(ctx, &map_b, wsplit ? (const void *)whi : w, N, K, bn);
@@ -411,7 +418,7 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
         splits = std::max(1, std::min(std::min(ctx->num_sms / std::max(tiles, 1), kb_all / 4), 16));
     }
     const int kb_per_split = (kb_all + splits - 1) / splits;
-    splits = (kb_all + kb_per_split - 1) / kb_per_split;
+    splits = pair ? plan.splits : (kb_all + kb_per_split - 1) / kb_per_split;
     void *partial = nullptr;
     if (rc == LUMEN_OK && splits > 1) rc = dev_alloc(ctx, (size_t)splits * M * N * sizeof(float), &partial);
     if (rc == LUMEN_OK) {
@@ -422,7 +429,14 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
         p.kb_per_split = kb_per_split;
         p.status = ctx->d_status;
 #define LUMEN_TC(NA_, NB_, BN_, SW_) launch_tc_kernel<NA_, NB_, BN_, SW_>(ctx, map_hi, map_lo, map_b, map_blo, p, M, N, s)
-        if (swap) rc = wsplit ? LUMEN_TC(2, 2, 64, true) : LUMEN_TC(1, 2, 64, true);
+        if (pair) {
+            GemmPairArgs g;
+            g.a_hi = hi; g.a_lo = lo;
+            g.w_hi = wsplit ? whi : static_cast<const __nv_bfloat16 *>(w); g.w_lo = wsplit ? wlo : nullptr;
+            g.M = M; g.K = K; g.N = N; g.c = p.c; g.residual = p.residual;
+            if (glu) { g.out_hi = fuse->next_hi; g.out_lo = fuse->next_lo; }
+            rc = launch_gemm_pair(ctx, g, plan, s);
+        } else if (swap) rc = wsplit ? LUMEN_TC(2, 2, 64, true) : LUMEN_TC(1, 2, 64, true);
         else if (wsplit) rc = bn == 128 ? LUMEN_TC(2, 2, 128, false) : bn == 64 ? LUMEN_TC(2, 2, 64, false) : LUMEN_TC(2, 2, 32, false);
         else rc = bn == 128 ? LUMEN_TC(2, 1, 128, false) : bn == 64 ? LUMEN_TC(2, 1, 64, false) : LUMEN_TC(2, 1, 32, false);
 #undef LUMEN_TC
@@ -437,7 +451,7 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
             else if (fuse->norm_w)  // c is complete (the product's epilogue added the residual): only the norm outputs are missing
                 rc = launch_sum_norm_split(ctx, c, 1, nullptr, M, N, nullptr, fuse->norm_w, fuse->eps, fuse->next_hi, fuse->next_lo, s);
         } else if (rc == LUMEN_OK && fuse && fuse->post == GemmFuse::kPostSwiglu) {
-            rc = launch_sum_swiglu_split(ctx, splits > 1 ? static_cast<const float *>(partial) : c, splits, M, N / 2, fuse->next_hi,
+            if (!glu) rc = launch_sum_swiglu_split(ctx, splits > 1 ? static_cast<const float *>(partial) : c, splits, M, N / 2, fuse->next_hi,
                                          fuse->next_lo, s);
         } else if (rc == LUMEN_OK && splits > 1) {
             const size_t mn = M * N;

@@ -26,6 +26,12 @@ __device__ __forceinline__ void split4(float4 v, uint2 *hi, uint2 *lo) {
     lo->y = (unsigned)__bfloat16_as_ushort(l2) | ((unsigned)__bfloat16_as_ushort(l3) << 16);
 }
 
+// SiLU::forward — src/layers/activation.rs:143-146
+__device__ __forceinline__ float silu_mul1(float g, float u) {
+    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-g)));
+    return __fmul_rn(__fmul_rn(g, sig), u);
+}
+
 // What follows the sum of a row.
 struct RowFinish {
     float *out;            // [rows, dim] the summed row (null: not stored)

@@ -110,6 +110,19 @@ def test_long_prompt_slices_tensor_core_prefill(L, oracle, over, wdt):
         assert rel_err(k, ocaches[l].k) < 5e-5 and rel_err(v, ocaches[l].v) < 5e-5
 
 
+@pytest.mark.parametrize("inter,prompt", [(136, 129), (200, 300), (264, 513), (128, 256)])
+@pytest.mark.parametrize("wdt", ["f32", "bf16"])
+def test_prefill_of_more_than_one_row_tile(L, oracle, inter, prompt, wdt):
+    """Prompts whose products run as 256-row tiles: gate and up in one tile with SwiGLU in its epilogue (edges of the tile in both
+    directions), and products in slices of K that the norm's kernel adds."""
+    cfg = small_cfg(hidden_size=128, num_attention_heads=2, num_key_value_heads=2, intermediate_size=inter, max_seq_len=520)
+    params = make_params(L, cfg, 31, std=0.08, round_bf16=(wdt == "bf16"), random_norms=True)
+    ids = np.random.default_rng(32).integers(0, cfg["vocab_size"], size=(1, prompt)).astype(np.float32)
+    got, _, _ = _gpu_run(L, cfg, params, ids, prompt, wdt)
+    want, _ = _oracle_run(oracle, cfg, params, ids, prompt, "f64")
+    assert rel_err(got, want) < TOL_F32
+
+
 def test_forward_last_and_device_entry_points(L, oracle):
     cfg = small_cfg()
     params = make_params(L, cfg, 31, std=0.08)

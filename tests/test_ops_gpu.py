@@ -87,6 +87,20 @@ def test_tensor_core_gemm_shapes(L, oracle, m, k, n, bf16):
     assert rel_err(got, want) < 2e-5, rel_err(got, want)
 
 
+@pytest.mark.parametrize("bf16", [True, False])
+@pytest.mark.parametrize("m,k,n", [(129, 8, 128), (256, 64, 256), (257, 72, 255), (300, 1000, 385), (2300, 328, 129), (5000, 136, 1030)])
+def test_paired_tile_edges(L, m, k, n, bf16):
+    """Products of more than 128 rows (256-row tiles by pairs of SMs): one row and one column beyond a tile, rows that are no whole
+    vector, fewer K blocks than ring stages, and more tiles than pairs of SMs (tile rows in several groups).  Tolerance as above:
+    operands are split in two bf16 halves, 2^-17 of each."""
+    rng = np.random.default_rng(m + k + n)
+    a = rng.standard_normal((m, k), dtype=np.float32)
+    w = rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.05)
+    wt = L.Tensor.from_bf16(w) if bf16 else L.Tensor.from_array_no_grad(w)
+    got = L.matmul(L.Tensor.from_array_no_grad(a), wt).data()
+    assert rel_err(got, a.astype(np.float64) @ wt.data().astype(np.float64).T) < 2e-5
+
+
 def test_matmul_batched_leading_dims_and_errors(L, oracle):
     rng = np.random.default_rng(0)
     a = rng.standard_normal((2, 3, 16), dtype=np.float32)
