@@ -467,10 +467,13 @@ int run_mega(lumen_llama *m, lumen_kv_cache **caches) {
     p.actT = p.qkvT + ((p.qkv_rows + 1) & ~1);
     p.partT = p.actT + ((p.I + 1) & ~1);
     p.epoch_base = ctx->mega_epoch;
-    // Attention work items = heads x splits, at most one per SM, with at least 128 rows per split.
+    p.past = (int)caches[0]->len;
+    // Attention work items = heads x splits, at most one per SM, with at least 256 rows per split (a split's rows
+    // are in shared memory before it starts, while every further split adds to what each CTA merges: one layer of TinyLlama at 1000
+    // positions, attention and merge, 12.1 us with 3 or 4 splits, 15.4 with one; of the 7B shape at 525 18.3 with 2, 18.7 with 4, 22.8 with one).
     const size_t len = caches[0]->len + 1;
     int nsplit = std::max(1, std::min(decode_mega_max_splits(), ctx->num_sms / std::max(1, p.Hq)));
-    nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, len / 128));
+    nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, len / 256));
     p.nsplit = nsplit;
     p.abort_flag = reinterpret_cast<int *>(ctx->d_mega_sync + 1);
     p.status = ctx->d_status;

@@ -55,6 +55,7 @@ constexpr int kRowBlock = 64;              // rows reduced together (one per con
 constexpr int kMaxSeg = 8;                 // segments a row is cut into at most
 constexpr int kPartCols = kMaxSeg;         // columns of the table of partial row sums: one per segment
 constexpr int kMaxSplit = 4;               // attention splits merged in the o_proj prologue
+constexpr int kKvTileRows = 64;            // cached rows of a K or V tile at most (two scores per lane)
 constexpr long long kWaitCycles = 400000000LL;  // ~0.2 s at 1.9 GHz
 constexpr long long kPrefetchGrace = 1000;      // a ring that has been full for this long is a stall, not back-pressure
 constexpr long long kPrefetchPace = 600;        // cycles between the L2 prefetches of consecutive 16 KB tiles (~54 KB/us)
@@ -109,6 +110,11 @@ __device__ __forceinline__ void bulk_load(void *dst_smem, const void *src, uint3
         ::"r"(smem_u32(dst_smem)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
         : "memory");
 }
+// The same without a cache hint.
+__device__ __forceinline__ void bulk_load_keep(void *dst_smem, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst_smem)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 // 3-D tiled TMA copy: box of the map at (0, unit, row) -> this CTA's shared memory.  The innermost coordinate is
 // always 0, so the 16-byte start rule of TMA holds.
 __device__ __forceinline__ void tensor_load(void *dst_smem, const CUtensorMap *map, int unit, int row, uint64_t *bar, uint64_t pol) {
@@ -118,9 +124,6 @@ __device__ __forceinline__ void tensor_load(void *dst_smem, const CUtensorMap *m
         : "memory");
 }
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory"); }
-struct ConsumerBar {
-    __device__ __forceinline__ void operator()() const { consumer_bar(); }
-};
 // A consumer barrier after which all consumer threads agree on whether the CTA is aborting.  Exits must be
 // uniform (a thread that left would make the next bar.sync wait forever), so the flag is sampled by
 // thread 0 before the barrier into a slot that alternates with `k`, and read by everyone after it.
@@ -313,20 +316,62 @@ __device__ __forceinline__ void prefetch_entry(const MegaParams &p, const uint4 
 // per copy by a single thread, which capped the stream at one tile per ~0.33 us.  A batch is issued in passes of
 // at most S tiles: within a pass no two tiles share a stage, so a stage's barrier is never tested for a use
 // before the use before it has been issued (a parity test tells two uses apart, not three).
-__device__ __forceinline__ void producer_loop(const MegaParams &p, Shared &sh, int cta, int lane) {
+// Cached rows of K and V travel through the ring too: an attention work item's rows do not depend on this token, so they
+// are in shared memory by the time its q has crossed.  Tiles of kv_tile_rows rows, K and V in turn.
+__host__ __device__ __forceinline__ int kv_tile_rows(int D, int stage_bytes) {
+    const int rows = stage_bytes / (4 * D);
+    return rows < kKvTileRows ? rows : kKvTileRows;
+}
+// The CTA's attention work of one layer: `items` work items (heads x context splits, dealt out in turn; more than one per CTA only
+// when there are more heads than CTAs, and then every item walks all rows), each over cached rows [j0, j1).
+struct KvWork {
+    int items, j0, j1, tile_rows, pairs;
+    __device__ __forceinline__ KvWork(const MegaParams &p, int stage_bytes, int cta, int nctas) {
+        const int all = p.Hq * p.nsplit;
+        items = cta < all ? (all - cta + nctas - 1) / nctas : 0;
+        const int total = p.past + 1, chunk = (total + p.nsplit - 1) / p.nsplit;
+        j0 = (cta % p.nsplit) * chunk;
+        j1 = min(min(total, j0 + chunk), p.past);
+        if (p.debug_flags & 1) j1 = j0;  // debug: nothing is streamed
+        tile_rows = kv_tile_rows(p.D, stage_bytes);
+        pairs = (max(0, j1 - j0) + tile_rows - 1) / tile_rows;
+    }
+    __device__ __forceinline__ int tiles() const { return 2 * items * pairs; }
+};
+// Entry r of a layer's K/V copies (see MegaParams::sched; bit 30 of w: no evict-first, the heads of a group read the same rows).
+__device__ __forceinline__ uint4 kv_entry(const MegaParams &p, const KvWork &kv, int layer, int r, int cta, int nctas) {
+    const int item = r / (2 * kv.pairs), t = r - item * 2 * kv.pairs;
+    const int h = (cta + item * nctas) / p.nsplit, hk = h / (p.Hq / p.Hkv);
+    const int row = kv.j0 + (t >> 1) * kv.tile_rows, rows = min(kv.tile_rows, kv.j1 - row);
+    const float *base = (t & 1) ? p.layers[layer].v_cache : p.layers[layer].k_cache;
+    const unsigned long long a = (unsigned long long)(uintptr_t)(base + ((size_t)hk * p.max_seq + row) * p.D);
+    const uint32_t bytes = (uint32_t)(rows * p.D * 4);
+    return make_uint4((uint32_t)a, (uint32_t)(a >> 32), bytes | ((uint32_t)(5 * layer + 1) << 16), bytes | 0x40000000u);
+}
+
+__device__ __forceinline__ void producer_loop(const MegaParams &p, Shared &sh, int cta, int nctas, int lane) {
     const uint64_t pol = make_evict_first_policy();
     const int nphases = 5 * p.L + 1;
     const uint4 *sched = p.sched + (size_t)cta * p.sched_stride;
-    const int n = p.sched_count[cta];
+    // The schedule is the same for every token but for the K/V tiles, which belong after the first layer's q/k/v tiles
+    // (`lead` entries) and then after every further `stretch` entries (o, gate/up, down, the next layer's q/k/v).
+    const int n_static = p.sched_count[cta], lead = p.sched_count[nctas + cta], stretch = p.sched_count[2 * nctas + cta];
+    const KvWork kv(p, sh.stage_bytes, cta, nctas);
+    const int kvn = kv.tiles(), n = n_static + p.L * kvn;
+    auto entry = [&](int v) {
+        if (v < lead || kvn == 0) return sched[v];
+        const int l = min((v - lead) / (kvn + stretch), p.L - 1), r = v - lead - l * (kvn + stretch);
+        return r < kvn ? kv_entry(p, kv, l, r, cta, nctas) : sched[lead + l * stretch + r - kvn];
+    };
     const uint32_t S = (uint32_t)sh.S;
     uint32_t tiles = 0;  // tiles before the current batch (the same in every lane)
     int last_ph = -1;    // trace: phase of the last entry of the previous batch
     bool carry_pf = false;
     bool ok = true;
-    uint4 nxt = lane < n ? sched[lane] : make_uint4(0u, 0u, 0u, 0u);
+    uint4 nxt = lane < n ? entry(lane) : make_uint4(0u, 0u, 0u, 0u);
     for (int base = 0; base < n && ok; base += 32) {
         const uint4 e = nxt;
-        if (base + 32 + lane < n) nxt = sched[base + 32 + lane];
+        if (base + 32 + lane < n) nxt = entry(base + 32 + lane);
         const bool valid = base + lane < n;
         const bool first = valid && (e.w & 0xffffu) != 0;  // first copy of a tile
         const uint32_t firsts = __ballot_sync(0xffffffffu, first);
@@ -360,7 +405,9 @@ __device__ __forceinline__ void producer_loop(const MegaParams &p, Shared &sh, i
                     if (e.w & 0x80000000u) {  // box of rows x one segment of the row length (3-D tiled copy)
                         tensor_load(dst, p.tmaps + (e.x & 0xffffu), (int)(e.x >> 16), (int)e.y, &sh.full[slot], pol);
                     } else {
-                        bulk_load(dst, reinterpret_cast<const char *>(((unsigned long long)e.y << 32) | e.x), e.z & 0xffffu, &sh.full[slot], pol);
+                        const char *src = reinterpret_cast<const char *>(((unsigned long long)e.y << 32) | e.x);
+                        if (e.w & 0x40000000u) bulk_load_keep(dst, src, e.z & 0xffffu, &sh.full[slot]);
+                        else bulk_load(dst, src, e.z & 0xffffu, &sh.full[slot], pol);
                     }
                     if (first) sh.issued[slot] = (int)use;
                     waiting = false;
@@ -475,8 +522,8 @@ template <int kBatch>  // 16-byte loads in flight per thread and pass
 __device__ __forceinline__ void poll_vector_pass(const MegaParams &p, Shared &sh, const uint4 *s4, int npairs, int base, uint32_t tag,
                                                  float *xs, int tid, int site, const StageOpts o, float &ss) {
     uint4 v[kBatch];
-    // up to 8 loads per thread the gains wait in registers; longer vectors fetch them after the wait instead
-    constexpr bool kEarlyGains = kBatch <= 8;
+    // up to 10 loads per thread the gains wait in registers; longer vectors fetch them after the wait instead
+    constexpr bool kEarlyGains = kBatch <= 10;
     float2 g[kEarlyGains ? kBatch : 1];
     if (kEarlyGains) {
 #pragma unroll
@@ -530,6 +577,7 @@ __device__ __forceinline__ bool poll_vector(const MegaParams &p, Shared &sh, con
     // costs a round trip through L2.  Every pass is such a round trip too.
     if (per_thread <= 4) poll_vector_pass<4>(p, sh, s4, npairs, 0, tag, xs, tid, site, o, ss);
     else if (per_thread <= 8) poll_vector_pass<8>(p, sh, s4, npairs, 0, tag, xs, tid, site, o, ss);
+    else if (per_thread <= 10) poll_vector_pass<10>(p, sh, s4, npairs, 0, tag, xs, tid, site, o, ss);
     else
         for (int base = 0; base < npairs; base += kConsumers * 13) poll_vector_pass<13>(p, sh, s4, npairs, base, tag, xs, tid, site, o, ss);
     publish_ss(sh, ss, tid);
@@ -935,6 +983,12 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
     }
     trace_stamp(p, cta, tid, 3 * ph + 1);
     trace_cta(p, cta, tid, 0, ph);
+    // The next RMSNorm's gains are read by every CTA at once, at the start of its phase: they should be in the L2 by then
+    // (from HBM, behind the stream of weights, they held up the 4096 numbers of the 7B shape by 8 us in every second phase).
+    if (stages_x && tid == 0) {
+        const float *next = g.kind == PH_QKV ? lw->norm2 : g.layer + 1 < p.L ? p.layers[g.layer + 1].norm1 : p.final_norm;
+        for (int k = cta * 32; k < p.H; k += nctas * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(next + k));
+    }
 
     // ---- tiles ------------------------------------------------------------------------------------------
     // Tiles are addressed in closed form (see PhaseTiles) and sit in ring slot (tiles consumed so far + t).
@@ -1068,62 +1122,179 @@ struct TaggedPartOut {
     }
 };
 
-// Waits for this step's q (head h), k and v (KV head hk) projections and copies them to shared memory
-// raw[3*D]; runs inside the attention item after its first K/V row requests are in flight.
-struct StageQKV {
-    const MegaParams *p;  // the kernel's __grid_constant__ block: taking its address costs nothing
-    volatile int *abort;  // (a pointer to the Shared struct itself would force it into local memory)
-    float *raw;
-    int h, hk, tid;
-    uint32_t tag;
-    __device__ __forceinline__ void operator()() const {
-        const int D = p->D, half = D / 2;
-        for (int t = tid; t < 3 * half; t += kConsumers) {
-            const int which = t / half, i = t % half;
-            const uint2 *src = which == 0 ? p->qkvT + (size_t)h * D
-                                          : p->qkvT + p->qd + (which == 2 ? p->kvd : 0) + (size_t)hk * D;
-            const uint4 *s4 = reinterpret_cast<const uint4 *>(src) + i;
-            const long long t0 = clock64();
-            int spins = 0;
-            uint4 v = ld_tagged2(s4);
-            while ((v.y != tag || v.w != tag) && poll_continue(*p, abort, spins, t0, 340, t)) v = ld_tagged2(s4);
-            *reinterpret_cast<float2 *>(raw + which * D + 2 * i) = make_float2(__uint_as_float(v.x), __uint_as_float(v.z));
-        }
-        consumer_bar();
+// Waits for this step's q (head h), k and v (KV head hk) projections and copies them to shared memory raw[3*D].
+__device__ __forceinline__ void stage_qkv(const MegaParams &p, volatile int *abort, float *raw, int h, int hk, int tid, uint32_t tag) {
+    const int D = p.D, half = D / 2;
+    for (int t = tid; t < 3 * half; t += kConsumers) {
+        const int which = t / half, i = t % half;
+        const uint2 *src = which == 0 ? p.qkvT + (size_t)h * D : p.qkvT + p.qd + (which == 2 ? p.kvd : 0) + (size_t)hk * D;
+        const uint4 *s4 = reinterpret_cast<const uint4 *>(src) + i;
+        const long long t0 = clock64();
+        int spins = 0;
+        uint4 v = ld_tagged2(s4);
+        while ((v.y != tag || v.w != tag) && poll_continue(p, abort, spins, t0, 340, t)) v = ld_tagged2(s4);
+        *reinterpret_cast<float2 *>(raw + which * D + 2 * i) = make_float2(__uint_as_float(v.x), __uint_as_float(v.z));
     }
-};
+    consumer_bar();
+}
 
-// Receives plain values only: a reference to the kernel's Shared struct inside the functors below would
-// push that struct into local memory.
-__device__ __forceinline__ void attention_items(const MegaParams &p, float *attn_smem, volatile int *abort, int layer, int ph, int past,
-                                             int cta, int nctas, int tid) {
-    const int items = p.Hq * p.nsplit;
-    const MegaLayer &l = p.layers[layer];
-    float *raw = attn_smem + attn_decode_smem_floats(1, p.D, kConsumerWarps);
-    DecodeParams dp;
-    dp.q = raw; dp.k_new = raw + p.D; dp.v_new = raw + 2 * p.D;
-    dp.q_stride = 0; dp.kv_stride = 0;
-    dp.k_cache = l.k_cache; dp.v_cache = l.v_cache; dp.d_len = l.d_len;
-    dp.Hq = p.Hq; dp.Hkv = p.Hkv; dp.D = p.D; dp.max_seq = p.max_seq;
-    dp.cos_t = p.cos_t; dp.sin_t = p.sin_t; dp.q_norm = l.qn; dp.k_norm = l.kn;
-    dp.norm_eps = p.eps; dp.scale = p.scale;
-    dp.part_m = nullptr; dp.part_l = nullptr; dp.part_ctx = nullptr;
-    dp.nsplit = p.nsplit;
-    const TaggedPartOut out{p.partT, 2 + p.D, p.nsplit, phase_tag(p, ph)};
-    for (int item = cta; item < items; item += nctas) {
-        const int h = item / p.nsplit, split = item % p.nsplit;
-        const StageQKV stage{&p, abort, raw, h, h / (p.Hq / p.Hkv), tid, phase_tag(p, ph - 1)};
-        // two lane layouts cover head_dim <= 128 (the launcher rejects larger heads)
-        if (p.D <= 64) attn_decode_item<1, 2, true, kConsumerWarps>(dp, attn_smem, 0, h, split, tid, past, ConsumerBar(), out, stage);
-        else attn_decode_item<1, 4, true, kConsumerWarps>(dp, attn_smem, 0, h, split, tid, past, ConsumerBar(), out, stage);
+// Scratch of an attention item in floats: q and the new k (rotated), q | k | v as they arrived, per-warp maximum, sum and context,
+// per-warp softmax weights of a tile.
+__host__ __device__ inline size_t mega_attn_floats(int D) { return 5 * (size_t)D + 16 + (size_t)kConsumerWarps * D + (size_t)kConsumerWarps * kKvTileRows; }
+
+// Waits for the next tile of the ring (position `slot`); the warp that owns the tile calls.
+__device__ __forceinline__ const float *ring_wait(const MegaParams &p, Shared &sh, uint32_t slot, int lane, int site, bool &have) {
+    const int rs = (int)(slot % (uint32_t)sh.S);
+    const uint32_t use = slot / (uint32_t)sh.S;
+    have = stage_use_seen(p, sh, rs, (int)use, site) && mbar_wait(p, sh, &sh.full[rs], use & 1, site + 1);
+    if (have && lane == 0) sh.seen[rs] = (int)use + 1;
+    return reinterpret_cast<const float *>(sh.stages + (size_t)rs * sh.stage_bytes);
+}
+__device__ __forceinline__ void ring_release(Shared &sh, uint32_t slot, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cnt(&sh.empty[slot % (uint32_t)sh.S], 1);
+}
+
+// One attention work item: head h, context split `split` (self_attention.rs:141-297; softmax(q.K^T * scale).V as pieces merged by
+// log-sum-exp).  The cached rows [kv.j0, kv.j1) are the next tiles of the ring, K and V in turn; a warp takes a pair of
+// tiles at a time: a lane forms the scores of one or two rows alone (16-byte reads in an order rotated by lane, so that the
+// 32 rows it reads side by side fall into different banks), the warp agrees on the tile's maximum, and the lanes then
+// share out the context's elements and walk the rows of V.  Row `past` (this token's) comes from shared memory.
+// VE = elements of the context per lane (2: D <= 64, 4: D <= 128).
+// Why through the ring: read straight from the cache, 28 to 56 rows per round trip to HBM, a layer's attention took 10.1 us for
+// TinyLlama at 1000 positions and 15.3 / 29.9 us for the 7B shape at 525 / 1900; from shared memory it takes 4.5 and 8.6 / 13.6 us
+// (3.8 us at 40 positions, where the exchange of q, k and v is all there is).
+template <int VE>
+__device__ __forceinline__ void attention_item(const MegaParams &p, Shared &sh, const MegaLayer &l, const KvWork &kv, RingPos &rp, int h, int split,
+                                               uint32_t tag, int ph, int tid) {
+    const int D = p.D, half = D / 2, lane = tid & 31, warp = tid >> 5, nch = D / 4;
+    const int G = p.Hq / p.Hkv, hk = h / G, past = p.past;
+    float *qs = sh.attn, *knew = qs + D, *raw = knew + D, *wm = raw + 3 * D, *wl = wm + 8, *wctx = wl + 8;
+    float *ws = wctx + kConsumerWarps * D + warp * kKvTileRows;
+    stage_qkv(p, sh.abort, raw, h, hk, tid, phase_tag(p, ph - 1));
+    const float *cos_row = p.cos_t + (size_t)past * half, *sin_row = p.sin_t + (size_t)past * half;
+    const int total = past + 1, chunk = (total + p.nsplit - 1) / p.nsplit;
+    const bool owns_new = past >= split * chunk && past < min(total, (split + 1) * chunk);
+    if (warp == 0) load_norm_rope<true>(qs, raw, D, l.qn, p.eps, cos_row, sin_row, lane);
+    if (owns_new && warp == kConsumerWarps - 1) {
+        load_norm_rope<true>(knew, raw + D, D, l.kn, p.eps, cos_row, sin_row, lane);
+        if (h % G == 0) {  // the first head of a KV head's group stores the row
+            float *k_row = l.k_cache + ((size_t)hk * p.max_seq + past) * D, *v_row = l.v_cache + ((size_t)hk * p.max_seq + past) * D;
+            for (int i = lane; i < D; i += 32) {
+                k_row[i] = knew[i];
+                v_row[i] = raw[2 * D + i];
+            }
+        }
+    }
+    consumer_bar();
+    float m = -INFINITY, lsum = 0.f, ctx[VE];  // lsum: this lane's share
+#pragma unroll
+    for (int i = 0; i < VE; ++i) ctx[i] = 0.f;
+    const int e0 = lane * VE;
+    const float4 *q4 = reinterpret_cast<const float4 *>(qs);
+    for (int pair = warp; pair < kv.pairs; pair += kConsumerWarps) {
+        const uint32_t slot = rp.n + 2u * (uint32_t)pair;
+        const int rows = min(kv.tile_rows, kv.j1 - (kv.j0 + pair * kv.tile_rows));
+        bool have;
+        const float4 *k4 = reinterpret_cast<const float4 *>(ring_wait(p, sh, slot, lane, 342, have));
+        float s[2] = {0.f, 0.f};
+        if (have) {
+            const int ra = min(lane, rows - 1), rb = min(lane + 32, rows - 1);
+            int c = lane % nch;
+            float t0[2] = {0.f, 0.f}, t1[2] = {0.f, 0.f};  // two chains per row
+            const bool second = rows > 32;
+#pragma unroll 4
+            for (int i = 0; i < nch; ++i) {
+                const float4 q = q4[c], a = k4[ra * nch + c];
+                t0[i & 1] = fmaf(q.w, a.w, fmaf(q.z, a.z, fmaf(q.y, a.y, fmaf(q.x, a.x, t0[i & 1]))));
+                if (second) {
+                    const float4 b = k4[rb * nch + c];
+                    t1[i & 1] = fmaf(q.w, b.w, fmaf(q.z, b.z, fmaf(q.y, b.y, fmaf(q.x, b.x, t1[i & 1]))));
+                }
+                c = c + 1 == nch ? 0 : c + 1;
+            }
+            s[0] = t0[0] + t0[1];
+            s[1] = t1[0] + t1[1];
+        }
+        ring_release(sh, slot, lane);
+        s[0] = lane < rows ? __fmul_rn(s[0], p.scale) : -INFINITY;
+        s[1] = lane + 32 < rows ? __fmul_rn(s[1], p.scale) : -INFINITY;
+        float top = fmaxf(s[0], s[1]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float mn = fmaxf(m, top), r = expf(m - mn);  // (a tile has at least one row; exp(-inf) = 0 on the first)
+        const float w0 = expf(s[0] - mn), w1 = expf(s[1] - mn);
+        lsum = fmaf(lsum, r, w0 + w1);
+        m = mn;
+        ws[lane] = w0;
+        ws[lane + 32] = w1;
+        __syncwarp();
+        const float *v = ring_wait(p, sh, slot + 1, lane, 344, have);
+#pragma unroll
+        for (int i = 0; i < VE; ++i) ctx[i] *= r;
+        if (have && e0 < D) {
+#pragma unroll 8
+            for (int j = 0; j < rows; ++j) {
+                const float w = ws[j];
+                if constexpr (VE == 4) {
+                    const float4 x = *reinterpret_cast<const float4 *>(v + j * D + e0);
+                    ctx[0] = fmaf(w, x.x, ctx[0]); ctx[1] = fmaf(w, x.y, ctx[1]); ctx[2] = fmaf(w, x.z, ctx[2]); ctx[3] = fmaf(w, x.w, ctx[3]);
+                } else {
+                    const float2 x = *reinterpret_cast<const float2 *>(v + j * D + e0);
+                    ctx[0] = fmaf(w, x.x, ctx[0]); ctx[1] = fmaf(w, x.y, ctx[1]);
+                }
+            }
+        }
+        ring_release(sh, slot + 1, lane);
+    }
+    if (owns_new && warp == kv.pairs % kConsumerWarps) {  // this token's row, by the warp that has least to do
+        float s = 0.f;
+        for (int i = lane; i < D; i += 32) s = fmaf(qs[i], knew[i], s);
+        s = __fmul_rn(warp_sum(s), p.scale);
+        const float mn = fmaxf(m, s), r = expf(m - mn), w = expf(s - mn);
+        lsum = fmaf(lsum, r, lane == 0 ? w : 0.f);
+        m = mn;
+#pragma unroll
+        for (int i = 0; i < VE; ++i) ctx[i] = e0 < D ? fmaf(w, raw[2 * D + e0 + i], ctx[i] * r) : 0.f;
+    }
+    rp.n += 2u * (uint32_t)kv.pairs;
+    // merge the warps
+    lsum = warp_sum(lsum);
+    if (lane == 0) {
+        wm[warp] = m;
+        wl[warp] = lsum;
+    }
+    if (e0 < D)
+#pragma unroll
+        for (int i = 0; i < VE; ++i) wctx[warp * D + e0 + i] = ctx[i];
+    consumer_bar();
+    const TaggedPartOut out{p.partT, 2 + D, p.nsplit, tag};
+    for (int e = tid; e < D; e += kConsumers) {
+        float M = -INFINITY, L = 0.f, c = 0.f;
+#pragma unroll
+        for (int w = 0; w < kConsumerWarps; ++w) M = fmaxf(M, wm[w]);
+#pragma unroll
+        for (int w = 0; w < kConsumerWarps; ++w) {
+            const float f = wm[w] == -INFINITY ? 0.f : expf(wm[w] - M);
+            L = fmaf(wl[w], f, L);
+            c = fmaf(wctx[w * D + e], f, c);
+        }
+        out(h, split, e, c, M, L);
     }
 }
 
-__device__ __forceinline__ bool attention_phase(const MegaParams &p, Shared &sh, int layer, int ph, int past, int cta, int nctas,
-                                                int tid, int &bk) {
-    if (cta >= p.Hq * p.nsplit) return true;  // no work item here: nothing to wait for
-    attention_items(p, sh.attn, sh.abort, layer, ph, past, cta, nctas, tid);
-    return consumer_bar_ok(sh.abort, sh.decision, tid, bk);
+__device__ __forceinline__ bool attention_phase(const MegaParams &p, Shared &sh, RingPos &rp, int layer, int ph, int cta, int nctas, int tid, int &bk) {
+    const KvWork kv(p, sh.stage_bytes, cta, nctas);
+    if (kv.items == 0) return true;  // no work item here: nothing to wait for
+    const MegaLayer &l = p.layers[layer];
+    for (int i = 0; i < kv.items; ++i) {
+        const int item = cta + i * nctas, h = item / p.nsplit, split = item % p.nsplit;
+        // two lane layouts cover head_dim <= 128 (the launcher rejects larger heads)
+        if (p.D <= 64) attention_item<2>(p, sh, l, kv, rp, h, split, phase_tag(p, ph), ph, tid);
+        else attention_item<4>(p, sh, l, kv, rp, h, split, phase_tag(p, ph), ph, tid);
+        if (!consumer_bar_ok(sh.abort, sh.decision, tid, bk)) return false;  // (the scratch is used again)
+    }
+    return true;
 }
 
 template <typename WT>
@@ -1131,7 +1302,6 @@ __device__ __forceinline__ void consumer_loop(const MegaParams &p, Shared &sh, i
     // Token id: f32 -> usize with Rust's saturating cast (embedding.rs:50); id >= vocab is the reference's
     // panic: record it and run nothing (every CTA takes the same branch).
     const float f = __ldcg(p.ids);
-    const int past = __ldcg(p.layers[0].d_len);  // context length before this token, the same for every layer
     const unsigned long long uid = (f != f || f <= 0.f) ? 0ull : (f >= 1.8e19f ? ~0ull : (unsigned long long)f);
     if (uid >= (unsigned long long)p.vocab) {
         if (cta == 0 && tid == 0 && atomicCAS(&p.status->code, 0, LUMEN_ERR_EMBED_RANGE) == 0) {
@@ -1157,7 +1327,7 @@ __device__ __forceinline__ void consumer_loop(const MegaParams &p, Shared &sh, i
         const Phase g = get_phase(p, p.layers, ph);
         trace_stamp(p, cta, tid, 3 * ph);
         if (g.kind == PH_ATT) {
-            if (!attention_phase(p, sh, g.layer, ph, past, cta, nctas, tid, bk)) return;
+            if (!attention_phase(p, sh, rp, g.layer, ph, cta, nctas, tid, bk)) return;
             trace_stamp(p, cta, tid, 3 * ph + 1);
             trace_stamp(p, cta, tid, 3 * ph + 2);
             if (cta < p.Hq * p.nsplit) trace_cta(p, cta, tid, 1, ph);
@@ -1191,9 +1361,10 @@ __device__ __forceinline__ void consumer_loop(const MegaParams &p, Shared &sh, i
             }
         }
     }
-    // c.len = new_len (self_attention.rs:179) for every layer's cache.  Every CTA read `past` before it did
-    // anything else, and the next launch starts only after this one has ended.
-    for (int l = tid; cta == 0 && l < p.L; l += kConsumers) *p.layers[l].d_len = past + 1;
+    // c.len = new_len (self_attention.rs:179) for every layer's cache, unless an earlier token that gave up is missing
+    // from it (its successors were already on their way; the host reads the length that is left here).
+    for (int l = tid; cta == 0 && l < p.L; l += kConsumers)
+        if (*p.layers[l].d_len == p.past) *p.layers[l].d_len = p.past + 1;
 }
 
 // The parameter block is __grid_constant__ so that helpers can take it by reference without the compiler
@@ -1217,7 +1388,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
     sh.xs = fl;
     sh.part = fl + mega_xs_floats(max(p.H, max(p.qd, p.I)));
     sh.red = fl + mega_table_floats(max(p.H, max(p.qd, p.I)));
-    sh.xraw = sh.red + kConsumerWarps;
+    sh.xraw = sh.red + 8;  // (what follows stays 16-byte aligned)
     sh.attn = sh.xraw + kRowBlock;
     sh.full = bars;
     sh.empty = bars + kMegaMaxStages;
@@ -1242,7 +1413,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
     __syncthreads();
     const int cta = blockIdx.x, nctas = gridDim.x;
     if (tid >= kConsumers) {
-        producer_loop(p, sh, cta, tid - kConsumers);
+        producer_loop(p, sh, cta, nctas, tid - kConsumers);
     } else {
         consumer_loop<WT>(p, sh, cta, nctas, tid);
     }
@@ -1252,8 +1423,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
 
 size_t decode_mega_smem_bytes(int stages, int stage_bytes, int head_dim, int kmax) {
     return (size_t)stages * stage_bytes +
-           (mega_table_floats(kmax) + kConsumerWarps + kRowBlock + attn_decode_smem_floats(1, head_dim, kConsumerWarps) + 3 * (size_t)head_dim) *
-               sizeof(float);
+           (mega_table_floats(kmax) + 8 + kRowBlock + mega_attn_floats(head_dim)) * sizeof(float);
 }
 
 int decode_mega_max_splits() { return kMaxSplit; }
@@ -1300,12 +1470,21 @@ void decode_mega_build_schedule(const MegaParams &p_in, const MegaLayer *host_la
     bool no_tensor = getenv("LUMEN_MEGA_NO_TENSOR_COPY") != nullptr;
     bool retry = false;
     std::vector<std::vector<uint4>> per;
+    std::vector<int> lead, stretch;
 build:
     tmaps.clear();
     per.assign(grid, std::vector<uint4>());
+    lead.assign(grid, 0);
+    stretch.assign(grid, 0);
     for (int ph = 0; ph < nphases; ++ph) {
         const Phase g = get_phase(p, host_layers, ph);
-        if (g.kind == PH_ATT) continue;
+        if (g.kind == PH_ATT) {  // the layer's K/V tiles belong here (all layers have the same shapes)
+            for (int cta = 0; cta < grid; ++cta) {
+                if (ph == PH_ATT) lead[cta] = (int)per[cta].size();
+                else stretch[cta] = ((int)per[cta].size() - lead[cta]) / g.layer;
+            }
+            continue;
+        }
         // Matrices whose rows are cut into segments get two tensor maps each (boxes of 4 rows and of 1 row).
         int map0[2] = {-1, -1};
         {
@@ -1374,9 +1553,11 @@ build:
     for (auto &v : per) mx = std::max(mx, v.size());
     stride = (int)((mx + 31) / 32 * 32);
     entries.assign((size_t)grid * stride, make_uint4(0u, 0u, 0u, 0u));
-    counts.resize(grid);
+    counts.resize(3 * (size_t)grid);
     for (int cta = 0; cta < grid; ++cta) {
         counts[cta] = (int)per[cta].size();
+        counts[grid + cta] = lead[cta];
+        counts[2 * grid + cta] = stretch[cta];
         std::copy(per[cta].begin(), per[cta].end(), entries.begin() + (size_t)cta * stride);
     }
 }

@@ -60,6 +60,7 @@ struct MegaParams {
     uint2 *partT;             // [Hq, nsplit, 2 + D]: {max}, {sum}, ctx[D] of every attention work item
     unsigned int epoch_base;
     int nsplit;
+    int past;  // context length before this token
     int *abort_flag;
     DeviceStatus *status;
     int stages, stage_bytes;            // filled by the launcher
@@ -76,7 +77,9 @@ struct MegaParams {
     //   had arrived, and [nph][kMegaTraceCtas] ns timestamp when the CTA had published the phase's results
     unsigned long long *trace;
     // Producer schedule: for CTA c the bulk copies of one token in issue order, sched[c * sched_stride + i],
-    // i < sched_count[c].  Entry = {src address lo, hi, copy bytes | phase << 16, tile bytes}; tile bytes is
+    // i < sched_count[c]; sched_count[grid + c] of them come before the first attention phase and
+    // sched_count[2 * grid + c] between two attention phases (the producer adds the copies of cached K and V rows there:
+    // their number grows with the context).  Entry = {src address lo, hi, copy bytes | phase << 16, tile bytes}; tile bytes is
     // non-zero on the first copy of a tile (= the transaction count of its stage) and 0 on the following ones.
     // The schedule depends only on the model's shapes and addresses, so it is built once on the host
     // (decode_mega_build_schedule) and the producer does no address arithmetic at all.
