@@ -23,7 +23,7 @@ struct DeviceStatus {
     int code;      // LUMEN_* code, 0 = ok
     int detail0;   // kernel-specific (e.g. the offending index)
     int detail1;
-    int pad;
+    int token;     // answer of the device sampler, fetched with the status
 };
 
 }  // namespace lumen
@@ -358,9 +358,8 @@ int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s
 bool attn_prefill_tc_usable(const AttnPrefillArgs &a);
 int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, const float *q_rot, cudaStream_t s);
 
-// Nucleus sampling of one logits vector on the device (sampler.cu); *token_dev is a device int.
-int launch_sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, float temperature, float top_p, float penalty,
-                        const int *recent_host, size_t n_recent, float r, int *token_dev, cudaStream_t s);
+// Nucleus sampling of one logits vector on the device (sampler.cu); waits for the stream.
+int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lumen_sample_params &sp, int32_t *token, cudaStream_t s);
 
 // LlamaKVCache::update: dst[h, start+s, :] = src[h, s, :].
 int launch_kv_slab_copy(lumen_ctx *ctx, const float *src, float *dst, size_t heads, size_t s_len, size_t d,

@@ -161,13 +161,7 @@ int lumen_model::forward_sample(const float *ids_host, size_t s, lumen_kv_cache 
     memcpy(io.h_ids, ids_host, s * sizeof(float));
     LUMEN_CUDA(ctx, cudaMemcpyAsync(io.ids, io.h_ids, s * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     LUMEN_TRY(run_forward(1, s, caches, true));  // last position's logits in io.logits[V]
-    int *token_dev = reinterpret_cast<int *>(io.ids);  // the id buffer is free again once the forward is enqueued behind it
-    LUMEN_TRY(launch_sample_top_p(ctx, io.logits, V, sp->temperature, sp->top_p, sp->repetition_penalty, sp->recent_tokens, sp->n_recent,
-                                  sp->uniform, token_dev, ctx->stream));
-    LUMEN_CUDA(ctx, cudaMemcpyAsync(io.h_ids, token_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    LUMEN_TRY(check_device_status(ctx));
-    memcpy(token_out, io.h_ids, sizeof(int));
-    return LUMEN_OK;
+    return sample_top_p(ctx, io.logits, V, *sp, token_out, ctx->stream);
 }
 
 int lumen_model::forward_device(const float *ids_dev, size_t b, size_t s, lumen_kv_cache **caches, size_t n_caches, float *logits_dev) {

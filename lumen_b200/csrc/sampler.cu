@@ -4,10 +4,17 @@
 // Same steps as the reference: repetition penalty over the recent tokens (one division per occurrence),
 // temperature (floored at 1e-5), softmax with 1/(sum + 1e-9), stable descending sort, nucleus cut at the
 // first rank where the cumulative probability reaches top_p (clamped to [1e-6, 1]), inverse-CDF walk over
-// probs[i] / cumulative with the caller's uniform draw.  The cumulative sums are added sequentially in f32 like
-// the reference's loops; the softmax denominator is a tree sum (the reference adds it sequentially), which
+// probs[i] / cumulative with the caller's uniform draw.  The cumulative sums carry the roundings of the reference's
+// sequential f32 loops; the softmax denominator is a tree sum (the reference adds it sequentially), which
 // moves every probability by the same last-ulp factor and the result only when the draw sits on a boundary.
-// The sort is cub::DeviceRadixSort (a library sort: this is not a hot loop).
+// One kernel on a cluster of eight SMs serves what chat loops ask for (sample_nucleus_kernel).  What it cannot hold
+// (nuclei that reach into probabilities below 2^-24, hundreds of nearly equal probabilities, vocabularies of more than
+// kNucleusMaxVocab, NaN) takes a kernel that forms the probabilities, cub::DeviceRadixSort (a library sort: not the hot
+// path) and a kernel that walks the sorted list.
+#include <climits>
+
+#include <cooperative_groups.h>
+
 #include <cub/cub.cuh>
 
 #include "common.cuh"
@@ -87,144 +94,454 @@ sample_prep_kernel(const float *__restrict__ logits, int n, float temperature, f
     }
 }
 
-// The reference adds the sorted probabilities one by one in f32 and stops at the first index where the
-// running sum reaches a threshold (main.rs:113-121 and :126-134).  With a flat distribution the rounding of
-// that sequential sum decides the index, so the order of the additions is kept: one thread adds the values in
-// order, 32 per test of the threshold (the block of 32 that crosses is then walked value by value), reading them
-// from shared memory, while the other three warps of the CTA stage the next 2048 values into the other half of a
-// double buffer (dividing by `scale` on the way: 1 for the cumulative probability, the nucleus mass for the
-// inverse-CDF walk).  What the walk costs is then the dependent chain of additions alone.  Returns the first
-// index < n whose running sum is >= threshold (n if none) and that running sum (the total if none).
-constexpr int kPickThreads = 128;
-constexpr int kPickChunk = 2048;
+// The reference adds the sorted probabilities one by one in f32 and stops at the first index where the running sum
+// reaches a threshold (main.rs:113-121 and :126-134).  With a flat distribution the rounding of that sequential sum
+// decides the index, so its roundings are kept, but not its order in time: while the sum stays within a binade, its
+// unit in the last place u is fixed and run / u is a whole number R, so that adding v >= 0 adds round(v / u) - which
+// depends on R only where v / u lies halfway between two whole numbers (the even sum wins), that is on R's parity.  A value is
+// therefore a function (parity of R) -> increment, the functions of consecutive values compose associatively, and a
+// block-wide scan gives every running sum exactly.  The value that takes R past 2^24 is added in f32 and the scan starts over
+// behind it with the next u: about one scan per doubling of the sum and one per 4096 values.  The first 256
+// values, over which the sum doubles most often, are added one by one.  (One thread adding everything takes 4 cycles a value:
+// 90 us for the two walks of a nucleus of 28800; a scan takes about 1 us.)
+constexpr int kPickThreads = 1024;
+constexpr int kPickWarps = kPickThreads / 32;
+constexpr int kPickHead = 256;             // values added one by one first
+constexpr uint32_t kPickFull = 1u << 24;   // R of the next binade
+constexpr uint32_t kPickSat = 1u << 30;    // increments saturate here: past the end of the binade they are not used
 
 struct PickShared {
-    __align__(16) float buf[2][kPickChunk];
+    __align__(16) float head[kPickHead];
+    uint2 total[2][kPickWarps];  // increments of a warp's values, for even and odd R (two sets: one is read while the next is written)
+    int at[2][kPickWarps];       // a warp's first value that ends the scan (INT_MAX: none),
+    uint32_t before[2][kPickWarps];  // R before it
+    float val[2][kPickWarps];        // and the value
     int found;
     float run;
 };
 
-__device__ __forceinline__ void stage_chunk(const float *__restrict__ vals, int n, int c0, float scale, float *dst, int first, int step) {
-    const int m = min(kPickChunk, n - c0);
-    for (int i = first; i < kPickChunk; i += step) dst[i] = i < m ? __fdiv_rn(vals[c0 + i], scale) : 0.f;  // zeros change no sum
+__device__ __forceinline__ uint2 pick_then(uint2 f, uint2 g) {  // f's values, then g's
+    return make_uint2(min(f.x + ((f.x & 1) ? g.y : g.x), kPickSat), min(f.y + ((f.y & 1) ? g.x : g.y), kPickSat));
+}
+__device__ __forceinline__ uint2 pick_inc(float w) {  // w = v / u < 2^24
+    const uint32_t q = (uint32_t)w;
+    const float frac = w - (float)q;
+    const uint32_t up = frac > 0.5f, tie = frac == 0.5f, odd = q & 1;
+    return make_uint2(q + (up | (tie & odd)), q + (up | (tie & (odd ^ 1))));
+}
+__device__ __forceinline__ uint2 pick_scan(uint2 f, int lane) {  // inclusive, over the warp's lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint2 g = make_uint2(__shfl_up_sync(0xffffffffu, f.x, o), __shfl_up_sync(0xffffffffu, f.y, o));
+        if (lane >= o) f = pick_then(g, f);
+    }
+    return f;
 }
 
-__device__ __forceinline__ int first_reaching(const float *__restrict__ vals, int n, float scale, float threshold, PickShared &sh,
-                                              float *sum_out) {
-    const int tid = threadIdx.x;
-    stage_chunk(vals, n, 0, scale, sh.buf[0], tid, kPickThreads);
-    if (tid == 0) {
-        sh.found = n;
-        sh.run = 0.f;
-    }
-    __syncthreads();
-    const int chunks = (n + kPickChunk - 1) / kPickChunk;
-    for (int c = 0; c < chunks; ++c) {
-        if (tid >= 32) {
-            if (c + 1 < chunks) stage_chunk(vals, n, (c + 1) * kPickChunk, scale, sh.buf[(c + 1) & 1], tid - 32, kPickThreads - 32);
-        } else if (tid == 0) {
-            const float *buf = sh.buf[c & 1];
-            const int c0 = c * kPickChunk, m = min(kPickChunk, n - c0);
-            float run = sh.run;
-            int found = n;
-            // 32 values per test of the threshold: eight 128-bit loads, then the dependent chain of 32 additions
-            for (int i = 0; i < m; i += 32) {
-                float4 v[8];
+// First index < n whose running sum of vals[i] / scale is >= threshold (n if none), and that running sum (the total if none).
+// vals is in descending order, all >= 0.  All kPickThreads threads call; the answers are the same in all of them.
+__device__ __forceinline__ int first_reaching(const float *vals, int n, float scale, float threshold, PickShared &sh, float *sum_out) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float run = 0.f;
+    int start = 0, turn = 0;  // values before `start` are in `run`
+    for (int base = 0; base < n; base += 4 * kPickThreads) {
+        const int i0 = base + 4 * tid;
+        float v[4];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const float4 *>(buf + i + 4 * j);
-                float t = run;
+        for (int q = 0; q < 4; ++q) v[q] = i0 + q < n ? __fdiv_rn(__ldcg(vals + i0 + q), scale) : 0.f;
+        if (base == 0) {
+            if (4 * tid < kPickHead) *reinterpret_cast<float4 *>(sh.head + 4 * tid) = make_float4(v[0], v[1], v[2], v[3]);
+            __syncthreads();
+            if (tid == 0) {
+                // 32 values per test of the threshold: eight 128-bit loads, then the dependent chain of 32 additions
+                const int m = min(n, kPickHead);
+                int found = -1;
+                for (int i = 0; i < m && found < 0; i += 32) {
+                    float4 x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    t = __fadd_rn(t, v[j].x);
-                    t = __fadd_rn(t, v[j].y);
-                    t = __fadd_rn(t, v[j].z);
-                    t = __fadd_rn(t, v[j].w);
-                }
-                if (t >= threshold) {  // the sums only grow: the crossing is inside these 32 (or in their zero padding)
-                    for (int j = 0; j < 32 && i + j < m; ++j) {
-                        run = __fadd_rn(run, buf[i + j]);
-                        if (run >= threshold) {
-                            found = c0 + i + j;
-                            break;
-                        }
+                    for (int j = 0; j < 8; ++j) x[j] = *reinterpret_cast<const float4 *>(sh.head + i + 4 * j);
+                    float t = run;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) t = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(t, x[j].x), x[j].y), x[j].z), x[j].w);
+                    if (!(t >= threshold)) {
+                        run = t;
+                        continue;
                     }
-                    if (found != n) break;
-                    continue;  // (only zero padding was left: t == run, and that was below the threshold)
+                    for (int j = i; j < m && found < 0; ++j) {  // the sums only grow: the crossing is inside these 32
+                        run = __fadd_rn(run, sh.head[j]);
+                        if (run >= threshold) found = j;
+                    }
                 }
-                run = t;
+                sh.found = found;
+                sh.run = run;
             }
-            sh.run = run;
-            sh.found = found;
+            __syncthreads();
+            run = sh.run;
+            start = kPickHead;
+            const int found = sh.found;
+            __syncthreads();  // everybody has read the words before the next walk writes them
+            if (found >= 0 || n <= kPickHead || !(run > 0.f)) {  // (NaN reaches nothing; behind a sum of zero there are only zeros)
+                *sum_out = run;
+                return found >= 0 ? found : n;
+            }
         }
-        __syncthreads();
-        const int f = sh.found;
-        __syncthreads();  // everybody has read the word before the walker writes it again
-        if (f != n) break;
+        while (start < min(n, base + 4 * kPickThreads)) {
+            // run in [2^(e-127), 2^(e-126)): u = 2^(e-150).  1 / n <= first value <= run < 2, so both powers are normal
+            const uint32_t e = __float_as_uint(run) >> 23;
+            const float per_u = __uint_as_float((277u - e) << 23), u = __uint_as_float((e - 23u) << 23);
+            const uint32_t r0 = (uint32_t)(run * per_u);
+            uint2 own[4], f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                own[q] = i0 + q >= start ? pick_inc(v[q] * per_u) : make_uint2(0u, 0u);
+                f = q == 0 ? own[0] : pick_then(f, own[q]);
+            }
+            const uint2 in = pick_scan(f, lane);
+            uint2 ex = make_uint2(__shfl_up_sync(0xffffffffu, in.x, 1), __shfl_up_sync(0xffffffffu, in.y, 1));
+            if (lane == 0) ex = make_uint2(0u, 0u);
+            if (lane == 31) sh.total[turn][warp] = in;
+            __syncthreads();
+            const uint2 w_in = pick_scan(sh.total[turn][lane], lane);
+            const int prev = max(warp - 1, 0);
+            uint2 w_ex = make_uint2(__shfl_sync(0xffffffffu, w_in.x, prev), __shfl_sync(0xffffffffu, w_in.y, prev));
+            if (warp == 0) w_ex = make_uint2(0u, 0u);
+            const uint2 all = make_uint2(__shfl_sync(0xffffffffu, w_in.x, 31), __shfl_sync(0xffffffffu, w_in.y, 31));
+            ex = pick_then(w_ex, ex);
+            uint32_t r = r0 + ((r0 & 1) ? ex.y : ex.x), before = r;
+            int at = INT_MAX;
+            float val = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t next = r + ((r & 1) ? own[q].y : own[q].x);
+                if (at == INT_MAX && (next >= kPickFull || (float)next * u >= threshold)) {
+                    at = i0 + q;
+                    before = r;
+                    val = v[q];
+                }
+                r = next;
+            }
+            const uint32_t hit = __ballot_sync(0xffffffffu, at != INT_MAX);
+            if (hit ? lane == __ffs(hit) - 1 : lane == 0) {
+                sh.at[turn][warp] = at;
+                sh.before[turn][warp] = before;
+                sh.val[turn][warp] = val;
+            }
+            __syncthreads();
+            const uint32_t hits = __ballot_sync(0xffffffffu, sh.at[turn][lane] != INT_MAX);
+            if (!hits) {
+                run = (float)(r0 + ((r0 & 1) ? all.y : all.x)) * u;
+                start = base + 4 * kPickThreads;
+            } else {
+                const int w = __ffs(hits) - 1;
+                run = __fadd_rn((float)sh.before[turn][w] * u, sh.val[turn][w]);
+                start = sh.at[turn][w] + 1;
+                if (run >= threshold) {
+                    *sum_out = run;
+                    __syncthreads();  // (the next walk starts with the same set)
+                    return start - 1;
+                }
+            }
+            turn ^= 1;
+        }
     }
-    const int found = sh.found;
-    *sum_out = sh.run;
-    __syncthreads();  // the buffers and the two words are reused by the next walk
-    return found;
+    *sum_out = run;
+    __syncthreads();
+    return n;
+}
+
+// Rank of the drawn token in the sorted list.  `all`: the list is complete; otherwise -1 where it ends before the nucleus does.
+__device__ __forceinline__ int pick_rank(const float *sorted_p, int n, bool all, float target, float r, PickShared &sh) {
+    float cumulative, acc;
+    const int at = first_reaching(sorted_p, n, 1.0f, target, sh, &cumulative);  // main.rs:113-121
+    if (at == n && !all) return -1;
+    const int cut = max(1, min(n, at + 1));
+    // main.rs:126-134: acc += probs[i] / cumulative; the first i with r <= acc, else the last of the nucleus
+    return min(first_reaching(sorted_p, cut, cumulative, r, sh, &acc), cut - 1);
 }
 
 __global__ void __launch_bounds__(kPickThreads)
-sample_pick_kernel(const float *__restrict__ sorted_p, const int *__restrict__ sorted_i, int n, float top_p, float r,
-                   int *__restrict__ token_out) {
+sample_pick_kernel(const float *__restrict__ sorted_p, const int *__restrict__ sorted_i, int n, float target, float r, int *__restrict__ token_out) {
     __shared__ PickShared sh;
-    const float target = fmaxf(fminf(fmaxf(top_p, 0.f), 1.f), 1e-6f);
-    float cumulative;
-    const int at = first_reaching(sorted_p, n, 1.0f, target, sh, &cumulative);  // main.rs:113-121
-    const int cut = max(1, min(n, at + 1));
-    float acc;
-    // main.rs:126-134: acc += probs[i] / cumulative; the first i with r <= acc, else the last of the nucleus
-    const int pick = first_reaching(sorted_p, cut, cumulative, r, sh, &acc);
-    if (threadIdx.x == 0) *token_out = sorted_i[min(pick, cut - 1)];
+    const int pick = pick_rank(sorted_p, n, true, target, r, sh);
+    if (threadIdx.x == 0) *token_out = sorted_i[pick];
+}
+
+// ---- one kernel ---------------------------------------------------------------------------------------------------
+// A cluster of eight CTAs holds the vocabulary in shared memory: CTA c owns the columns [128 c, 128 c + 128) of every 1024
+// logits, the columns whose partial sums sample_prep_kernel's threads 128 c .. 128 c + 127 form, so that both kernels add the softmax
+// denominator in the same order and agree on every bit of a probability.
+// Only the nucleus is sorted.  The probabilities are counted by exponent and seven bits of mantissa (128 bins per octave, 24
+// octaves); from the counts and the bins' lower edges every CTA finds the bin that certainly completes the nucleus, and the
+// offsets of the bins in descending order.  The candidates are scattered into their bins (global memory: tens of KB in the L2), and
+// a candidate's rank within its bin is the number of larger ones (an equal probability of a smaller index is larger: the sort
+// is stable).  CTA 0 then walks the list as the general path does.
+// What bounds it is the chain of passes and cluster barriers, not bytes.  32000 logits of which some hundred to a thousand make the
+// nucleus: 33 us against 100 us for the seven kernels of the general path, 56 us against 140 us for the whole call.
+namespace cg = cooperative_groups;
+constexpr int kCluster = 8;
+constexpr int kNucleusBins = 24 * 128;
+constexpr int kBinsPerThread = kNucleusBins / kPrepThreads;
+constexpr uint32_t kTopBin = 0x3f800000u >> 16;  // of probability 1
+constexpr int kMaxBin = 512;                      // ranking is quadratic in a bin's size
+constexpr int kNucleusMaxVocab = 256 * 1024;      // 128 KB of shared memory per CTA
+static_assert(kPrepThreads == kPickThreads && kBinsPerThread * kPrepThreads == kNucleusBins, "");
+
+struct NucleusArgs {
+    const float *logits;
+    int n;
+    float temperature, penalty, target, r;
+    unsigned long long *cand;  // [n] probability bits : ~index
+    float *sorted_p;           // [n]
+    int *sorted_i;             // [n]
+    int *token;                // the token, or -1: not served here
+    int n_recent;
+    int recent[kMaxRecent];
+};
+
+struct NucleusShared {
+    int hist[kNucleusBins], cursor[kNucleusBins], first[kNucleusBins + 1];  // counts here; next place; first place of a bin
+    __align__(16) unsigned long long window[kPrepThreads / 32][32];
+    float red[33], top, part[4];
+    int scan_n[32];
+    float scan_m[32];
+    int last_bin, crowded;
+    PickShared pick;
+};
+
+__device__ __forceinline__ int bin_of(float p) { return (int)kTopBin - (int)(__float_as_uint(p) >> 16); }
+
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads) sample_nucleus_kernel(const __grid_constant__ NucleusArgs a) {
+    extern __shared__ __align__(16) unsigned char nucleus_smem[];
+    NucleusShared &sh = *reinterpret_cast<NucleusShared *>(nucleus_smem);
+    float *vals = reinterpret_cast<float *>(nucleus_smem + sizeof(NucleusShared));
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank(), n = a.n;
+    const int slots = (n + 1023) / 1024 * 128;
+    auto index_of = [&](int s) { return (s >> 7) * 1024 + rank * 128 + (s & 127); };
+#pragma unroll 4
+    for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? a.logits[index_of(s)] : -INFINITY;
+    for (int b = tid; b < kNucleusBins; b += kPrepThreads) sh.hist[b] = 0;
+    if (tid == 0) {
+        sh.last_bin = INT_MAX;
+        sh.crowded = 0;
+    }
+    __syncthreads();
+    if (a.penalty > 1.0f && tid < a.n_recent) {
+        // the first occurrence of a token applies one division per occurrence (main.rs:83-89)
+        const int t = a.recent[tid];
+        bool first = t >= 0 && t < n && ((t >> 7) & (kCluster - 1)) == rank;
+        for (int k = 0; k < tid && first; ++k) first = a.recent[k] != t;
+        if (first) {
+            float &x = vals[(t >> 10) * 128 + (t & 127)];
+            for (int k = tid; k < a.n_recent; ++k)
+                if (a.recent[k] == t) x = __fdiv_rn(x, a.penalty);
+        }
+    }
+    __syncthreads();
+    const float temp = fmaxf(a.temperature, 1e-5f);
+    float mx = -INFINITY;
+    for (int s = tid; s < slots; s += kPrepThreads) {
+        const float x = __fdiv_rn(vals[s], temp);
+        vals[s] = x;
+        if (index_of(s) < n) mx = fmaxf(mx, x);
+    }
+    mx = block_reduce(mx, sh.red, true);
+    if (tid == 0) sh.top = mx;
+    cluster.sync();
+#pragma unroll
+    for (int c = 0; c < kCluster; ++c) mx = fmaxf(mx, *cluster.map_shared_rank(&sh.top, c));
+    for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? expf(__fsub_rn(vals[s], mx)) : 0.f;
+    __syncthreads();
+    if (tid < 128) {
+        float sum = 0.f;
+#pragma unroll 8
+        for (int s = tid; s < slots; s += 128) sum += vals[s];  // (adding the zeros behind the end changes nothing)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) sh.part[warp] = sum;
+    }
+    cluster.sync();
+    float sum = *cluster.map_shared_rank(&sh.part[lane & 3], lane >> 2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float inv = __fdiv_rn(1.0f, __fadd_rn(sum, 1e-9f));
+    const bool finite = inv > 0.f && inv < INFINITY;  // (the same in every CTA)
+    for (int s = tid; s < slots; s += kPrepThreads) {
+        const float p = __fmul_rn(vals[s], inv);
+        vals[s] = p;
+        const int b = bin_of(p);
+        if (finite && b < kNucleusBins && index_of(s) < n) atomicAdd(&sh.hist[b], 1);
+    }
+    cluster.sync();
+    // Thread t's bins; all CTAs form the same totals in the same order.
+    int total[kBinsPerThread], lower[kBinsPerThread], count = 0;  // lower: of the CTAs before this one
+    float mass = 0.f;
+#pragma unroll
+    for (int j = 0; j < kBinsPerThread; ++j) {
+        const int b = tid * kBinsPerThread + j;
+        total[j] = lower[j] = 0;
+#pragma unroll
+        for (int c = 0; c < kCluster; ++c) {
+            const int h = *cluster.map_shared_rank(&sh.hist[b], c);
+            if (c < rank) lower[j] += h;
+            total[j] += h;
+        }
+        count += total[j];
+        mass += (float)total[j] * __uint_as_float((kTopBin - (uint32_t)b) << 16);
+    }
+    int count_in = count;
+    float mass_in = mass;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int c = __shfl_up_sync(0xffffffffu, count_in, o);
+        const float m = __shfl_up_sync(0xffffffffu, mass_in, o);
+        if (lane >= o) {
+            count_in += c;
+            mass_in += m;
+        }
+    }
+    if (lane == 31) {
+        sh.scan_n[warp] = count_in;
+        sh.scan_m[warp] = mass_in;
+    }
+    __syncthreads();
+    int at = count_in - count, counted = 0;
+    float reached = mass_in - mass;
+    for (int w = 0; w < kPrepThreads / 32; ++w) {
+        if (w < warp) {
+            at += sh.scan_n[w];
+            reached += sh.scan_m[w];
+        }
+        counted += sh.scan_n[w];
+    }
+    const float need = a.target * (1.0f + 1.0f / 4096);  // (the sequential sum may round down a little; checked by the walk)
+#pragma unroll
+    for (int j = 0; j < kBinsPerThread; ++j) {
+        const int b = tid * kBinsPerThread + j;
+        sh.first[b] = at;
+        sh.cursor[b] = at + lower[j];
+        at += total[j];
+        reached += (float)total[j] * __uint_as_float((kTopBin - (uint32_t)b) << 16);
+        if (reached >= need) atomicMin(&sh.last_bin, b);
+    }
+    if (tid == kPrepThreads - 1) sh.first[kNucleusBins] = at;
+    __syncthreads();
+    int last = sh.last_bin;
+    const bool all = last == INT_MAX;  // the whole vocabulary is the list, if the bins hold it
+    if (all) last = kNucleusBins - 1;
+#pragma unroll
+    for (int j = 0; j < kBinsPerThread; ++j)
+        if (tid * kBinsPerThread + j <= last && total[j] > kMaxBin) sh.crowded = 1;
+    __syncthreads();
+    if (!finite || sh.crowded || (all && counted != n)) {
+        if (rank == 0 && tid == 0) *a.token = -1;
+        cluster.sync();  // the others may still read this CTA's counts
+        return;
+    }
+    const int cands = sh.first[last + 1];
+    for (int s = tid; s < slots; s += kPrepThreads) {
+        const float p = vals[s];
+        const int b = bin_of(p), i = index_of(s);
+        if (b <= last && i < n) a.cand[atomicAdd(&sh.cursor[b], 1)] = ((unsigned long long)__float_as_uint(p) << 32) | (uint32_t)~i;
+    }
+    __threadfence();
+    cluster.sync();
+    // A warp ranks 32 neighbours at a time against the bins that they lie in.
+    for (int p0 = (rank * (kPrepThreads / 32) + warp) * 32; p0 < cands; p0 += kCluster * kPrepThreads) {
+        const int live = min(32, cands - p0);
+        const unsigned long long own = lane < live ? __ldcg(a.cand + p0 + lane) : 0;
+        const int b = bin_of(__uint_as_float((uint32_t)(own >> 32)));
+        const int w0 = sh.first[__shfl_sync(0xffffffffu, b, 0)], w1 = sh.first[__shfl_sync(0xffffffffu, b, live - 1) + 1];
+        int larger = 0;
+        unsigned long long next = w0 + lane < w1 ? __ldcg(a.cand + w0 + lane) : 0;
+        for (int w = w0; w < w1; w += 32) {
+            sh.window[warp][lane] = next;
+            __syncwarp();
+            next = w + 32 + lane < w1 ? __ldcg(a.cand + w + 32 + lane) : 0;
+#pragma unroll 8
+            for (int j = 0; j < 32; j += 2) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2 *>(&sh.window[warp][j]);
+                larger += (k.x > own) + (k.y > own);
+            }
+            __syncwarp();
+        }
+        if (lane < live) {
+            a.sorted_p[w0 + larger] = __uint_as_float((uint32_t)(own >> 32));
+            a.sorted_i[w0 + larger] = (int)~(uint32_t)own;
+        }
+    }
+    __threadfence();
+    cluster.sync();
+    if (rank != 0) return;
+    const int pick = pick_rank(a.sorted_p, cands, all, a.target, a.r, sh.pick);
+    if (tid == 0) *a.token = pick < 0 ? -1 : __ldcg(a.sorted_i + pick);
 }
 
 }  // namespace
 
-// logits_dev[vocab] -> *token_dev (device int).  Asynchronous on `s`.
-int launch_sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, float temperature, float top_p, float penalty,
-                        const int *recent_host, size_t n_recent, float r, int *token_dev, cudaStream_t s) {
+// logits_dev[vocab] -> *token (waits for the stream).
+int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lumen_sample_params &sp, int32_t *token, cudaStream_t s) {
     if (vocab == 0 || vocab > (size_t)1 << 30) return set_error(ctx, LUMEN_ERR_SHAPE, "sample: vocabulary of %zu", vocab);
-    if (n_recent > (size_t)kMaxRecent) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "sample: %zu recent tokens, at most %d", n_recent, kMaxRecent);
+    if (sp.n_recent > (size_t)kMaxRecent) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "sample: %zu recent tokens, at most %d", sp.n_recent, kMaxRecent);
     const int n = (int)vocab;
-    size_t sort_bytes = 0;
-    cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, (const float *)nullptr, (float *)nullptr, (const int *)nullptr,
-                                              (int *)nullptr, n, 0, 32, s);
-    const size_t nf = ((size_t)n + 63) & ~(size_t)63;
-    const size_t bytes = 4 * nf * 4 + kMaxRecent * sizeof(int) + ((sort_bytes + 255) & ~(size_t)255);
+    const size_t nf = ((size_t)n + 63) & ~(size_t)63, list_bytes = 4 * nf * 4 + kMaxRecent * sizeof(int);
     // scratch kept with the context (grown when a larger vocabulary comes along): no allocation per token
-    if (ctx->sampler_ws_bytes < bytes) {
+    auto ensure_ws = [&](size_t bytes) -> int {
+        if (ctx->sampler_ws_bytes >= bytes) return LUMEN_OK;
         LUMEN_CUDA(ctx, cudaStreamSynchronize(s));
         if (ctx->sampler_ws) cudaFree(ctx->sampler_ws);
         ctx->sampler_ws = nullptr;
         ctx->sampler_ws_bytes = 0;
         LUMEN_CUDA(ctx, cudaMalloc(&ctx->sampler_ws, bytes));
         ctx->sampler_ws_bytes = bytes;
+        return LUMEN_OK;
+    };
+    int *token_dev = &ctx->d_status->token;  // comes back with the status
+    const float target = fmaxf(fminf(fmaxf(sp.top_p, 0.f), 1.f), 1e-6f);
+    // A nucleus of (nearly) everything reaches into the probabilities that the bins leave out.
+    if (n <= kNucleusMaxVocab && target < 0.999f) {
+        LUMEN_TRY(ensure_ws(list_bytes));
+        const size_t smem = sizeof(NucleusShared) + (size_t)(n + 1023) / 1024 * 128 * sizeof(float);
+        static bool attr_set[64] = {false};
+        const int dev = ctx->device >= 0 && ctx->device < 64 ? ctx->device : 0;
+        if (!attr_set[dev]) {
+            const size_t most = sizeof(NucleusShared) + kNucleusMaxVocab / kCluster * sizeof(float);
+            LUMEN_CUDA(ctx, cudaFuncSetAttribute(sample_nucleus_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+            attr_set[dev] = true;
+        }
+        char *ws = static_cast<char *>(ctx->sampler_ws);
+        NucleusArgs a;
+        a.logits = logits_dev; a.n = n; a.temperature = sp.temperature; a.penalty = sp.repetition_penalty; a.target = target; a.r = sp.uniform;
+        a.cand = reinterpret_cast<unsigned long long *>(ws);
+        a.sorted_p = reinterpret_cast<float *>(ws + 8 * nf); a.sorted_i = reinterpret_cast<int *>(ws + 12 * nf); a.token = token_dev;
+        a.n_recent = (int)sp.n_recent;
+        for (size_t i = 0; i < sp.n_recent; ++i) a.recent[i] = sp.recent_tokens[i];
+        sample_nucleus_kernel<<<kCluster, kPrepThreads, smem, s>>>(a);
+        LUMEN_LAUNCHED(ctx);
+        LUMEN_TRY(check_device_status(ctx));
+        if (ctx->h_status->token >= 0) {
+            *token = ctx->h_status->token;
+            return LUMEN_OK;
+        }
     }
+    size_t sort_bytes = 0;
+    LUMEN_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, (const float *)nullptr, (float *)nullptr, (const int *)nullptr,
+                                                              (int *)nullptr, n, 0, 32, s));
+    LUMEN_TRY(ensure_ws(list_bytes + ((sort_bytes + 255) & ~(size_t)255)));
     void *ws = ctx->sampler_ws;
     float *probs = static_cast<float *>(ws), *probs_sorted = probs + nf;
     int *idx = reinterpret_cast<int *>(probs_sorted + nf), *idx_sorted = idx + nf;
     int *recent_dev = idx_sorted + nf;
     void *sort_ws = recent_dev + kMaxRecent;
-    int rc = LUMEN_OK;
-    cudaError_t e = cudaSuccess;
-    if (n_recent) e = cudaMemcpyAsync(recent_dev, recent_host, n_recent * sizeof(int), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-        sample_prep_kernel<<<1, kPrepThreads, 0, s>>>(logits_dev, n, temperature, penalty, recent_dev, (int)n_recent, probs, idx);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) ctx->launches += 1;
-    }
-    if (e == cudaSuccess)
-        e = cub::DeviceRadixSort::SortPairsDescending(sort_ws, sort_bytes, probs, probs_sorted, idx, idx_sorted, n, 0, 32, s);
-    if (e == cudaSuccess) {
-        sample_pick_kernel<<<1, kPickThreads, 0, s>>>(probs_sorted, idx_sorted, n, top_p, r, token_dev);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) ctx->launches += 1;
-    }
-    if (e != cudaSuccess) rc = cuda_fail(ctx, e, "sample_top_p");
-    return rc;
+    if (sp.n_recent) LUMEN_CUDA(ctx, cudaMemcpyAsync(recent_dev, sp.recent_tokens, sp.n_recent * sizeof(int), cudaMemcpyHostToDevice, s));
+    sample_prep_kernel<<<1, kPrepThreads, 0, s>>>(logits_dev, n, sp.temperature, sp.repetition_penalty, recent_dev, (int)sp.n_recent, probs, idx);
+    LUMEN_LAUNCHED(ctx);
+    LUMEN_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(sort_ws, sort_bytes, probs, probs_sorted, idx, idx_sorted, n, 0, 32, s));
+    sample_pick_kernel<<<1, kPickThreads, 0, s>>>(probs_sorted, idx_sorted, n, target, sp.uniform, token_dev);
+    LUMEN_LAUNCHED(ctx);
+    LUMEN_TRY(check_device_status(ctx));
+    *token = ctx->h_status->token;
+    return LUMEN_OK;
 }
 
 }  // namespace lumen

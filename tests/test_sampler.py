@@ -54,6 +54,45 @@ def test_device_sampler_matches_oracle(L, ctx, oracle, vocab, scale):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [1, 2, 33, 256, 257, 1023, 1025, 4099, 32000, 151936, 262144, 262145])
+@pytest.mark.parametrize("shape", ["peaked", "broad", "close", "masked", "equal"])
+def test_sampler_paths_draw_from_the_nucleus(L, ctx, vocab, shape):
+    """Edges of the sampler's cluster kernel (vocabulary, nuclei of one to 10^5 tokens, crowded bins) and of the general path behind it.
+
+    Bound: the drawn token's interval of the cumulative distribution, in 64 bits over the stable order, holds the draw.  A sum
+    of n probabilities in f32 is off by at most n * 2^-24 of itself, and so is the nucleus' mass; tokens of nearly equal probability may change
+    places, which moves an interval by less than their spread (expf is good to 2 ulp: 2^-22 of a probability per place)."""
+    rng = np.random.default_rng(vocab * 7 + len(shape))
+    lg = rng.standard_normal(vocab) * {"peaked": 3.0, "broad": 0.9, "close": 0.02, "masked": 1.0, "equal": 0.0}[shape]
+    if shape == "peaked":
+        lg[rng.permutation(vocab)[: max(1, vocab // 64)]] += 5.0
+    if shape == "masked":
+        lg[rng.random(vocab) < 0.4] = -np.inf
+        lg[vocab // 2] = 1.0
+    lg = lg.astype(np.float32)
+    t = L.Tensor.from_array_no_grad(lg)
+    for temp, top_p, pen, recent in [(0.8, 0.9, 1.05, rng.integers(0, vocab, 96).tolist()), (1.0, 0.95, 1.0, []), (0.6, 0.99, 1.3, [vocab - 1] * 2), (1.0, 0.9995, 1.0, [])]:
+        z = lg.copy()
+        for tok in recent if pen > 1 else []:
+            z[tok] = np.float32(z[tok] / np.float32(pen))
+        z = (z / np.float32(temp)).astype(np.float32)
+        p = np.exp(z.astype(np.float64) - z.max())
+        p /= p.sum()
+        order = np.argsort(-z, kind="stable")
+        cum = np.cumsum(p[order])
+        m = min(int(np.searchsorted(cum, np.float64(np.float32(top_p)))) + 1, vocab)
+        place = np.empty(vocab, np.int64)
+        place[order] = np.arange(vocab)
+        slack = 3 * vocab * 2.0 ** -24 + 2.0 ** -22 + 2 * p[order[m - 1]]
+        for u in list(rng.random(6).astype(np.float32)) + [np.float32(0), np.float32(1)]:
+            got = L.sample_top_p(ctx, t.data_ptr, vocab, temp, top_p, pen, recent, float(u))
+            i = place[got]
+            assert cum[i] - p[got] <= top_p * (1 + slack), (temp, top_p, u)
+            top = cum[m - 1]
+            assert (cum[i] - p[got]) / top - slack / top <= u <= cum[i] / top + slack / top or i >= m - 1, (temp, top_p, u, i, m)
+
+
+@pytest.mark.gpu
 def test_forward_sample_equals_forward_then_oracle_sampler(L, oracle):
     cfg = small_cfg()
     params = make_params(L, cfg, 17, std=0.3)
