@@ -10,6 +10,8 @@
 // shared memory and read back as conflict-free 128-bit words.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "decoder_kernels.cuh"
 #include "gemv_rows.cuh"
 
@@ -340,98 +342,124 @@ __global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const Ge
 }
 
 // ---- [K,N] row-major layout ---------------------------------------------------------------------
-// y[n] = sum_k w[k,n] x[k].  A thread owns VEC adjacent columns and walks a slice of k; slices are
-// summed by a second kernel in slice order (deterministic, no atomics).
-constexpr int kKnThreads = 128;
+// y[n] = sum_k w[k,n] x[k].  A warp walks rows of a tile of columns, LW lanes side by side (16 bytes each: VEC adjacent columns a
+// lane) and 32 / LW rows at once; the CTA's eight warps take the rows in turn, the CTAs of a cluster take a slice of K each.  Partial
+// sums meet in shared memory and, across the slices, in `part` (slices added in order: deterministic, no atomics).
+// Rows that do not start on 16 bytes (N not a multiple of VEC) are read in whole aligned vectors all the same: a thread's rows
+// lie a multiple of eight apart, so all of them are `shift` elements off alignment, and its sums belong `shift` columns further
+// left; a tile is one vector narrower than what a warp reads.
+// Why this split: HBM wants some 45 KB in flight per SM (two or three CTAs of 256 threads with eight 16-byte loads each), in lines
+// of 128 bytes or more; everything behind that is overhead.  [4096,11008] bf16: 21.9 us (4.1 TB/s), against 34.8 us with 108 slices
+// per column, whose sums a second kernel had to read back (10.9 us of it).
+constexpr int kKnWarps = 8, kKnUnroll = 8, kKnChunk = 2048, kKnSplits = 8;
+__host__ __device__ constexpr int kn_tile_cols(int lw, int vec, bool whole) { return (whole ? lw : lw - 1) * vec; }
 
-template <typename WT>
-__global__ void __launch_bounds__(kKnThreads)
-gemv_kn_partial_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *__restrict__ part, size_t K,
-                       size_t N, size_t k_per_split) {
-    constexpr int VEC = 16 / sizeof(WT);
-    const size_t col0 = ((size_t)blockIdx.x * kKnThreads + threadIdx.x) * VEC;
-    const size_t k0 = (size_t)blockIdx.y * k_per_split;
-    const size_t k1 = min(K, k0 + k_per_split);
-    __shared__ float xs[1024];
+template <typename WT, int LW>
+__global__ void __launch_bounds__(kKnWarps * 32, 3)
+gemv_kn_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *part, float *__restrict__ y, size_t K, size_t N, size_t k_per_split) {
+    constexpr int VEC = 16 / sizeof(WT), RPW = 32 / LW, ROWS = kKnWarps * RPW;
+    static_assert(ROWS % 8 == 0, "a thread's rows share their alignment");
+    __shared__ float xs[kKnChunk];
+    __shared__ __align__(16) float red[kKnWarps * 32 * VEC];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane % LW, row = warp * RPW + lane / LW;
+    const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    const int tile = kn_tile_cols(LW, VEC, N % VEC == 0);
+    const size_t c0 = (size_t)blockIdx.x * tile, k0 = min(K, (size_t)blockIdx.y * k_per_split), k1 = min(K, k0 + k_per_split), total = K * N;
+    auto shift_of = [&](int r) { return (int)(((k0 + r) % VEC * (N % VEC) + c0) % VEC); };
+    const int shift = shift_of(row);
+    const bool active = c0 + (size_t)sub * VEC < N + shift;
+    const size_t first = (k0 + row) * N + c0 - shift + (size_t)sub * VEC;  // of this thread's elements
+    auto fetch = [&](size_t kk) {  // row k0 + row + kk
+        const size_t at = first + kk * N;
+        if (aligned && at + VEC <= total) return __ldcs(reinterpret_cast<const uint4 *>(w + at));
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);  // the last elements of the matrix, or a matrix that starts anywhere
+        WT *e = reinterpret_cast<WT *>(&v);
+        for (int i = 0; i < VEC; ++i)
+            if (at + i < total) e[i] = w[at + i];
+        return v;
+    };
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
-    const bool vec_ok = (N % VEC == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    for (size_t kb = k0; kb < k1; kb += 1024) {
-        const size_t kn = min((size_t)1024, k1 - kb);
-        __syncthreads();
-        for (size_t i = threadIdx.x; i < kn; i += kKnThreads) xs[i] = x[kb + i];
-        __syncthreads();
-        if (col0 >= N) continue;
-        if (vec_ok) {
-            constexpr int U = 8;
-            for (size_t kk = 0; kk < kn; kk += U) {
-                uint4 wv[U];
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t kb = k0; kb < k1; kb += kKnChunk) {
+        const int kn = (int)min((size_t)kKnChunk, k1 - kb);
+        uint4 wv[kKnUnroll];
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    wv[u] = (kk + u < kn) ? __ldcs(reinterpret_cast<const uint4 *>(w + (kb + kk + u) * N + col0))
-                                          : make_uint4(0u, 0u, 0u, 0u);
+        for (int u = 0; u < kKnUnroll; ++u) wv[u] = active && row + u * ROWS < kn ? fetch(kb - k0 + u * ROWS) : zero;
+        __syncthreads();
+        for (int i = tid; i < kn; i += kKnWarps * 32) xs[i] = x[kb + i];
+        __syncthreads();
+        for (int r = row; r < kn;) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const float xv = (kk + u < kn) ? xs[kk + u] : 0.f;
-                    if constexpr (sizeof(WT) == 4) {
-                        acc[0] = fmaf(__uint_as_float(wv[u].x), xv, acc[0]);
-                        acc[1] = fmaf(__uint_as_float(wv[u].y), xv, acc[1]);
-                        acc[2] = fmaf(__uint_as_float(wv[u].z), xv, acc[2]);
-                        acc[3] = fmaf(__uint_as_float(wv[u].w), xv, acc[3]);
-                    } else {
-                        acc[0] = fmaf(bf16_lo(wv[u].x), xv, acc[0]);
-                        acc[1] = fmaf(bf16_hi(wv[u].x), xv, acc[1]);
-                        acc[2] = fmaf(bf16_lo(wv[u].y), xv, acc[2]);
-                        acc[3] = fmaf(bf16_hi(wv[u].y), xv, acc[3]);
-                        acc[4] = fmaf(bf16_lo(wv[u].z), xv, acc[4]);
-                        acc[5] = fmaf(bf16_hi(wv[u].z), xv, acc[5]);
-                        acc[6] = fmaf(bf16_lo(wv[u].w), xv, acc[6]);
-                        acc[7] = fmaf(bf16_hi(wv[u].w), xv, acc[7]);
-                    }
+            for (int u = 0; u < kKnUnroll; ++u) {
+                const float xv = r + u * ROWS < kn ? xs[r + u * ROWS] : 0.f;
+                if constexpr (sizeof(WT) == 4) {
+                    acc[0] = fmaf(__uint_as_float(wv[u].x), xv, acc[0]);
+                    acc[1] = fmaf(__uint_as_float(wv[u].y), xv, acc[1]);
+                    acc[2] = fmaf(__uint_as_float(wv[u].z), xv, acc[2]);
+                    acc[3] = fmaf(__uint_as_float(wv[u].w), xv, acc[3]);
+                } else {
+                    acc[0] = fmaf(bf16_lo(wv[u].x), xv, acc[0]);
+                    acc[1] = fmaf(bf16_hi(wv[u].x), xv, acc[1]);
+                    acc[2] = fmaf(bf16_lo(wv[u].y), xv, acc[2]);
+                    acc[3] = fmaf(bf16_hi(wv[u].y), xv, acc[3]);
+                    acc[4] = fmaf(bf16_lo(wv[u].z), xv, acc[4]);
+                    acc[5] = fmaf(bf16_hi(wv[u].z), xv, acc[5]);
+                    acc[6] = fmaf(bf16_lo(wv[u].w), xv, acc[6]);
+                    acc[7] = fmaf(bf16_hi(wv[u].w), xv, acc[7]);
                 }
             }
-        } else {
-            for (size_t kk = 0; kk < kn; ++kk) {
+            r += kKnUnroll * ROWS;
 #pragma unroll
-                for (int v = 0; v < VEC; ++v) {
-                    if (col0 + v < N) {
-                        float wv;
-                        if constexpr (sizeof(WT) == 4) wv = reinterpret_cast<const float *>(w)[(kb + kk) * N + col0 + v];
-                        else wv = __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(w)[(kb + kk) * N + col0 + v]);
-                        acc[v] = fmaf(wv, xs[kk], acc[v]);
-                    }
-                }
-            }
+            for (int u = 0; u < kKnUnroll; ++u) wv[u] = active && r + u * ROWS < kn ? fetch(kb - k0 + (r - row) + u * ROWS) : zero;
         }
     }
 #pragma unroll
-    for (int v = 0; v < VEC; ++v)
-        if (col0 + v < N) part[(size_t)blockIdx.y * N + col0 + v] = acc[v];
-}
-
-__global__ void gemv_kn_reduce_kernel(const float *__restrict__ part, float *__restrict__ y, size_t N, int splits) {
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int i = 0; i < splits; ++i) s += part[(size_t)i * N + n];
-    y[n] = s;
+    for (int v = 0; v < VEC; v += 4)
+        *reinterpret_cast<float4 *>(red + (warp * 32 + lane) * VEC + v) = make_float4(acc[v], acc[v + 1], acc[v + 2], acc[v + 3]);
+    __syncthreads();
+    const bool sliced = gridDim.y > 1;
+    for (int c = tid; c < tile && c0 + c < N; c += kKnWarps * 32) {
+        float s = 0.f;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) s += red[r * LW * VEC + c + shift_of(r)];
+        if (sliced) part[(size_t)blockIdx.y * N + c0 + c] = s;
+        else y[c0 + c] = s;
+    }
+    if (!sliced) return;
+    __threadfence();
+    cooperative_groups::this_cluster().sync();  // (grid.y is the cluster)
+    const int per = (tile + gridDim.y - 1) / gridDim.y, end = min(tile, (int)(blockIdx.y + 1) * per);
+    for (int c = blockIdx.y * per + tid; c < end && c0 + c < N; c += kKnWarps * 32) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < (int)gridDim.y; ++i) s += __ldcg(part + (size_t)i * N + c0 + c);
+        y[c0 + c] = s;
+    }
 }
 
 struct KnPlan {
-    int col_blocks, splits;
+    int lanes, col_blocks, splits;
     size_t k_per_split;
 };
 
+// Tiles as wide as leave two CTAs per SM with K cut in eight; no more slices than that takes (a slice has at least four
+// rows per thread).
 KnPlan plan_kn(size_t K, size_t N, int vec, int num_sms) {
     KnPlan p;
-    p.col_blocks = (int)((N + (size_t)kKnThreads * vec - 1) / ((size_t)kKnThreads * vec));
-    int want = (num_sms * 8 + p.col_blocks - 1) / p.col_blocks;  // aim at ~8 CTAs per SM
-    size_t max_splits = (K + 31) / 32;                            // at least 32 k per slice
-    int splits = (int)std::min<size_t>((size_t)std::max(want, 1), max_splits);
-    splits = std::min(splits, 256);
-    p.k_per_split = (K + splits - 1) / splits;
-    p.splits = (int)((K + p.k_per_split - 1) / p.k_per_split);
+    const size_t want = 2 * (size_t)num_sms;
+    size_t blocks = 0;
+    for (p.lanes = 32; p.lanes >= 8; p.lanes /= 2) {
+        const size_t tile = kn_tile_cols(p.lanes, vec, N % vec == 0);
+        blocks = (N + tile - 1) / tile;
+        if (blocks * kKnSplits >= want || p.lanes == 8) break;
+    }
+    p.col_blocks = (int)blocks;
+    const size_t rows = (size_t)kKnWarps * 32 / p.lanes;
+    p.splits = 1;
+    while (p.splits < kKnSplits && blocks * p.splits < want && K > (size_t)p.splits * rows * 4) p.splits *= 2;
+    p.k_per_split = ((K + p.splits - 1) / p.splits + rows - 1) / rows * rows;
     return p;
 }
 
@@ -551,17 +579,20 @@ size_t gemv_kn_scratch_bytes(size_t K, size_t N, int num_sms) {
 
 int launch_gemv_kn(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype wdt, float *y, size_t K, size_t N,
                    float *scratch, cudaStream_t s) {
-    const int vec = wdt == LUMEN_F32 ? 4 : 8;
-    KnPlan p = plan_kn(K, N, vec, ctx->num_sms);
-    dim3 grid(p.col_blocks, p.splits);
-    if (wdt == LUMEN_F32)
-        gemv_kn_partial_kernel<float><<<grid, kKnThreads, 0, s>>>(x, static_cast<const float *>(w), scratch, K, N,
-                                                                   p.k_per_split);
-    else
-        gemv_kn_partial_kernel<__nv_bfloat16>
-            <<<grid, kKnThreads, 0, s>>>(x, static_cast<const __nv_bfloat16 *>(w), scratch, K, N, p.k_per_split);
-    LUMEN_LAUNCHED(ctx);
-    gemv_kn_reduce_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(scratch, y, N, p.splits);
+    const KnPlan p = plan_kn(K, N, wdt == LUMEN_F32 ? 4 : 8, ctx->num_sms);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.col_blocks, p.splits);
+    cfg.blockDim = dim3(kKnWarps * 32);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {1, (unsigned)p.splits, 1};
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+#define LUMEN_KN(T_, L_) cudaLaunchKernelEx(&cfg, gemv_kn_kernel<T_, L_>, x, static_cast<const T_ *>(w), scratch, y, K, N, p.k_per_split)
+    if (wdt == LUMEN_F32) LUMEN_CUDA(ctx, p.lanes == 32 ? LUMEN_KN(float, 32) : p.lanes == 16 ? LUMEN_KN(float, 16) : LUMEN_KN(float, 8));
+    else LUMEN_CUDA(ctx, p.lanes == 32 ? LUMEN_KN(__nv_bfloat16, 32) : p.lanes == 16 ? LUMEN_KN(__nv_bfloat16, 16) : LUMEN_KN(__nv_bfloat16, 8));
+#undef LUMEN_KN
     LUMEN_LAUNCHED(ctx);
     return LUMEN_OK;
 }

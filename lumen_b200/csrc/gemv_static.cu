@@ -7,9 +7,8 @@
 
 namespace {
 
-// Room for the partial sums: splits * N floats.  The launcher aims at about 8 CTAs per SM, which puts
-// splits * N near 1184 * 1024 floats (4.7 MB) whatever N is, so 8 MiB covers N up to several hundred
-// thousand columns on a 148-SM part; larger requests are refused, never truncated.
+// Room for the partial sums: splits * N floats, of at most eight splits, and one only where the columns alone fill the
+// device, so 8 MiB covers N up to two million columns; larger requests are refused, never truncated.
 constexpr size_t kStaticScratchBytes = 8u << 20;
 static __device__ __align__(256) float g_kn_scratch[kStaticScratchBytes / sizeof(float)];
 
@@ -57,7 +56,7 @@ int lumen_gemv_kn_static(lumen_ctx *ctx, const float *x_dev, const void *w_dev, 
             scratch = g_scratch_ptr[cur] = static_cast<float *>(p);
         }
     }
-    // Nothing has to start at zero: the first kernel writes every partial sum that the second one reads.
+    // Nothing has to start at zero: the kernel writes every partial sum that it reads.
     return launch_gemv_kn(ctx, x_dev, w_dev, w_dtype, y_dev, k, n, scratch, ctx->stream);
 }
 

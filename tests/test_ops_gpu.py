@@ -143,6 +143,33 @@ def test_gemv_kn_layout_raw_pointers(L, oracle, ctx, k, n, bf16):
     assert rel_err(y[pad:-pad], oracle.matmul(x[None], w_nk, "f64")[0]) < 2e-6
 
 
+@pytest.mark.parametrize("k,n", [(1, 1), (7, 9), (64, 8), (65, 130), (256, 127), (300, 33), (511, 2049), (2049, 1031), (4097, 257), (1000, 40000), (70, 99001), (12288, 128)])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_gemv_kn_edges(L, ctx, k, n, offset, bf16):
+    """Tiles of columns and slices of K with remainders, rows that start at every alignment, a matrix that does not start on 16 bytes; what
+    surrounds the matrix is infinite."""
+    rng = np.random.default_rng(k * 31 + n)
+    x = rng.standard_normal(k, dtype=np.float32)
+    w = rng.standard_normal((k, n), dtype=np.float32) * np.float32(0.02)
+    flat = np.full(k * n + 64, np.inf, np.float32)
+    flat[offset:offset + k * n] = w.reshape(-1)
+    if bf16:
+        wt = L.Tensor.from_bf16(flat[None])
+        bits = w.view(np.uint32)
+        w = (bits + np.uint32(0x7fff) + ((bits >> np.uint32(16)) & np.uint32(1)) & np.uint32(0xffff0000)).view(np.float32)
+    else:
+        wt = L.Tensor.from_array_no_grad(flat[None])
+    xt = L.Tensor.from_array_no_grad(x)
+    y = L.Tensor.from_array_no_grad(np.full(n + 2, 5.0, np.float32))
+    L.gemv(ctx, xt.data_ptr, wt.data_ptr + offset * (2 if bf16 else 4), L.BF16 if bf16 else L.F32, True, k, n, y.data_ptr + 4)
+    got = y.data()
+    assert got[0] == 5.0 and got[-1] == 5.0
+    want = x.astype(np.float64) @ w.astype(np.float64)
+    # f32 sums of k products: at most k * 2^-24 of the sum of their sizes, of which chains of k / 64 and trees use a few
+    assert np.abs(got[1:-1] - want).max() <= 2.0 ** -24 * (8 + k / 32) * (np.abs(x) @ np.abs(w)).max()
+
+
 def test_linear_with_bias(L, oracle):
     rng = np.random.default_rng(3)
     x = rng.standard_normal((2, 4, 24), dtype=np.float32)
