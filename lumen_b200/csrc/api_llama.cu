@@ -14,8 +14,10 @@
 #include <map>
 #include <tuple>
 
+#include "attn_rows.cuh"
 #include "common.cuh"
 #include "decode_mega.cuh"
+#include "gemm_rows.cuh"
 #include "model_base.cuh"
 #include "tp_plan.cuh"
 
@@ -40,6 +42,7 @@ struct Workspace {
     // bf16 hi/lo split of the activations the next tensor-core product reads (written by the kernel that finishes the
     // previous product): the normed rows [M, H], and the SwiGLU rows [M, I_l] (the product that writes them still reads the former)
     __nv_bfloat16 *p_hi = nullptr, *p_lo = nullptr, *g_hi = nullptr, *g_lo = nullptr;
+    float *ss = nullptr;  // sums of squares of the residual stream (see GemmRowsArgs)
     size_t part_bytes = 0;
     float *h_ids = nullptr;     // pinned
     float *h_logits = nullptr;  // pinned
@@ -112,20 +115,20 @@ int ensure_workspace(lumen_llama *m, size_t M) {
         off += align_up(elems * sizeof(float), 256);
         return o;
     };
-    size_t o_x = take(M * m->H), o_nx = take(M * m->H), o_qkv = take(M * qkvd), o_att = take(M * m->qd_l);
+    size_t o_x = take(M * m->H), o_nx = take(M * m->H), o_qkv = take(M * qkvd), o_att = take(2 * M * m->qd_l);  // (f32, then the bf16 pair)
     // gate and up are adjacent: the fused step runs them as one product into [M, 2 * I_l]
     size_t o_act = take(M * m->inter_l), o_gate = take(2 * M * m->inter_l);
     auto half = [](size_t n) { return (n + 1) / 2 + 8; };
     size_t o_phi = take(half(M * m->H)), o_plo = take(half(M * m->H)), o_ghi = take(half(M * m->inter_l)), o_glo = take(half(M * m->inter_l));
     size_t o_logits = take(M * m->V), o_ll = take(T > 1 ? T * M * m->vocab_l : 0), o_last = take(M * m->H);
-    size_t o_part = take(w.part_bytes / sizeof(float)), o_ids = take(M);
+    size_t o_part = take(w.part_bytes / sizeof(float)), o_ids = take(M), o_ss = take(gemm_rows_ss_floats(m->H));
     LUMEN_CUDA(ctx, cudaMalloc(&w.base, off));
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w.base + o); };
     w.x = at(o_x); w.nx = at(o_nx); w.qkv = at(o_qkv); w.att = at(o_att); w.act = at(o_act); w.gate = at(o_gate);
     w.up = w.gate + M * m->inter_l; w.p_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_phi)); w.p_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_plo));
     w.g_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_ghi)); w.g_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_glo));
     w.logits = at(o_logits); w.logits_local = at(o_ll); w.last_x = at(o_last); w.part = at(o_part);
-    w.ids = at(o_ids);
+    w.ids = at(o_ids); w.ss = at(o_ss);
     LUMEN_CUDA(ctx, cudaMallocHost(&w.h_ids, std::max<size_t>(M, 1) * sizeof(float)));
     w.h_logits_elems = std::min<size_t>(M * m->V, (size_t)16 << 20);  // pinned staging up to 64 MB
     LUMEN_CUDA(ctx, cudaMallocHost(&w.h_logits, std::max<size_t>(w.h_logits_elems, 1) * sizeof(float)));
@@ -169,6 +172,7 @@ struct StepPlan {
     size_t B, S, M;
     bool decode;
     int nsplit;
+    int parts = 0;  // of a context in launch_attn_rows (0: the general kernel)
 };
 
 // Enqueues one forward pass over ws.ids[M] on the context stream.  `last_only` restricts the final norm
@@ -227,6 +231,35 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         LUMEN_TRY(launch_attn_prefill(ctx, a, s));
         return launch_bump_len(ctx, c->d_len, (int)p.S, s);
     };
+    // Few rows: every product leaves what the next one reads (gemm_rows.cu), five kernels per block.  In decode steps a kernel is
+    // launched while its predecessor runs and asks for its weights or cached rows before it waits for it.
+    bool few = fuse && !tp && H % 4 == 0 && (wdt == LUMEN_BF16 || m->wsplit_valid);
+    for (size_t l = 0; few && l < m->L; ++l) {
+        const LayerW &lw = m->layers[l];
+        few = gemm_rows_usable(wdt, M, H, qkvd, lw.wqkv) && gemm_rows_usable(wdt, M, m->qd_l, H, lw.wo) &&
+              gemm_rows_usable(wdt, M, H, 2 * m->inter_l, lw.wgate) && gemm_rows_usable(wdt, M, m->inter_l, H, lw.wdown);
+    }
+    const bool rows_attn = few && p.decode && p.parts > 0;
+    struct PdlScope {
+        lumen_ctx *ctx;
+        ~PdlScope() { ctx->pdl = false; }
+    } pdl_scope{ctx};
+    __nv_bfloat16 *const att_hi = reinterpret_cast<__nv_bfloat16 *>(w.att + M * m->qd_l), *const att_lo = att_hi + M * m->qd_l;
+    auto rows_args = [&](const void *wmat, size_t rows, size_t K, size_t N, const __nv_bfloat16 *hi, const __nv_bfloat16 *lo, int n_ss) {
+        GemmRowsArgs g;
+        GemmFuse split;
+        use_weight_split(m, wmat, split);
+        g.w_hi = split.w_hi ? split.w_hi : static_cast<const __nv_bfloat16 *>(wmat);
+        g.w_lo = split.w_lo;
+        g.M = (int)rows; g.N = (int)N; g.K = (int)K; g.x_hi = hi; g.x_lo = lo; g.ss_in = w.ss; g.n_ss = n_ss; g.eps = eps;
+        return g;
+    };
+    auto rows_residual = [&](const void *wmat, size_t K, const __nv_bfloat16 *hi, const __nv_bfloat16 *lo, const float *next_gain, int *advance) {
+        GemmRowsArgs g = rows_args(wmat, M, K, H, hi, lo, 0);
+        g.epi = GemmRowsArgs::kResidual; g.x = w.x; g.gain = next_gain; g.hi = w.p_hi; g.lo = w.p_lo; g.ss_out = w.ss; g.advance = advance;
+        return launch_gemm_rows(ctx, g, s);
+    };
+    const int ss_tiles = (int)((H + 127) / 128);
     // Row-parallel product of the fused step: x = x + a . W^T summed over the ranks, and the split of RMSNorm(x) * norm_w
     // for the next product (norm_w null after the last block).  `a` null: the activations are the SwiGLU pair.
     auto row_parallel = [&](const float *a, const void *wmat, size_t K, const float *norm_w) -> int {
@@ -251,10 +284,33 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     };
 
     LUMEN_TRY(launch_embedding(ctx, w.ids, m->embed, wdt, w.x, M, m->V, H, s));
+    ctx->pdl = rows_attn;  // (the embedding has waited for everything before the step)
     bool nx_ready = false;  // w.nx (or, fused, the pair) already holds Norm(x) of the block about to run
     for (size_t l = 0; l < m->L; ++l) {
         const LayerW &lw = m->layers[l];
         lumen_kv_cache *c = caches[l];
+        if (few) {
+            if (l == 0) LUMEN_TRY(launch_rows_start(ctx, w.x, lw.norm1, M, H, w.p_hi, w.p_lo, w.ss, s));
+            GemmRowsArgs g = rows_args(lw.wqkv, M, H, qkvd, w.p_hi, w.p_lo, l == 0 ? 1 : ss_tiles);
+            g.c = w.qkv;
+            LUMEN_TRY(launch_gemm_rows(ctx, g, s));
+            if (rows_attn) {
+                AttnRowsArgs r;
+                r.qkv = w.qkv; r.stride = qkvd; r.k_cache = c->k; r.v_cache = c->v; r.d_len = c->d_len; r.max_seq = c->max_seq;
+                r.cos_t = m->cos_t; r.sin_t = m->sin_t; r.q_norm = lw.qn; r.k_norm = lw.kn; r.norm_eps = eps; r.scale = scale;
+                r.out_hi = att_hi; r.out_lo = att_lo; r.status = ctx->d_status;
+                LUMEN_TRY(launch_attn_rows(ctx, r, p.B, m->hq_l, m->hkv_l, m->D, p.parts, s));
+            } else {
+                LUMEN_TRY(attend(lw, c));
+                LUMEN_TRY(launch_split_bf16(ctx, w.att, att_hi, att_lo, M * m->qd_l, s));
+            }
+            LUMEN_TRY(rows_residual(lw.wo, m->qd_l, att_hi, att_lo, lw.norm2, rows_attn ? c->d_len : nullptr));
+            g = rows_args(lw.wgate, M, H, 2 * m->inter_l, w.p_hi, w.p_lo, ss_tiles);
+            g.epi = GemmRowsArgs::kSwiglu; g.hi = w.g_hi; g.lo = w.g_lo;
+            LUMEN_TRY(launch_gemm_rows(ctx, g, s));
+            LUMEN_TRY(rows_residual(lw.wdown, m->inter_l, w.g_hi, w.g_lo, l + 1 < m->L ? m->layers[l + 1].norm1 : m->final_norm, nullptr));
+            continue;
+        }
         if (fuse) {
             if (!nx_ready) LUMEN_TRY(launch_sum_norm_split(ctx, w.x, 1, nullptr, M, H, nullptr, lw.norm1, eps, w.p_hi, w.p_lo, s));
             GemmFuse fq;
@@ -312,7 +368,13 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         rows = p.B;
     }
     float *lg = tp ? w.logits_local + (size_t)ctx->tp_rank * rows * m->vocab_l : w.logits;
-    if (rows <= vec_rows && rows * H * 4 <= 200 * 1024) {
+    if (!tp && rows > vec_rows && H % 4 == 0 && (wdt == LUMEN_BF16 || m->wsplit_valid) && gemm_rows_usable(wdt, rows, H, m->vocab_l, m->lm_head)) {
+        const bool ready = few && xin == w.x;  // (the last block left the pair)
+        if (!ready) LUMEN_TRY(launch_rows_start(ctx, xin, m->final_norm, rows, H, w.p_hi, w.p_lo, w.ss, s));
+        GemmRowsArgs g = rows_args(m->lm_head, rows, H, m->vocab_l, w.p_hi, w.p_lo, ready ? ss_tiles : 1);
+        g.c = lg;
+        LUMEN_TRY(launch_gemm_rows(ctx, g, s));
+    } else if (rows <= vec_rows && rows * H * 4 <= 200 * 1024) {
         GemvArgs g;
         g.x = xin; g.w = m->lm_head; g.wdt = wdt; g.y = lg; g.M = (int)rows; g.K = H; g.N = m->vocab_l; g.ldy = m->vocab_l;
         g.norm_w = m->final_norm; g.norm_eps = eps;
@@ -510,7 +572,8 @@ int run_forward(lumen_llama *m, size_t b, size_t s, lumen_kv_cache **caches, boo
     StepPlan p{b, s, b * s, s == 1, 1};
     if (p.M > 8) LUMEN_TRY(ensure_weight_split(m));  // (outside any stream capture; the streaming kernels of <= 8 rows read f32)
     if (p.decode) p.nsplit = pick_decode_splits(m, b, caches[0]->len + 1);
-    const int rc = p.decode ? m->run_graphed(std::make_tuple(b, p.nsplit, (const void *)caches[0]->k),
+    if (p.decode) p.parts = attn_rows_splits(b, m->hq_l, m->hkv_l, m->D, caches[0]->len + 1, ctx->num_sms);
+    const int rc = p.decode ? m->run_graphed(std::make_tuple(b, p.nsplit * 16 + p.parts, (const void *)caches[0]->k),
                                              [&] { return enqueue_forward(m, p, caches, last_only); })
                             : enqueue_forward(m, p, caches, last_only);
     if (rc == LUMEN_OK)

@@ -123,6 +123,23 @@ def test_prefill_of_more_than_one_row_tile(L, oracle, inter, prompt, wdt):
     assert rel_err(got, want) < TOL_F32
 
 
+@pytest.mark.parametrize("heads,kv,dim,hidden,inter,batch,prompt", [
+    (8, 1, 64, 512, 200, 16, 40), (4, 2, 64, 136, 136, 33, 5), (2, 2, 128, 264, 72, 64, 1), (4, 1, 128, 1032, 1352, 9, 300), (8, 1, 128, 256, 4104, 17, 2),
+    (2, 1, 64, 128, 64, 32, 130), (4, 4, 64, 256, 392, 48, 17)])
+@pytest.mark.parametrize("wdt", ["f32", "bf16"])
+def test_batched_steps_as_a_chain_of_products(L, oracle, heads, kv, dim, hidden, inter, batch, prompt, wdt):
+    """Batched decode steps (products with their epilogues in thread-block clusters, attention in one kernel): every group size and
+    head dimension it serves, rows at the edges of 16, 32 and 64, widths with remainders of 64 and 128, contexts in one and in several
+    parts; short prompts of as many rows take the same products."""
+    cfg = small_cfg(hidden_size=hidden, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, intermediate_size=inter, qk_norm=dim == 128,
+                    max_seq_len=320)
+    params = make_params(L, cfg, 41, std=0.08, round_bf16=(wdt == "bf16"), random_norms=True)
+    ids = np.random.default_rng(batch).integers(0, cfg["vocab_size"], size=(batch, prompt + 4)).astype(np.float32)
+    got, _, _ = _gpu_run(L, cfg, params, ids, prompt, wdt)
+    want, _ = _oracle_run(oracle, cfg, params, ids, prompt, "f64")
+    assert rel_err(got, want) < TOL_F32
+
+
 def test_forward_last_and_device_entry_points(L, oracle):
     cfg = small_cfg()
     params = make_params(L, cfg, 31, std=0.08)
