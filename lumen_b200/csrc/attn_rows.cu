@@ -159,15 +159,20 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArg
     const float4 *q4 = reinterpret_cast<const float4 *>(qs) + part * A::kVec;
     float *ws = wsoft + warp * TR * G;
     bool alive = true;
-    for (int it = 0; j < jc; j += step, ++it) {
-        const int rows = min(TR, jc - j);
-        alive = __all_sync(0xffffffffu, tc::bar_wait(&kbar[warp], (uint32_t)(it & 1), p.status, 570));
+    // The cached tiles of this warp, then, for the warp that has least to do, this token's row as a tile of one row.
+    const int cached = jc > j ? (jc - j + step - 1) / step : 0;
+    const bool takes_new = owns_new && warp == (max(jc - j0, 0) + TR - 1) / TR % kArWarps;
+#pragma unroll 1
+    for (int it = 0; it < cached + takes_new; ++it, j += step) {
+        const bool fresh = it == cached;
+        const int rows = fresh ? 1 : min(TR, jc - j);
+        if (!fresh) alive = __all_sync(0xffffffffu, tc::bar_wait(&kbar[warp], (uint32_t)(it & 1), p.status, 570));
         if (!alive) break;
         float s[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) s[g] = 0.f;
-        const float4 *k4 = reinterpret_cast<const float4 *>(kt) + r_l * (D / 4) + part * A::kVec;
-#pragma unroll 4
+        const float4 *k4 = reinterpret_cast<const float4 *>(fresh ? knew : kt) + min(r_l, rows - 1) * (D / 4) + part * A::kVec;
+#pragma unroll 2
         for (int i = 0; i < A::kVec; ++i) {
             const int at = (i + r_l) % A::kVec;
             const float4 k = k4[at];
@@ -201,19 +206,25 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArg
             for (int i = 0; i < A::kEl; ++i) ctx[g][i] *= r;
         }
         __syncwarp();
-        alive = __all_sync(0xffffffffu, tc::bar_wait(&vbar[warp], (uint32_t)(it & 1), p.status, 571));
+        if (!fresh) alive = __all_sync(0xffffffffu, tc::bar_wait(&vbar[warp], (uint32_t)(it & 1), p.status, 571));
         if (!alive) break;
-#pragma unroll 4
+        const float *v_tile = fresh ? vnew : vt;
+#pragma unroll 2
         for (int r = 0; r < rows; ++r) {
-            float v[A::kEl];
-            if constexpr (A::kEl == 4) *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(vt + r * D + e0);
-            else *reinterpret_cast<float2 *>(v) = *reinterpret_cast<const float2 *>(vt + r * D + e0);
+            float v[A::kEl], w[G];
+            if constexpr (A::kEl == 4) *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(v_tile + r * D + e0);
+            else *reinterpret_cast<float2 *>(v) = *reinterpret_cast<const float2 *>(v_tile + r * D + e0);
+            if constexpr (G % 4 == 0) {
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const float w = ws[r * G + g];
+                for (int g = 0; g < G; g += 4) *reinterpret_cast<float4 *>(w + g) = *reinterpret_cast<const float4 *>(ws + r * G + g);
+            } else {
 #pragma unroll
-                for (int i = 0; i < A::kEl; ++i) ctx[g][i] = fmaf(w, v[i], ctx[g][i]);
+                for (int g = 0; g < G; ++g) w[g] = ws[r * G + g];
             }
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int i = 0; i < A::kEl; ++i) ctx[g][i] = fmaf(w[g], v[i], ctx[g][i]);
         }
         __syncwarp();
         fetch(vt, vbase, j + step, &vbar[warp], v_issued);
@@ -224,29 +235,18 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArg
         if (v_issued) while (!tc::bar_try(&vbar[warp], (uint32_t)(v_issued - 1) & 1) && clock64() - t0 < tc::kTcWaitCycles) {}
     }
     __syncwarp();
-    if (owns_new) {  // this token's row: the warps share out the heads
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            if (g % kArWarps != warp) continue;
-            float s = 0.f;
-            for (int i = lane; i < D; i += 32) s = fmaf(qs[g * D + i], knew[i], s);
-            s = __fmul_rn(attn_warp_sum(s), p.scale);
-            const float mn = fmaxf(m[g], s), r = expf(m[g] - mn), w = expf(s - mn);
-            m[g] = mn;
-            l[g] = fmaf(l[g], r, lane == 0 ? w : 0.f);
-#pragma unroll
-            for (int i = 0; i < A::kEl; ++i) ctx[g][i] = fmaf(w, vnew[e0 + i], ctx[g][i] * r);
-        }
-    }
     // ---- the warps' parts, then the cluster's ----
     __syncthreads();  // the tiles are no longer read
     float *wctx = tiles + warp * G * D;
 #pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int g = 0; g < G; ++g) l[g] += __shfl_xor_sync(0xffffffffu, l[g], o);
+#pragma unroll
     for (int g = 0; g < G; ++g) {
-        const float sum = attn_warp_sum(l[g]);
         if (lane == 0) {
             wm[warp * G + g] = m[g];
-            wl[warp * G + g] = sum;
+            wl[warp * G + g] = l[g];
         }
 #pragma unroll
         for (int i = 0; i < A::kEl; ++i) wctx[g * D + e0 + i] = ctx[g][i];
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kArThreads) attn_rows_kernel(const AttnRowsArg
         p.out_hi[at] = h;
         p.out_lo[at] = __float2bfloat16_rn(v - __bfloat162float(h));
     };
-#pragma unroll
+#pragma unroll 1
     for (int idx = tid; idx < G * D; idx += kArThreads) {
         const int g = idx / D;
         float M = -INFINITY, L = 0.f, c = 0.f;

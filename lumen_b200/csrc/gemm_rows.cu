@@ -17,10 +17,11 @@
 //   - hi and lo of the activations are one operand of twice the columns: two MMAs per step of K with f32 weights, not three, and even
 //     and odd steps have accumulators of their own (a chain of small MMAs into one accumulator is bound by their latency).
 //
-// TinyLlama f32, 16 sequences: 40 steps and the prefill of 64 positions 84 -> 63.6 ms (a step 1.9 -> 1.37 ms); 9 layers of the Qwen3-8B
-// shape, 64 sequences: 32 steps and a prefill of 60 positions 95 -> 83.5 ms.
+// TinyLlama f32, 16 sequences: 40 steps and the prefill of 64 positions 84 -> 60.8 ms (a step 1.9 -> 1.3 ms); 9 layers of the Qwen3-8B
+// shape, 64 sequences: 32 steps and a prefill of 60 positions 95 -> 81.3 ms.
 //
-// Thread 0 is the TMA producer, thread 32 issues the MMAs, the last two warps form 1 / rms meanwhile; all four warps are the epilogue.
+// Thread 0 is the TMA producer, thread 32 issues the MMAs, warps 2 and 3 form 1 / rms meanwhile; all eight warps are the epilogue (its code runs
+// once per CTA, so it is bound by latencies and by the way of the instructions themselves: short loops, little unrolling).
 // Every wait is bounded; after a failure the CTA skips its arithmetic but takes part in every barrier of the cluster.
 #include <algorithm>
 
@@ -36,7 +37,7 @@ namespace {
 using namespace tc;
 namespace cg = cooperative_groups;
 
-constexpr int kRowsThreads = 128;
+constexpr int kRowsThreads = 256;
 constexpr int kRowsRing = 111 * 1024;
 constexpr size_t kRowsL2 = (size_t)64 << 20;  // bytes that the CTAs of one product may request ahead for the L2
 
@@ -91,10 +92,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int inter = a.N / 2;
     const int n0 = tile * (EPI == GemmRowsArgs::kSwiglu ? 64 : 128), n1 = EPI == GemmRowsArgs::kSwiglu ? inter + n0 : n0 + 64;  // rows of W of the two halves
     const int kb_all = (a.K + kBK - 1) / kBK, kb0 = rank * p.kb_per, nkb = max(0, min(kb_all, kb0 + p.kb_per) - kb0);
+    // The tiles walk K from different steps on: they read the same activations, and all at once they would queue for the same lines of the L2.
+    const int turn = nkb ? tile % nkb : 0;
+    auto k_of = [&](int kb) { return (kb0 + (kb + turn < nkb ? kb + turn : kb + turn - nkb)) * kBK; };
     auto weights = [&](int kb) {
         unsigned char *st = ring + (size_t)(kb % kStages) * G::kStageBytes;
         uint64_t *bar = &full[kb % kStages];
-        const int kx = (kb0 + kb) * kBK;
+        const int kx = k_of(kb);
         bar_expect(bar, G::kStageBytes);
         tma_load_2d(st, &map_w, kx, n0, bar);
         tma_load_2d(st + G::kHalfBytes, &map_w, kx, n1, bar);
@@ -136,8 +140,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 weights(kb);
             }
             unsigned char *st = ring + (size_t)s * G::kStageBytes + NW * G::kWBytes;
-            tma_load_2d(st, &map_x, (kb0 + kb) * kBK, 0, &full[s]);
-            tma_load_2d(st + G::kXBytes, &map_xlo, (kb0 + kb) * kBK, 0, &full[s]);
+            tma_load_2d(st, &map_x, k_of(kb), 0, &full[s]);
+            tma_load_2d(st + G::kXBytes, &map_xlo, k_of(kb), 0, &full[s]);
         }
     } else if (tid == 32) {
         bool ok = true;
@@ -159,12 +163,12 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
         if (!ok) failed = 1;
         umma_commit(&done);
-    } else if (warp >= 2) {
+    } else if (warp == 2 || warp == 3) {
         if (tid == 96) {
             // what the ring cannot take goes to the L2: HBM would otherwise idle while the kernel before this one ends
             const int end = min(nkb, ahead + p.l2_ahead);
             for (int kb = ahead; kb < end; ++kb) {
-                const int kx = (kb0 + kb) * kBK;
+                const int kx = k_of(kb);
                 prefetch_2d(&map_w, kx, n0);
                 prefetch_2d(&map_w, kx, n1);
                 if (NW == 2) {
@@ -192,9 +196,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     float *red = reinterpret_cast<float *>(ring);
     const bool good = have && !failed;
     if (good) {
-        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
+        for (int c0 = 16 * (warp >> 2); c0 < BN; c0 += 32) {  // (warps w and w + 4 read the same lanes)
             uint32_t v[G::kAccs][16];
 #pragma unroll
             for (int q = 0; q < G::kAccs; ++q) tmem_ld16_issue(taddr + (uint32_t)(q * BN + c0), v[q]);
@@ -204,7 +208,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 float sum = __uint_as_float(v[0][j]);
 #pragma unroll
                 for (int q = 1; q < G::kAccs; ++q) sum += __uint_as_float(v[q][j]);
-                if (c0 + j < a.M) red[(c0 + j) * 128 + tid] = nkb ? sum : 0.f;
+                if (c0 + j < a.M) red[(c0 + j) * 128 + (tid & 127)] = nkb ? sum : 0.f;
             }
         }
     } else if (tid == 0) {
@@ -220,7 +224,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (splits > 1) cluster.sync();
     // Rows m, m + by, ... of a column: the sum of the slices, in order.  The loads of a batch of rows from four CTAs are in flight
     // together: a trip to another SM's shared memory takes some 0.5 us.
-    constexpr int kBatch = BN == 16 ? 4 : 8;
+    constexpr int kBatch = BN == 16 ? 2 : 4;
     auto sums = [&](float (&v)[kBatch], int m, int by, int col) {
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) v[q] = 0.f;
@@ -230,6 +234,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 if (m + q * by < a.M) v[q] = red[(m + q * by) * 128 + col];
             return;
         }
+#pragma unroll 1
         for (int r0 = 0; r0 < splits; r0 += 4) {
             float t[4][kBatch];
 #pragma unroll
@@ -246,8 +251,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     };
     if (good) {
         if constexpr (EPI == GemmRowsArgs::kSwiglu) {
-            const int col = n0 + (tid & 63), by = 2 * splits;
-            for (int m0 = rank * 2 + (tid >> 6); m0 < a.M; m0 += kBatch * by) {
+            const int col = n0 + (tid & 63), by = 4 * splits;
+#pragma unroll 1
+            for (int m0 = rank * 4 + (tid >> 6); m0 < a.M; m0 += kBatch * by) {
                 float g[kBatch], u[kBatch];
                 sums(g, m0, by, tid & 63);
                 sums(u, m0, by, 64 + (tid & 63));
@@ -262,20 +268,21 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 }
             }
         } else if constexpr (EPI == GemmRowsArgs::kResidual) {
-            const int col = n0 + tid;
+            const int col = n0 + (tid & 127), by = 2 * splits;
             const float g = col < a.N ? a.gain[col] : 0.f;
-            for (int m0 = rank; m0 < a.M; m0 += kBatch * splits) {
+#pragma unroll 1
+            for (int m0 = rank + splits * (tid >> 7); m0 < a.M; m0 += kBatch * by) {
                 float v[kBatch], x[kBatch];
 #pragma unroll
                 for (int q = 0; q < kBatch; ++q) {
-                    const int m = m0 + q * splits;
+                    const int m = m0 + q * by;
                     x[q] = m < a.M && col < a.N ? a.x[(size_t)m * a.N + col] : 0.f;
                 }
-                sums(v, m0, splits, tid);
+                sums(v, m0, by, tid & 127);
 #pragma unroll
                 for (int q = 0; q < kBatch; ++q) {
-                    const int m = m0 + q * splits;
-                    if (m >= a.M) break;  // (the same in all threads)
+                    const int m = m0 + q * by;
+                    if (m >= a.M) break;  // (the same in a warp)
                     float ss = 0.f;
                     if (col < a.N) {
                         const size_t at = (size_t)m * a.N + col;
@@ -289,20 +296,21 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    if (lane == 0) ss_s[warp][m] = ss;
+                    if (lane == 0) ss_s[warp & 3][m] = ss;
                 }
             }
             __syncthreads();
             if (tid < a.M && tid % splits == rank) a.ss_out[tile * 64 + tid] = (ss_s[0][tid] + ss_s[1][tid]) + (ss_s[2][tid] + ss_s[3][tid]);
             if (a.advance && blockIdx.x == 0 && tid == 0) *a.advance += 1;
         } else {
-            const int col = n0 + tid;
-            for (int m0 = rank; m0 < a.M; m0 += kBatch * splits) {
+            const int col = n0 + (tid & 127), by = 2 * splits;
+#pragma unroll 1
+            for (int m0 = rank + splits * (tid >> 7); m0 < a.M; m0 += kBatch * by) {
                 float v[kBatch];
-                sums(v, m0, splits, tid);
+                sums(v, m0, by, tid & 127);
 #pragma unroll
                 for (int q = 0; q < kBatch; ++q) {
-                    const int m = m0 + q * splits;
+                    const int m = m0 + q * by;
                     if (m < a.M && col < a.N) a.c[(size_t)m * a.N + col] = __fmul_rn(v[q], inv_s[m]);
                 }
             }
