@@ -208,6 +208,8 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
                gemm_tc_usable(wdt, M, m->inter_l, H, lw.wdown);
     }
 
+    // The attention's result as the pair that the output projection reads (prompts of the fused path, and batched steps below).
+    __nv_bfloat16 *const att_hi = reinterpret_cast<__nv_bfloat16 *>(w.att + M * m->qd_l), *const att_lo = att_hi + M * m->qd_l;
     auto attend = [&](const LayerW &lw, lumen_kv_cache *c) -> int {
         if (p.decode) {
             AttnDecodeArgs a;
@@ -228,6 +230,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         a.cos_t = m->cos_t; a.sin_t = m->sin_t;
         a.q_norm = lw.qn; a.k_norm = lw.kn; a.norm_eps = eps;
         a.scale = scale; a.causal = 1; a.out = w.att;
+        if (fuse) { a.out_hi = att_hi; a.out_lo = att_lo; }
         LUMEN_TRY(launch_attn_prefill(ctx, a, s));
         return launch_bump_len(ctx, c->d_len, (int)p.S, s);
     };
@@ -244,7 +247,6 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         lumen_ctx *ctx;
         ~PdlScope() { ctx->pdl = false; }
     } pdl_scope{ctx};
-    __nv_bfloat16 *const att_hi = reinterpret_cast<__nv_bfloat16 *>(w.att + M * m->qd_l), *const att_lo = att_hi + M * m->qd_l;
     auto rows_args = [&](const void *wmat, size_t rows, size_t K, size_t N, const __nv_bfloat16 *hi, const __nv_bfloat16 *lo, int n_ss) {
         GemmRowsArgs g;
         GemmFuse split;
@@ -261,11 +263,12 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     };
     const int ss_tiles = (int)((H + 127) / 128);
     // Row-parallel product of the fused step: x = x + a . W^T summed over the ranks, and the split of RMSNorm(x) * norm_w
-    // for the next product (norm_w null after the last block).  `a` null: the activations are the SwiGLU pair.
+    // for the next product (norm_w null after the last block).  `a` null: the activations are the SwiGLU pair; otherwise the attention's.
     auto row_parallel = [&](const float *a, const void *wmat, size_t K, const float *norm_w) -> int {
         GemmFuse f;
         use_weight_split(m, wmat, f);
         if (!a) { f.a_hi = w.g_hi; f.a_lo = w.g_lo; }
+        else if (!p.decode) { f.a_hi = att_hi; f.a_lo = att_lo; }
         if (!tp) {
             f.post = GemmFuse::kPostNorm; f.norm_w = norm_w; f.eps = eps; f.next_hi = w.p_hi; f.next_lo = w.p_lo;
             return launch_gemm_tc(ctx, a, wmat, wdt, w.x, M, K, H, res_x, s, nullptr, &f);
@@ -302,7 +305,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
                 LUMEN_TRY(launch_attn_rows(ctx, r, p.B, m->hq_l, m->hkv_l, m->D, p.parts, s));
             } else {
                 LUMEN_TRY(attend(lw, c));
-                LUMEN_TRY(launch_split_bf16(ctx, w.att, att_hi, att_lo, M * m->qd_l, s));
+                if (p.decode) LUMEN_TRY(launch_split_bf16(ctx, w.att, att_hi, att_lo, M * m->qd_l, s));
             }
             LUMEN_TRY(rows_residual(lw.wo, m->qd_l, att_hi, att_lo, lw.norm2, rows_attn ? c->d_len : nullptr));
             g = rows_args(lw.wgate, M, H, 2 * m->inter_l, w.p_hi, w.p_lo, ss_tiles);

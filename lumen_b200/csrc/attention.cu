@@ -565,6 +565,7 @@ int launch_attn_decode(lumen_ctx *ctx, const AttnDecodeArgs &a, cudaStream_t s) 
 int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s) {
     if (a.D == 0 || a.D > 256 || (a.D & 1)) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "attention: head_dim %zu", a.D);
     if (a.Hkv == 0 || a.Hq % a.Hkv) return set_error(ctx, LUMEN_ERR_SHAPE, "attention: Hq %zu not a multiple of Hkv %zu", a.Hq, a.Hkv);
+    if (attn_prefill_tc_usable(a)) return launch_attn_prefill_tc(ctx, a, s);
     PrefillParams p;
     p.q = a.q; p.k = a.k; p.v = a.v; p.q_stride = a.q_stride; p.kv_stride = a.kv_stride;
     p.k_cache = a.k_cache; p.v_cache = a.v_cache;
@@ -577,11 +578,6 @@ int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s
     p.q_rot = static_cast<float *>(qrot);
     attn_prefill_prep_kernel<<<dim3((unsigned)a.S, (unsigned)a.B), kThreads, kWarps * a.D * sizeof(float), s>>>(p);
     LUMEN_LAUNCHED(ctx);
-    if (attn_prefill_tc_usable(a)) {
-        const int rc = launch_attn_prefill_tc(ctx, a, p.q_rot, s);
-        const int rc2 = dev_free(ctx, qrot);
-        return rc != LUMEN_OK ? rc : rc2;
-    }
     dim3 grid((unsigned)((a.S + kWarps - 1) / kWarps), (unsigned)a.Hq, (unsigned)a.B);
     switch (pick_ni(a.D)) {
         case 1: attn_prefill_kernel<1><<<grid, kThreads, 0, s>>>(p); break;
@@ -591,6 +587,7 @@ int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s
     }
     LUMEN_LAUNCHED(ctx);
     LUMEN_TRY(dev_free(ctx, qrot));
+    if (a.out_hi) LUMEN_TRY(launch_split_bf16(ctx, a.out, a.out_hi, a.out_lo, a.B * a.S * a.Hq * a.D, s));
     return LUMEN_OK;
 }
 

@@ -13,7 +13,7 @@
 //     held in registers: ctx = ctx * exp(m_old - m_new) + O_tile.
 // f32 values go through the tensor cores as hi + lo bf16 pairs (hi = bf16(x), lo = bf16(x - hi)) and three of the
 // four cross products are accumulated in f32, which keeps products to ~2^-17 relative: the result agrees with
-// the f32 reference to ~1e-5.  Q, K and V^T are split (and V transposed) by small kernels beforehand; rows
+// the f32 reference to ~1e-5.  Q, K and V^T are split (and rotated, or transposed) by small kernels beforehand; rows
 // beyond the context are zero so that masked weights (exactly 0) meet finite values.
 //
 // The same kernel serves latent attention over expanded keys and values (launch_latent_prefill): Q, K and V are single bf16
@@ -24,6 +24,7 @@
 // Every wait is bounded; a wait that gives up records LUMEN_ERR_TIMEOUT, the CTA leaves its loop at the next
 // block-wide barrier, lets the copies in flight land, frees its tensor memory and returns.
 #include <algorithm>
+#include <type_traits>
 
 #include "decoder_kernels.cuh"
 #include "tc_common.cuh"
@@ -366,7 +367,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
                 const float inv = __fdiv_rn(1.0f, CHUNK ? xch[0][row] + xch[1][row] : __fadd_rn(xch[0][row] + xch[1][row], 1e-9f));
                 const size_t orow = (size_t)b * p.S + (i0 + row);
                 if constexpr (PAIR) {
-                    float *o = p.out + (orow * p.Hq + h) * DV + half * kDH;
+                    const size_t at = (orow * p.Hq + h) * DV + half * kDH;
+                    float *o = p.out + at;
+                    if (p.out_hi) {
+#pragma unroll
+                        for (int e = 0; e < kDH; e += 8) {
+                            uint32_t hi[4], lo[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const float x = __fmul_rn(ctx[e + 2 * u], inv), y = __fmul_rn(ctx[e + 2 * u + 1], inv);
+                                hi[u] = pack_bf16(x, y);
+                                lo[u] = pack_bf16(x - __uint_as_float(hi[u] << 16), y - __uint_as_float(hi[u] & 0xffff0000u));
+                            }
+                            *reinterpret_cast<uint4 *>(p.out_hi + at + e) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                            *reinterpret_cast<uint4 *>(p.out_lo + at + e) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        }
+                    } else
 #pragma unroll
                     for (int e = 0; e < kDH; e += 4)
                         *reinterpret_cast<float4 *>(o + e) = make_float4(__fmul_rn(ctx[e], inv), __fmul_rn(ctx[e + 1], inv),
@@ -415,29 +431,103 @@ __device__ __forceinline__ void split_store(float x, __nv_bfloat16 *hi, __nv_bfl
     lo[i] = __float2bfloat16_rn(x - __bfloat162float(h));
 }
 
-// q_rot [B, S, Hq, D] f32 -> hi / lo [B, Hq, s_pad, D] bf16, rows s >= S zero.  One thread per element.
-__global__ void fa_split_q_kernel(const float *__restrict__ q_rot, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                  int S, int Hq, int D, int s_pad, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int e = (int)(i % D);
-    const size_t row = i / D;
-    const int s = (int)(row % s_pad);
-    const size_t bh = row / s_pad;
-    const size_t b = bh / Hq, h = bh % Hq;
-    split_store(s < S ? q_rot[((b * S + s) * Hq + h) * D + e] : 0.f, hi, lo, i);
+// What the projections left, as the tensor cores and the cache want it: q rotated into hi / lo [B, Hq, s_pad, D] (rows s >= S zero), k
+// rotated and v copied into the cache at past + s, and, where nothing was cached before (khi not null), k into hi / lo
+// [B, Hkv, l_pad, D] as well (rows s >= S zero).  grid (s_pad, B), a warp per head vector: a lane holds D / 32 neighbours, its partner in
+// the rotation is the lane 16 further.  Bound by HBM: 8192 positions of 32 + 16 heads of 128 numbers in 115 us (3.8 TB/s), against
+// 121 + 178 + 36 us for a rotation through shared memory and two kernels that split its results element by element.
+template <int D>
+__global__ void __launch_bounds__(256) fa_pack_kernel(const AttnPrefillArgs a, __nv_bfloat16 *__restrict__ qhi, __nv_bfloat16 *__restrict__ qlo,
+                                                      __nv_bfloat16 *__restrict__ khi, __nv_bfloat16 *__restrict__ klo, int s_pad, int l_pad, bool vec) {
+    constexpr int E = D / 32;
+    using V = typename std::conditional<E == 4, float4, float2>::type;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.x, b = blockIdx.y, e0 = lane * E;
+    const int S = (int)a.S, Hq = (int)a.Hq, Hkv = (int)a.Hkv;
+    const size_t row = (size_t)b * S + s, pos = a.past + s;
+    const bool live = s < S;
+    float co[E], sn[E], gq[E], gk[E];
+    const bool rot = a.cos_t != nullptr && live;
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+        const int j = (e0 + i) % (D / 2);
+        co[i] = rot ? a.cos_t[pos * (D / 2) + j] : 1.f;
+        sn[i] = rot ? a.sin_t[pos * (D / 2) + j] : 0.f;
+        gq[i] = a.q_norm ? a.q_norm[e0 + i] : 1.f;
+        gk[i] = a.k_norm ? a.k_norm[e0 + i] : 1.f;
+    }
+    auto pair_out = [&](__nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t at, const float (&v)[E]) {
+        uint32_t h[E / 2], l[E / 2];
+#pragma unroll
+        for (int i = 0; i < E / 2; ++i) {
+            h[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+            l[i] = pack_bf16(v[2 * i] - __uint_as_float(h[i] << 16), v[2 * i + 1] - __uint_as_float(h[i] & 0xffff0000u));
+        }
+        if constexpr (E == 4) {
+            *reinterpret_cast<uint2 *>(hi + at) = make_uint2(h[0], h[1]);
+            *reinterpret_cast<uint2 *>(lo + at) = make_uint2(l[0], l[1]);
+        } else {
+            *reinterpret_cast<uint32_t *>(hi + at) = h[0];
+            *reinterpret_cast<uint32_t *>(lo + at) = l[0];
+        }
+    };
+#pragma unroll 2
+    for (int h = warp; h < Hq + 2 * Hkv; h += 8) {
+        const bool is_q = h < Hq, is_k = !is_q && h < Hq + Hkv;
+        const int hk = is_q ? 0 : is_k ? h - Hq : h - Hq - Hkv;
+        float v[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = 0.f;
+        if (live) {
+            const float *src = is_q ? a.q + row * a.q_stride + (size_t)h * D : (is_k ? a.k : a.v) + row * a.kv_stride + (size_t)hk * D;
+            if (vec) {
+                *reinterpret_cast<V *>(v) = *reinterpret_cast<const V *>(src + e0);
+            } else {
+#pragma unroll
+                for (int i = 0; i < E; ++i) v[i] = src[e0 + i];
+            }
+            if (is_q || is_k) {
+                if (is_q ? a.q_norm != nullptr : a.k_norm != nullptr) {  // RMSNorm of the head (rms_norm.rs:49-56)
+                    float ss = 0.f;
+#pragma unroll
+                    for (int i = 0; i < E; ++i) ss = fmaf(v[i], v[i], ss);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)D), a.norm_eps)));
+#pragma unroll
+                    for (int i = 0; i < E; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], inv), is_q ? gq[i] : gk[i]);
+                }
+                if (rot) {  // encoding.rs:195-203
+#pragma unroll
+                    for (int i = 0; i < E; ++i) {
+                        const float other = __shfl_xor_sync(0xffffffffu, v[i], 16);
+                        v[i] = lane < 16 ? __fsub_rn(__fmul_rn(v[i], co[i]), __fmul_rn(other, sn[i])) : __fadd_rn(__fmul_rn(v[i], co[i]), __fmul_rn(other, sn[i]));
+                    }
+                }
+            }
+        }
+        if (is_q) {
+            pair_out(qhi, qlo, (((size_t)b * Hq + h) * s_pad + s) * D + e0, v);
+            continue;
+        }
+        if (is_k && khi && s < l_pad) pair_out(khi, klo, (((size_t)b * Hkv + hk) * l_pad + s) * D + e0, v);
+        if (live) *reinterpret_cast<V *>((is_k ? a.k_cache : a.v_cache) + (((size_t)b * Hkv + hk) * a.max_seq + pos) * D + e0) = *reinterpret_cast<const V *>(v);
+    }
 }
 
-// K cache [B*Hkv, max_seq, D] f32 -> hi / lo [B*Hkv, l_pad, D] bf16, rows >= total zero.
-__global__ void fa_split_k_kernel(const float *__restrict__ k_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                  int total, int max_seq, int D, int l_pad, size_t n) {
+// K cache [B*Hkv, max_seq, D] f32 -> hi / lo [B*Hkv, l_pad, D] bf16, rows >= total zero.  One thread per four elements (D is a multiple of 64).
+__global__ void __launch_bounds__(256) fa_split_k_kernel(const float *__restrict__ k_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
+                                                         int total, int max_seq, int D, int l_pad, size_t n4) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int e = (int)(i % D);
-    const size_t row = i / D;
+    if (i >= n4) return;
+    const int per = D / 4, e = (int)(i % per) * 4;
+    const size_t row = i / per;
     const int j = (int)(row % l_pad);
     const size_t bh = row / l_pad;
-    split_store(j < total ? k_cache[(bh * max_seq + j) * D + e] : 0.f, hi, lo, i);
+    const float4 v = j < total ? *reinterpret_cast<const float4 *>(k_cache + (bh * max_seq + j) * D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t h0 = pack_bf16(v.x, v.y), h1 = pack_bf16(v.z, v.w);
+    reinterpret_cast<uint2 *>(hi)[i] = make_uint2(h0, h1);
+    reinterpret_cast<uint2 *>(lo)[i] = make_uint2(pack_bf16(v.x - __uint_as_float(h0 << 16), v.y - __uint_as_float(h0 & 0xffff0000u)),
+                                                  pack_bf16(v.z - __uint_as_float(h1 << 16), v.w - __uint_as_float(h1 & 0xffff0000u)));
 }
 
 // V cache [B*Hkv, max_seq, D] f32 -> transposed hi / lo [B*Hkv, D, l_pad] bf16, columns >= total zero.
@@ -513,21 +603,22 @@ int launch_fa(lumen_ctx *ctx, const CUtensorMap *maps, const FaParams &p, dim3 g
 
 }  // namespace
 
-// Head dimensions 64 and 128, prompts of at least 64 positions (shorter ones leave most of a 128-row tile empty
-// and stay on the warp-per-row kernel).  LUMEN_NO_TC_ATTN=1 switches the path off.
+// Head dimensions 64 and 128, prompts of at least 64 positions.  Shorter ones leave most of a 128-row tile empty and stay on the
+// warp-per-row kernel unless there is much of them: that kernel takes 0.4 ns per pair of positions and head (437 us for 64 sequences x 32
+// heads x 60 positions, 108 us and 20 us more for packing here), and this path some 20 us however little there is to do.  LUMEN_NO_TC_ATTN=1 switches the path off.
 bool attn_prefill_tc_usable(const AttnPrefillArgs &a) {
     static const bool off = [] {
         const char *e = getenv("LUMEN_NO_TC_ATTN");
         return e && e[0] == '1';
     }();
-    if (off || (a.D != 64 && a.D != 128) || a.S < 64) return false;
+    if (off || (a.D != 64 && a.D != 128)) return false;
+    if (a.S < 64 && (a.S < 16 || a.B * a.Hq * a.S * (a.past + a.S) < ((size_t)1 << 20))) return false;
     const size_t l_pad = (a.past + a.S + 63) / 64 * 64, s_pad = (a.S + 127) / 128 * 128;
     // tensor-map coordinates are 32-bit row numbers
     return a.B * a.Hq * s_pad < ((size_t)1 << 31) && a.B * a.Hkv * l_pad < ((size_t)1 << 31) && a.B <= 65535 && a.Hq <= 65535;
 }
 
-// q_rot: the rotated queries [B, S, Hq, D]; the cache already holds rows 0 .. past + S - 1.
-int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, const float *q_rot, cudaStream_t s) {
+int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s) {
     const size_t total = a.past + a.S;
     const size_t l_pad = (total + 63) / 64 * 64, s_pad = (a.S + kBQ - 1) / kBQ * kBQ;
     const size_t nq = a.B * a.Hq * s_pad * a.D, nkv = a.B * a.Hkv * l_pad * a.D;
@@ -541,10 +632,16 @@ int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, const float
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, what);
         else ctx->launches += 1;
     };
-    fa_split_q_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(q_rot, qhi, qlo, (int)a.S, (int)a.Hq, (int)a.D, (int)s_pad, nq);
-    launched("fa_split_q_kernel launch");
-    if (rc == LUMEN_OK) {
-        fa_split_k_kernel<<<(unsigned)((nkv + 255) / 256), 256, 0, s>>>(a.k_cache, khi, klo, (int)total, (int)a.max_seq, (int)a.D, (int)l_pad, nkv);
+    const bool fresh = a.past == 0;
+    const bool vec = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0 &&
+                     a.q_stride % 4 == 0 && a.kv_stride % 4 == 0;
+    const dim3 pack_grid((unsigned)s_pad, (unsigned)a.B);
+    __nv_bfloat16 *kh = fresh ? khi : nullptr, *kl = fresh ? klo : nullptr;
+    if (a.D == 64) fa_pack_kernel<64><<<pack_grid, 256, 0, s>>>(a, qhi, qlo, kh, kl, (int)s_pad, (int)l_pad, vec);
+    else fa_pack_kernel<128><<<pack_grid, 256, 0, s>>>(a, qhi, qlo, kh, kl, (int)s_pad, (int)l_pad, vec);
+    launched("fa_pack_kernel launch");
+    if (rc == LUMEN_OK && !fresh) {
+        fa_split_k_kernel<<<(unsigned)((nkv / 4 + 255) / 256), 256, 0, s>>>(a.k_cache, khi, klo, (int)total, (int)a.max_seq, (int)a.D, (int)l_pad, nkv / 4);
         launched("fa_split_k_kernel launch");
     }
     if (rc == LUMEN_OK) {
@@ -562,7 +659,7 @@ int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, const float
     if (rc == LUMEN_OK) rc = make_map(ctx, &maps[5], vlo, a.B * a.Hkv * a.D, l_pad, (int)a.D);
     if (rc == LUMEN_OK) {
         FaParams p{};
-        p.out = a.out;
+        p.out = a.out; p.out_hi = a.out_hi; p.out_lo = a.out_lo;
         p.S = (int)a.S; p.Hq = (int)a.Hq; p.Hkv = (int)a.Hkv; p.past = (int)a.past; p.total = (int)total; p.causal = a.causal;
         p.s_pad = (int)s_pad;
         p.k_rows_b = (int)(a.Hkv * l_pad); p.k_rows_h = (int)l_pad; p.kb_main = (int)(a.D / kBK);

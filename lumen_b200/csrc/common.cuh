@@ -351,12 +351,12 @@ struct AttnPrefillArgs {
     float scale = 0.f;
     int causal = 1;
     float *out = nullptr;
+    __nv_bfloat16 *out_hi = nullptr, *out_lo = nullptr;  // the result as a bf16 pair (then `out` is scratch)
 };
 int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s);
-// Tensor-core prefill attention (attn_prefill_tc.cu): q_rot holds the rotated queries [B, S, Hq, D] and the
-// cache rows 0 .. past + S - 1 are already written.
+// Tensor-core prefill attention (attn_prefill_tc.cu), the rotation and the cache's new rows included.
 bool attn_prefill_tc_usable(const AttnPrefillArgs &a);
-int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, const float *q_rot, cudaStream_t s);
+int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s);
 
 // Nucleus sampling of one logits vector on the device (sampler.cu); waits for the stream.
 int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lumen_sample_params &sp, int32_t *token, cudaStream_t s);

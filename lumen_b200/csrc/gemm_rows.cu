@@ -11,14 +11,14 @@
 //   - RMSNorm is a scalar per row, so it is left to the next product: a product's epilogue adds the residual, and writes x, the pair
 //     (hi, lo) of x * gains, and its tile's sum of squares; the next product's epilogue multiplies by 1 / rms.  No kernel has to see a whole row;
 //   - SwiGLU: a tile is 64 rows of gate and the 64 rows of up that go with them;
-//   - programmatic dependent launch: a CTA asks for its first weights (and, for the L2, for those behind them), then waits for the
-//     kernel before it.  The ring is small enough (111 KB) for two CTAs per SM, so that the next product's CTAs find room
-//     before this one's end;
+//   - programmatic dependent launch: a CTA asks for its first weights, then waits for the kernel before it.  The ring is small
+//     enough (111 KB) for two CTAs per SM, so that the next product's CTAs find room before this one's end.  (Asking for the rest too, up to
+//     64 MB for the L2, gained nothing with 16 rows and cost 3 % with 64: the way from the L2 to the SMs is busy enough);
 //   - hi and lo of the activations are one operand of twice the columns: two MMAs per step of K with f32 weights, not three, and even
 //     and odd steps have accumulators of their own (a chain of small MMAs into one accumulator is bound by their latency).
 //
 // TinyLlama f32, 16 sequences: 40 steps and the prefill of 64 positions 84 -> 60.8 ms (a step 1.9 -> 1.3 ms); 9 layers of the Qwen3-8B
-// shape, 64 sequences: 32 steps and a prefill of 60 positions 95 -> 81.3 ms.
+// shape, 64 sequences: a step 1.9 -> 1.5 ms.
 //
 // Thread 0 is the TMA producer, thread 32 issues the MMAs, warps 2 and 3 form 1 / rms meanwhile; all eight warps are the epilogue (its code runs
 // once per CTA, so it is bound by latencies and by the way of the instructions themselves: short loops, little unrolling).
@@ -39,7 +39,6 @@ namespace cg = cooperative_groups;
 
 constexpr int kRowsThreads = 256;
 constexpr int kRowsRing = 111 * 1024;
-constexpr size_t kRowsL2 = (size_t)64 << 20;  // bytes that the CTAs of one product may request ahead for the L2
 
 template <int NW, int BN>
 struct RowsGeom {
@@ -55,13 +54,9 @@ struct RowsGeom {
 struct RowsParams {
     GemmRowsArgs a;
     int kb_per, splits;
-    int l2_ahead;  // steps of K requested for the L2 at the start
     DeviceStatus *status;
 };
 
-__device__ __forceinline__ void prefetch_2d(const CUtensorMap *map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
 // 16 consecutive accumulator columns of this thread's lane; usable after tmem_ld_wait().
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -164,20 +159,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (!ok) failed = 1;
         umma_commit(&done);
     } else if (warp == 2 || warp == 3) {
-        if (tid == 96) {
-            // what the ring cannot take goes to the L2: HBM would otherwise idle while the kernel before this one ends
-            const int end = min(nkb, ahead + p.l2_ahead);
-            for (int kb = ahead; kb < end; ++kb) {
-                const int kx = k_of(kb);
-                prefetch_2d(&map_w, kx, n0);
-                prefetch_2d(&map_w, kx, n1);
-                if (NW == 2) {
-                    prefetch_2d(&map_wlo, kx, n0);
-                    prefetch_2d(&map_wlo, kx, n1);
-                }
-            }
-        }
-        __syncwarp();
         pdl_wait();
         const int m = tid - 64;
         if (m < a.M) {
@@ -370,7 +351,6 @@ int launch_rows_t(lumen_ctx *ctx, const GemmRowsArgs &a, cudaStream_t s) {
     p.splits = 1;
     while (p.splits < 8 && tiles * p.splits * 100 < ctx->num_sms * 85 && kb_all >= 8 * p.splits) p.splits *= 2;
     p.kb_per = (kb_all + p.splits - 1) / p.splits;
-    p.l2_ahead = (int)(kRowsL2 / ((size_t)std::min(tiles * p.splits, 2 * ctx->num_sms) * NW * G::kWBytes));
     return launch_pdl_cluster(ctx, kernel, (unsigned)p.splits, dim3((unsigned)(tiles * p.splits)), dim3(kRowsThreads), smem, s, mw, mwlo, mx, mxlo, p);
 }
 

@@ -41,46 +41,48 @@ struct RowFinish {
     __nv_bfloat16 *hi, *lo;  // [rows, dim] bf16 split of Norm(row) (null: not stored)
 };
 
-// acc[k] = sum over `splits` slices (added in slice order) of part[slice][row] (+ residual[row]): the thread's share of a row.
-__device__ __forceinline__ void row_load_sum(float4 (&acc)[kRowVecs], const float *part, int splits, size_t mn, const float *residual,
+// NV: float4 per thread, NV * 1024 >= row length.  acc[k] = sum over `splits` slices (added in slice order) of part[slice][row] (+ residual[row]): the thread's share of a row.
+template <int NV>
+__device__ __forceinline__ void row_load_sum(float4 (&acc)[NV], const float *part, int splits, size_t mn, const float *residual,
                                              size_t base, int nvec, int tid) {
     {
         const float4 *p0 = reinterpret_cast<const float4 *>(part + base);
 #pragma unroll
-        for (int k = 0; k < kRowVecs; ++k)
+        for (int k = 0; k < NV; ++k)
             if (tid + 256 * k < nvec) acc[k] = p0[tid + 256 * k];
     }
 #pragma unroll 4
     for (int sl = 1; sl < splits; ++sl) {
         const float4 *ps = reinterpret_cast<const float4 *>(part + (size_t)sl * mn + base);
-        float4 t[kRowVecs];
+        float4 t[NV];
 #pragma unroll
-        for (int k = 0; k < kRowVecs; ++k)
+        for (int k = 0; k < NV; ++k)
             if (tid + 256 * k < nvec) t[k] = ps[tid + 256 * k];
 #pragma unroll
-        for (int k = 0; k < kRowVecs; ++k)
+        for (int k = 0; k < NV; ++k)
             if (tid + 256 * k < nvec) acc[k] = add4(acc[k], t[k]);
     }
     if (residual) {
         const float4 *pr = reinterpret_cast<const float4 *>(residual + base);
-        float4 t[kRowVecs];
+        float4 t[NV];
 #pragma unroll
-        for (int k = 0; k < kRowVecs; ++k)
+        for (int k = 0; k < NV; ++k)
             if (tid + 256 * k < nvec) t[k] = pr[tid + 256 * k];
 #pragma unroll
-        for (int k = 0; k < kRowVecs; ++k)
+        for (int k = 0; k < NV; ++k)
             if (tid + 256 * k < nvec) acc[k] = add4(t[k], acc[k]);
     }
 }
 
 // Stores the row and, with gains, RMSNorm::forward of it (src/layers/norm/rms_norm.rs:49-56: rms = sqrt(ss/dim + eps),
 // o = (x * (1/rms)) * w) as f32 and/or as the bf16 hi/lo pair.  `red` is 8 floats of shared memory; all 256 threads call.
-__device__ __forceinline__ void row_finish(const float4 (&v)[kRowVecs], const RowFinish &f, size_t base, int dim, int nvec, int tid,
+template <int NV>
+__device__ __forceinline__ void row_finish(const float4 (&v)[NV], const RowFinish &f, size_t base, int dim, int nvec, int tid,
                                            float *red) {
     float ss = 0.f;
     float4 *o4 = f.out ? reinterpret_cast<float4 *>(f.out + base) : nullptr;
 #pragma unroll
-    for (int k = 0; k < kRowVecs; ++k)
+    for (int k = 0; k < NV; ++k)
         if (tid + 256 * k < nvec) {
             if (o4) o4[tid + 256 * k] = v[k];
             ss = fmaf(v[k].x, v[k].x, ss);
@@ -104,7 +106,7 @@ __device__ __forceinline__ void row_finish(const float4 (&v)[kRowVecs], const Ro
     uint2 *h2 = f.hi ? reinterpret_cast<uint2 *>(f.hi + base) : nullptr;
     uint2 *l2 = f.hi ? reinterpret_cast<uint2 *>(f.lo + base) : nullptr;
 #pragma unroll
-    for (int k = 0; k < kRowVecs; ++k)
+    for (int k = 0; k < NV; ++k)
         if (tid + 256 * k < nvec) {
             const float4 g = g4[tid + 256 * k];
             const float4 n = make_float4(__fmul_rn(__fmul_rn(v[k].x, inv), g.x), __fmul_rn(__fmul_rn(v[k].y, inv), g.y),

@@ -140,6 +140,30 @@ def test_batched_steps_as_a_chain_of_products(L, oracle, heads, kv, dim, hidden,
     assert rel_err(got, want) < TOL_F32
 
 
+@pytest.mark.parametrize("kv,dim,prompts", [(2, 64, (48, 17)), (4, 128, (50, 31, 64)), (8, 64, (63,))])
+def test_many_short_prompts_on_the_tensor_cores(L, oracle, kv, dim, prompts):
+    """Prompts of fewer than 64 positions of many sequences take the tensor-core attention (8 heads x 64 sequences x positions squared >= 2^20),
+    into an empty cache and behind rows that are there already."""
+    cfg = small_cfg(hidden_size=128, num_attention_heads=8, num_key_value_heads=kv, head_dim=dim, intermediate_size=136, qk_norm=dim == 128, max_seq_len=160)
+    params = make_params(L, cfg, 51, std=0.08, random_norms=True)
+    ids = np.random.default_rng(kv).integers(0, cfg["vocab_size"], size=(64, sum(prompts))).astype(np.float32)
+    model = L.LlamaModel(cfg_obj(L, cfg))
+    model.load_state(params)
+    caches = model.init_kv_caches(64)
+    ref = oracle.Llama(cfg, params, "f64")
+    rcaches = ref.init_kv_caches(64)
+    at = 0
+    with L.no_grad():
+        for n in prompts:
+            got = model.forward(ids[:, at:at + n], caches, 0)
+            want = ref.forward(ids[:, at:at + n], rcaches)
+            at += n
+            assert rel_err(got, want) < TOL_F32
+    for l in range(cfg["num_hidden_layers"]):
+        k, v = caches[l].read()
+        assert rel_err(k, rcaches[l].k) < 5e-5 and rel_err(v, rcaches[l].v) < 5e-5
+
+
 def test_forward_last_and_device_entry_points(L, oracle):
     cfg = small_cfg()
     params = make_params(L, cfg, 31, std=0.08)
