@@ -276,7 +276,7 @@ sample_pick_kernel(const float *__restrict__ sorted_p, const int *__restrict__ s
 // a candidate's rank within its bin is the number of larger ones (an equal probability of a smaller index is larger: the sort
 // is stable).  CTA 0 then walks the list as the general path does.
 // What bounds it is the chain of passes and cluster barriers, not bytes.  32000 logits of which some hundred to a thousand make the
-// nucleus: 33 us against 100 us for the seven kernels of the general path, 56 us against 140 us for the whole call.
+// nucleus: 24 us against 100 us for the seven kernels of the general path, 48 us against 140 us for the whole call.
 namespace cg = cooperative_groups;
 constexpr int kCluster = 8;
 constexpr int kNucleusBins = 24 * 128;
@@ -302,6 +302,7 @@ struct NucleusShared {
     int hist[kNucleusBins], cursor[kNucleusBins], first[kNucleusBins + 1];  // counts here; next place; first place of a bin
     __align__(16) unsigned long long window[kPrepThreads / 32][32];
     float red[33], top, part[4];
+    int recent[kMaxRecent];
     int scan_n[32];
     float scan_m[32];
     int last_bin, crowded;
@@ -321,6 +322,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
 #pragma unroll 4
     for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? a.logits[index_of(s)] : -INFINITY;
     for (int b = tid; b < kNucleusBins; b += kPrepThreads) sh.hist[b] = 0;
+    if (tid < a.n_recent) sh.recent[tid] = a.recent[tid];
     if (tid == 0) {
         sh.last_bin = INT_MAX;
         sh.crowded = 0;
@@ -328,13 +330,18 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     __syncthreads();
     if (a.penalty > 1.0f && tid < a.n_recent) {
         // the first occurrence of a token applies one division per occurrence (main.rs:83-89)
-        const int t = a.recent[tid];
-        bool first = t >= 0 && t < n && ((t >> 7) & (kCluster - 1)) == rank;
-        for (int k = 0; k < tid && first; ++k) first = a.recent[k] != t;
-        if (first) {
-            float &x = vals[(t >> 10) * 128 + (t & 127)];
-            for (int k = tid; k < a.n_recent; ++k)
-                if (a.recent[k] == t) x = __fdiv_rn(x, a.penalty);
+        const int t = sh.recent[tid];
+        int times = 0, before = 0;
+#pragma unroll 4
+        for (int k = 0; k < a.n_recent; ++k) {
+            const int same = sh.recent[k] == t;
+            times += same;
+            before += k < tid ? same : 0;
+        }
+        if (before == 0 && t >= 0 && t < n && ((t >> 7) & (kCluster - 1)) == rank) {
+            float x = vals[(t >> 10) * 128 + (t & 127)];
+            for (int k = 0; k < times; ++k) x = __fdiv_rn(x, a.penalty);
+            vals[(t >> 10) * 128 + (t & 127)] = x;
         }
     }
     __syncthreads();
@@ -348,8 +355,15 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     mx = block_reduce(mx, sh.red, true);
     if (tid == 0) sh.top = mx;
     cluster.sync();
+    // (one warp reads the other CTAs' numbers: all of them at once would queue for the same words)
+    if (warp == 0) {
+        float t = *cluster.map_shared_rank(&sh.top, lane & (kCluster - 1));
 #pragma unroll
-    for (int c = 0; c < kCluster; ++c) mx = fmaxf(mx, *cluster.map_shared_rank(&sh.top, c));
+        for (int o = kCluster / 2; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+        if (lane == 0) sh.red[32] = t;
+    }
+    __syncthreads();
+    mx = sh.red[32];
     for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? expf(__fsub_rn(vals[s], mx)) : 0.f;
     __syncthreads();
     if (tid < 128) {
@@ -361,10 +375,14 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
         if (lane == 0) sh.part[warp] = sum;
     }
     cluster.sync();
-    float sum = *cluster.map_shared_rank(&sh.part[lane & 3], lane >> 2);
+    if (warp == 0) {
+        float sum = *cluster.map_shared_rank(&sh.part[lane & 3], lane >> 2);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float inv = __fdiv_rn(1.0f, __fadd_rn(sum, 1e-9f));
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) sh.red[0] = sum;
+    }
+    __syncthreads();
+    const float inv = __fdiv_rn(1.0f, __fadd_rn(sh.red[0], 1e-9f));
     const bool finite = inv > 0.f && inv < INFINITY;  // (the same in every CTA)
     for (int s = tid; s < slots; s += kPrepThreads) {
         const float p = __fmul_rn(vals[s], inv);
@@ -405,15 +423,21 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
         sh.scan_m[warp] = mass_in;
     }
     __syncthreads();
-    int at = count_in - count, counted = 0;
-    float reached = mass_in - mass;
-    for (int w = 0; w < kPrepThreads / 32; ++w) {
-        if (w < warp) {
-            at += sh.scan_n[w];
-            reached += sh.scan_m[w];
+    int w_count = sh.scan_n[lane];  // the 32 warps' totals, scanned by every warp
+    float w_mass = sh.scan_m[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int c = __shfl_up_sync(0xffffffffu, w_count, o);
+        const float m = __shfl_up_sync(0xffffffffu, w_mass, o);
+        if (lane >= o) {
+            w_count += c;
+            w_mass += m;
         }
-        counted += sh.scan_n[w];
     }
+    const int counted = __shfl_sync(0xffffffffu, w_count, 31), n_before = __shfl_sync(0xffffffffu, w_count, max(warp - 1, 0));
+    const float m_before = __shfl_sync(0xffffffffu, w_mass, max(warp - 1, 0));
+    int at = (warp ? n_before : 0) + count_in - count;
+    float reached = (warp ? m_before : 0.f) + mass_in - mass;
     const float need = a.target * (1.0f + 1.0f / 4096);  // (the sequential sum may round down a little; checked by the walk)
 #pragma unroll
     for (int j = 0; j < kBinsPerThread; ++j) {
