@@ -445,7 +445,7 @@ struct KnPlan {
 };
 
 // Tiles as wide as leave two CTAs per SM with K cut in eight; no more slices than that takes (a slice has at least four
-// rows per thread).
+// rows per thread), and no more CTAs than are resident, three per SM (500 CTAs for [4096,32000] bf16 took 63 us, 250 take 57).
 KnPlan plan_kn(size_t K, size_t N, int vec, int num_sms) {
     KnPlan p;
     const size_t want = 2 * (size_t)num_sms;
@@ -458,7 +458,7 @@ KnPlan plan_kn(size_t K, size_t N, int vec, int num_sms) {
     p.col_blocks = (int)blocks;
     const size_t rows = (size_t)kKnWarps * 32 / p.lanes;
     p.splits = 1;
-    while (p.splits < kKnSplits && blocks * p.splits < want && K > (size_t)p.splits * rows * 4) p.splits *= 2;
+    while (p.splits < kKnSplits && blocks * p.splits < want && 2 * blocks * p.splits <= 3 * (size_t)num_sms && K > (size_t)p.splits * rows * 4) p.splits *= 2;
     p.k_per_split = ((K + p.splits - 1) / p.splits + rows - 1) / rows * rows;
     return p;
 }
