@@ -17,7 +17,7 @@
 //   - hi and lo of the activations are one operand of twice the columns: two MMAs per step of K with f32 weights, not three, and even
 //     and odd steps have accumulators of their own (a chain of small MMAs into one accumulator is bound by their latency).
 //
-// TinyLlama f32, 16 sequences: 40 steps and the prefill of 64 positions 84 -> 60.8 ms (a step 1.9 -> 1.3 ms); 9 layers of the Qwen3-8B
+// TinyLlama f32, 16 sequences: 40 steps and the prefill of 64 positions 84 -> 59.7 ms (a step 1.9 -> 1.3 ms); 9 layers of the Qwen3-8B
 // shape, 64 sequences: a step 1.9 -> 1.5 ms.
 //
 // Thread 0 is the TMA producer, thread 32 issues the MMAs, warps 2 and 3 form 1 / rms meanwhile; all eight warps are the epilogue (its code runs
