@@ -8,6 +8,7 @@
 // reference: rotate q/k at positions past..past+S, slab write, causal mask j > past+i, softmax with
 // `1/(sum + 1e-9)`, P.V, output in [B,S,H,D] order.
 #include "attn_decode.cuh"
+#include "row_finish.cuh"
 
 namespace lumen {
 namespace {
@@ -48,6 +49,7 @@ struct PrefillParams {
     int causal;
     float *q_rot;  // [B,S,Hq,D]
     float *out;    // [B,S,Hq,D]
+    __nv_bfloat16 *out_hi, *out_lo;  // the same as a pair (attn_prefill_tile_kernel; null: f32)
 };
 
 // One warp per head vector of (b, s): heads 0..Hq-1 are q (rotated into q_rot), Hq..Hq+Hkv-1 are k
@@ -82,6 +84,128 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_prep_kernel(PrefillPara
         }
         __syncwarp();
     }
+}
+
+// Prompts of fewer than 64 positions whose context fits 64 rows: one CTA per (head, sequence), everything in shared memory, f32
+// throughout.  A thread forms a 4 x 4 block of the scores (rows ty + 16 i, cached rows tx + 16 j; rows padded by four numbers, so that
+// 16-byte reads of eight neighbouring rows hit different banks), then 4 rows x D / 16 numbers of the result.  Bound by the
+// FMA pipe: 2 x 64 x 64 x D FMAs per CTA however short the prompt, which is why fewer than 32 positions (that kernel: 124 us for 32) or fewer CTAs than SMs stay with a warp per query row.
+// 64 sequences x 32 heads x 60 positions of 128 numbers: 180 us against 437.  grid (Hq, B).
+constexpr int kTileRows = 64;
+template <int D>
+constexpr size_t prefill_tile_floats() { return (size_t)3 * kTileRows * (D + 4); }
+
+template <int D>
+__global__ void __launch_bounds__(256, 2) attn_prefill_tile_kernel(PrefillParams p) {
+    constexpr int LD = D + 4, LP = kTileRows + 4, V4 = D / 4;
+    extern __shared__ __align__(16) float smem[];
+    float *qs = smem, *ks = qs + kTileRows * LD, *vs = ks + kTileRows * LD, *ps = qs;  // (the weights take the place of q)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.x, b = blockIdx.y, hk = h / (p.Hq / p.Hkv);
+    const int total = p.past + p.S;
+    const float *kbase = p.k_cache + ((size_t)b * p.Hkv + hk) * p.max_seq * D, *vbase = p.v_cache + ((size_t)b * p.Hkv + hk) * p.max_seq * D;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < kTileRows * V4; i += 256) {
+        const int r = i / V4, e = (i % V4) * 4;
+        *reinterpret_cast<float4 *>(qs + r * LD + e) = r < p.S ? *reinterpret_cast<const float4 *>(p.q_rot + (((size_t)b * p.S + r) * p.Hq + h) * D + e) : zero;
+        *reinterpret_cast<float4 *>(ks + r * LD + e) = r < total ? *reinterpret_cast<const float4 *>(kbase + (size_t)r * D + e) : zero;
+        *reinterpret_cast<float4 *>(vs + r * LD + e) = r < total ? *reinterpret_cast<const float4 *>(vbase + (size_t)r * D + e) : zero;
+    }
+    __syncthreads();
+    const int tx = tid & 15, ty = tid >> 4;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+    for (int e = 0; e < D; e += 4) {
+        float4 q[4], k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            q[i] = *reinterpret_cast<const float4 *>(qs + (ty + 16 * i) * LD + e);
+            k[i] = *reinterpret_cast<const float4 *>(ks + (tx + 16 * i) * LD + e);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                acc[i][j] = fmaf(q[i].w, k[j].w, fmaf(q[i].z, k[j].z, fmaf(q[i].y, k[j].y, fmaf(q[i].x, k[j].x, acc[i][j]))));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i, last = p.causal ? min(total - 1, p.past + r) : total - 1;  // mask j > past + i
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ps[r * LP + tx + 16 * j] = tx + 16 * j <= last ? __fmul_rn(acc[i][j], p.scale) : -INFINITY;
+    }
+    __syncthreads();
+    for (int r = warp; r < p.S; r += kWarps) {  // weights of a row by a warp: exp(s - max) / (sum + 1e-9)
+        const float s0 = ps[r * LP + lane], s1 = ps[r * LP + lane + 32];
+        float m = fmaxf(s0, s1);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float w0 = expf(s0 - m), w1 = expf(s1 - m);
+        const float inv = __fdiv_rn(1.0f, __fadd_rn(attn_warp_sum(w0 + w1), 1e-9f));
+        ps[r * LP + lane] = __fmul_rn(w0, inv);
+        ps[r * LP + lane + 32] = __fmul_rn(w1, inv);
+    }
+    __syncthreads();
+    constexpr int NB = D / 64;  // groups of four numbers per thread: tx * 4 + 64 n
+    float4 c[4][NB];
+    int end[4];  // (rows behind a position are not its business, whatever they hold)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) end[i] = p.causal ? min(total, p.past + ty + 16 * i + 1) : total;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) c[i][n] = zero;
+#pragma unroll 4
+    for (int j = 0; j < total; ++j) {
+        float4 v[NB];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) v[n] = *reinterpret_cast<const float4 *>(vs + j * LD + tx * 4 + 64 * n);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (j >= end[i]) continue;
+            const float w = ps[(ty + 16 * i) * LP + j];
+#pragma unroll
+            for (int n = 0; n < NB; ++n) {
+                c[i][n].x = fmaf(w, v[n].x, c[i][n].x); c[i][n].y = fmaf(w, v[n].y, c[i][n].y);
+                c[i][n].z = fmaf(w, v[n].z, c[i][n].z); c[i][n].w = fmaf(w, v[n].w, c[i][n].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
+        if (r >= p.S) continue;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            const size_t at = (((size_t)b * p.S + r) * p.Hq + h) * D + tx * 4 + 64 * n;
+            if (p.out_hi) {
+                uint2 hi, lo;
+                split4(c[i][n], &hi, &lo);
+                *reinterpret_cast<uint2 *>(p.out_hi + at) = hi;
+                *reinterpret_cast<uint2 *>(p.out_lo + at) = lo;
+            } else {
+                *reinterpret_cast<float4 *>(p.out + at) = c[i][n];
+            }
+        }
+    }
+}
+
+template <int D>
+int launch_prefill_tile(lumen_ctx *ctx, const PrefillParams &p, dim3 grid, cudaStream_t s) {
+    constexpr size_t smem = prefill_tile_floats<D>() * sizeof(float);
+    static bool attr_set[64] = {false};
+    const int dev = ctx->device >= 0 && ctx->device < 64 ? ctx->device : 0;
+    if (!attr_set[dev]) {
+        LUMEN_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_tile_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set[dev] = true;
+    }
+    attn_prefill_tile_kernel<D><<<grid, 256, smem, s>>>(p);
+    LUMEN_LAUNCHED(ctx);
+    return LUMEN_OK;
 }
 
 // One warp per query row; grid (ceil(S/kWarps), Hq, B).
@@ -578,6 +702,14 @@ int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s
     p.q_rot = static_cast<float *>(qrot);
     attn_prefill_prep_kernel<<<dim3((unsigned)a.S, (unsigned)a.B), kThreads, kWarps * a.D * sizeof(float), s>>>(p);
     LUMEN_LAUNCHED(ctx);
+    p.out_hi = a.out_hi; p.out_lo = a.out_lo;
+    if ((a.D == 64 || a.D == 128) && a.S >= 32 && a.past + a.S <= (size_t)kTileRows && a.B <= 65535 && a.B * a.Hq >= (size_t)ctx->num_sms &&
+        ((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_hi) | reinterpret_cast<uintptr_t>(a.out_lo)) & 15) == 0) {
+        const dim3 g((unsigned)a.Hq, (unsigned)a.B);
+        const int rc = a.D == 64 ? launch_prefill_tile<64>(ctx, p, g, s) : launch_prefill_tile<128>(ctx, p, g, s);
+        const int rc2 = dev_free(ctx, qrot);
+        return rc != LUMEN_OK ? rc : rc2;
+    }
     dim3 grid((unsigned)((a.S + kWarps - 1) / kWarps), (unsigned)a.Hq, (unsigned)a.B);
     switch (pick_ni(a.D)) {
         case 1: attn_prefill_kernel<1><<<grid, kThreads, 0, s>>>(p); break;

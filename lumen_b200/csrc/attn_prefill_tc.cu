@@ -603,16 +603,14 @@ int launch_fa(lumen_ctx *ctx, const CUtensorMap *maps, const FaParams &p, dim3 g
 
 }  // namespace
 
-// Head dimensions 64 and 128, prompts of at least 64 positions.  Shorter ones leave most of a 128-row tile empty and stay on the
-// warp-per-row kernel unless there is much of them: that kernel takes 0.4 ns per pair of positions and head (437 us for 64 sequences x 32
-// heads x 60 positions, 108 us and 20 us more for packing here), and this path some 20 us however little there is to do.  LUMEN_NO_TC_ATTN=1 switches the path off.
+// Head dimensions 64 and 128, prompts of at least 64 positions (shorter ones leave most of a 128-row tile empty and stay on the
+// f32 kernels).  LUMEN_NO_TC_ATTN=1 switches the path off.
 bool attn_prefill_tc_usable(const AttnPrefillArgs &a) {
     static const bool off = [] {
         const char *e = getenv("LUMEN_NO_TC_ATTN");
         return e && e[0] == '1';
     }();
-    if (off || (a.D != 64 && a.D != 128)) return false;
-    if (a.S < 64 && (a.S < 16 || a.B * a.Hq * a.S * (a.past + a.S) < ((size_t)1 << 20))) return false;
+    if (off || (a.D != 64 && a.D != 128) || a.S < 64) return false;
     const size_t l_pad = (a.past + a.S + 63) / 64 * 64, s_pad = (a.S + 127) / 128 * 128;
     // tensor-map coordinates are 32-bit row numbers
     return a.B * a.Hq * s_pad < ((size_t)1 << 31) && a.B * a.Hkv * l_pad < ((size_t)1 << 31) && a.B <= 65535 && a.Hq <= 65535;
