@@ -123,7 +123,7 @@ int lumen_gemv(lumen_ctx *ctx, const float *x_dev, const void *w_dev, lumen_dtyp
  *  - Set-up: the first call for a device resolves the array's address (cudaGetSymbolAddress, which may load
  *    the module); make that call before any stream capture begins.
  *  - Limit: sizes whose partial sums exceed 8 MiB are refused with LUMEN_ERR_UNSUPPORTED (on 148 SMs that is
- *    beyond roughly 800k columns); nothing is truncated.  Use lumen_gemv there.
+ *    beyond roughly two million columns); nothing is truncated.  Use lumen_gemv there.
  *  - Nothing has to be zeroed: each call overwrites every partial sum it later reads.
  *  - The array is one per device: two calls in flight at once on the same device (other streams, other
  *    contexts) race on it; calls on one context's stream are ordered and safe. */

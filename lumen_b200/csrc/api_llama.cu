@@ -194,8 +194,8 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
 
     // Fused step (tiled products only): every product's finishing kernel writes what the next product reads, as the bf16
     // hi/lo pair in w.p_hi / w.p_lo (SwiGLU: w.g_hi / w.g_lo), and gate and up run as one product over their adjacent weights.  Per block:
-    // qkv product + split-K sum, attention, o_proj (split + product + finisher), gate/up (product + finisher),
-    // down (product + finisher) = 11 launches instead of 20.
+    // qkv product (+ sum of slices), attention (its result as the pair for prompts), o_proj (product + finisher), gate/up (product, +
+    // finisher up to 128 rows), down (product + finisher).  At most 64 rows: see `few` below.
     static const bool no_fuse = [] {
         const char *e = getenv("LUMEN_NO_STEP_FUSE");
         return e && e[0] == '1';

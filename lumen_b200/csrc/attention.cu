@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_prep_kernel(PrefillPara
 // Prompts of fewer than 64 positions whose context fits 64 rows: one CTA per (head, sequence), everything in shared memory, f32
 // throughout.  A thread forms a 4 x 4 block of the scores (rows ty + 16 i, cached rows tx + 16 j; rows padded by four numbers, so that
 // 16-byte reads of eight neighbouring rows hit different banks), then 4 rows x D / 16 numbers of the result.  Bound by the
-// FMA pipe: 2 x 64 x 64 x D FMAs per CTA however short the prompt, which is why fewer than 32 positions (that kernel: 124 us for 32) or fewer CTAs than SMs stay with a warp per query row.
+// FMA pipe: 2 x 64 x 64 x D FMAs per CTA however short the prompt, so a prompt of 32 costs as much as one of 63: shorter ones, and
+// fewer CTAs than SMs, stay with a warp per query row.
 // 64 sequences x 32 heads x 60 positions of 128 numbers: 180 us against 437.  grid (Hq, B).
 constexpr int kTileRows = 64;
 template <int D>
