@@ -607,7 +607,12 @@ int lumen_llama::set_param(const char *name, const void *host_data, const size_t
     lumen_llama *m = this;
     const lumen_dtype wdt = m->cfg.weight_dtype;
     const size_t se = dtype == LUMEN_F32 ? 4 : 2, e = m->esz, H = m->H;
-    m->wsplit_valid = false;  // (the kept bf16 split of the f32 weights is rebuilt before its next use)
+    if (m->wsplit_valid) {
+        // The kept bf16 split of the f32 weights is rebuilt before its next use; steps captured meanwhile still read the old one.
+        LUMEN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        m->drop_graphs();
+        m->wsplit_valid = false;
+    }
     // Which part of the tensor this rank keeps comes from the shard plan; what is left here is where it goes.
     TpSlice sl;
     long li = -1;

@@ -219,6 +219,27 @@ def test_persistent_kernel_equals_per_op_path(L, oracle, monkeypatch, over, wdt)
         assert rel_err(k, oc[l].k) < 1e-5 and rel_err(v, oc[l].v) < 1e-5
 
 
+@pytest.mark.parametrize("batch", [8, 9])
+def test_parameters_set_between_steps(L, batch):
+    """Wide f32 models send eight rows through the products of the kept bf16 weight split, in captured steps: after set_param
+    they follow the new weights (as a model that never had others), whether the split is rebuilt first (nine rows) or not."""
+    cfg = small_cfg(intermediate_size=6408)
+    old, new = (make_params(L, cfg, seed, std=0.08) for seed in (71, 72))
+    ids = np.random.default_rng(73).integers(0, cfg["vocab_size"], size=(batch, 7)).astype(np.float32)
+    model = L.LlamaModel(cfg_obj(L, cfg))
+    model.load_state(old)
+    caches = model.init_kv_caches(batch)
+    with L.no_grad():
+        model.forward(ids[:, :3], caches, 0)
+        for t in range(3, 7):
+            model.forward(ids[:, t:t + 1], caches, 0)
+        model.load_state(new)
+        model.reset_kv_caches(caches)
+        got = np.concatenate([model.forward(ids[:, t:t + 1], caches, 0) for t in range(7)], axis=1)
+    want, _, _ = _gpu_run(L, cfg, new, ids, 1)
+    assert rel_err(got, want) < TOL_F32
+
+
 def test_reset_and_reuse_caches(L):
     cfg = small_cfg()
     params = make_params(L, cfg, 51, std=0.08)
