@@ -8,6 +8,7 @@
 // reference: rotate q/k at positions past..past+S, slab write, causal mask j > past+i, softmax with
 // `1/(sum + 1e-9)`, P.V, output in [B,S,H,D] order.
 #include "attn_decode.cuh"
+#include "ring.cuh"
 #include "row_finish.cuh"
 
 namespace lumen {
@@ -386,7 +387,9 @@ __global__ void __launch_bounds__((tiled_warps<D>() * 32), 1) attn_decode_tiled_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    int issued = 0;  // tiles of this warp whose copies are on their way
     auto load_tile = [&](int jt, int buf) {
+        if (jt < j1) ++issued;
         if (jt < j1 && lane == 0) {
             const uint32_t bytes = (uint32_t)min(TR, j1 - jt) * D * sizeof(float);
             uint64_t *bar = &bars[warp * NS + buf];
@@ -546,8 +549,9 @@ __global__ void __launch_bounds__((tiled_warps<D>() * 32), 1) attn_decode_tiled_
     }
     if (!alive) {  // a wait gave up: let this warp's copies that are still in flight land before the CTA exits
         for (int sb = 0; sb < NS; ++sb) {
+            const int uses = ring_uses(issued, sb, NS);
             const long long t0 = clock64();
-            while (!tile_bar_try(&bars[warp * NS + sb], 0) && !tile_bar_try(&bars[warp * NS + sb], 1) && clock64() - t0 < 200000000LL) {}
+            while (uses && !tile_bar_try(&bars[warp * NS + sb], ring_last_parity(uses)) && clock64() - t0 < 200000000LL) {}
         }
     }
     float *wctx = ktile;  // this warp's first K tile is free now: [GT][D]

@@ -141,6 +141,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
 
     float ctx[kDH];
     float l = 0.f;
+    int k_issued = 0, v_issued = 0;  // tiles whose copies are on their way (producer thread)
     if (warp == kFaWorkers / 32 + 1) {
         if ((tid & 31) == 0) {
             // ---- TMA producer: Q once, then K and V^T of tile j + 2 as soon as tile j has released its half stage ----
@@ -161,6 +162,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
                         tma_load_2d(st + kb * G::kKTile, &map_klo, p.r_col0 + (kb - p.kb_main) * kBK, r_row0 + j * kBKV, &k_full[s]);
                     if (PAIR) tma_load_2d(st + (kKB + kb) * G::kKTile, &map_klo, k_col0 + kb * kBK, k_row0 + j * kBKV, &k_full[s]);
                 }
+                ++k_issued;
             };
             auto load_v = [&](int j) {
                 const int s = j % G::kStages;
@@ -168,6 +170,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
                 bar_expect(&v_full[s], G::kVBytes);
                 tma_load_2d(st + G::kKBytes, &map_vhi, v_col0 + j * kBKV, v_row0, &v_full[s]);
                 if (PAIR) tma_load_2d(st + G::kKBytes + G::kVTile, &map_vlo, j * kBKV, v_row0, &v_full[s]);
+                ++v_issued;
             };
             bar_expect(&q_bar, G::kQBytes);
 #pragma unroll
@@ -410,14 +413,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
             }
         }
     } else if (tid == kFaWorkers + 32) {
-        // A wait gave up: let the copies that are still in flight land before the CTA exits (bounded).
-        const long long t0 = clock64();
-        while (!bar_try(&q_bar, 0) && clock64() - t0 < kTcWaitCycles) {}
-        for (int s = 0; s < G::kStages; ++s) {
-            const long long t1 = clock64();
-            while (!bar_try(&k_full[s], 0) && !bar_try(&k_full[s], 1) && clock64() - t1 < kTcWaitCycles) {}
-            while (!bar_try(&v_full[s], 0) && !bar_try(&v_full[s], 1) && clock64() - t1 < kTcWaitCycles) {}
-        }
+        drain_ring(&q_bar, 1, 1);  // a wait gave up
+        drain_ring(k_full, G::kStages, k_issued);
+        drain_ring(v_full, G::kStages, v_issued);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

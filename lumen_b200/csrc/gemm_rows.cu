@@ -124,6 +124,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
+    int issued = 0;  // steps whose copies are on their way (thread 0)
     if (tid == 0) {
         pdl_wait();
         for (int kb = 0; kb < nkb; ++kb) {
@@ -138,6 +139,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             unsigned char *st = ring + (size_t)s * G::kStageBytes + NW * G::kWBytes;
             tma_load_2d(st, &map_x, k_of(kb), 0, &full[s]);
             tma_load_2d(st + G::kXBytes, &map_xlo, k_of(kb), 0, &full[s]);
+            ++issued;  // (the weights requested ahead are all among these: nothing before step `ahead` can fail)
         }
     } else if (tid == 32) {
         bool ok = true;
@@ -194,10 +196,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
         }
     } else if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {  // (bounded) let the copies in flight land
-            const long long t0 = clock64();
-            while (!bar_try(&full[s], 0) && !bar_try(&full[s], 1) && clock64() - t0 < kTcWaitCycles) {}
-        }
+        drain_ring(full, kStages, issued);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -131,6 +131,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
 
+    int issued = 0;  // steps whose copies are on their way (thread 0)
     if (tid == 0) {
         // ---- producer ----
         for (int kb = 0; kb < nkb; ++kb) {
@@ -146,6 +147,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
             if (NA == 2) tma_load_2d(st + kABytes, &map_alo, kx, a0, &full[s]);
             tma_load_2d(st + NA * kABytes, &map_b, kx, b_load, &full[s]);
             if (NB == 2) tma_load_2d(st + NA * kABytes + kBBytes, &map_blo, kx, b_load, &full[s]);
+            ++issued;
         }
     } else if (tid == 32) {
         // ---- MMA issuer ----
@@ -271,11 +273,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
         }
         }
     } else if (tid == 0) {
-        // A wait gave up: let the copies that are still in flight land before the CTA exits (bounded).
-        for (int s = 0; s < kStages; ++s) {
-            const long long t0 = clock64();
-            while (!bar_try(&full[s], 0) && !bar_try(&full[s], 1) && clock64() - t0 < kTcWaitCycles) {}
-        }
+        drain_ring(full, kStages, issued);  // a wait gave up
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -224,6 +224,7 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
+    int issued = 0;  // chunks whose copies are on their way (producer thread)
 
     if (warp == kWorkers / 32 + 1) {
         if ((tid & 31) == 0) {
@@ -240,6 +241,7 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
                     tma_load_2d(st + 2 * kStA + k * kStB, &map_khi, x, bh * p.dim + n0, &full[s]);
                     tma_load_2d(st + 2 * kStA + (2 + k) * kStB, &map_klo, x, bh * p.dim + n0, &full[s]);
                 }
+                ++issued;
             }
         }
         __syncwarp();
@@ -333,12 +335,7 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
         if (tid == 0) tma_store_wait();
     }
     __syncthreads();
-    if (*failed && tid == kWorkers + 32) {  // copies in flight land before the CTA exits (bounded)
-        for (int s = 0; s < kStStages; ++s) {
-            const long long t0 = clock64();
-            while (!bar_try(&full[s], 0) && !bar_try(&full[s], 1) && clock64() - t0 < kTcWaitCycles) {}
-        }
-    }
+    if (*failed && tid == kWorkers + 32) drain_ring(full, kStStages, issued);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kWorkers / 32)
@@ -401,17 +398,17 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
+    int issued = 0;  // stages whose copies are on their way (producer thread)
     auto inter_cols = [&](int j) { return tmem + ((j & 1) ? 3u : 1u) * 128u; };
     auto intra_cols = [&](int j) { return tmem + ((j & 1) ? 0u : 2u) * 128u; };
 
     if (warp == kWorkers / 32 + 1) {
         if ((tid & 31) == 0) {
             const int row0 = b * p.S + p.t0 + c * kC;
-            int it = 0;
             // a free stage, announced with its bytes
             auto next = [&](uint32_t bytes) -> unsigned char * {
-                const int s = it % G::kStages;
-                if (it >= G::kStages && !wait_or_failed(&empty[s], (uint32_t)((it / G::kStages - 1) & 1), failed, p.status, 740)) return nullptr;
+                const int s = issued % G::kStages;
+                if (issued >= G::kStages && !wait_or_failed(&empty[s], (uint32_t)((issued / G::kStages - 1) & 1), failed, p.status, 740)) return nullptr;
                 bar_expect(&full[s], bytes);
                 return ring + (size_t)s * kOutStage;
             };
@@ -419,28 +416,28 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
             for (int kb = 0; kb < KB; ++kb) tma_load_3d(q_s + kb * kTile, &map_q, kb * kBK, h, row0, &q_bar);
 #pragma unroll 1
-            for (int kb = 0; kb < KB; ++kb, ++it) {
+            for (int kb = 0; kb < KB; ++kb, ++issued) {
                 unsigned char *st = next(kTile);
                 if (!st) break;
-                tma_load_3d(st, &map_k, kb * kBK, h, row0, &full[it % G::kStages]);
+                tma_load_3d(st, &map_k, kb * kBK, h, row0, &full[issued % G::kStages]);
             }
 #pragma unroll 1
             for (int j = 0; j < nj && !*failed; ++j) {
                 const int d0 = (j0 + j) * 128;
                 if (has_prev)
 #pragma unroll 1
-                    for (int kb = 0; kb < KB; ++kb, ++it) {
+                    for (int kb = 0; kb < KB; ++kb, ++issued) {
                         unsigned char *st = next(2 * kTile);
                         if (!st) break;
                         const int y = (int)(bc * p.vdim) + d0;
-                        tma_load_2d(st, &map_shi, kb * kBK, y, &full[it % G::kStages]);
-                        tma_load_2d(st + kTile, &map_slo, kb * kBK, y, &full[it % G::kStages]);
+                        tma_load_2d(st, &map_shi, kb * kBK, y, &full[issued % G::kStages]);
+                        tma_load_2d(st + kTile, &map_slo, kb * kBK, y, &full[issued % G::kStages]);
                     }
                 unsigned char *st = next(2 * kTile);
                 if (!st) break;
 #pragma unroll
-                for (int k = 0; k < 2; ++k) tma_load_2d(st + k * kTile, &map_v, c * kC + k * kBK, bh * p.vdim + d0, &full[it % G::kStages]);
-                ++it;
+                for (int k = 0; k < 2; ++k) tma_load_2d(st + k * kTile, &map_v, c * kC + k * kBK, bh * p.vdim + d0, &full[issued % G::kStages]);
+                ++issued;
             }
         }
         __syncwarp();
@@ -608,12 +605,8 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     }
     __syncthreads();
     if (*failed && tid == kWorkers + 32) {  // copies in flight land before the CTA exits (bounded)
-        const long long t0 = clock64();
-        while (!bar_try(&q_bar, 0) && clock64() - t0 < kTcWaitCycles) {}
-        for (int s = 0; s < G::kStages; ++s) {
-            const long long t1 = clock64();
-            while (!bar_try(&full[s], 0) && !bar_try(&full[s], 1) && clock64() - t1 < kTcWaitCycles) {}
-        }
+        drain_ring(&q_bar, 1, 1);
+        drain_ring(full, G::kStages, issued);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "ring.cuh"
 
 namespace lumen {
 namespace tc {
@@ -35,6 +36,14 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, DeviceS
         }
     }
     return true;
+}
+// After a wait that gave up: the copies of the first `steps` steps of a ring land before the CTA may end (bounded).
+__device__ __forceinline__ void drain_ring(uint64_t *full, int stages, int steps) {
+    for (int s = 0; s < stages; ++s) {
+        const int uses = ring_uses(steps, s, stages);
+        const long long t0 = clock64();
+        while (uses && !bar_try(&full[s], ring_last_parity(uses)) && clock64() - t0 < kTcWaitCycles) {}
+    }
 }
 // 2-D tiled TMA load: box (kBK elements, rows) at element coordinates (x, y = row).  x is a multiple of
 // 64 bf16 elements = 128 bytes, so the 16-byte start rule of TMA holds.
