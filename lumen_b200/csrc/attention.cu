@@ -439,7 +439,7 @@ __global__ void __launch_bounds__((tiled_warps<D>() * 32), 1) attn_decode_tiled_
     bool alive = true;
     for (int jt = jw0; jt < j1 && alive; jt += kStep, buf = (buf + 1 == NS ? 0 : buf + 1), ++it) {
         load_tile(jt + (NS - 1) * kStep, buf == 0 ? NS - 1 : buf - 1);  // into the stage released by the previous iteration
-        alive = tile_bar_wait(&bars[warp * NS + buf], (uint32_t)(it / NS) & 1u, p.status);
+        alive = __all_sync(0xffffffffu, tile_bar_wait(&bars[warp * NS + buf], (uint32_t)(it / NS) & 1u, p.status));
         float4 *k4 = reinterpret_cast<float4 *>(ktile + buf * TR * D);
         float4 *v4 = reinterpret_cast<float4 *>(vtile + buf * TR * D);
         const int nvalid = min(TR, j1 - jt);

@@ -175,10 +175,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     pdl_wait();
     const bool have = bar_wait(&done, 0, p.status, 562);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    __syncthreads();
+    const bool good = __syncthreads_and(have) && !failed;  // (waits of a CTA may end differently near their limit: one answer for all, there are barriers ahead)
     // The accumulator as red[m][column of the tile], where the ring was: every copy has landed and been read.
     float *red = reinterpret_cast<float *>(ring);
-    const bool good = have && !failed;
     if (good) {
         const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll 1
@@ -197,6 +196,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     } else if (tid == 0) {
         drain_ring(full, kStages, issued);
+        drain_ring(&done, 1, 1);  // (the MMAs that were issued, before their tensor memory is given back)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -175,8 +175,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
     // ---- epilogue: all four warps ----
     const bool have = bar_wait(&done, 0, p.status, 520);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (have && !failed) {
+    if (__syncthreads_and(have) && !failed) {  // (one answer for the CTA: what follows is done by whole warps)
         const int arow = a0 + warp * 32 + lane;  // this thread's row of the tile's 128-row side
         const bool empty_slice = nkb == 0;       // nothing was accumulated: the tile's contribution is zero
         if constexpr (EPI == GemmBf16Args::kGated || EPI == GemmBf16Args::kGatedGelu) {
@@ -274,6 +273,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
         }
     } else if (tid == 0) {
         drain_ring(full, kStages, issued);  // a wait gave up
+        drain_ring(&done, 1, 1);            // (the MMAs that were issued, before their tensor memory is given back)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

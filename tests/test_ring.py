@@ -22,3 +22,13 @@ def test_no_wait_for_either_parity():
     either = re.compile(r"bar_try\(([^;]*?), 0\)\s*&&\s*!\s*\w*bar_try\(\1, 1\)")
     bad = [f"{p.name}: {m.group(0)}" for p in sorted(CSRC.glob("*.cu*")) for m in either.finditer(p.read_text())]
     assert not bad, bad
+
+
+def test_answers_of_bounded_waits_are_agreed_on():
+    """Threads of a CTA may see a wait end differently near its limit; where whole warps or the CTA meet again behind it, they take one answer."""
+    for name in ("gemm_rows.cu", "gemm_tc.cu"):
+        text = (CSRC / name).read_text()
+        assert len(re.findall(r"const bool have = bar_wait\(&done", text)) == len(re.findall(r"__syncthreads_and\(have\)", text)) == 1, name
+        assert not re.search(r"\bhave && ", text), name
+    waits = re.findall(r"alive = (.*)bar_wait", (CSRC / "attention.cu").read_text() + (CSRC / "attn_rows.cu").read_text())
+    assert len(waits) == 3 and all("__all_sync" in w for w in waits), waits
