@@ -143,6 +143,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     } else if (tid == 32) {
         bool ok = true;
+        pdl_wait();  // (the limit of a wait is for this kernel's copies, not for the kernel before)
         for (int kb = 0; kb < nkb && ok; ++kb) {
             const int s = kb % kStages;
             ok = bar_wait(&full[s], (uint32_t)((kb / kStages) & 1), p.status, 561);

@@ -32,3 +32,14 @@ def test_answers_of_bounded_waits_are_agreed_on():
         assert not re.search(r"\bhave && ", text), name
     waits = re.findall(r"alive = (.*)bar_wait", (CSRC / "attention.cu").read_text() + (CSRC / "attn_rows.cu").read_text())
     assert len(waits) == 3 and all("__all_sync" in w for w in waits), waits
+
+
+def test_limits_start_behind_the_kernel_before():
+    """Kernels that start early count their bounded waits from the end of their predecessor: no wait on a barrier before pdl_wait()."""
+    for name in ("gemm_rows.cu", "attn_rows.cu"):
+        text = (CSRC / name).read_text()
+        body = text[text.index("    pdl_launch();"):]
+        branches = re.split(r"\n    \} else if \(", body[: body.index("bar_wait(&done") if "bar_wait(&done" in body else len(body)])
+        for b in branches:
+            if "bar_wait(" in b:
+                assert "pdl_wait()" in b[: b.index("bar_wait(")], (name, b[:60])
