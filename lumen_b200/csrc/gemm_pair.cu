@@ -297,30 +297,6 @@ int launch_pair_t(lumen_ctx *ctx, const GemmPairArgs &g, const PairParams &p, cu
 
 }  // namespace
 
-GemmPairPlan plan_gemm_pair(size_t M, size_t K, size_t N, int products, bool swiglu, bool may_split, int num_sms) {
-    // Cycles of the fullest pair of SMs: its tiles one after the other, and what is not overlapped (ring fill, last epilogue).
-    // A 128-wide tile takes more than half of a 256-wide one's time (its operands are 40 KB per 64 numbers of K instead of 48).
-    const size_t pairs = (size_t)std::max(1, num_sms / 2), kb_all = (K + kBK - 1) / kBK, tm = (M + kPairRows - 1) / kPairRows;
-    const size_t width = swiglu ? N / 2 : N;
-    GemmPairPlan best;
-    double best_cost = 0;
-    for (int bn : {256, 128}) {
-        const size_t cols = swiglu ? bn / 2 : bn, tiles = tm * ((width + cols - 1) / cols);
-        for (size_t splits = 1; splits <= (may_split ? 4 : 1); ++splits) {
-            const size_t per = (kb_all + splits - 1) / splits;
-            if (splits > 1 && (per < 8 || (kb_all + per - 1) / per != splits)) continue;
-            const size_t waves = (tiles * splits + pairs - 1) / pairs;
-            const double cost = (double)waves * per * products * (bn == 256 ? 512 : 330) + 4000 +
-                                (splits > 1 ? (double)(splits + 1) * M * N * 4 / 2500 : 0);  // slices written and read again
-            if (!best.bn || cost < best_cost) {
-                best = GemmPairPlan{bn, (int)splits, (int)per};
-                best_cost = cost;
-            }
-        }
-    }
-    return best;
-}
-
 int launch_gemm_pair(lumen_ctx *ctx, const GemmPairArgs &g, const GemmPairPlan &plan, cudaStream_t s) {
     PairParams p{};
     p.c = g.c; p.residual = g.residual; p.hi = g.out_hi; p.lo = g.out_lo;

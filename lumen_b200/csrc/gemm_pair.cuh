@@ -2,13 +2,10 @@
 #pragma once
 
 #include "common.cuh"
+#include "gemm_plan.cuh"
 
 namespace lumen {
 
-// Tile width, slices of K and 64-number blocks of K per slice.
-struct GemmPairPlan {
-    int bn = 0, splits = 1, kb_per_split = 0;
-};
 struct GemmPairArgs {
     const __nv_bfloat16 *a_hi = nullptr, *a_lo = nullptr;  // activations [M, K]
     const __nv_bfloat16 *w_hi = nullptr, *w_lo = nullptr;  // weights [N, K]; w_lo null: bf16 weights
@@ -19,7 +16,6 @@ struct GemmPairArgs {
     // here, [M, N / 2], instead of c.
     __nv_bfloat16 *out_hi = nullptr, *out_lo = nullptr;
 };
-GemmPairPlan plan_gemm_pair(size_t M, size_t K, size_t N, int products, bool swiglu, bool may_split, int num_sms);
 int launch_gemm_pair(lumen_ctx *ctx, const GemmPairArgs &g, const GemmPairPlan &plan, cudaStream_t s);
 
 }  // namespace lumen

@@ -396,11 +396,14 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
         return e && e[0] == '1';
     }();
     const bool swap = M <= 64 && !no_swap;
-    // More than one row of 128-row tiles: pairs of SMs (gemm_pair.cu).
-    const bool pair = M > (size_t)kBM && N >= 128;
-    const bool glu = pair && fuse && fuse->post == GemmFuse::kPostSwiglu && !tp && N % 16 == 0 && fuse->next_hi != hi && fuse->next_lo != lo;
-    // (slices of K are added by the kernel that reads the product anyway)
-    const GemmPairPlan plan = pair ? plan_gemm_pair(M, K, N, wsplit ? 3 : 2, glu, tp || (fuse && fuse->post == GemmFuse::kPostNorm), ctx->num_sms) : GemmPairPlan();
+    // More than one row of 128-row tiles: pairs of SMs (gemm_pair.cu), for plain products where they are faster.
+    const bool many = M > (size_t)kBM && N >= 128;
+    const bool glu = many && fuse && fuse->post == GemmFuse::kPostSwiglu && !tp && N % 16 == 0 && fuse->next_hi != hi && fuse->next_lo != lo;
+    const bool may_split = tp || (fuse && fuse->post == GemmFuse::kPostNorm);  // (slices of K are added by the kernel that reads the product anyway)
+    const GemmPairPlan plan = !many ? GemmPairPlan()
+                              : glu || may_split ? plan_gemm_pair(M, K, N, wsplit ? 3 : 2, glu, may_split, ctx->num_sms)
+                                                 : plan_gemm_plain(M, K, N, !wsplit, ctx->num_sms);
+    const bool pair = plan.bn != 0;
     CUtensorMap map_hi, map_lo, map_b, map_blo;  // 128-row side (hi, lo), BN-row side (hi, lo)
     const int bn = swap ? 64 : pick_bn(M, N, ctx->num_sms);
     if (pair) {

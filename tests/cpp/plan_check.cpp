@@ -1,0 +1,25 @@
+// Prints the plan of products, one per line of its input:
+//   plain M K N bf16   ->  bn splits kb_per_split          (bn 0: 128 x 128 tiles of single SMs)
+//   pair M K N products swiglu may_split   ->  the same
+#include <cstdio>
+#include <cstring>
+
+#include "gemm_plan.cuh"
+
+int main() {
+    char kind[16];
+    size_t m, k, n;
+    while (std::scanf("%15s %zu %zu %zu", kind, &m, &k, &n) == 4) {
+        int a = 0, b = 0, c = 0;
+        lumen::GemmPairPlan p;
+        if (!std::strcmp(kind, "plain")) {
+            if (std::scanf("%d", &a) != 1) return 1;
+            p = lumen::plan_gemm_plain(m, k, n, a != 0, 148);
+        } else {
+            if (std::scanf("%d %d %d", &a, &b, &c) != 3) return 1;
+            p = lumen::plan_gemm_pair(m, k, n, a, b != 0, c != 0, 148);
+        }
+        std::printf("%d %d %d\n", p.bn, p.splits, p.kb_per_split);
+    }
+    return 0;
+}

@@ -1,0 +1,51 @@
+"""Which kernel multiplies many rows: the rules of dispatch on the CPU, against what was measured on a B200 (148 SMs)."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    out = tmp_path_factory.mktemp("plan") / "plan_check"
+    r = subprocess.run(["g++", "-std=c++17", "-Wall", "-Wextra", "-Werror", "-I", str(ROOT / "lumen_b200" / "csrc"), str(ROOT / "tests" / "cpp" / "plan_check.cpp"),
+                        "-o", str(out)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+    def run(*line):
+        r = subprocess.run([str(out)], input=" ".join(str(int(x) if isinstance(x, bool) else x) for x in line), capture_output=True, text=True, timeout=60)
+        return tuple(int(x) for x in r.stdout.split())
+
+    return run
+
+
+# m, k, n, bf16 weights, microseconds of the whole product with 128 x 128 tiles of single SMs, 256 x 128 and 256 x 256 tiles of pairs
+MEASURED = [
+    (129, 5632, 2048, True, 48.9, 56.1, 67.0), (192, 2048, 256, True, 25.5, 29.0, 35.4), (257, 2048, 5632, True, 29.2, 49.4, 39.8),
+    (384, 2048, 11264, True, 49.1, 68.3, 62.5), (512, 4096, 6144, True, 75.4, 82.7, 61.2), (768, 4096, 4096, True, 73.7, 80.5, 58.3),
+    (1025, 1024, 1024, True, 21.6, 24.2, 28.5), (1025, 2048, 2048, True, 29.6, 49.6, 39.3), (1777, 4096, 4096, True, 136.6, 148.9, 106.4),
+    (2048, 2048, 256, True, 29.0, 33.2, 39.7), (2048, 5632, 2048, True, 100.2, 110.7, 83.1), (4096, 4096, 12288, True, 814.8, 736.8, 579.3),
+    (257, 4096, 12288, False, 179.3, 206.1, 207.3), (640, 576, 1536, False, 25.9, 29.1, 35.7), (768, 12288, 4096, False, 324.2, 331.6, 266.1),
+    (1777, 4096, 4096, False, 206.0, 207.8, 167.5), (8192, 11008, 4096, False, 1860.5, 2141.6, 1570.0),
+]
+
+
+@pytest.mark.parametrize("m,k,n,bf16,single,pair128,pair256", MEASURED)
+def test_plain_products_take_the_kernel_that_was_faster(plan, m, k, n, bf16, single, pair128, pair256):
+    times = {0: single, 128: pair128, 256: pair256}
+    bn, splits, per = plan("plain", m, k, n, bf16)
+    assert times[bn] <= 1.1 * min(times.values()) and splits == 1 and per * 64 >= k
+
+
+def test_plans_cover_the_whole_of_k(plan):
+    for m in (129, 300, 1025, 8192):
+        for k in (8, 64, 520, 1096, 2008, 4096, 11008):
+            for n in (128, 136, 1032, 4096):
+                for products in (2, 3):
+                    for kind in ((False, False), (False, True), (True, False)):
+                        bn, splits, per = plan("pair", m, k, n, products, *kind)
+                        assert bn in (128, 256) and 1 <= splits <= 4 and (splits - 1) * per * 64 < k <= splits * per * 64
+                bn, splits, per = plan("plain", m, k, n, True)
+                assert bn in (0, 128, 256) and splits == 1 and per * 64 >= k
