@@ -325,18 +325,6 @@ int launch_t(lumen_ctx *ctx, const AttnRowsArgs &a, size_t B, size_t Hkv, int sp
 
 }  // namespace
 
-// Up to eight parts of a context: as many as leave every SM two CTAs and a part 96 rows (a tile of rows per warp takes about 3 us; a step of
-// four TinyLlama layers, 16 sequences at 1900 positions: 383 us with eight parts, 479 with four, 402 with the general kernel and its merge).
-// Longer contexts of few sequences want more parts than a cluster has: they take the general kernel.
-int attn_rows_splits(size_t B, size_t Hq, size_t Hkv, size_t D, size_t len, int num_sms) {
-    if ((D != 64 && D != 128) || Hkv == 0 || Hq % Hkv) return 0;
-    const size_t G = Hq / Hkv;
-    if ((G != 1 && G != 2 && G != 4 && G != 8) || (B * Hkv * 8 < (size_t)num_sms && len > 4096)) return 0;
-    int n = 1;
-    while (n < 8 && B * Hkv * n < 2 * (size_t)num_sms && len >= 96 * (size_t)n) n *= 2;
-    return n;
-}
-
 int launch_attn_rows(lumen_ctx *ctx, const AttnRowsArgs &a, size_t B, size_t Hq, size_t Hkv, size_t D, int splits, cudaStream_t s) {
     const size_t G = Hkv ? Hq / Hkv : 0;
 #define LUMEN_AR(D_) (G == 8 ? launch_t<D_, 8>(ctx, a, B, Hkv, splits, s) : G == 4 ? launch_t<D_, 4>(ctx, a, B, Hkv, splits, s) \

@@ -1,6 +1,7 @@
 // Decode attention of a batched step (attn_rows.cu).
 #pragma once
 
+#include "attn_plan.cuh"
 #include "common.cuh"
 
 namespace lumen {
@@ -16,8 +17,7 @@ struct AttnRowsArgs {
     __nv_bfloat16 *out_hi = nullptr, *out_lo = nullptr;  // [B, Hq * D]
     DeviceStatus *status = nullptr;
 };
-// Parts of the context for launch_attn_rows; 0: this geometry is not served.
-int attn_rows_splits(size_t B, size_t Hq, size_t Hkv, size_t D, size_t len, int num_sms);
+// `splits`: of attn_rows_splits, not 0.
 int launch_attn_rows(lumen_ctx *ctx, const AttnRowsArgs &a, size_t B, size_t Hq, size_t Hkv, size_t D, int splits, cudaStream_t s);
 
 }  // namespace lumen

@@ -140,6 +140,40 @@ def test_batched_steps_as_a_chain_of_products(L, oracle, heads, kv, dim, hidden,
     assert rel_err(got, want) < TOL_F32
 
 
+@pytest.mark.parametrize("heads,kv,dim,batch,at", [(8, 1, 64, 20, 2597), (8, 1, 64, 80, 1197), (4, 1, 64, 24, 3497), (4, 1, 64, 80, 1747), (8, 1, 128, 9, 381),
+                                                    (4, 2, 128, 12, 765), (2, 2, 64, 9, 1021), (4, 1, 128, 40, 4093), (8, 4, 64, 10, 2047)])
+@pytest.mark.parametrize("wdt", ["f32", "bf16"])
+def test_batched_steps_over_long_contexts(L, oracle, heads, kv, dim, batch, at, wdt):
+    """Batched decode steps over caches that hold hundreds to thousands of rows already (written from the host): contexts in eight, four and two
+    parts, and both sides of the lengths from which the general attention kernel serves them."""
+    cfg = small_cfg(hidden_size=128, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, intermediate_size=136, qk_norm=dim == 128, max_seq_len=at + 8)
+    params = make_params(L, cfg, 81, std=0.08, round_bf16=(wdt == "bf16"), random_norms=True)
+    rng = np.random.default_rng(at)
+    ids = rng.integers(0, cfg["vocab_size"], size=(batch, 6)).astype(np.float32)
+    model = L.LlamaModel(cfg_obj(L, cfg, wdt))
+    model.load_state(params)
+    caches = model.init_kv_caches(batch)
+    ref = oracle.Llama(cfg, params, "f64")
+    rcaches = ref.init_kv_caches(batch)
+    for c, r in zip(caches, rcaches):
+        k, v = (rng.standard_normal((batch, kv, at + 8, dim), dtype=np.float32) for _ in range(2))
+        c.write(k, v, at)
+        r.k[:], r.v[:] = k, v
+        r.len = at
+    with L.no_grad():
+        for t in range(6):
+            got = model.forward(ids[:, t:t + 1], caches, 0)
+            assert rel_err(got, ref.forward(ids[:, t:t + 1], rcaches)) < TOL_F32, t
+    # Rows of the second layer have five products behind them (q/k/v, o, gate and up, down, q/k/v), each of two operands that a bf16 pair
+    # holds to 2^-17.  Keys are turned by angles from f32 tables, which are off by up to position * 2^-23 (a frequency and a product, rounded), while the
+    # 64-bit oracle's are not: 5e-5 as in the other tests was exceeded from position 2597 on (5.03e-5; 8.7e-5 at 3497).
+    tol = 5 * 2 * 2.0 ** -17
+    for c, r in zip(caches, rcaches):
+        k, v = c.read()
+        assert c.len == at + 6 and rel_err(k[:, :, at:at + 6], r.k[:, :, at:at + 6]) < tol + (at + 6) * 2.0 ** -23
+        assert rel_err(v[:, :, at:at + 6], r.v[:, :, at:at + 6]) < tol
+
+
 @pytest.mark.parametrize("kv,dim,prompts", [(2, 64, (32, 32, 17)), (4, 128, (63, 33)), (8, 64, (5, 59)), (4, 128, (31, 33, 64))])
 def test_many_short_prompts(L, oracle, kv, dim, prompts):
     """Prompts of fewer than 64 positions of many sequences: attention in one tile where the context fits 64 rows (both edges of its range), into an

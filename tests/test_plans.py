@@ -1,4 +1,4 @@
-"""Which kernel multiplies many rows: the rules of dispatch on the CPU, against what was measured on a B200 (148 SMs)."""
+"""Which kernel multiplies many rows, and which attends in a batched decode step: the rules of dispatch on the CPU, against what was measured on a B200 (148 SMs)."""
 import subprocess
 from pathlib import Path
 
@@ -49,3 +49,19 @@ def test_plans_cover_the_whole_of_k(plan):
                         assert bn in (128, 256) and 1 <= splits <= 4 and (splits - 1) * per * 64 < k <= splits * per * 64
                 bn, splits, per = plan("plain", m, k, n, True)
                 assert bn in (0, 128, 256) and splits == 1 and per * 64 >= k
+
+
+# sequences, query heads, KV heads, head size, positions, microseconds of a step of four layers with the batched kernel and with the general one
+ATTENDED = [
+    (64, 32, 4, 64, 500, 318.1, 343.5), (64, 32, 4, 64, 1500, 501.2, 457.9), (64, 32, 4, 64, 4096, 927.2, 770.2), (32, 32, 4, 64, 1000, 276.8, 286.6),
+    (32, 32, 4, 64, 2000, 372.8, 340.2), (16, 32, 4, 64, 2000, 257.7, 295.9), (16, 32, 4, 64, 4096, 364.1, 335.6), (8, 32, 4, 64, 3000, 278.7, 250.2),
+    (4, 32, 4, 64, 3000, 232.4, 262.9), (2, 32, 4, 64, 2000, 188.9, 263.4), (64, 32, 8, 64, 1000, 490.2, 498.0), (64, 32, 8, 64, 2000, 710.2, 661.3),
+    (16, 32, 8, 64, 1500, 266.4, 273.2), (16, 32, 8, 64, 4096, 460.9, 395.0), (4, 32, 8, 64, 4096, 272.6, 252.1), (64, 16, 8, 64, 4096, 938.4, 973.1),
+    (64, 32, 8, 128, 4096, 1741.9, 2046.6), (64, 32, 4, 128, 4096, 1284.9, 1497.7), (32, 16, 16, 128, 4096, 1552.8, 1987.0), (64, 16, 16, 64, 4096, 1724.6, 1886.1),
+]
+
+
+@pytest.mark.parametrize("b,hq,hkv,d,at,rows,general", ATTENDED)
+def test_batched_steps_take_the_attention_that_was_faster(plan, b, hq, hkv, d, at, rows, general):
+    (parts,) = plan("attn", b, hq, hkv, d, at)
+    assert (rows if parts else general) <= 1.02 * min(rows, general) and parts in (0, 1, 2, 4, 8)
