@@ -27,7 +27,6 @@ using namespace tc;
 constexpr int kPairThreads = 192;
 constexpr int kPairRows = 256;          // rows of a tile, 128 per CTA
 constexpr int kGroupRows = 8;           // tile rows walked together
-constexpr uint32_t kPeerMask = 0xFEFFFFFFu;  // shared::cluster address of the same variable in the pair's first CTA
 
 template <int NA, int NB, int BN>
 struct PairGeom {
@@ -54,10 +53,15 @@ __device__ __forceinline__ uint32_t cta_rank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// 2-D tiled load into this CTA's shared memory that signals the barrier of the pair's first CTA.
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+__device__ __forceinline__ uint32_t in_first(const void *p) {  // shared::cluster address of the same variable in the pair's first CTA
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(saddr(p)));
+    return a;
+}
+// 2-D tiled load into this CTA's shared memory that signals a barrier of the pair's first CTA (an address of in_first).
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(saddr(dst)), "l"(map), "r"(x), "r"(y), "r"(saddr(bar) & kPeerMask) : "memory");
+                 ::"r"(saddr(dst)), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -70,8 +74,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
                  ::"r"(saddr(bar)), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void arrive_first(uint64_t *bar) {  // at the barrier of the pair's first CTA
-    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %0, 0;\n mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n}"
-                 ::"r"(saddr(bar)) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_first(bar)) : "memory");
 }
 
 struct PairTile {
@@ -135,6 +138,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     if (warp == 0) {
         if (lane == 0) {
             // ---- producer: this CTA's rows of A and its half of the tile's weight rows ----
+            const uint32_t full0 = in_first(full);
             int i = 0;
             for (int item = first; item < items && !failed; item += step) {
                 const PairTile t = pair_tile(item, tm, tn, kCols);
@@ -148,10 +152,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
                     unsigned char *st = ring + (size_t)s * G::kStageBytes;
                     if (rank == 0) bar_expect(&full[s], 2 * G::kStageBytes);
                     const int kx = (kb0 + kb) * kBK;
-                    tma_load_2d_pair(st, &map_ahi, kx, ay, &full[s]);
-                    if (NA == 2) tma_load_2d_pair(st + G::kABytes, &map_alo, kx, ay, &full[s]);
-                    tma_load_2d_pair(st + NA * G::kABytes, &map_b, kx, by, &full[s]);
-                    if (NB == 2) tma_load_2d_pair(st + NA * G::kABytes + G::kBBytes, &map_blo, kx, by, &full[s]);
+                    const uint32_t bar = full0 + s * (uint32_t)sizeof(full[0]);
+                    tma_load_2d_pair(st, &map_ahi, kx, ay, bar);
+                    if (NA == 2) tma_load_2d_pair(st + G::kABytes, &map_alo, kx, ay, bar);
+                    tma_load_2d_pair(st + NA * G::kABytes, &map_b, kx, by, bar);
+                    if (NB == 2) tma_load_2d_pair(st + NA * G::kABytes + G::kBBytes, &map_blo, kx, by, bar);
                 }
             }
             // the last stages have been read (and their copies landed) before the CTA may end

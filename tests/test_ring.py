@@ -43,3 +43,10 @@ def test_limits_start_behind_the_kernel_before():
         for b in branches:
             if "bar_wait(" in b:
                 assert "pdl_wait()" in b[: b.index("bar_wait(")], (name, b[:60])
+
+
+def test_peer_addresses_come_from_mapa():
+    """Where the window of a cluster's other CTA lies is the machine's business: addresses in it come from mapa, not from masked bits."""
+    for p in sorted(CSRC.glob("*.cu*")):
+        assert not re.search(r"0xF[0-9A-Fa-f]FFFFFF|kPeerMask", p.read_text()), p.name
+    assert "mapa.shared::cluster" in (CSRC / "gemm_pair.cu").read_text()
