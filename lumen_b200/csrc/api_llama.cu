@@ -40,8 +40,9 @@ struct Workspace {
     float *x = nullptr, *nx = nullptr, *qkv = nullptr, *att = nullptr, *act = nullptr, *gate = nullptr, *up = nullptr;
     float *logits = nullptr, *logits_local = nullptr, *last_x = nullptr, *part = nullptr, *ids = nullptr;
     // bf16 hi/lo split of the activations the next tensor-core product reads (written by the kernel that finishes the
-    // previous product): the normed rows [M, H], and the SwiGLU rows [M, I_l] (the product that writes them still reads the former)
-    __nv_bfloat16 *p_hi = nullptr, *p_lo = nullptr, *g_hi = nullptr, *g_lo = nullptr;
+    // previous product): the normed rows [M, H]; the SwiGLU rows [M, I_l] (the product that writes them still reads the former) where `act` is, which
+    // only unfused steps use; and the attention's rows [M, qd_l] where `gate` and `up` are, written after the attention has been read and read before the next
+    __nv_bfloat16 *p_hi = nullptr, *p_lo = nullptr, *g_hi = nullptr, *g_lo = nullptr, *att_hi = nullptr, *att_lo = nullptr;
     float *ss = nullptr;  // sums of squares of the residual stream (see GemmRowsArgs)
     size_t part_bytes = 0;
     float *h_ids = nullptr;     // pinned
@@ -115,18 +116,20 @@ int ensure_workspace(lumen_llama *m, size_t M) {
         off += align_up(elems * sizeof(float), 256);
         return o;
     };
-    size_t o_x = take(M * m->H), o_nx = take(M * m->H), o_qkv = take(M * qkvd), o_att = take(2 * M * m->qd_l);  // (f32, then the bf16 pair)
+    size_t o_x = take(M * m->H), o_nx = take(M * m->H), o_qkv = take(M * qkvd), o_att = take(M * m->qd_l);
     // gate and up are adjacent: the fused step runs them as one product into [M, 2 * I_l]
-    size_t o_act = take(M * m->inter_l), o_gate = take(2 * M * m->inter_l);
-    auto half = [](size_t n) { return (n + 1) / 2 + 8; };
-    size_t o_phi = take(half(M * m->H)), o_plo = take(half(M * m->H)), o_ghi = take(half(M * m->inter_l)), o_glo = take(half(M * m->inter_l));
+    auto half = [](size_t n) { return (n + 15) / 16 * 8; };  // floats that hold n bf16 numbers (whole 16-byte words)
+    const size_t att_half = half(M * m->qd_l), act_half = half(M * m->inter_l);
+    size_t o_act = take(2 * act_half), o_gate = take(std::max(2 * M * m->inter_l, 2 * att_half));
+    size_t o_phi = take(half(M * m->H)), o_plo = take(half(M * m->H));
     size_t o_logits = take(M * m->V), o_ll = take(T > 1 ? T * M * m->vocab_l : 0), o_last = take(M * m->H);
     size_t o_part = take(w.part_bytes / sizeof(float)), o_ids = take(M), o_ss = take(gemm_rows_ss_floats(m->H));
     LUMEN_CUDA(ctx, cudaMalloc(&w.base, off));
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w.base + o); };
     w.x = at(o_x); w.nx = at(o_nx); w.qkv = at(o_qkv); w.att = at(o_att); w.act = at(o_act); w.gate = at(o_gate);
     w.up = w.gate + M * m->inter_l; w.p_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_phi)); w.p_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_plo));
-    w.g_hi = reinterpret_cast<__nv_bfloat16 *>(at(o_ghi)); w.g_lo = reinterpret_cast<__nv_bfloat16 *>(at(o_glo));
+    w.g_hi = reinterpret_cast<__nv_bfloat16 *>(w.act); w.g_lo = w.g_hi + 2 * act_half;
+    w.att_hi = reinterpret_cast<__nv_bfloat16 *>(w.gate); w.att_lo = w.att_hi + 2 * att_half;
     w.logits = at(o_logits); w.logits_local = at(o_ll); w.last_x = at(o_last); w.part = at(o_part);
     w.ids = at(o_ids); w.ss = at(o_ss);
     LUMEN_CUDA(ctx, cudaMallocHost(&w.h_ids, std::max<size_t>(M, 1) * sizeof(float)));
@@ -209,7 +212,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     }
 
     // The attention's result as the pair that the output projection reads (prompts of the fused path, and batched steps below).
-    __nv_bfloat16 *const att_hi = reinterpret_cast<__nv_bfloat16 *>(w.att + M * m->qd_l), *const att_lo = att_hi + M * m->qd_l;
+    __nv_bfloat16 *const att_hi = w.att_hi, *const att_lo = w.att_lo;
     auto attend = [&](const LayerW &lw, lumen_kv_cache *c) -> int {
         if (p.decode) {
             AttnDecodeArgs a;

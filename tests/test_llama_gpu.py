@@ -174,6 +174,29 @@ def test_batched_steps_over_long_contexts(L, oracle, heads, kv, dim, batch, at, 
         assert rel_err(v[:, :, at:at + 6], r.v[:, :, at:at + 6]) < tol
 
 
+def test_workspace_of_a_long_prompt(L):
+    """Device memory that a prompt's activations take: no more than its buffers, with the bf16 pairs of the attention's and the SwiGLU rows inside
+    buffers that are free at that time (a model of the same sizes has run before, so that nothing else is allocated)."""
+    import torch
+    rows, h, i, heads, d = 8192, 128, 4096, 2, 64
+    cfg = small_cfg(hidden_size=h, num_attention_heads=heads, num_key_value_heads=1, head_dim=d, intermediate_size=i, max_seq_len=rows)
+    params = make_params(L, cfg, 91, std=0.05)
+    ids = np.random.default_rng(92).integers(0, cfg["vocab_size"], size=(1, rows)).astype(np.float32)
+    kept = []
+    for _ in range(2):
+        model = L.LlamaModel(cfg_obj(L, cfg, "bf16"))
+        model.load_state(params)
+        caches = model.init_kv_caches(1)
+        kept.append((model, caches))
+        before = torch.cuda.mem_get_info()[0]
+        with L.no_grad():
+            model.forward(ids, caches, 0, last_only=True)
+        took = before - torch.cuda.mem_get_info()[0]
+    # x, normed x, last x, q/k/v, attention, SwiGLU, gate and up, normed pair, logits, ids, pieces of split decode attention
+    per_row = 4 * (3 * h + (heads + 2) * d + heads * d + i + 2 * i + h + cfg["vocab_size"] + 1 + 64 * heads * (d + 2))
+    assert took <= rows * per_row + (8 << 20), (took, rows * per_row)  # (allocations come in 2 MB pages)
+
+
 @pytest.mark.parametrize("kv,dim,prompts", [(2, 64, (32, 32, 17)), (4, 128, (63, 33)), (8, 64, (5, 59)), (4, 128, (31, 33, 64))])
 def test_many_short_prompts(L, oracle, kv, dim, prompts):
     """Prompts of fewer than 64 positions of many sequences: attention in one tile where the context fits 64 rows (both edges of its range), into an
