@@ -8,6 +8,17 @@ import numpy as np
 TOL_F32 = 1e-4
 TOL_BF16 = 1e-2
 
+# Sizes at which products run on pairs of SMs (test_plans.py checks that they do).
+# m, k, n of plain products; all take the 256-wide tile but the last, whose f32 form takes the 128-wide one (and bf16 single SMs)
+PAIRED_PRODUCTS = [(129, 1096, 9601), (513, 1160, 4865), (1281, 1160, 1921), (2300, 1544, 1031), (9473, 1096, 129), (5000, 1032, 1030)]
+# hidden size, intermediate size, positions of a prompt, slices of K of its down product, tile widths of that and of its gate-and-up product,
+# with bf16 and with f32 weights
+PAIRED_PROMPTS = [
+    (128, 136, 129, (1, 1), (128, 128), (128, 128)), (128, 200, 300, (1, 1), (128, 128), (128, 128)), (128, 264, 513, (1, 1), (128, 128), (128, 128)),
+    (128, 128, 256, (1, 1), (128, 128), (128, 128)), (128, 1096, 129, (2, 2), (128, 128), (128, 128)), (128, 1544, 300, (3, 3), (128, 128), (128, 128)),
+    (128, 2008, 513, (4, 4), (128, 128), (256, 256)), (768, 2248, 1500, (2, 4), (128, 256), (128, 128)),
+]
+
 
 def rel_err(a, b) -> float:
     a = np.asarray(a, dtype=np.float64)

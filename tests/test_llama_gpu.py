@@ -8,7 +8,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
-from helpers import TOL_BF16, TOL_F32, cfg_obj, make_params, rel_err, small_cfg
+from helpers import PAIRED_PROMPTS, TOL_BF16, TOL_F32, cfg_obj, make_params, rel_err, small_cfg
 
 pytestmark = pytest.mark.gpu
 GOLD = Path(__file__).resolve().parent / "golden"
@@ -110,12 +110,12 @@ def test_long_prompt_slices_tensor_core_prefill(L, oracle, over, wdt):
         assert rel_err(k, ocaches[l].k) < 5e-5 and rel_err(v, ocaches[l].v) < 5e-5
 
 
-@pytest.mark.parametrize("inter,prompt", [(136, 129), (200, 300), (264, 513), (128, 256)])
+@pytest.mark.parametrize("hidden,inter,prompt", [c[:3] for c in PAIRED_PROMPTS])
 @pytest.mark.parametrize("wdt", ["f32", "bf16"])
-def test_prefill_of_more_than_one_row_tile(L, oracle, inter, prompt, wdt):
+def test_prefill_of_more_than_one_row_tile(L, oracle, hidden, inter, prompt, wdt):
     """Prompts whose products run as 256-row tiles: gate and up in one tile with SwiGLU in its epilogue (edges of the tile in both
-    directions), and products in slices of K that the norm's kernel adds."""
-    cfg = small_cfg(hidden_size=128, num_attention_heads=2, num_key_value_heads=2, intermediate_size=inter, max_seq_len=520)
+    directions, both widths), and products in one to four slices of K that the norm's kernel adds (test_plans.py checks which size takes what)."""
+    cfg = small_cfg(hidden_size=hidden, num_attention_heads=hidden // 64, num_key_value_heads=2, intermediate_size=inter, max_seq_len=prompt + 8)
     params = make_params(L, cfg, 31, std=0.08, round_bf16=(wdt == "bf16"), random_norms=True)
     ids = np.random.default_rng(32).integers(0, cfg["vocab_size"], size=(1, prompt)).astype(np.float32)
     got, _, _ = _gpu_run(L, cfg, params, ids, prompt, wdt)
@@ -125,14 +125,14 @@ def test_prefill_of_more_than_one_row_tile(L, oracle, inter, prompt, wdt):
 
 @pytest.mark.parametrize("heads,kv,dim,hidden,inter,batch,prompt", [
     (8, 1, 64, 512, 200, 16, 40), (4, 2, 64, 136, 136, 33, 5), (2, 2, 128, 264, 72, 64, 1), (4, 1, 128, 1032, 1352, 9, 300), (8, 1, 128, 256, 4104, 17, 2),
-    (2, 1, 64, 128, 64, 32, 130), (4, 4, 64, 256, 392, 48, 17)])
+    (2, 1, 64, 128, 64, 32, 130), (4, 4, 64, 256, 392, 48, 17), (4, 1, 64, 128, 136, 10, 33), (4, 2, 128, 256, 200, 21, 9), (8, 1, 64, 256, 136, 9, 384)])
 @pytest.mark.parametrize("wdt", ["f32", "bf16"])
 def test_batched_steps_as_a_chain_of_products(L, oracle, heads, kv, dim, hidden, inter, batch, prompt, wdt):
     """Batched decode steps (products with their epilogues in thread-block clusters, attention in one kernel): every group size and
-    head dimension it serves, rows at the edges of 16, 32 and 64, widths with remainders of 64 and 128, contexts in one and in several
+    head dimension it serves, rows at the edges of 16, 32 and 64, widths with remainders of 64 and 128, contexts in one to eight
     parts; short prompts of as many rows take the same products."""
     cfg = small_cfg(hidden_size=hidden, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, intermediate_size=inter, qk_norm=dim == 128,
-                    max_seq_len=320)
+                    max_seq_len=400)
     params = make_params(L, cfg, 41, std=0.08, round_bf16=(wdt == "bf16"), random_norms=True)
     ids = np.random.default_rng(batch).integers(0, cfg["vocab_size"], size=(batch, prompt + 4)).astype(np.float32)
     got, _, _ = _gpu_run(L, cfg, params, ids, prompt, wdt)

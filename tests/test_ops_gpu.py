@@ -7,7 +7,7 @@ compared within f32 rounding and against the f64 shadow."""
 import numpy as np
 import pytest
 
-from helpers import rel_err
+from helpers import PAIRED_PRODUCTS, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -88,11 +88,11 @@ def test_tensor_core_gemm_shapes(L, oracle, m, k, n, bf16):
 
 
 @pytest.mark.parametrize("bf16", [True, False])
-@pytest.mark.parametrize("m,k,n", [(129, 8, 128), (256, 64, 256), (257, 72, 255), (300, 1000, 385), (2300, 328, 129), (5000, 136, 1030)])
+@pytest.mark.parametrize("m,k,n", [(129, 8, 128), (256, 64, 256), (257, 72, 255), (300, 1000, 385), (2300, 328, 129), (5000, 136, 1030)] + PAIRED_PRODUCTS)
 def test_paired_tile_edges(L, m, k, n, bf16):
-    """Products of more than 128 rows (256-row tiles by pairs of SMs): one row and one column beyond a tile, rows that are no whole
-    vector, fewer K blocks than ring stages, and more tiles than pairs of SMs (tile rows in several groups).  Tolerance as above:
-    operands are split in two bf16 halves, 2^-17 of each."""
+    """Products of more than 128 rows, by single SMs and (the sizes of PAIRED_PRODUCTS, see test_plans.py) by pairs of SMs: one row and one
+    column beyond a tile, rows that are no whole vector, fewer K blocks than ring stages, and more tiles than pairs of SMs (tile rows in several
+    groups).  Tolerance as above: operands are split in two bf16 halves, 2^-17 of each."""
     rng = np.random.default_rng(m + k + n)
     a = rng.standard_normal((m, k), dtype=np.float32)
     w = rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.05)

@@ -4,6 +4,8 @@ from pathlib import Path
 
 import pytest
 
+from helpers import PAIRED_PRODUCTS, PAIRED_PROMPTS
+
 ROOT = Path(__file__).resolve().parents[1]
 
 
@@ -37,6 +39,17 @@ def test_plain_products_take_the_kernel_that_was_faster(plan, m, k, n, bf16, sin
     times = {0: single, 128: pair128, 256: pair256}
     bn, splits, per = plan("plain", m, k, n, bf16)
     assert times[bn] <= 1.1 * min(times.values()) and splits == 1 and per * 64 >= k
+
+
+def test_sizes_of_the_gpu_tests_reach_what_they_claim(plan):
+    for m, k, n in PAIRED_PRODUCTS[:-1]:
+        assert plan("plain", m, k, n, True)[0] == plan("plain", m, k, n, False)[0] == 256
+    assert plan("plain", *PAIRED_PRODUCTS[-1], False)[0] == 128 and plan("plain", *PAIRED_PRODUCTS[-1], True)[0] == 0
+    for h, inter, prompt, slices, down, gate_up in PAIRED_PROMPTS:
+        for bf16 in (True, False):
+            products = 2 if bf16 else 3
+            assert plan("pair", prompt, inter, h, products, False, True)[:2] == (down[not bf16], slices[not bf16])
+            assert plan("pair", prompt, h, 2 * inter, products, True, False)[0] == gate_up[not bf16]
 
 
 def test_plans_cover_the_whole_of_k(plan):
