@@ -17,16 +17,11 @@ namespace {
 constexpr int kThreads = kAttnThreads;
 constexpr int kWarps = kAttnWarps;
 
-struct SyncThreads {
-    __device__ __forceinline__ void operator()() const { __syncthreads(); }
-};
-
 // grid (nsplit, Hkv * (G/GT), B)
 template <int GT, int NI>
 __global__ void __launch_bounds__(kThreads) attn_decode_kernel(DecodeParams p) {
     extern __shared__ __align__(16) float smem[];
-    attn_decode_item<GT, NI, false, kWarps>(p, smem, blockIdx.z, blockIdx.y, blockIdx.x, threadIdx.x, *p.d_len, SyncThreads(),
-                                    PartOut{&p}, NoStage());
+    attn_decode_item<GT, NI>(p, smem, blockIdx.z, blockIdx.y, blockIdx.x, threadIdx.x, *p.d_len);
 }
 
 // Merge the splits; grid (B*Hq).  Thread 0 of block 0 advances the cache length afterwards
@@ -90,8 +85,8 @@ __global__ void __launch_bounds__(kThreads) attn_prefill_prep_kernel(PrefillPara
 // Prompts of fewer than 64 positions whose context fits 64 rows: one CTA per (head, sequence), everything in shared memory, f32
 // throughout.  A thread forms a 4 x 4 block of the scores (rows ty + 16 i, cached rows tx + 16 j; rows padded by four numbers, so that
 // 16-byte reads of eight neighbouring rows hit different banks), then 4 rows x D / 16 numbers of the result.  Bound by the
-// FMA pipe: 2 x 64 x 64 x D FMAs per CTA however short the prompt, so a prompt of 32 costs as much as one of 63: shorter ones, and
-// fewer CTAs than SMs, stay with a warp per query row.
+// FMA pipe: the scores take 64 x 64 x D FMAs per CTA however short the prompt (the product with V ends with the context, and in rows
+// with their position).  Prompts of fewer than 32 positions, and fewer CTAs than SMs, stay with a warp per query row.
 // 64 sequences x 32 heads x 60 positions of 128 numbers: 180 us against 437.  grid (Hq, B).
 constexpr int kTileRows = 64;
 template <int D>
@@ -406,13 +401,13 @@ __global__ void __launch_bounds__((tiled_warps<D>() * 32), 1) attn_decode_tiled_
     // Stage and rotate the query heads and this step's k (as in the other kernel).
     for (int g = warp; g < GT; g += NW) {
         const float *src = p.q + (size_t)b * p.q_stride + (size_t)(h0 + g) * D;
-        load_norm_rope<false>(qs + g * D, src, D, p.q_norm, p.norm_eps, cos_row, sin_row, lane);
+        load_norm_rope(qs + g * D, src, D, p.q_norm, p.norm_eps, cos_row, sin_row, lane);
     }
     const bool owns_new = (past >= j0 && past < j1);
     const float *vnew_src = p.v_new + (size_t)b * p.kv_stride + (size_t)hk * D;
     if (owns_new && warp == NW - 1) {
         const float *ksrc = p.k_new + (size_t)b * p.kv_stride + (size_t)hk * D;
-        load_norm_rope<false>(knew, ksrc, D, p.k_norm, p.norm_eps, cos_row, sin_row, lane);
+        load_norm_rope(knew, ksrc, D, p.k_norm, p.norm_eps, cos_row, sin_row, lane);
         if (ygroup % groups_per_kv == 0) {
             float *k_row = p.k_cache + (((size_t)b * p.Hkv + hk) * p.max_seq + past) * D;
             float *v_row = p.v_cache + (((size_t)b * p.Hkv + hk) * p.max_seq + past) * D;

@@ -1,5 +1,5 @@
-// Device code of the decode (S == 1) attention step, shared by the stand-alone kernel and the
-// whole-step persistent kernel.
+// Device code of the decode (S == 1) attention step: the work item of the general kernel (attention.cu), and the head norm and
+// rotation that the persistent kernel uses too.
 //
 // Restates src/layers/attention/self_attention.rs:141-297 of the reference: rotate the new k into cache
 // row `len`, copy v, rotate q, then softmax(q.K^T * scale).V over rows 0..=len with the
@@ -118,8 +118,9 @@ struct DecodeParams {
 // Rows of K and V a warp keeps in flight, as a function of the elements per lane NI = ceil(D / 32).
 __host__ __device__ constexpr int attn_rows_in_flight(int NI) { return NI <= 2 ? 8 : (NI == 4 ? 4 : 2); }
 
-__host__ __device__ inline size_t attn_decode_smem_floats(int GT, int D, int warps = kAttnWarps) {
+__host__ __device__ inline size_t attn_decode_smem_floats(int GT, int D) {
     // q heads, rotated new k, per-warp (max, sum), per-warp ctx, per-warp softmax weights of one chunk + rescale factors
+    constexpr int warps = kAttnWarps;
     return (size_t)GT * D + D + 2 * warps * GT + (size_t)warps * GT * D + (size_t)warps * (8 * GT + GT);
 }
 
@@ -149,35 +150,13 @@ __device__ __forceinline__ void attn_reduce_multi(float (&a)[NV], int lane) {
     }
 }
 
-// Default sink of an item's result: the plain partial arrays of DecodeParams.
-struct PartOut {
-    const DecodeParams *p;
-    __device__ __forceinline__ void operator()(size_t row, int split, int e, float c, float M, float L) const {
-        const size_t o = row * p->nsplit + split;
-        p->part_ctx[o * p->D + e] = c;
-        if (e == 0) {
-            p->part_m[o] = M;
-            p->part_l[o] = L;
-        }
-    }
-};
-
 // One work item: batch row b, KV head group `ygroup` (= hk * (G/GT) + group), context split `split`.
-// Executed by NW warps (tid = 0 .. 32*NW-1) that share `smem` and the barrier `bar()`.
-// GT query heads per item, NI = ceil(D/32) elements per lane.
-// LOCAL_IN: p.q / p.k_new / p.v_new point at this item's vectors already staged in shared memory
-// ([GT*D], [D], [D]) instead of the global projection buffer.
-// out(row = b*Hq + head, split, e, ctx_e, max, sum) receives the item's partial result.
-// The first K/V rows of every warp are requested before q is staged: cached rows do not depend on this
-// step's projections, so their round trip overlaps the wait for q.
-// stage() runs after those requests are issued and before q is read: the persistent kernel waits there
-// for the projections of this step (and copies them to shared memory); elsewhere it is a no-op.
-struct NoStage {
-    __device__ __forceinline__ void operator()() const {}
-};
-template <int GT, int NI, bool LOCAL_IN, int NW, typename Bar, typename Out, typename Stage>
-__device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *smem, int b, int ygroup, int split, int tid,
-                                                 int past, Bar bar, Out out, Stage stage) {
+// Executed by a CTA of kAttnThreads threads.  GT query heads per item, NI = ceil(D/32) elements per lane.  The item's maximum, sum and
+// context go to the partial arrays of DecodeParams.  The first K/V rows of every warp are requested before q is staged: cached rows do
+// not depend on this step's projections, so their round trip overlaps q's.
+template <int GT, int NI>
+__device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *smem, int b, int ygroup, int split, int tid, int past) {
+    constexpr int NW = kAttnWarps;
     const int D = p.D;
     float *qs = smem;                        // [GT][D]
     float *knew = qs + GT * D;               // [D]
@@ -222,31 +201,30 @@ __device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *s
     };
     int jb = j0 + warp * UN;
     if (jb < j1) load_chunk(jb, kra, vra);
-    stage();
 
     // Stage and rotate the GT query heads (one warp per head, round robin).
     for (int g = warp; g < GT; g += NW) {
-        const float *src = LOCAL_IN ? p.q + (size_t)g * D : p.q + (size_t)b * p.q_stride + (size_t)(h0 + g) * D;
-        load_norm_rope<LOCAL_IN>(qs + g * D, src, D, p.q_norm, p.norm_eps, cos_row, sin_row, lane);
+        const float *src = p.q + (size_t)b * p.q_stride + (size_t)(h0 + g) * D;
+        load_norm_rope(qs + g * D, src, D, p.q_norm, p.norm_eps, cos_row, sin_row, lane);
     }
     // Every item whose range holds row `past` rotates the new k into shared memory and uses that copy
     // (and v_new straight from the projection), so no item reads the cache row written during this step;
     // the first head group of each KV head also stores the row into the cache.
     const bool owns_new = (past >= j0 && past < j1);
-    const float *vnew_src = LOCAL_IN ? p.v_new : p.v_new + (size_t)b * p.kv_stride + (size_t)hk * D;
+    const float *vnew_src = p.v_new + (size_t)b * p.kv_stride + (size_t)hk * D;
     if (owns_new && warp == NW - 1) {
-        const float *ksrc = LOCAL_IN ? p.k_new : p.k_new + (size_t)b * p.kv_stride + (size_t)hk * D;
-        load_norm_rope<LOCAL_IN>(knew, ksrc, D, p.k_norm, p.norm_eps, cos_row, sin_row, lane);
+        const float *ksrc = p.k_new + (size_t)b * p.kv_stride + (size_t)hk * D;
+        load_norm_rope(knew, ksrc, D, p.k_norm, p.norm_eps, cos_row, sin_row, lane);
         if (ygroup % groups_per_kv == 0) {
             float *k_row = p.k_cache + (((size_t)b * p.Hkv + hk) * p.max_seq + past) * D;
             float *v_row = p.v_cache + (((size_t)b * p.Hkv + hk) * p.max_seq + past) * D;
             for (int i = lane; i < D; i += 32) {
                 k_row[i] = knew[i];
-                v_row[i] = LOCAL_IN ? vnew_src[i] : __ldcg(vnew_src + i);
+                v_row[i] = __ldcg(vnew_src + i);
             }
         }
     }
-    bar();
+    __syncthreads();
 
     // A chunk of UN rows x GT heads is handled at once: the UN*GT dot products are summed across the lanes
     // by one butterfly, after which each score lives in one lane (value g*UN + u in lane idx0 .. ), the
@@ -283,7 +261,7 @@ __device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *s
                     for (int i = 0; i < NI; ++i) {
                         const int e = lane + 32 * i;
                         kr[u][i] = (e < D) ? knew[e] : 0.f;
-                        vr[u][i] = (e < D) ? (LOCAL_IN ? vnew_src[e] : __ldcg(vnew_src + e)) : 0.f;
+                        vr[u][i] = (e < D) ? __ldcg(vnew_src + e) : 0.f;
                     }
                 }
             }
@@ -363,8 +341,8 @@ __device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *s
             if (e < D) wctx[(warp * GT + g) * D + e] = ctx[g][i];
         }
     }
-    bar();
-    for (int idx = tid; idx < GT * D; idx += (NW * 32)) {
+    __syncthreads();
+    for (int idx = tid; idx < GT * D; idx += kAttnThreads) {
         const int g = idx / D, e = idx % D;
         float M = -INFINITY;
 #pragma unroll
@@ -377,9 +355,13 @@ __device__ __forceinline__ void attn_decode_item(const DecodeParams &p, float *s
             L = fmaf(wl[w * GT + g], f, L);
             c = fmaf(wctx[(w * GT + g) * D + e], f, c);
         }
-        out((size_t)b * p.Hq + h0 + g, split, e, c, M, L);
+        const size_t o = ((size_t)b * p.Hq + h0 + g) * p.nsplit + split;
+        p.part_ctx[o * D + e] = c;
+        if (e == 0) {
+            p.part_m[o] = M;
+            p.part_l[o] = L;
+        }
     }
-    bar();  // shared memory may be reused by the caller's next item
 }
 
 // Merges the splits of one (b, head) row: element e of out = ctx * (1/(l + 1e-9)) (self_attention.rs:287-290).

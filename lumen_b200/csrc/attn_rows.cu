@@ -9,8 +9,6 @@
 // conflicts), and the lanes share out the context's elements for P.V.  Some 40 KB of shared memory and 128 threads: 512 CTAs (64 sequences of
 // eight KV heads) are resident at once, and the products before and after find room beside them.  Steps of two Qwen3-8B layers with 64
 // sequences at 60 / 250 / 1000 positions: 520 / 574 / 925 us, with the general kernel and its merge 573 / 626 / 1063.
-#include <algorithm>
-
 #include <cooperative_groups.h>
 
 #include "attn_decode.cuh"
