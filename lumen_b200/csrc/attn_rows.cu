@@ -8,7 +8,8 @@
 // lanes form the scores of one row for all heads of the group from 16-byte reads in an order rotated by row (no bank
 // conflicts), and the lanes share out the context's elements for P.V.  Some 40 KB of shared memory and 128 threads: 512 CTAs (64 sequences of
 // eight KV heads) are resident at once, and the products before and after find room beside them.  Steps of two Qwen3-8B layers with 64
-// sequences at 60 / 250 / 1000 positions: 520 / 574 / 925 us, with the general kernel and its merge 573 / 626 / 1063.
+// sequences at 60 / 250 / 1000 / 4096 positions: 518 / 569 / 719 / 1257 us (rows beyond 1000 positions at 6.0 TB/s), with the general kernel and its merge
+// 571 / 619 / 785 / 1413.  Which lengths come here: attn_plan.cuh.
 #include <cooperative_groups.h>
 
 #include "attn_decode.cuh"
