@@ -93,7 +93,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     unsigned char *q_s = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *ring = q_s + G::kQBytes;
     unsigned char *p_s = ring + G::kStages * G::kStageBytes;
-    __shared__ uint64_t q_bar, k_full[G::kStages], v_full[G::kStages], k_free[G::kStages], v_free[G::kStages], s_bar[2], o_bar, p_bar;
+    __shared__ uint64_t q_bar, k_full[G::kStages], v_full[G::kStages], k_free[G::kStages], v_free[G::kStages], s_bar[2], o_bar, p_bar, quiet;
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
     // [column half][row]: row maxima, at the end the row sums.  One copy is enough: a thread writes its next value
@@ -125,6 +125,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
         bar_init(&s_bar[0], 1);
         bar_init(&s_bar[1], 1);
         bar_init(&o_bar, 1);
+        bar_init(&quiet, 1);
         bar_init(&p_bar, kFaWorkers);
         failed_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -416,6 +417,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
         drain_ring(&q_bar, 1, 1);  // a wait gave up
         drain_ring(k_full, G::kStages, k_issued);
         drain_ring(v_full, G::kStages, v_issued);
+    } else if (tid == kFaWorkers) {
+        drain_mmas(&quiet);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -99,7 +99,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     constexpr int kStages = G::kStages, kCols = SWIGLU ? BN / 2 : BN;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *ring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[kStages], empty[kStages], tfull[2], tempty[2];
+    __shared__ uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], quiet;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -122,6 +122,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
             bar_init(&tfull[b], 1);
             bar_init(&tempty[b], 8);  // four epilogue warps of two CTAs
         }
+        bar_init(&quiet, 1);
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -270,6 +271,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (failed && rank == 0 && tid == 32) {  // a wait gave up: the MMAs under way end before their tensor memory is given back
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(&quiet)) : "memory");
+        drain_ring(&quiet, 1, 1);
+    }
     cluster_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");

@@ -195,7 +195,7 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
                    const Seg p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *ring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[kStStages], empty[kStStages], d_full[2], d_free[2];
+    __shared__ uint64_t full[kStStages], empty[kStStages], d_full[2], d_free[2], quiet;
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
     __shared__ float decay[kSegChunks];
@@ -212,6 +212,7 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
             bar_init(&d_full[s], 1);
             bar_init(&d_free[s], kWorkers);
         }
+        bar_init(&quiet, 1);
         failed_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -335,7 +336,8 @@ mlstm_state_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_const
         if (tid == 0) tma_store_wait();
     }
     __syncthreads();
-    if (*failed && tid == kWorkers + 32) drain_ring(full, kStStages, issued);
+    if (*failed && tid == kWorkers + 32) drain_ring(full, kStStages, issued);  // a wait gave up: what is under way ends first
+    if (*failed && tid == kWorkers) drain_mmas(&quiet);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kWorkers / 32)
@@ -363,7 +365,7 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     extern __shared__ unsigned char smem_raw[];
     unsigned char *q_s = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *p_s = q_s + G::kQ, *ring = p_s + G::kP;
-    __shared__ uint64_t q_bar, full[G::kStages], empty[G::kStages], s_bar, p_bar, o_full[2], o_free[2];
+    __shared__ uint64_t q_bar, full[G::kStages], empty[G::kStages], s_bar, p_bar, o_full[2], o_free[2], quiet;
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
     __shared__ float a2_s[kC], xch[2][kC];
@@ -381,6 +383,7 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             bar_init(&empty[s], 1);
         }
         bar_init(&s_bar, 1);
+        bar_init(&quiet, 1);
         bar_init(&p_bar, kWorkers);
         for (int s = 0; s < 2; ++s) {
             bar_init(&o_full[s], 1);
@@ -608,6 +611,7 @@ mlstm_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         drain_ring(&q_bar, 1, 1);
         drain_ring(full, G::kStages, issued);
     }
+    if (*failed && tid == kWorkers) drain_mmas(&quiet);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kWorkers / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

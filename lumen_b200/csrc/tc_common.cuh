@@ -83,6 +83,12 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar)) : "memory");
 }
+// The same for MMAs, before their tensor memory is given back: called by the thread that issued them, with a barrier for one arrival that is
+// used for nothing else.
+__device__ __forceinline__ void drain_mmas(uint64_t *bar) {
+    umma_commit(bar);
+    drain_ring(bar, 1, 1);
+}
 // 32 consecutive accumulator columns of this thread's lane (lane = 32 * (warp % 4) + lane id); the values may be
 // used after tmem_ld_wait().
 __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&v)[32]) {

@@ -50,3 +50,11 @@ def test_peer_addresses_come_from_mapa():
     for p in sorted(CSRC.glob("*.cu*")):
         assert not re.search(r"0xF[0-9A-Fa-f]FFFFFF|kPeerMask", p.read_text()), p.name
     assert "mapa.shared::cluster" in (CSRC / "gemm_pair.cu").read_text()
+
+
+def test_tensor_memory_is_kept_until_the_mmas_end():
+    """Every kernel that gives tensor memory back waits, after a wait that gave up, for a barrier that its last MMAs arrive at."""
+    for p in sorted(CSRC.glob("*.cu")):
+        text = p.read_text()
+        waits = re.findall(r"drain_mmas\(&\w+\)|drain_ring\(&(?:done|quiet), 1, 1\)", text)
+        assert text.count("tcgen05.dealloc") == len(waits), p.name
