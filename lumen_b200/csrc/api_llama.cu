@@ -77,11 +77,9 @@ struct lumen_llama : lumen_model {
     MegaLayer *d_mega_layers = nullptr;
     uint4 *d_sched = nullptr;      // producer schedule of the persistent kernel (see MegaParams::sched)
     int *d_sched_count = nullptr;
-    size_t sched_capacity = 0;
     int sched_stride = 0;
     CUtensorMap *d_tmaps = nullptr;   // tensor maps of the segmented matrices (see MegaParams::tmaps); null when there are none
-    size_t tmaps_capacity = 0;
-    const void *mega_key = nullptr;  // first cache's k pointer the layer table was built for
+    std::vector<MegaLayer> mega_table;  // what d_mega_layers holds (empty: nothing yet)
     unsigned long long *d_trace = nullptr;  // phase timestamps of the last persistent step (LUMEN_DECODE_TRACE=1)
 
     ~lumen_llama() override;
@@ -444,50 +442,44 @@ int run_mega(lumen_llama *m, lumen_kv_cache **caches) {
     p.qkv_rows = (int)m->qkv_rows; p.qd = (int)m->qd_l; p.kvd = (int)m->kvd_l; p.max_seq = (int)caches[0]->max_seq;
     p.wbf16 = m->cfg.weight_dtype == LUMEN_BF16;
     p.embed = m->embed; p.final_norm = m->final_norm; p.lm_head = m->lm_head;
-    if (m->mega_key != (const void *)caches[0]->k || !m->d_mega_layers) {
-        // (Re)build what depends on addresses: the layer table and the producer's copy schedule.
-        std::vector<MegaLayer> host(m->L);
-        for (size_t l = 0; l < m->L; ++l) {
-            const LayerW &lw = m->layers[l];
-            host[l] = MegaLayer{lw.wqkv, lw.wo, lw.wgate, lw.wup, lw.wdown, lw.norm1, lw.norm2, lw.qn, lw.kn,
-                                caches[l]->k, caches[l]->v, caches[l]->d_len};
-        }
+    // The layer table holds addresses of weights and of this call's caches: it goes to the device again when one of them differs
+    // (a few KB in stream order, so that steps in flight still read the former one).  The copy schedule and its tensor maps
+    // depend on the weights alone and are built once: a server that takes turns between conversations paid 3 ms a
+    // turn (TinyLlama; 250,000 entries) while they were rebuilt with the table.
+    std::vector<MegaLayer> host(m->L);
+    for (size_t l = 0; l < m->L; ++l) {
+        const LayerW &lw = m->layers[l];
+        host[l] = MegaLayer{lw.wqkv, lw.wo, lw.wgate, lw.wup, lw.wdown, lw.norm1, lw.norm2, lw.qn, lw.kn,
+                            caches[l]->k, caches[l]->v, caches[l]->d_len};
+    }
+    const size_t table_bytes = m->L * sizeof(MegaLayer);
+    if (!m->d_sched) {
         std::vector<uint4> entries;
         std::vector<int> counts;
         int stride = 0;
         std::vector<CUtensorMap> tmaps;
         decode_mega_build_schedule(p, host.data(), ctx->num_sms, entries, counts, stride, tmaps);
-        LUMEN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // earlier launches may still read the tables
-        if (!m->d_mega_layers) LUMEN_CUDA(ctx, cudaMalloc(&m->d_mega_layers, std::max<size_t>(m->L, 1) * sizeof(MegaLayer)));
-        if (m->d_sched && m->sched_capacity < entries.size()) {
-            cudaFree(m->d_sched);
-            m->d_sched = nullptr;
-        }
-        if (!m->d_sched) {
-            LUMEN_CUDA(ctx, cudaMalloc(&m->d_sched, entries.size() * sizeof(uint4)));
-            m->sched_capacity = entries.size();
-        }
+        if (!m->d_mega_layers) LUMEN_CUDA(ctx, cudaMalloc(&m->d_mega_layers, table_bytes));
         if (!m->d_sched_count) LUMEN_CUDA(ctx, cudaMalloc(&m->d_sched_count, counts.size() * sizeof(int)));
-        if (m->d_tmaps && m->tmaps_capacity < tmaps.size()) {
-            cudaFree(m->d_tmaps);
-            m->d_tmaps = nullptr;
-        }
-        if (!tmaps.empty()) {
-            if (!m->d_tmaps) {
-                LUMEN_CUDA(ctx, cudaMalloc(&m->d_tmaps, tmaps.size() * sizeof(CUtensorMap)));
-                m->tmaps_capacity = tmaps.size();
-            }
-            LUMEN_CUDA(ctx, cudaMemcpy(m->d_tmaps, tmaps.data(), tmaps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
-        } else if (m->d_tmaps) {
-            cudaFree(m->d_tmaps);
-            m->d_tmaps = nullptr;
-            m->tmaps_capacity = 0;
-        }
-        LUMEN_CUDA(ctx, cudaMemcpy(m->d_mega_layers, host.data(), m->L * sizeof(MegaLayer), cudaMemcpyHostToDevice));
-        LUMEN_CUDA(ctx, cudaMemcpy(m->d_sched, entries.data(), entries.size() * sizeof(uint4), cudaMemcpyHostToDevice));
         LUMEN_CUDA(ctx, cudaMemcpy(m->d_sched_count, counts.data(), counts.size() * sizeof(int), cudaMemcpyHostToDevice));
+        if (!tmaps.empty()) {
+            if (!m->d_tmaps) LUMEN_CUDA(ctx, cudaMalloc(&m->d_tmaps, tmaps.size() * sizeof(CUtensorMap)));
+            LUMEN_CUDA(ctx, cudaMemcpy(m->d_tmaps, tmaps.data(), tmaps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+        }
         m->sched_stride = stride;
-        m->mega_key = caches[0]->k;
+        uint4 *sched = nullptr;
+        LUMEN_CUDA(ctx, cudaMalloc(&sched, entries.size() * sizeof(uint4)));
+        const cudaError_t e = cudaMemcpy(sched, entries.data(), entries.size() * sizeof(uint4), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(sched);
+            return cuda_fail(ctx, e, "cudaMemcpy(copy schedule)");
+        }
+        m->d_sched = sched;  // (last: what is there is complete)
+    }
+    if (m->mega_table.size() != m->L || memcmp(m->mega_table.data(), host.data(), table_bytes) != 0) {
+        m->mega_table.clear();
+        LUMEN_CUDA(ctx, cudaMemcpyAsync(m->d_mega_layers, host.data(), table_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        m->mega_table = std::move(host);
     }
     p.layers = m->d_mega_layers;
     p.sched = m->d_sched; p.sched_count = m->d_sched_count; p.sched_stride = m->sched_stride;

@@ -276,6 +276,36 @@ def test_persistent_kernel_equals_per_op_path(L, oracle, monkeypatch, over, wdt)
         assert rel_err(k, oc[l].k) < 1e-5 and rel_err(v, oc[l].v) < 1e-5
 
 
+def test_caches_in_turn(L):
+    """The persistent kernel follows the caches of each call: two conversations of one model in turn, and caches whose first layer alone is shared."""
+    cfg = small_cfg()
+    params = make_params(L, cfg, 66, std=0.08)
+    ids = np.random.default_rng(67).integers(0, cfg["vocab_size"], size=(2, 14)).astype(np.float32)
+    want = [_gpu_run(L, cfg, params, ids[i:i + 1], 3)[0][:, 3:] for i in range(2)]
+    model = L.LlamaModel(cfg_obj(L, cfg))
+    model.load_state(params)
+    caches = [model.init_kv_caches(1) for _ in range(2)]
+    with L.no_grad():
+        for i in range(2):
+            model.forward(ids[i:i + 1, :3], caches[i], 0)
+        for t in range(3, 14):
+            for i in range(2):
+                got = model.forward(ids[i:i + 1, t:t + 1], caches[i], 0)
+                assert np.array_equal(got[:, 0], want[i][:, t - 3]), (t, i)
+        third = model.init_kv_caches(1)
+        mixed = [third[0]] + list(caches[1][1:])  # (the first layer's memory is another one, the others' are not)
+        model.reset_kv_caches(mixed)
+        for part in (ids[1:2, :3], *(ids[1:2, t:t + 1] for t in range(3, 6))):
+            got = model.forward(part, mixed, 0)
+        assert np.array_equal(got[:, 0], want[1][:, 2])
+        model.reset_kv_caches(caches[0])
+        swapped = [third[0]] + list(caches[0][1:])  # the same first layer, other layers behind it
+        model.reset_kv_caches(swapped)
+        for part in (ids[0:1, :3], *(ids[0:1, t:t + 1] for t in range(3, 6))):
+            got = model.forward(part, swapped, 0)
+        assert np.array_equal(got[:, 0], want[0][:, 2])
+
+
 @pytest.mark.parametrize("batch", [8, 9])
 def test_parameters_set_between_steps(L, batch):
     """Wide f32 models send eight rows through the products of the kept bf16 weight split, in captured steps: after set_param
