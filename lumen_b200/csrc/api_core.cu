@@ -156,6 +156,8 @@ int lumen_ctx_create(int device, int tp_rank, int tp_size, const void *nccl_uniq
     if ((e = cudaMalloc(&ctx->d_status, sizeof(DeviceStatus))) != cudaSuccess) return fail(e, "cudaMalloc(status)");
     if ((e = cudaMemset(ctx->d_status, 0, sizeof(DeviceStatus))) != cudaSuccess) return fail(e, "cudaMemset(status)");
     if ((e = cudaMallocHost(&ctx->h_status, sizeof(DeviceStatus))) != cudaSuccess) return fail(e, "cudaMallocHost(status)");
+    if ((e = cudaMallocHost(&ctx->h_answer, sizeof(*ctx->h_answer))) != cudaSuccess) return fail(e, "cudaMallocHost(answer)");
+    *ctx->h_answer = 0;
     if ((e = cudaMalloc(&ctx->d_mega_sync, 16)) != cudaSuccess) return fail(e, "cudaMalloc(barrier)");
     if ((e = cudaMemset(ctx->d_mega_sync, 0, 16)) != cudaSuccess) return fail(e, "cudaMemset(barrier)");
     if (tp_size > 1) {
@@ -189,6 +191,7 @@ int lumen_ctx_destroy(lumen_ctx *ctx) {
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_mega_sync) cudaFree(ctx->d_mega_sync);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->h_answer) cudaFreeHost(ctx->h_answer);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return LUMEN_OK;

@@ -37,6 +37,8 @@ struct lumen_ctx {
     void *nccl_comm = nullptr;  // ncclComm_t when tp_size > 1
     lumen::DeviceStatus *d_status = nullptr;
     lumen::DeviceStatus *h_status = nullptr;  // pinned mirror
+    unsigned long long *h_answer = nullptr;   // pinned: the device sampler's answer, turn << 32 | token
+    unsigned int answer_turn = 0;
     char err[512] = {0};
     bool pdl = false;  // launch_pdl may overlap kernels now (set by steps that consist of such launches alone)
     unsigned long long launches = 0;  // kernels enqueued so far (graph replays add their node count)

@@ -140,6 +140,7 @@ __device__ __forceinline__ uint2 pick_scan(uint2 f, int lane) {  // inclusive, o
 
 // First index < n whose running sum of vals[i] / scale is >= threshold (n if none), and that running sum (the total if none).
 // vals is in descending order, all >= 0.  All kPickThreads threads call; the answers are the same in all of them.
+template <bool SHARED>  // where the list is
 __device__ __forceinline__ int first_reaching(const float *vals, int n, float scale, float threshold, PickShared &sh, float *sum_out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float run = 0.f;
@@ -148,7 +149,7 @@ __device__ __forceinline__ int first_reaching(const float *vals, int n, float sc
         const int i0 = base + 4 * tid;
         float v[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = i0 + q < n ? __fdiv_rn(__ldcg(vals + i0 + q), scale) : 0.f;
+        for (int q = 0; q < 4; ++q) v[q] = i0 + q < n ? __fdiv_rn(SHARED ? vals[i0 + q] : __ldcg(vals + i0 + q), scale) : 0.f;
         if (base == 0) {
             if (4 * tid < kPickHead) *reinterpret_cast<float4 *>(sh.head + 4 * tid) = make_float4(v[0], v[1], v[2], v[3]);
             __syncthreads();
@@ -250,19 +251,20 @@ __device__ __forceinline__ int first_reaching(const float *vals, int n, float sc
 }
 
 // Rank of the drawn token in the sorted list.  `all`: the list is complete; otherwise -1 where it ends before the nucleus does.
+template <bool SHARED>
 __device__ __forceinline__ int pick_rank(const float *sorted_p, int n, bool all, float target, float r, PickShared &sh) {
     float cumulative, acc;
-    const int at = first_reaching(sorted_p, n, 1.0f, target, sh, &cumulative);  // main.rs:113-121
+    const int at = first_reaching<SHARED>(sorted_p, n, 1.0f, target, sh, &cumulative);  // main.rs:113-121
     if (at == n && !all) return -1;
     const int cut = max(1, min(n, at + 1));
     // main.rs:126-134: acc += probs[i] / cumulative; the first i with r <= acc, else the last of the nucleus
-    return min(first_reaching(sorted_p, cut, cumulative, r, sh, &acc), cut - 1);
+    return min(first_reaching<SHARED>(sorted_p, cut, cumulative, r, sh, &acc), cut - 1);
 }
 
 __global__ void __launch_bounds__(kPickThreads)
 sample_pick_kernel(const float *__restrict__ sorted_p, const int *__restrict__ sorted_i, int n, float target, float r, int *__restrict__ token_out) {
     __shared__ PickShared sh;
-    const int pick = pick_rank(sorted_p, n, true, target, r, sh);
+    const int pick = pick_rank<false>(sorted_p, n, true, target, r, sh);
     if (threadIdx.x == 0) *token_out = sorted_i[pick];
 }
 
@@ -272,19 +274,24 @@ sample_pick_kernel(const float *__restrict__ sorted_p, const int *__restrict__ s
 // denominator in the same order and agree on every bit of a probability.
 // Only the nucleus is sorted.  The probabilities are counted by exponent and seven bits of mantissa (128 bins per octave, 24
 // octaves); from the counts and the bins' lower edges every CTA finds the bin that certainly completes the nucleus, and the
-// offsets of the bins in descending order.  The candidates are scattered into their bins (global memory: tens of KB in the L2), and
+// offsets of the bins in descending order.  The candidates are scattered into their bins (up to 2048 into CTA 0's shared memory, which
+// ranks them alone; longer lists in global memory, tens of KB in the L2, ranked by all CTAs), and
 // a candidate's rank within its bin is the number of larger ones (an equal probability of a smaller index is larger: the sort
 // is stable).  CTA 0 then walks the list as the general path does.
-// What bounds it is the chain of passes and cluster barriers, not bytes.  32000 logits of which some hundred to a thousand make the
-// nucleus: 48 us a call against 140 us with the seven kernels of the general path (100 us of it theirs).
+// What bounds it is the chain of passes and cluster barriers, not bytes: hence one barrier per reduction (every warp hands its number to
+// every CTA), counts of 16 bits (eight remote reads a thread), no trip to the L2 for short lists, and an answer that the
+// host picks up by itself.  32000 logits of which some hundred to a thousand make the nucleus: 29 us a call (49 with remote reads behind
+// local reductions, lists in the L2, and a copy and a wait for the stream behind the kernel; 140 with the seven kernels of the general path).
 namespace cg = cooperative_groups;
 constexpr int kCluster = 8;
 constexpr int kNucleusBins = 24 * 128;
-constexpr int kBinsPerThread = kNucleusBins / kPrepThreads;
+constexpr int kBinsPerThread = 4, kBinThreads = kNucleusBins / kBinsPerThread;
+constexpr int kNear = 2048;  // a list of up to this many stays in the first CTA's shared memory
 constexpr uint32_t kTopBin = 0x3f800000u >> 16;  // of probability 1
 constexpr int kMaxBin = 512;                      // ranking is quadratic in a bin's size
 constexpr int kNucleusMaxVocab = 256 * 1024;      // 128 KB of shared memory per CTA
-static_assert(kPrepThreads == kPickThreads && kBinsPerThread * kPrepThreads == kNucleusBins, "");
+static_assert(kPrepThreads == kPickThreads && kBinsPerThread * kBinThreads == kNucleusBins && kBinThreads <= kPrepThreads && kBinThreads % 32 == 0, "");
+static_assert(kNucleusMaxVocab / kCluster < 65536, "a CTA's counts take 16 bits");
 
 struct NucleusArgs {
     const float *logits;
@@ -293,15 +300,21 @@ struct NucleusArgs {
     unsigned long long *cand;  // [n] probability bits : ~index
     float *sorted_p;           // [n]
     int *sorted_i;             // [n]
-    int *token;                // the token, or -1: not served here
+    const int *status;         // what kernels before this one reported
+    unsigned long long *answer;  // pinned host memory: turn << 32 | token; the token is -1 where it is not served here, -2 after a report
+    unsigned int turn;
     int n_recent;
     int recent[kMaxRecent];
 };
 
 struct NucleusShared {
-    int hist[kNucleusBins], cursor[kNucleusBins], first[kNucleusBins + 1];  // counts here; next place; first place of a bin
+    __align__(16) unsigned int hist[kNucleusBins / 2];          // counts here, two bins to a word
+    int cursor[kNucleusBins], first[kNucleusBins + 1];          // next place; first place of a bin
     __align__(16) unsigned long long window[kPrepThreads / 32][32];
-    float red[33], top, part[4];
+    __align__(16) unsigned long long cand[kNear];               // the first CTA's: candidates in their bins,
+    float near_p[kNear];                                        // in order
+    int near_i[kNear];
+    float top[kCluster * kPrepThreads / 32], part[kCluster * 4];  // every warp's, of all CTAs
     int recent[kMaxRecent];
     int scan_n[32];
     float scan_m[32];
@@ -319,30 +332,43 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank(), n = a.n;
     const int slots = (n + 1023) / 1024 * 128;
     auto index_of = [&](int s) { return (s >> 7) * 1024 + rank * 128 + (s & 127); };
-#pragma unroll 4
-    for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? a.logits[index_of(s)] : -INFINITY;
-    for (int b = tid; b < kNucleusBins; b += kPrepThreads) sh.hist[b] = 0;
+    auto answer = [&](int token) {  // one word, so that its turn says that the token is there
+        const unsigned int t = __ldcg(a.status) ? (unsigned int)-2 : (unsigned int)token;
+        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(a.answer), "l"((unsigned long long)a.turn << 32 | t) : "memory");
+    };
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // (this CTA runs: the others may write to its shared memory)
+    for (int s = tid; s < slots; s += kPrepThreads) {
+        if (index_of(s) < n)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(vals + s)), "l"(a.logits + index_of(s)) : "memory");
+        else vals[s] = -INFINITY;
+    }
+    for (int b = tid; b < kNucleusBins / 2; b += kPrepThreads) sh.hist[b] = 0;
     if (tid < a.n_recent) sh.recent[tid] = a.recent[tid];
     if (tid == 0) {
         sh.last_bin = INT_MAX;
         sh.crowded = 0;
     }
     __syncthreads();
+    // (the recent tokens are counted while the logits are on their way)
+    int times = 0, token = -1;  // occurrences of thread t's recent token, if it is the first and in this CTA's columns
     if (a.penalty > 1.0f && tid < a.n_recent) {
         // the first occurrence of a token applies one division per occurrence (main.rs:83-89)
-        const int t = sh.recent[tid];
-        int times = 0, before = 0;
-#pragma unroll 4
+        token = sh.recent[tid];
+        int before = 0;
+#pragma unroll 8
         for (int k = 0; k < a.n_recent; ++k) {
-            const int same = sh.recent[k] == t;
+            const int same = sh.recent[k] == token;
             times += same;
             before += k < tid ? same : 0;
         }
-        if (before == 0 && t >= 0 && t < n && ((t >> 7) & (kCluster - 1)) == rank) {
-            float x = vals[(t >> 10) * 128 + (t & 127)];
-            for (int k = 0; k < times; ++k) x = __fdiv_rn(x, a.penalty);
-            vals[(t >> 10) * 128 + (t & 127)] = x;
-        }
+        if (before != 0 || token < 0 || token >= n || ((token >> 7) & (kCluster - 1)) != rank) token = -1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (token >= 0) {
+        float x = vals[(token >> 10) * 128 + (token & 127)];
+        for (int k = 0; k < times; ++k) x = __fdiv_rn(x, a.penalty);
+        vals[(token >> 10) * 128 + (token & 127)] = x;
     }
     __syncthreads();
     const float temp = fmaxf(a.temperature, 1e-5f);
@@ -352,18 +378,16 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
         vals[s] = x;
         if (index_of(s) < n) mx = fmaxf(mx, x);
     }
-    mx = block_reduce(mx, sh.red, true);
-    if (tid == 0) sh.top = mx;
-    cluster.sync();
-    // (one warp reads the other CTAs' numbers: all of them at once would queue for the same words)
-    if (warp == 0) {
-        float t = *cluster.map_shared_rank(&sh.top, lane & (kCluster - 1));
+    // Every warp hands its maximum to every CTA, so that one barrier is all that lies between.
 #pragma unroll
-        for (int o = kCluster / 2; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
-        if (lane == 0) sh.red[32] = t;
-    }
-    __syncthreads();
-    mx = sh.red[32];
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (lane < kCluster) *cluster.map_shared_rank(&sh.top[rank * (kPrepThreads / 32) + warp], lane) = mx;
+    cluster.sync();
+#pragma unroll
+    for (int q = 0; q < kCluster; ++q) mx = fmaxf(mx, sh.top[q * 32 + lane]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     for (int s = tid; s < slots; s += kPrepThreads) vals[s] = index_of(s) < n ? expf(__fsub_rn(vals[s], mx)) : 0.f;
     __syncthreads();
     if (tid < 128) {
@@ -372,40 +396,44 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
         for (int s = tid; s < slots; s += 128) sum += vals[s];  // (adding the zeros behind the end changes nothing)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) sh.part[warp] = sum;
+        if (lane < kCluster) *cluster.map_shared_rank(&sh.part[rank * 4 + warp], lane) = sum;
     }
     cluster.sync();
-    if (warp == 0) {
-        float sum = *cluster.map_shared_rank(&sh.part[lane & 3], lane >> 2);
+    float sum = sh.part[lane];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) sh.red[0] = sum;
-    }
-    __syncthreads();
-    const float inv = __fdiv_rn(1.0f, __fadd_rn(sh.red[0], 1e-9f));
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float inv = __fdiv_rn(1.0f, __fadd_rn(sum, 1e-9f));
     const bool finite = inv > 0.f && inv < INFINITY;  // (the same in every CTA)
     for (int s = tid; s < slots; s += kPrepThreads) {
         const float p = __fmul_rn(vals[s], inv);
         vals[s] = p;
         const int b = bin_of(p);
-        if (finite && b < kNucleusBins && index_of(s) < n) atomicAdd(&sh.hist[b], 1);
+        if (finite && b < kNucleusBins && index_of(s) < n) atomicAdd(&sh.hist[b >> 1], b & 1 ? 0x10000u : 1u);
     }
     cluster.sync();
     // Thread t's bins; all CTAs form the same totals in the same order.
     int total[kBinsPerThread], lower[kBinsPerThread], count = 0;  // lower: of the CTAs before this one
     float mass = 0.f;
 #pragma unroll
-    for (int j = 0; j < kBinsPerThread; ++j) {
-        const int b = tid * kBinsPerThread + j;
-        total[j] = lower[j] = 0;
+    for (int j = 0; j < kBinsPerThread; ++j) total[j] = lower[j] = 0;
+    if (tid < kBinThreads) {
+        uint2 h[kCluster];
+#pragma unroll
+        for (int c = 0; c < kCluster; ++c) h[c] = *cluster.map_shared_rank(reinterpret_cast<uint2 *>(sh.hist) + tid, c);
 #pragma unroll
         for (int c = 0; c < kCluster; ++c) {
-            const int h = *cluster.map_shared_rank(&sh.hist[b], c);
-            if (c < rank) lower[j] += h;
-            total[j] += h;
+            const int n_c[kBinsPerThread] = {(int)(h[c].x & 0xffffu), (int)(h[c].x >> 16), (int)(h[c].y & 0xffffu), (int)(h[c].y >> 16)};
+#pragma unroll
+            for (int j = 0; j < kBinsPerThread; ++j) {
+                if (c < rank) lower[j] += n_c[j];
+                total[j] += n_c[j];
+            }
         }
+    }
+#pragma unroll
+    for (int j = 0; j < kBinsPerThread; ++j) {
         count += total[j];
-        mass += (float)total[j] * __uint_as_float((kTopBin - (uint32_t)b) << 16);
+        mass += (float)total[j] * __uint_as_float((kTopBin - (uint32_t)(tid * kBinsPerThread + j)) << 16);
     }
     int count_in = count;
     float mass_in = mass;
@@ -442,13 +470,14 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
 #pragma unroll
     for (int j = 0; j < kBinsPerThread; ++j) {
         const int b = tid * kBinsPerThread + j;
+        if (tid >= kBinThreads) break;
         sh.first[b] = at;
         sh.cursor[b] = at + lower[j];
         at += total[j];
         reached += (float)total[j] * __uint_as_float((kTopBin - (uint32_t)b) << 16);
         if (reached >= need) atomicMin(&sh.last_bin, b);
     }
-    if (tid == kPrepThreads - 1) sh.first[kNucleusBins] = at;
+    if (tid == kBinThreads - 1) sh.first[kNucleusBins] = at;
     __syncthreads();
     int last = sh.last_bin;
     const bool all = last == INT_MAX;  // the whole vocabulary is the list, if the bins hold it
@@ -458,11 +487,35 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
         if (tid * kBinsPerThread + j <= last && total[j] > kMaxBin) sh.crowded = 1;
     __syncthreads();
     if (!finite || sh.crowded || (all && counted != n)) {
-        if (rank == 0 && tid == 0) *a.token = -1;
+        if (rank == 0 && tid == 0) answer(-1);
         cluster.sync();  // the others may still read this CTA's counts
         return;
     }
     const int cands = sh.first[last + 1];
+    if (cands <= kNear) {
+        // The first CTA alone: candidates into their bins over its shared memory, ranked and walked there.
+        for (int s = tid; s < slots; s += kPrepThreads) {
+            const float p = vals[s];
+            const int b = bin_of(p), i = index_of(s);
+            if (b <= last && i < n)
+                *cluster.map_shared_rank(&sh.cand[atomicAdd(&sh.cursor[b], 1)], 0) = ((unsigned long long)__float_as_uint(p) << 32) | (uint32_t)~i;
+        }
+        cluster.sync();
+        if (rank != 0) return;
+        for (int c = tid; c < cands; c += kPrepThreads) {
+            const unsigned long long own = sh.cand[c];
+            const int b = bin_of(__uint_as_float((uint32_t)(own >> 32))), w0 = sh.first[b], w1 = sh.first[b + 1];
+            int larger = 0;
+#pragma unroll 4
+            for (int w = w0; w < w1; ++w) larger += sh.cand[w] > own;
+            sh.near_p[w0 + larger] = __uint_as_float((uint32_t)(own >> 32));
+            sh.near_i[w0 + larger] = (int)~(uint32_t)own;
+        }
+        __syncthreads();
+        const int pick = pick_rank<true>(sh.near_p, cands, all, a.target, a.r, sh.pick);
+        if (tid == 0) answer(pick < 0 ? -1 : sh.near_i[pick]);
+        return;
+    }
     for (int s = tid; s < slots; s += kPrepThreads) {
         const float p = vals[s];
         const int b = bin_of(p), i = index_of(s);
@@ -497,8 +550,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     __threadfence();
     cluster.sync();
     if (rank != 0) return;
-    const int pick = pick_rank(a.sorted_p, cands, all, a.target, a.r, sh.pick);
-    if (tid == 0) *a.token = pick < 0 ? -1 : __ldcg(a.sorted_i + pick);
+    const int pick = pick_rank<false>(a.sorted_p, cands, all, a.target, a.r, sh.pick);
+    if (tid == 0) answer(pick < 0 ? -1 : __ldcg(a.sorted_i + pick));
 }
 
 }  // namespace
@@ -537,16 +590,37 @@ int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lu
         NucleusArgs a;
         a.logits = logits_dev; a.n = n; a.temperature = sp.temperature; a.penalty = sp.repetition_penalty; a.target = target; a.r = sp.uniform;
         a.cand = reinterpret_cast<unsigned long long *>(ws);
-        a.sorted_p = reinterpret_cast<float *>(ws + 8 * nf); a.sorted_i = reinterpret_cast<int *>(ws + 12 * nf); a.token = token_dev;
+        a.sorted_p = reinterpret_cast<float *>(ws + 8 * nf); a.sorted_i = reinterpret_cast<int *>(ws + 12 * nf);
+        a.status = &ctx->d_status->code;
+        a.answer = ctx->h_answer; a.turn = ++ctx->answer_turn;
         a.n_recent = (int)sp.n_recent;
         for (size_t i = 0; i < sp.n_recent; ++i) a.recent[i] = sp.recent_tokens[i];
         sample_nucleus_kernel<<<kCluster, kPrepThreads, smem, s>>>(a);
         LUMEN_LAUNCHED(ctx);
-        LUMEN_TRY(check_device_status(ctx));
-        if (ctx->h_status->token >= 0) {
-            *token = ctx->h_status->token;
+        // The kernel stores its answer to pinned memory of the host, which watches the word; the stream is asked now and then, so that a
+        // failure ends the watch.
+        int got = -1;
+        for (unsigned int spins = 1;; ++spins) {
+            const unsigned long long v = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
+            if ((unsigned int)(v >> 32) == a.turn) {
+                got = (int)(unsigned int)v;
+                break;
+            }
+            if ((spins & 0xffff) == 0 && cudaStreamQuery(s) != cudaErrorNotReady) {
+                LUMEN_TRY(check_device_status(ctx));
+                const unsigned long long last = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
+                if ((unsigned int)(last >> 32) == a.turn) got = (int)(unsigned int)last;
+                break;
+            }
+#if defined(__x86_64__)
+            __builtin_ia32_pause();
+#endif
+        }
+        if (got >= 0) {
+            *token = got;
             return LUMEN_OK;
         }
+        if (got == -2) LUMEN_TRY(check_device_status(ctx));
     }
     size_t sort_bytes = 0;
     LUMEN_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, (const float *)nullptr, (float *)nullptr, (const int *)nullptr,

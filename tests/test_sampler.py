@@ -94,6 +94,20 @@ def test_sampler_paths_draw_from_the_nucleus(L, ctx, vocab, shape):
 
 
 @pytest.mark.gpu
+def test_lists_on_both_sides_of_the_shared_memory(L, ctx, oracle):
+    """Lists of up to 2048 candidates stay in one SM's shared memory, longer ones cross the L2: nearly all of m likely tokens make the list."""
+    rng = np.random.default_rng(12)
+    mismatches = 0
+    for m in range(2040, 2200, 10):
+        lg = np.full(9000, -30.0, np.float32)
+        lg[rng.permutation(9000)[:m]] = (rng.standard_normal(m) * 0.7).astype(np.float32)
+        t = L.Tensor.from_array_no_grad(lg)
+        for u in list(rng.random(5).astype(np.float32)) + [np.float32(0), np.float32(1)]:
+            mismatches += L.sample_top_p(ctx, t.data_ptr, 9000, 1.0, 0.99, 1.0, [], float(u)) != oracle.sample_top_p(lg, 1.0, 0.99, 1.0, [], float(u))
+    assert mismatches <= 2, mismatches  # (as above: draws within an ulp of a boundary)
+
+
+@pytest.mark.gpu
 def test_forward_sample_equals_forward_then_oracle_sampler(L, oracle):
     cfg = small_cfg()
     params = make_params(L, cfg, 17, std=0.3)
