@@ -216,6 +216,7 @@ int lumen_gemv(lumen_ctx *ctx, const float *x_dev, const void *w_dev, lumen_dtyp
     if (w_dtype != LUMEN_F32 && w_dtype != LUMEN_BF16) return set_error(ctx, LUMEN_ERR_DTYPE, "gemv: dtype %d", (int)w_dtype);
     if (k == 0 || n == 0) return LUMEN_OK;
     if (!layout_kn) {
+        if (gemv_vec_usable(w_dev, w_dtype, k)) return launch_gemv_vec(ctx, x_dev, w_dev, w_dtype, y_dev, k, n, ctx->stream);
         if (k * 4 > 200 * 1024) return launch_gemm_nk(ctx, x_dev, w_dev, w_dtype, y_dev, 1, k, n, nullptr, ctx->stream);
         GemvArgs g;
         g.x = x_dev; g.w = w_dev; g.wdt = w_dtype; g.y = y_dev; g.M = 1; g.K = k; g.N = n; g.ldy = n;

@@ -257,6 +257,10 @@ int launch_gemv_nk(lumen_ctx *ctx, const GemvArgs &a, cudaStream_t s);
 int launch_gemv_gate_up(lumen_ctx *ctx, const float *x, const void *w_gate, const void *w_up, lumen_dtype wdt,
                         float *out, int M, size_t K, size_t I, const float *norm_w, float norm_eps, cudaStream_t s);
 
+// y = W x for one vector, as a call of its own (gemv_vec_kernel); usable: rows of whole aligned 16-byte vectors.
+bool gemv_vec_usable(const void *w, lumen_dtype wdt, size_t K);
+int launch_gemv_vec(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype wdt, float *y, size_t K, size_t N, cudaStream_t s);
+
 // y[n] = sum_k w[k, n] * x[k]; w is [K,N] row-major.  Uses `scratch` (>= gemv_kn_scratch_bytes) for
 // split-K partial sums.
 size_t gemv_kn_scratch_bytes(size_t K, size_t N, int num_sms);                           // either weight type

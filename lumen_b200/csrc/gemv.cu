@@ -116,6 +116,54 @@ gemv_nk_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *__r
     }
 }
 
+// One vector, nothing before or behind the product, rows of whole 16-byte vectors: launched so that it may start while the call before it
+// still runs (programmatic dependent launch).  Until that one is complete nothing is read - x and W may be its result - but the first
+// rows are handed to the L2, which is where all SMs meet.  Then a warp has 2 x kAhead vectors of its rows in flight,
+// the first of them requested before x is staged and the next row's while a row is summed up.  WPR warps share a row where rows
+// are fewer than warps would be.
+// What bounds it: launch, first bytes and staging for matrices of a few MB, HBM for large ones.  Calls behind one another, other weights every time:
+// f32 [256,2048] 6.7 -> 2.65 us (three quarters of it the overlap), [4096,4096] 15.7 -> 12.3, [32000,4096] 79.9 -> 75.9 (6.9 TB/s);
+// bf16 [4096,4096] 11.7 -> 8.8, [12288,12288] 62.3 -> 54.9 (5.5 TB/s).
+template <typename WT, int WPR>
+__global__ void __launch_bounds__(kThreads, 4) gemv_vec_kernel(const float *x, const WT *w, float *y, int K, size_t N) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float red[kWarps];
+    constexpr int VEC = 16 / sizeof(WT), kRows = kWarps / WPR;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = warp % WPR;
+    const int nv = K / VEC, per = (nv + WPR - 1) / WPR, v0 = min(nv, part * per), vn = min(nv - v0, per);
+    const size_t row0 = (size_t)blockIdx.x * kRows + warp / WPR, step = (size_t)gridDim.x * kRows;
+    auto at = [&](size_t r) { return reinterpret_cast<const uint4 *>(w + r * K) + v0; };
+    pdl_launch();
+    if (row0 < N)
+        for (int i = lane * 8; i < min(vn, 512); i += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(at(row0) + i));
+    pdl_wait();
+    uint4 cur[kAhead];
+    if (row0 < N) batch_load<true>(at(row0), 0, vn, lane, cur);
+    if (K % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+#pragma unroll 4
+        for (int k = tid; k < K / 4; k += kThreads) reinterpret_cast<float4 *>(smem)[k] = reinterpret_cast<const float4 *>(x)[k];
+    } else {
+        for (int k = tid; k < K; k += kThreads) smem[k] = x[k];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (size_t base = (size_t)blockIdx.x * kRows; base < N; base += step) {
+        const size_t row = base + warp / WPR;
+        float v = 0.f;
+        if (row < N) v = row_dot_ahead<WT, true>(at(row), smem + v0 * VEC, vn, lane, cur, row + step < N ? at(row + step) : nullptr);
+        v = warp_sum(v);
+        if (WPR > 1) {  // the row's slices meet in its first warp
+            if (lane == 0) red[warp] = v;
+            __syncthreads();
+            v = 0.f;
+#pragma unroll
+            for (int i = 0; i < WPR; ++i) v += red[(warp / WPR) * WPR + i];
+            __syncthreads();
+        }
+        if (lane == 0 && part == 0 && row < N) y[row] = v;
+    }
+}
+
 // gate/up pair: out[m,i] = silu(gate_i . x_m) * (up_i . x_m)  (src/models/llama.rs:59-63,
 // src/layers/activation.rs:143-146: sig = 1/(1+exp(-g)); g*sig).
 template <typename WT, int MB>
@@ -349,14 +397,14 @@ __global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const Ge
 // lie a multiple of eight apart, so all of them are `shift` elements off alignment, and its sums belong `shift` columns further
 // left; a tile is one vector narrower than what a warp reads.
 // Why this split: HBM wants some 45 KB in flight per SM (two or three CTAs of 256 threads with eight 16-byte loads each), in lines
-// of 128 bytes or more; everything behind that is overhead.  [4096,11008] bf16: 21.9 us (4.1 TB/s), against 34.8 us with 108 slices
-// per column, whose sums a second kernel had to read back (10.9 us of it).
+// of 128 bytes or more; everything behind that is overhead: calls overlap like those of gemv_vec_kernel.  [4096,11008] bf16, calls behind one
+// another: 18.4 us (4.9 TB/s; 21.9 without the overlap, 34.8 with 108 slices per column, whose sums a second kernel had to read back).
 constexpr int kKnWarps = 8, kKnUnroll = 8, kKnChunk = 2048, kKnSplits = 8;
 __host__ __device__ constexpr int kn_tile_cols(int lw, int vec, bool whole) { return (whole ? lw : lw - 1) * vec; }
 
 template <typename WT, int LW>
 __global__ void __launch_bounds__(kKnWarps * 32, 3)
-gemv_kn_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *part, float *__restrict__ y, size_t K, size_t N, size_t k_per_split) {
+gemv_kn_kernel(const float *x, const WT *w, float *part, float *y, size_t K, size_t N, size_t k_per_split) {
     constexpr int VEC = 16 / sizeof(WT), RPW = 32 / LW, ROWS = kKnWarps * RPW;
     static_assert(ROWS % 8 == 0, "a thread's rows share their alignment");
     __shared__ float xs[kKnChunk];
@@ -371,13 +419,17 @@ gemv_kn_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *par
     const size_t first = (k0 + row) * N + c0 - shift + (size_t)sub * VEC;  // of this thread's elements
     auto fetch = [&](size_t kk) {  // row k0 + row + kk
         const size_t at = first + kk * N;
-        if (aligned && at + VEC <= total) return __ldcs(reinterpret_cast<const uint4 *>(w + at));
+        if (aligned && at + VEC <= total) return ld_live_u4(reinterpret_cast<const uint4 *>(w + at));
         uint4 v = make_uint4(0u, 0u, 0u, 0u);  // the last elements of the matrix, or a matrix that starts anywhere
         WT *e = reinterpret_cast<WT *>(&v);
         for (int i = 0; i < VEC; ++i)
             if (at + i < total) e[i] = w[at + i];
         return v;
     };
+    if (active && k0 + row < k1)
+#pragma unroll 1
+        for (int u = 0; u < kKnUnroll && k0 + row + u * ROWS < k1; ++u) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + min(first + (size_t)u * ROWS * N, total - 1)));
+    pdl_wait();
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
@@ -415,6 +467,7 @@ gemv_kn_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *par
             for (int u = 0; u < kKnUnroll; ++u) wv[u] = active && r + u * ROWS < kn ? fetch(kb - k0 + (r - row) + u * ROWS) : zero;
         }
     }
+    pdl_launch();  // (from the start on, the next call's CTAs would take turns with this one's: [4096,32000] bf16 58.2 us instead of 55.8)
 #pragma unroll
     for (int v = 0; v < VEC; v += 4)
         *reinterpret_cast<float4 *>(red + (warp * 32 + lane) * VEC + v) = make_float4(acc[v], acc[v + 1], acc[v + 2], acc[v + 3]);
@@ -520,6 +573,29 @@ int launch_gemv_nk(lumen_ctx *ctx, const GemvArgs &a, cudaStream_t s) {
     }
 }
 
+// y = W x for one vector (see gemv_vec_kernel); false: not a call for it.
+bool gemv_vec_usable(const void *w, lumen_dtype wdt, size_t K) {
+    return K % (wdt == LUMEN_F32 ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && K * 4 <= 100 * 1024;
+}
+int launch_gemv_vec(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype wdt, float *y, size_t K, size_t N, cudaStream_t s) {
+    const size_t smem = K * sizeof(float), row_bytes = K * (wdt == LUMEN_F32 ? 4 : 2), want = (size_t)ctx->num_sms * 4 * kWarps;
+    // warps per row: enough warps for four CTAs per SM, a slice of at least 1 KB each
+    int wpr = 1;
+    while (wpr < 8 && N * wpr * 2 <= want && row_bytes >= 2048u * wpr) wpr *= 2;
+    const int grid = std::min(pick_grid(ctx, N * wpr, smem), ctx->num_sms * 4);
+    const bool pdl = ctx->pdl;
+    ctx->pdl = true;
+    int rc;
+#define LUMEN_VEC(T_, W_) rc = set_smem(ctx, gemv_vec_kernel<T_, W_>, smem); if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_kernel<T_, W_>, grid, kThreads, smem, s, x, static_cast<const T_ *>(w), y, (int)K, N)
+#define LUMEN_VEC_T(T_) do { if (wpr == 8) { LUMEN_VEC(T_, 8); } else if (wpr == 4) { LUMEN_VEC(T_, 4); } else if (wpr == 2) { LUMEN_VEC(T_, 2); } else { LUMEN_VEC(T_, 1); } } while (0)
+    if (wdt == LUMEN_F32) LUMEN_VEC_T(float);
+    else LUMEN_VEC_T(__nv_bfloat16);
+#undef LUMEN_VEC_T
+#undef LUMEN_VEC
+    ctx->pdl = pdl;
+    return rc;
+}
+
 int launch_gemv_gate_up(lumen_ctx *ctx, const float *x, const void *w_gate, const void *w_up, lumen_dtype wdt,
                         float *out, int M, size_t K, size_t I, const float *norm_w, float norm_eps, cudaStream_t s) {
     if (M < 1 || M > 8) return set_error(ctx, LUMEN_ERR_INVALID, "gate_up: M=%d outside 1..8", M);
@@ -584,11 +660,13 @@ int launch_gemv_kn(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype wd
     cfg.gridDim = dim3(p.col_blocks, p.splits);
     cfg.blockDim = dim3(kKnWarps * 32);
     cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim = {1, (unsigned)p.splits, 1};
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {1, (unsigned)p.splits, 1};
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
 #define LUMEN_KN(T_, L_) cudaLaunchKernelEx(&cfg, gemv_kn_kernel<T_, L_>, x, static_cast<const T_ *>(w), scratch, y, K, N, p.k_per_split)
     if (wdt == LUMEN_F32) LUMEN_CUDA(ctx, p.lanes == 32 ? LUMEN_KN(float, 32) : p.lanes == 16 ? LUMEN_KN(float, 16) : LUMEN_KN(float, 8));
     else LUMEN_CUDA(ctx, p.lanes == 32 ? LUMEN_KN(__nv_bfloat16, 32) : p.lanes == 16 ? LUMEN_KN(__nv_bfloat16, 16) : LUMEN_KN(__nv_bfloat16, 8));

@@ -15,6 +15,13 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ float4 ld_stream_f4(const float4 *p) { return __ldcs(p); }
 __device__ __forceinline__ uint4 ld_stream_u4(const uint4 *p) { return __ldcs(p); }
 
+// The same for what an earlier kernel may have written: stays behind pdl_wait() (the compiler may move __ldcs).
+__device__ __forceinline__ uint4 ld_live_u4(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
@@ -102,11 +109,12 @@ __device__ __forceinline__ void row_dot(const WT *__restrict__ wrow, const float
 // an earlier kernel still runs) and the next few KB of the row handed to the L2 (not more: all rows of a large matrix at once
 // would push one another out).  n: vectors of the row.
 constexpr int kAhead = 4;  // (registers: more would reduce the CTAs an SM holds)
-__device__ __forceinline__ void batch_load(const uint4 *__restrict__ row, int base, int n, int lane, uint4 (&v)[kAhead]) {
+template <bool LIVE = false>  // LIVE: see ld_live_u4
+__device__ __forceinline__ void batch_load(const uint4 *row, int base, int n, int lane, uint4 (&v)[kAhead]) {
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
         const int i = base + u * 32 + lane;
-        v[u] = i < n ? ld_stream_u4(row + i) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = i < n ? (LIVE ? ld_live_u4(row + i) : ld_stream_u4(row + i)) : make_uint4(0u, 0u, 0u, 0u);
     }
 }
 __device__ __forceinline__ void row_ahead(const uint4 *__restrict__ row, int n, int lane, uint4 (&pre)[kAhead]) {
@@ -134,16 +142,16 @@ __device__ __forceinline__ float vec_dot(uint4 w, const float *x, float acc) {
         return fmaf(bf16_hi(w.w), x1.w, acc);
     }
 }
-template <typename WT>
-__device__ __forceinline__ float row_dot_ahead(const uint4 *__restrict__ row, const float *xs, int n, int lane, uint4 (&cur)[kAhead],
-                                               const uint4 *__restrict__ next_row = nullptr) {  // its first batch is left in cur
+template <typename WT, bool LIVE = false>
+__device__ __forceinline__ float row_dot_ahead(const uint4 *row, const float *xs, int n, int lane, uint4 (&cur)[kAhead],
+                                               const uint4 *next_row = nullptr) {  // its first batch is left in cur
     constexpr int VEC = 16 / sizeof(WT);
     float acc = 0.f;
 #pragma unroll 1
     for (int base = 0; base < n; base += kAhead * 32) {
         uint4 next[kAhead];
-        if (next_row && base + kAhead * 32 >= n) batch_load(next_row, 0, n, lane, next);
-        else batch_load(row, base + kAhead * 32, n, lane, next);
+        if (next_row && base + kAhead * 32 >= n) batch_load<LIVE>(next_row, 0, n, lane, next);
+        else batch_load<LIVE>(row, base + kAhead * 32, n, lane, next);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
             const int i = base + u * 32 + lane;

@@ -142,6 +142,52 @@ def test_gemv_kn_layout_raw_pointers(L, oracle, ctx, k, n, bf16):
     assert np.all(y[:pad] == 12345.0) and np.all(y[-pad:] == 12345.0)
     assert rel_err(y[pad:-pad], oracle.matmul(x[None], w_nk, "f64")[0]) < 2e-6
 
+@pytest.mark.parametrize("k,n", [(4, 1), (8, 9), (2052, 5), (512, 2368), (512, 2369), (1024, 1184), (1032, 1185), (4096, 592), (4096, 593), (8200, 3), (8192, 297)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_gemv_warps_per_row(L, oracle, ctx, k, n, bf16):
+    """[N,K] products on raw pointers on both sides of every change of the warps that share a row, and rows that end inside a warp's step.
+    A lane adds at most K / 32 products one after the other: sqrt(K) roundings of 2^-24 at most in the mean."""
+    k += -k % (8 if bf16 else 4)
+    rng = np.random.default_rng(k + n)
+    x, w = rng.standard_normal(k, dtype=np.float32), rng.standard_normal((n, k), dtype=np.float32)
+    if bf16:
+        w = oracle.round_bf16(w)
+    xt, wt = L.Tensor.from_array_no_grad(x), L.Tensor.from_bf16(w) if bf16 else L.Tensor.from_array_no_grad(w)
+    y = L.Tensor.from_array_no_grad(np.full(n + 64, 777.0, np.float32))
+    L.gemv(ctx, xt.data_ptr, wt.data_ptr, L.BF16 if bf16 else L.F32, False, k, n, y.data_ptr + 128)
+    got = y.data()
+    assert np.all(got[:32] == 777.0) and np.all(got[-32:] == 777.0)
+    want = w.astype(np.float64) @ x
+    assert np.abs(got[32:-32] - want).max() < 4 * 2.0 ** -24 * np.sqrt(k) * np.sqrt((w.astype(np.float64) ** 2 @ x.astype(np.float64) ** 2).max())
+
+
+@pytest.mark.parametrize("kn", [False, True])
+def test_gemv_calls_that_feed_each_other(L, ctx, kn):
+    """A product may start while the one before it still runs: vectors and matrix rows that the one before writes are read after it."""
+    n = 1024
+    rng = np.random.default_rng(17)
+    a, b = (rng.standard_normal((n, n), dtype=np.float32) / np.float32(n ** 0.5) for _ in range(2))
+    x = rng.standard_normal(n, dtype=np.float32)
+
+    def chain(wait):
+        wa, wb = L.Tensor.from_array_no_grad(a), L.Tensor.from_array_no_grad(b)
+        v = [L.Tensor.from_array_no_grad(x), L.Tensor.from_array_no_grad(np.zeros(n, np.float32))]
+        for i in range(60):
+            if i % 3 == 2:  # a row of the matrix that comes next
+                L.gemv(ctx, v[i % 2].data_ptr, wa.data_ptr, L.F32, kn, n, n, wb.data_ptr + 4 * n * (i % n))
+                if wait:
+                    ctx.synchronize()
+            L.gemv(ctx, v[i % 2].data_ptr, (wa if i % 2 else wb).data_ptr, L.F32, kn, n, n, v[(i + 1) % 2].data_ptr)
+            if wait:
+                ctx.synchronize()
+        return v[0].data()
+
+    want = chain(True)
+    assert np.isfinite(want).all() and np.abs(want).max() > 0
+    for _ in range(3):
+        assert np.array_equal(chain(False), want)
+
+
 
 @pytest.mark.parametrize("k,n", [(1, 1), (7, 9), (64, 8), (65, 130), (256, 127), (300, 33), (511, 2049), (2049, 1031), (4097, 257), (1000, 40000), (70, 99001), (12288, 128)])
 @pytest.mark.parametrize("offset", [0, 1])
