@@ -551,7 +551,7 @@ bool mega_usable(lumen_llama *m, size_t b, size_t s) {
     const int T = m->ctx->tp_size;
     if (T != 1 && T != 2 && T != 4 && T != 8) return false;
     MegaParams p{};
-    p.H = (int)m->H; p.I = (int)m->inter_l; p.qd = (int)m->qd_l; p.D = (int)m->D;
+    p.H = (int)m->H; p.I = (int)m->inter_l; p.V = (int)m->vocab_l; p.qd = (int)m->qd_l; p.D = (int)m->D;
     p.qkv_rows = (int)m->qkv_rows; p.kvd = (int)m->kvd_l;
     p.wbf16 = m->cfg.weight_dtype == LUMEN_BF16;
     char why[128];

@@ -21,8 +21,11 @@
 // The only CTA-wide barrier is at the end of a row block, where the partial sums of a row are added, the
 // fused epilogue runs (1/rms, residual add, SiLU*mul) and the results are published.  Phases of a layer:
 // qkv | attention | o_proj(+residual) | gate/up(+SiLU*mul) | down(+residual).
-// The arithmetic on tiles that already sit in shared memory is what the token's time is made of (measured
-// with the copies switched off), so the kernel is kept free of register spills: with the L1 squeezed by
+// With the copies switched off a token still takes two thirds of its time: the exchanges, and the code between them, which runs once
+// per phase at some four cycles an instruction (time stamps of a phase, in cycles: 900 to 2400 from the input to the first tile,
+// 1600 to 2300 for that tile, 560 to 1200 for the epilogue).  So what does not depend on the input is settled before the wait for it, words that
+// have arrived are not polled again, and the epilogue is kept short: TinyLlama f32 884 -> 839 us a token, bf16 667 -> 630,
+// Llama-2-7B bf16 2613 -> 2537.  And the kernel is kept free of register spills: with the L1 squeezed by
 // ~220 KB of shared memory a spill reload inside the tile loop is a round trip through L2.
 //
 // Activations cross CTAs through global memory (L2) as tagged words {f32 bits, tag}: a consumer polls
@@ -35,6 +38,7 @@
 // device status word, raises an abort flag that the other CTAs poll, waits (bounded) for its own bulk
 // copies still in flight and returns; the kernel never traps or spins forever.
 #include <algorithm>
+#include <cfloat>
 #include <cstdlib>
 
 #include "attn_decode.cuh"
@@ -254,6 +258,9 @@ __host__ __device__ __forceinline__ Phase get_phase(const MegaParams &p, const M
     return g;
 }
 
+// CTA c's rows of n: [row_share(n, c), row_share(n, c + 1)).  (32 bits: a division is a long stretch of instructions.)
+__host__ __device__ __forceinline__ int row_share(int n, int cta, int nctas) { return (int)((unsigned)n * (unsigned)cta / (unsigned)nctas); }
+
 // The CTA's tiles of one phase, in the order both the producer and the consumers walk them.
 // A tile is up to R rows (4, or 8 for very short rows) x one segment of the row length.  Rows longer than a
 // quarter of a ring stage are cut into nseg = 2 or 4 segments of whole steps (a step = 32 consecutive 16-byte
@@ -262,14 +269,14 @@ __host__ __device__ __forceinline__ Phase get_phase(const MegaParams &p, const M
 // stage.  Tile t of the phase = (chunk of R rows, matrix, segment): t = (chunk * nmat + mat) * nseg + seg.
 // The partial row sums of the segments of a row land in different columns of the row-sum table.
 struct PhaseTiles {
-    long r0, r1;  // the CTA's rows of the matrix (or matrices)
+    int r0, r1;  // the CTA's rows of the matrix (or matrices)
     int nmat, R, nseg, per, njl, rowbytes, nrows, chunks;
     __host__ __device__ PhaseTiles(const Phase &g, int esz, int stage_bytes, int cta, int nctas) {
         rowbytes = g.K * esz;
         nmat = g.nmat;
-        r0 = (long)g.N * cta / nctas;
-        r1 = (long)g.N * (cta + 1) / nctas;
-        nrows = (int)(r1 - r0);
+        r0 = row_share(g.N, cta, nctas);
+        r1 = row_share(g.N, cta + 1, nctas);
+        nrows = r1 - r0;
         njl = (rowbytes / 16 + 31) / 32;  // steps of a lane through a whole row
         // Four whole rows per stage where they fit; otherwise four rows x segments of stage_bytes / 4 bytes each (a
         // whole number of blocks of four steps, the unit of the consumers' inner loop).
@@ -535,13 +542,18 @@ __device__ __forceinline__ void poll_vector_pass(const MegaParams &p, Shared &sh
     const long long t0 = clock64();
     int spins = 0;
     bool done = false, alive = true;
+    // Only what is still missing is asked for again: every CTA polls the whole vector, and 148 times 16 to 45 KB a round trip is what the
+    // L2 delivers in that time; words that have arrived need not queue in front of those that have not.
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+        const uint32_t none = base + tid + kConsumers * u < npairs ? ~tag : tag;
+        v[u] = make_uint4(0u, none, 0u, none);
+    }
     while (!done && alive) {
         done = true;
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            const int idx = base + tid + kConsumers * u;
-            v[u] = idx < npairs ? ld_tagged2(s4 + idx) : make_uint4(0u, tag, 0u, tag);
-        }
+        for (int u = 0; u < kBatch; ++u)
+            if (v[u].y != tag || v[u].w != tag) v[u] = ld_tagged2(s4 + base + tid + kConsumers * u);
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) done = done && v[u].y == tag && v[u].w == tag;
         if (!done) alive = poll_continue(p, sh.abort, spins, t0, site, base);
@@ -735,20 +747,26 @@ __device__ __forceinline__ void poll_attention_pass(const MegaParams &p, Shared 
     const long long t0 = clock64();
     int spins = 0;
     bool done = false, alive = true;
+    // (as in poll_vector_pass: what has arrived is not asked for again)
+#pragma unroll
+    for (int b = 0; b < VB; ++b)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const uint32_t none = s < p.nsplit && vbase + tid + kConsumers * b < nv4 ? ~tag : tag;
+            ml[b][s] = make_uint4(0xff800000u, none, 0u, none);  // {max = -inf, sum = 0}
+            c01[b][s] = c23[b][s] = make_uint4(0u, none, 0u, none);
+        }
     while (!done && alive) {
         done = true;
 #pragma unroll
         for (int b = 0; b < VB; ++b) {
-            const int v = vbase + tid + kConsumers * b;
-            const int k0 = v * 4, h = k0 / p.D, e0 = k0 % p.D;
+            const int k0 = (vbase + tid + kConsumers * b) * 4, h = k0 / p.D, e0 = k0 % p.D;
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                const bool oks = s < p.nsplit && v < nv4;
-                const uint4 *rec = reinterpret_cast<const uint4 *>(p.partT + ((size_t)(oks ? h : 0) * p.nsplit + (oks ? s : 0)) * rec_words);
-                const uint4 ok_word = make_uint4(0xff800000u, tag, 0u, tag);  // {max = -inf, sum = 0}
-                ml[b][s] = oks ? ld_tagged2(rec) : ok_word;
-                c01[b][s] = oks ? ld_tagged2(rec + 1 + e0 / 2) : make_uint4(0u, tag, 0u, tag);
-                c23[b][s] = oks ? ld_tagged2(rec + 2 + e0 / 2) : make_uint4(0u, tag, 0u, tag);
+                const uint4 *rec = reinterpret_cast<const uint4 *>(p.partT + ((size_t)h * p.nsplit + s) * rec_words);
+                if (ml[b][s].y != tag || ml[b][s].w != tag) ml[b][s] = ld_tagged2(rec);
+                if (c01[b][s].y != tag || c01[b][s].w != tag) c01[b][s] = ld_tagged2(rec + 1 + e0 / 2);
+                if (c23[b][s].y != tag || c23[b][s].w != tag) c23[b][s] = ld_tagged2(rec + 2 + e0 / 2);
             }
         }
 #pragma unroll
@@ -932,12 +950,27 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
     else if (g.kind == PH_GATEUP) so.gains = lw->norm2;
     else if (g.kind == PH_LMHEAD) so.gains = p.final_norm;
     const bool normed = so.gains != nullptr;
-    const long r0h = (long)p.H * cta / nctas, r1h = (long)p.H * (cta + 1) / nctas;
+    const int r0h = row_share(p.H, cta, nctas), r1h = row_share(p.H, cta + 1, nctas);
     if (stages_x) {
         so.xraw = sh.xraw;
-        so.r0 = (int)r0h;
-        so.r1 = (int)r1h;
+        so.r0 = r0h;
+        so.r1 = r1h;
     }
+    // The next RMSNorm's gains are read by every CTA at once, at the start of its phase: they should be in the L2 by then
+    // (from HBM, behind the stream of weights, they held up the 4096 numbers of the 7B shape by 8 us in every second phase).
+    if (stages_x && tid == 0) {
+        const float *next = g.kind == PH_QKV ? lw->norm2 : g.layer + 1 < p.L ? p.layers[g.layer + 1].norm1 : p.final_norm;
+        for (int k = cta * 32; k < p.H; k += nctas * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(next + k));
+    }
+    // This warp's first tile, its coordinates and ring position (carried along from tile to tile, no divisions in the loop).  All of
+    // this is settled before the wait for the input: code that runs once costs some four cycles an instruction, and what stands
+    // between the input and the first tile is paid in every phase by every CTA.
+    const int nmat = ti.nmat, nseg = ti.nseg, tpc = nmat * nseg;  // tpc: tiles per chunk of rows
+    int t = warp, chunk = t / tpc, mat = (t - chunk * tpc) / nseg, seg = t - chunk * tpc - mat * nseg;
+    uint32_t slot = rp.n + (uint32_t)t, use = slot / (uint32_t)sh.S;
+    int rs = (int)(slot - use * (uint32_t)sh.S);
+    float inv_k = __frcp_rn((float)g.K);
+    asm volatile("" : "+r"(t), "+r"(chunk), "+r"(mat), "+r"(seg), "+r"(slot), "+r"(use), "+r"(rs), "+f"(inv_k));
     const int njl4 = (njl + 3) & ~3;  // the inner loop takes four steps at a time
     for (int k = g.K + tid; k < njl4 * 32 * XPV; k += kConsumers) xs[k] = 0.f;  // zero padding up to whole blocks of steps
     if (g.kind == PH_QKV && g.layer == 0) {
@@ -957,20 +990,10 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
         else if (g.kind == PH_DOWN) ok = poll_vector(p, sh, p.actT, g.K, tag, xs, tid, bk, 330 + g.kind);
         else if (p.tp_size == 1) ok = poll_vector(p, sh, xsrc, g.K, tag, xs, tid, bk, 330 + g.kind, so);
         else if (p.xrT)
-            ok = reduce_then_poll_x(p, sh, xsrc, p.xrT + (size_t)(g.kind == PH_GATEUP ? 0 : 1) * p.x_slot_words, g.K, tag, xs, tid, bk, (int)r0h,
-                                    (int)r1h, so);
+            ok = reduce_then_poll_x(p, sh, xsrc, p.xrT + (size_t)(g.kind == PH_GATEUP ? 0 : 1) * p.x_slot_words, g.K, tag, xs, tid, bk, r0h, r1h, so);
         else ok = poll_x_sum(p, sh, xsrc, g.K, tag, xs, tid, bk, so);
         if (!ok) return false;
         if (p.trace && cta == 0 && tid == 0) p.trace[4 * (5 * p.L + 1) + 1 + ph] = globaltimer_ns();
-    }
-    // RMSNorm::forward (rms_norm.rs:49-56): rms = sqrt(ss/dim + eps), inv = 1/rms.  The vector in shared memory
-    // carries the gains; inv multiplies the row sums in the epilogue.
-    float inv = 1.f;
-    if (normed) {
-        float tot = 0.f;
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) tot += sh.red[w];
-        inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(tot, (float)g.K), p.eps)));
     }
     if (stages_x || owes_sums) {
         // keep this thread's row of the residual stream (all ranks' partial sums added, before the gains)
@@ -983,37 +1006,22 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
     }
     trace_stamp(p, cta, tid, 3 * ph + 1);
     trace_cta(p, cta, tid, 0, ph);
-    // The next RMSNorm's gains are read by every CTA at once, at the start of its phase: they should be in the L2 by then
-    // (from HBM, behind the stream of weights, they held up the 4096 numbers of the 7B shape by 8 us in every second phase).
-    if (stages_x && tid == 0) {
-        const float *next = g.kind == PH_QKV ? lw->norm2 : g.layer + 1 < p.L ? p.layers[g.layer + 1].norm1 : p.final_norm;
-        for (int k = cta * 32; k < p.H; k += nctas * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(next + k));
-    }
-
     // ---- tiles ------------------------------------------------------------------------------------------
     // Tiles are addressed in closed form (see PhaseTiles) and sit in ring slot (tiles consumed so far + t).
-    // Warp w owns tiles w, w + 4, ...  Rows are reduced and published in blocks of at most kRowBlock (a block
+    // Warp w owns tiles w, w + 7, ...  Rows are reduced and published in blocks of at most kRowBlock (a block
     // never splits a chunk of rows).
     constexpr int XQ = VecTraits<WT>::XQ;
-    const int R = ti.R, nmat = ti.nmat, nseg = ti.nseg;
+    const int R = ti.R;
     const int nrows_cta = ti.nrows;
     const int chunks = ((p.debug_flags & 1) && !(p.debug_flags & 16)) ? 0 : ti.chunks;
     const bool dry = (p.debug_flags & 16) != 0;  // debug: no copies are issued (bit 0); run the arithmetic on whatever the ring holds
     const int chunks_per_block = kRowBlock / R;
-    const int tpc = nmat * nseg;  // tiles per chunk of rows
     // rows of a segment tile that came as a box sit a whole segment slot apart (the box is zero-filled past the row end)
     const bool boxed = nseg > 1 && p.tmaps != nullptr;
     for (int cb = 0; cb < chunks; cb += chunks_per_block) {
         const int cend = min(chunks, cb + chunks_per_block);
-        const int t0 = cb * tpc, t1 = cend * tpc;
+        const int t1 = cend * tpc;
         const int row0_blk = cb * R;  // first row of the block, relative to the CTA's first row
-        // Warp w owns tiles w, w + W, ... of the phase.  The tile's coordinates and its ring position are carried
-        // along incrementally (no divisions in the loop).
-        int t = t0 + (warp + kConsumerWarps - t0 % kConsumerWarps) % kConsumerWarps;
-        int chunk = t / tpc, mat = (t - chunk * tpc) / nseg, seg = t - chunk * tpc - mat * nseg;
-        uint32_t slot = rp.n + (uint32_t)t;
-        int rs = (int)(slot % (uint32_t)sh.S);
-        uint32_t use = slot / (uint32_t)sh.S;
         for (; t < t1; t += kConsumerWarps) {
             const int rrel = chunk * R;
             const int nr = min(R, nrows_cta - rrel);
@@ -1047,14 +1055,30 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
         }
         // End of a row block: add the warps' partial sums, run the epilogue and publish.
         const int nrows = min(cend * R, nrows_cta) - row0_blk;
+        // RMSNorm::forward (rms_norm.rs:49-56): inv = 1 / sqrt(ss / dim + eps).  The vector in shared memory carries the gains; inv
+        // multiplies the row sums.  One Newton step takes the reciprocal root to the last bit or the one before.
+        float inv = 1.f;
+        if (normed) {
+            float ss = 0.f;
+#pragma unroll
+            for (int w = 0; w < kConsumerWarps; ++w) ss += sh.red[w];
+            const float a = fmaf(ss, inv_k, p.eps), y = rsqrtf(a);
+            inv = a > FLT_MAX ? 0.f : fmaf(0.5f * y, fmaf(-a * y, y, 1.0f), y);  // (a sum that overflows: 1 / infinity)
+        }
         if (!consumer_bar_ok(sh.abort, sh.decision, tid, bk)) return false;
         if (tid < nrows) {
             // the segments of the row, added in order
-            const float *pr = sh.part + (size_t)tid * kPartCols;
-            float acc = pr[0];
-            for (int c = 1; c < nseg; ++c) acc += pr[c];
-            const float tot = __fmul_rn(acc, inv);
-            const long row = ti.r0 + row0_blk + tid;
+            auto row_sum = [&](const float *pr) {
+                const float4 a = *reinterpret_cast<const float4 *>(pr), b = *reinterpret_cast<const float4 *>(pr + 4);
+                const float c[kPartCols] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                float v = c[0];
+#pragma unroll
+                for (int i = 1; i < kPartCols; ++i)
+                    if (i < nseg) v += c[i];
+                return v;
+            };
+            const float tot = __fmul_rn(row_sum(sh.part + tid * kPartCols), inv);
+            const int row = ti.r0 + row0_blk + tid;
             const uint32_t tag = phase_tag(p, ph);
             switch (g.kind) {
                 case PH_QKV:
@@ -1076,11 +1100,8 @@ __device__ __forceinline__ bool gemv_phase(const MegaParams &p, Shared &sh, cons
                     break;
                 }
                 case PH_GATEUP: {  // SiLU (activation.rs:143-146) then gate_act * up (llama.rs:61-63)
-                    const float *pu = sh.part + ((size_t)kRowBlock + tid) * kPartCols;
-                    float accu = pu[0];
-                    for (int c = 1; c < nseg; ++c) accu += pu[c];
-                    const float up = __fmul_rn(accu, inv);
-                    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-tot)));
+                    const float up = __fmul_rn(row_sum(sh.part + (kRowBlock + tid) * kPartCols), inv);
+                    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-tot)));
                     st_tagged(p.actT + row, __fmul_rn(__fmul_rn(tot, sig), up), tag);
                     break;
                 }
@@ -1591,6 +1612,10 @@ int decode_mega_supported(const MegaParams &p, char *why, size_t why_len) {
     }
     if (p.D > 128 || (p.D % 4)) {
         snprintf(why, why_len, "head_dim %d is not a multiple of 4 up to 128", p.D);
+        return 0;
+    }
+    if (p.V > 1 << 24 || p.I > 1 << 24) {
+        snprintf(why, why_len, "more than %d rows", 1 << 24);
         return 0;
     }
     if (p.qkv_rows % 2 || p.qd % 4 || p.kvd % 2) {
