@@ -556,7 +556,8 @@ int lumen_decoder::step_row(lumen_kv_cache **caches) {
     int cur = 0;
     Pending pend;
     // y = w . x, where x is the residual after the pending output (which is thereby settled), normed with norm_w if given
-    auto from_residual = [&](const void *w, size_t N, float *out, StepFinish::Kind act, size_t layer, const float *norm_w = nullptr) -> int {
+    auto from_residual = [&](const void *w, size_t N, float *out, StepFinish::Kind act, size_t layer, const float *norm_w = nullptr,
+                             lumen_kv_cache **end_of = nullptr) -> int {
         GemvStepArgs g;
         g.res = ws.x[cur]; g.eps = cfg.norm_eps; g.w = w; g.wdt = dt; g.K = W; g.N = N; g.out = out; g.act = act; g.norm_w = norm_w;
         if (pend.y) {
@@ -566,6 +567,9 @@ int lumen_decoder::step_row(lumen_kv_cache **caches) {
         }
         if (act == StepFinish::kSideGate) {
             g.ids = ws.ids; g.table = side_embed + layer * cfg.side_dim * esz; g.table_ld = L * cfg.side_dim; g.table_rows = V;
+        }
+        if (end_of) {
+            g.ids = ws.ids; g.d_lens = end_of[0]->d_len; g.last_tok = end_of[0]->last_tok; g.layers = (int)L;
         }
         return launch_gemv_step(ctx, g, s);
     };
@@ -616,8 +620,7 @@ int lumen_decoder::step_row(lumen_kv_cache **caches) {
             LUMEN_TRY(plain(ws.side.f, w.side_proj, cfg.side_dim, w.side_norm));
         }
     }
-    LUMEN_TRY(from_residual(head, V, ws.logits, StepFinish::kStore, 0, final_gain));
-    return launch_advance(ctx, caches[0]->d_len, L, ws.ids, caches[0]->last_tok, 1, 1, s);
+    return from_residual(head, V, ws.logits, StepFinish::kStore, 0, final_gain, caches);
 }
 
 // c = a . w^T, then `fin` (null: c is the result).  `pair`: multiply the hi/lo pair of the activations instead of hi alone.

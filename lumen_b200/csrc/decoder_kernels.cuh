@@ -99,6 +99,9 @@ struct GemvStepArgs {
     const float *ids = nullptr;
     const void *table = nullptr;
     size_t table_ld = 0, table_rows = 0;
+    // the last product of a step also ends it (launch_advance of one row): nothing behind it in the step reads these
+    int *d_lens = nullptr, *last_tok = nullptr;
+    int layers = 0;
 };
 int launch_gemv_step(lumen_ctx *ctx, const GemvStepArgs &a, cudaStream_t s);
 

@@ -121,6 +121,14 @@ def test_attention_alone(L, dtype, a):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [2048, 2052])
+def test_widest_rows_with_gains_in_shared_memory(L, dtype, width):
+    """One-row products keep the gains of both norms in shared memory up to 2048 numbers and read them when they need them beyond."""
+    cfg = K.config([(K.attn(heads=2, kv_heads=1, dim=16, vdim=16, chunk=100, rot_dims=8, scaling=None, scale=0.3), 24)], width=width)
+    _check(L, cfg, K.weights(L, cfg, 16), _ids(9, 16), ([1], [4, 1]), dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("scaling", [dict(factor=8.0, low=1.0, high=4.0, original=256), dict(factor=2.0, low=3.0, high=9.0, original=1000), None])
 def test_frequency_scaling(L, dtype, scaling):
     """Large queries and keys, so that angles decide; every pair of the three ranges of wavelengths is there."""
