@@ -227,7 +227,7 @@ struct GroupedArgs {
     __nv_bfloat16 *out_hi = nullptr, *out_lo = nullptr;
 };
 constexpr size_t kGroupedMaxDim = 512;
-int grouped_pick_splits(const GroupedArgs &a, int num_sms);
+int grouped_pick_splits(const GroupedArgs &a, int num_sms);  // 0: no pieces to merge, all in one launch
 // Keys (normed, rotated) and values -> cache, for layers with keys and values of their own; with q also the queries
 // (normed, rotated) as bf16 [B, H, s_pad, width].
 int launch_grouped_append(lumen_ctx *ctx, const GroupedArgs &a, __nv_bfloat16 *q, size_t s_pad, size_t width, cudaStream_t s);

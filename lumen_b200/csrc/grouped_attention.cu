@@ -422,6 +422,7 @@ int group_of(const GroupedArgs &a) {  // query heads a CTA takes
 // As many CTAs as the device holds, pieces that give every warp something, partial results within the workspace (see
 // ensure_workspace).
 int grouped_pick_splits(const GroupedArgs &a, int num_sms) {
+    if (grouped_one_usable(a)) return 0;
     const bool mma = grouped_mma_usable(a);
     const size_t rows = a.B * a.S, r = a.H / a.G, items = rows * a.G * (mma ? (r + kMmaHeads - 1) / kMmaHeads : r / group_of(a));
     const size_t total = a.past + a.S, len = a.chunk ? std::min(total, a.chunk) : total, piece = mma ? 128 : 64;
@@ -457,7 +458,7 @@ int launch_grouped_attention(lumen_ctx *ctx, const GroupedArgs &a, bool append, 
         case 2: rc = f32 ? launch_rows_g<float, 2>(ctx, a, append, s) : launch_rows_g<__nv_bfloat16, 2>(ctx, a, append, s); break;
         default: rc = f32 ? launch_rows_g<float, 1>(ctx, a, append, s) : launch_rows_g<__nv_bfloat16, 1>(ctx, a, append, s); break;
     }
-    if (rc != LUMEN_OK) return rc;
+    if (rc != LUMEN_OK || a.nsplit == 0) return rc;
     return launch_pdl(ctx, grouped_merge_kernel, dim3((unsigned)a.H, (unsigned)std::min<size_t>(a.B * a.S, 65535)), kMergeThreads, 0, s, a);
 }
 

@@ -11,6 +11,7 @@ constexpr int kMmaHeads = 8;   // query heads a CTA of the MMA kernel takes
 
 // The one-row kernel on the tensor cores (bf16 cache): one CTA per (piece, key head and up to kMmaHeads of its query heads, row).
 bool grouped_mma_usable(const GroupedArgs &a);
+bool grouped_one_usable(const GroupedArgs &a);  // one row, attention and merge in one launch (nsplit == 0)
 int launch_grouped_mma(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s);
 
 __device__ __forceinline__ int chunk_start(int pos, size_t chunk) { return chunk ? (int)((size_t)pos / chunk * chunk) : 0; }

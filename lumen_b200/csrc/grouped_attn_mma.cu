@@ -7,7 +7,13 @@
 //   O^T [values, 8 heads] += V^T P^T: a lane loads 16 bytes (8 values) of four rows; bytes of two rows are paired into the operands
 //                               of one MMA per value of the eight, P^T comes from the scores by 8 x 8 transposes
 // so that no tile passes through shared memory.  The weights P enter as a bf16 hi + lo pair.
+//
+// ONE: the one row of a step.  The pieces of its context are the CTAs of a cluster, which hand one another their sums: sink, gate and
+// the division follow in the same launch, each CTA for its share of the output (a merge of its own was one launch of six in an
+// attention layer's step, 6 us by itself).  Eight pieces, up to kOneRows cached rows.
 #include <algorithm>
+
+#include <cooperative_groups.h>
 
 #include "grouped_attention.cuh"
 #include "mma_common.cuh"
@@ -19,10 +25,12 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kTileRows = 16, kStep = kWarps * kTileRows;
+constexpr int kOnePieces = 8;       // ONE
+constexpr size_t kOneRows = 4096;   // (four steps of a CTA; beyond, as many pieces as there are SMs pay for the merge)
 
 // KB: blocks of 32 numbers of a key; VB: blocks of 64 numbers of a value.
-// grid (pieces, G * groups of kMmaHeads query heads, rows)
-template <int KB, int VB>
+// grid (pieces, G * groups of kMmaHeads query heads, rows); ONE: clusters of (pieces, 1, 1), one row
+template <int KB, int VB, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedArgs a, int append) {
     extern __shared__ __align__(16) float smem[];
     const int dim = (int)a.dim, vdim = (int)a.vdim, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -33,14 +41,17 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedA
     const int R = (int)(a.H / a.G), groups = (R + kMmaHeads - 1) / kMmaHeads, hk = (int)blockIdx.y / groups, first = ((int)blockIdx.y % groups) * kMmaHeads;
     const int heads = min(kMmaHeads, R - first), h0 = hk * R + first;
     const float scale2 = a.scale * 1.4426950408889634f;  // weights are powers of two: exp(s scale - m) = 2^(s scale log2(e) - m')
+    namespace cg = cooperative_groups;
+    const int pieces = ONE ? kOnePieces : a.nsplit;
+    if (ONE) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // (this CTA runs: the others may write to its shared memory)
     pdl_launch();
     bool ahead = append;  // (the cached rows of a layer that appends are older than this step, see grouped_rows_kernel)
     if (!ahead) pdl_wait();
     for (size_t m = blockIdx.z; m < a.B * a.S; m += gridDim.z) {
         const size_t b = m / a.S;
         const int pos = *a.d_len + (int)(m - b * a.S), lo = chunk_start(pos, a.chunk), len = pos + 1 - lo;
-        const int per = piece_rows(len, a.nsplit), j0 = lo + (int)blockIdx.x * per, j1 = min(pos + 1, j0 + per);
-        if (j0 >= j1) {  // (the same for the whole CTA)
+        const int per = piece_rows(len, pieces), j0 = lo + (int)blockIdx.x * per, j1 = min(pos + 1, j0 + per);
+        if (!ONE && j0 >= j1) {  // (the same for the whole CTA)
             if (ahead) pdl_wait();
             ahead = false;
             continue;
@@ -80,7 +91,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedA
         const float *cos_row = a.cos_t + pos * half, *sin_row = a.sin_t + pos * half;
         if (warp < heads) head_norm_rotate(buf, u + (size_t)(h0 + warp) * dim, dim, a.q_gain, a.eps, (int)a.rot_dims, cos_row, sin_row, lane);
         for (int e = lane; e < KB * 32; e += 32) qs[warp][e] = __float2bfloat16_rn(warp < heads && e < dim ? buf[e] : 0.f);
-        if (append && j1 == pos + 1 && warp == kWarps - 1) {
+        if (append && j1 == pos + 1 && j0 < j1 && warp == kWarps - 1) {
             // every group of query heads writes the row that it reads below (the same numbers)
             __syncwarp();
             head_norm_rotate(buf, u + a.u_k + (size_t)hk * dim, dim, a.k_gain, a.eps, (int)a.rot_dims, cos_row, sin_row, lane);
@@ -167,6 +178,13 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedA
                     if (vb * 64 + 8 * g + e < vdim) wctx[(warp * kMmaHeads + 2 * t + c) * vdim + vb * 64 + 8 * g + e] = o[e][2 * vb + c];
         }
         __syncthreads();
+        cg::cluster_group cluster = cg::this_cluster();
+        const int mine = (int)blockIdx.x, n_out = heads * vdim, slice = (n_out + kOnePieces - 1) / kOnePieces;  // ONE: outputs of a CTA
+        float *got = wctx + kWarps * kMmaHeads * vdim, *got_m = got + kOnePieces * slice, *got_l = got_m + kOnePieces * kMmaHeads;
+        if (ONE) {
+            __syncwarp();
+            asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        }
         for (int i = tid; i < heads * vdim; i += kThreads) {
             const int hd = i / vdim, e = i - hd * vdim;
             float M = -INFINITY, L = 0.f, c = 0.f;
@@ -174,16 +192,50 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedA
             for (int w = 0; w < kWarps; ++w) M = fmaxf(M, wm[w * kMmaHeads + hd]);
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) {
-                const float f = tc::ex2(wm[w * kMmaHeads + hd] - M);  // (a warp without tiles: 2^-inf = 0)
+                // (a warp without tiles: 2^-inf = 0; ONE: so is a piece without rows)
+                const float f = tc::ex2(wm[w * kMmaHeads + hd] - (ONE && M == -INFINITY ? 0.f : M));
                 L = fmaf(wl[w * kMmaHeads + hd], f, L);
                 c = fmaf(wctx[(w * kMmaHeads + hd) * vdim + e], f, c);
             }
-            const size_t row = (m * a.H + h0 + hd) * a.nsplit + blockIdx.x;
-            a.part_ctx[row * vdim + e] = c;
-            if (e == 0) {
-                a.part_ml[row * 2] = M * 0.6931471805599453f;
-                a.part_ml[row * 2 + 1] = L;
+            if constexpr (ONE) {
+                const int to = i / slice;
+                *cluster.map_shared_rank(got + mine * slice + (i - to * slice), to) = c;
+                if (e < kOnePieces) {
+                    *cluster.map_shared_rank(got_m + mine * kMmaHeads + hd, e) = M;
+                    *cluster.map_shared_rank(got_l + mine * kMmaHeads + hd, e) = L;
+                }
+            } else {
+                const size_t row = (m * a.H + h0 + hd) * a.nsplit + blockIdx.x;
+                a.part_ctx[row * vdim + e] = c;
+                if (e == 0) {
+                    a.part_ml[row * 2] = M * 0.6931471805599453f;
+                    a.part_ml[row * 2 + 1] = L;
+                }
             }
+        }
+        if constexpr (ONE) {
+            static_assert(kMmaHeads * 128 / kOnePieces <= kThreads, "an output per thread");
+            const int i = mine * slice + tid, hd = i / vdim, e = i - hd * vdim;
+            const bool has = tid < slice && i < n_out;
+            const float sink = has ? a.sink[h0 + hd] * 1.4426950408889634f : 0.f, gate = has ? u[a.u_gate + h0 + hd] : 0.f;  // (maxima are in powers of two)
+            cluster.sync();
+            if (has) {
+                float M = sink, c = 0.f;
+#pragma unroll
+                for (int q = 0; q < kOnePieces; ++q) M = fmaxf(M, got_m[q * kMmaHeads + hd]);
+                float L = exp2f(sink - M);
+#pragma unroll
+                for (int q = 0; q < kOnePieces; ++q) {
+                    const float f = exp2f(got_m[q * kMmaHeads + hd] - M);  // (a piece without rows: 2^-inf = 0)
+                    L = fmaf(got_l[q * kMmaHeads + hd], f, L);
+                    c = fmaf(got[q * slice + tid], f, c);
+                }
+                c *= __fdiv_rn(sigmoid_f(gate), L);
+                const size_t at = (size_t)(h0 + hd) * vdim + e;
+                if (a.out) a.out[at] = c;
+                if (a.out_hi) store_split(c, a.out_hi, a.out_lo, at);
+            }
+            return;
         }
         __syncthreads();
     }
@@ -191,11 +243,16 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_mma_kernel(const GroupedA
 
 template <int KB, int VB>
 int launch(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s) {
-    const size_t smem = (kWarps * a.dim + 2 * kWarps * kMmaHeads + (size_t)kWarps * kMmaHeads * a.vdim) * sizeof(float);
-    if (smem > 40 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_mma_kernel<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const size_t r = a.H / a.G, groups = (r + kMmaHeads - 1) / kMmaHeads;
+    size_t smem = (kWarps * a.dim + 2 * kWarps * kMmaHeads + (size_t)kWarps * kMmaHeads * a.vdim) * sizeof(float);
+    if (a.nsplit == 0) {
+        smem += (kMmaHeads * a.vdim + kOnePieces + 2 * kOnePieces * kMmaHeads) * sizeof(float);
+        if (smem > 40 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_mma_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return launch_pdl_cluster(ctx, grouped_mma_kernel<KB, VB, true>, kOnePieces, dim3(kOnePieces, (unsigned)(a.G * groups)), dim3(kThreads), smem, s, a, append ? 1 : 0);
+    }
+    if (smem > 40 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_mma_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((unsigned)a.nsplit, (unsigned)(a.G * groups), (unsigned)std::min<size_t>(a.B * a.S, 65535));
-    return launch_pdl(ctx, grouped_mma_kernel<KB, VB>, grid, kThreads, smem, s, a, append ? 1 : 0);
+    return launch_pdl(ctx, grouped_mma_kernel<KB, VB, false>, grid, kThreads, smem, s, a, append ? 1 : 0);
 }
 
 }  // namespace
@@ -203,6 +260,11 @@ int launch(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s) {
 // Heads of at most 128 numbers in whole 16-byte pieces.
 bool grouped_mma_usable(const GroupedArgs &a) {
     return a.dt == LUMEN_BF16 && a.dim <= 128 && a.vdim <= 128 && a.dim % 8 == 0 && a.vdim % 8 == 0;
+}
+
+bool grouped_one_usable(const GroupedArgs &a) {
+    const size_t total = a.past + a.S;
+    return a.B * a.S == 1 && grouped_mma_usable(a) && (a.chunk ? std::min(total, a.chunk) : total) <= kOneRows;
 }
 
 int launch_grouped_mma(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s) {

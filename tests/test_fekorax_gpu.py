@@ -128,6 +128,12 @@ def test_widest_rows_with_gains_in_shared_memory(L, dtype, width):
     _check(L, cfg, K.weights(L, cfg, 16), _ids(9, 16), ([1], [4, 1]), dtype)
 
 
+def test_steps_across_the_length_of_one_launch(L):
+    """Eight pieces that hand one another their sums up to 4096 rows, more pieces and a merge beyond; sizes that leave the last shares short."""
+    cfg = K.config([(K.attn(heads=5, kv_heads=1, dim=24, vdim=40, chunk=6000, rot_dims=8, scaling=None, scale=0.1), None)])
+    _check(L, cfg, K.weights(L, cfg, 15), _ids(4101, 15), ([4091] + [1] * 10,), "bf16")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("scaling", [dict(factor=8.0, low=1.0, high=4.0, original=256), dict(factor=2.0, low=3.0, high=9.0, original=1000), None])
 def test_frequency_scaling(L, dtype, scaling):
