@@ -49,7 +49,6 @@ __device__ __forceinline__ void head_norm_rope(float *buf, int D, const float *n
 // then normalises (optional) and rotates it into shared memory `buf[D]`.  Same arithmetic as
 // head_norm_rope; the loads are issued before anything depends on them so the whole step costs one
 // memory round trip.  Called by one warp.
-template <bool LOCAL = false>
 __device__ __forceinline__ void load_norm_rope(float *buf, const float *src, int D, const float *norm_w, float eps,
                                                const float *cos_row, const float *sin_row, int lane) {
     const int half = D / 2;
@@ -57,7 +56,7 @@ __device__ __forceinline__ void load_norm_rope(float *buf, const float *src, int
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
         const int i = lane + 32 * t;
-        v[t] = (i < D) ? (LOCAL ? src[i] : __ldcg(src + i)) : 0.f;  // LOCAL: src is already in shared memory
+        v[t] = (i < D) ? __ldcg(src + i) : 0.f;
         nw[t] = (norm_w && i < D) ? __ldg(norm_w + i) : 1.f;
     }
 #pragma unroll

@@ -61,7 +61,7 @@ constexpr int kPartCols = kMaxSeg;         // columns of the table of partial ro
 constexpr int kMaxSplit = 4;               // attention splits merged in the o_proj prologue
 constexpr int kKvTileRows = 64;            // cached rows of a K or V tile at most (two scores per lane)
 constexpr long long kWaitCycles = 400000000LL;  // ~0.2 s at 1.9 GHz
-constexpr long long kPrefetchGrace = 1000;      // a ring that has been full for this long is a stall, not back-pressure
+constexpr long long kPrefetchGrace = 300;       // a ring that has been full for this long is a stall, not back-pressure (1000: TinyLlama f32 835 us instead of 831)
 constexpr long long kPrefetchPace = 600;        // cycles between the L2 prefetches of consecutive 16 KB tiles (~54 KB/us)
 
 // Floats of the staged input vector of a phase (up to kmax elements, zero-padded to four whole steps of a
@@ -592,7 +592,7 @@ __device__ __forceinline__ bool poll_vector(const MegaParams &p, Shared &sh, con
     else if (per_thread <= 10) poll_vector_pass<10>(p, sh, s4, npairs, 0, tag, xs, tid, site, o, ss);
     else
         for (int base = 0; base < npairs; base += kConsumers * 13) poll_vector_pass<13>(p, sh, s4, npairs, base, tag, xs, tid, site, o, ss);
-    publish_ss(sh, ss, tid);
+    if (o.gains) publish_ss(sh, ss, tid);  // (a norm follows)
     return consumer_bar_ok(sh.abort, sh.decision, tid, bk);
 }
 
@@ -791,7 +791,7 @@ __device__ __forceinline__ void poll_attention_pass(const MegaParams &p, Shared 
         for (int s = 0; s < NS; ++s) {
             const float ms = __uint_as_float(ml[b][s].x);
             if (ms != -INFINITY) {
-                const float f = expf(ms - M);
+                const float f = NS == 1 ? 1.f : expf(ms - M);
                 L = fmaf(__uint_as_float(ml[b][s].z), f, L);
                 c.x = fmaf(__uint_as_float(c01[b][s].x), f, c.x);
                 c.y = fmaf(__uint_as_float(c01[b][s].z), f, c.y);
@@ -799,7 +799,7 @@ __device__ __forceinline__ void poll_attention_pass(const MegaParams &p, Shared 
                 c.w = fmaf(__uint_as_float(c23[b][s].z), f, c.w);
             }
         }
-        const float inv = __fdiv_rn(1.0f, __fadd_rn(L, 1e-9f));
+        const float inv = __frcp_rn(__fadd_rn(L, 1e-9f));
         reinterpret_cast<float4 *>(xs)[v] =
             make_float4(__fmul_rn(c.x, inv), __fmul_rn(c.y, inv), __fmul_rn(c.z, inv), __fmul_rn(c.w, inv));
     }
@@ -1159,9 +1159,9 @@ __device__ __forceinline__ void stage_qkv(const MegaParams &p, volatile int *abo
     consumer_bar();
 }
 
-// Scratch of an attention item in floats: q and the new k (rotated), q | k | v as they arrived, per-warp maximum, sum and context,
-// per-warp softmax weights of a tile.
-__host__ __device__ inline size_t mega_attn_floats(int D) { return 5 * (size_t)D + 16 + (size_t)kConsumerWarps * D + (size_t)kConsumerWarps * kKvTileRows; }
+// Scratch of an attention item in floats: cos and sin of this token's position (for the whole token), q and the new k (rotated),
+// q | k | v as they arrived, per-warp maximum, sum and context, per-warp softmax weights of a tile.
+__host__ __device__ inline size_t mega_attn_floats(int D) { return 6 * (size_t)D + 16 + (size_t)kConsumerWarps * D + (size_t)kConsumerWarps * kKvTileRows; }
 
 // Waits for the next tile of the ring (position `slot`); the warp that owns the tile calls.
 __device__ __forceinline__ const float *ring_wait(const MegaParams &p, Shared &sh, uint32_t slot, int lane, int site, bool &have) {
@@ -1174,6 +1174,34 @@ __device__ __forceinline__ const float *ring_wait(const MegaParams &p, Shared &s
 __device__ __forceinline__ void ring_release(Shared &sh, uint32_t slot, int lane) {
     __syncwarp();
     if (lane == 0) mbar_arrive_cnt(&sh.empty[slot % (uint32_t)sh.S], 1);
+}
+
+// RMSNorm (gains in g, where there are any) and rotation of one head vector, shared memory to shared memory; a lane has pairs of elements.
+template <int VE>
+__device__ __forceinline__ void norm_rotate(float *dst, const float *src, int half, const float (&g)[VE], bool normed, float eps, const float *cos_row,
+                                            const float *sin_row, int lane) {
+    float lo[VE / 2], hi[VE / 2], inv = 1.f, ss = 0.f;
+#pragma unroll
+    for (int t = 0; t < VE / 2; ++t) {
+        const int j = lane + 32 * t;
+        lo[t] = j < half ? src[j] : 0.f;
+        hi[t] = j < half ? src[j + half] : 0.f;
+        ss = fmaf(lo[t], lo[t], fmaf(hi[t], hi[t], ss));
+    }
+    if (normed) inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(warp_sum(ss), (float)(2 * half)), eps)));
+#pragma unroll
+    for (int t = 0; t < VE / 2; ++t) {
+        const int j = lane + 32 * t;
+        if (j >= half) continue;
+        if (normed) {
+            lo[t] = __fmul_rn(__fmul_rn(lo[t], inv), g[2 * t]);
+            hi[t] = __fmul_rn(__fmul_rn(hi[t], inv), g[2 * t + 1]);
+        }
+        const float c = cos_row[j], s = sin_row[j];
+        dst[j] = __fsub_rn(__fmul_rn(lo[t], c), __fmul_rn(hi[t], s));
+        dst[j + half] = __fadd_rn(__fmul_rn(hi[t], c), __fmul_rn(lo[t], s));
+    }
+    __syncwarp();
 }
 
 // One attention work item: head h, context split `split` (self_attention.rs:141-297; softmax(q.K^T * scale).V as pieces merged by
@@ -1190,15 +1218,22 @@ __device__ __forceinline__ void attention_item(const MegaParams &p, Shared &sh, 
                                                uint32_t tag, int ph, int tid) {
     const int D = p.D, half = D / 2, lane = tid & 31, warp = tid >> 5, nch = D / 4;
     const int G = p.Hq / p.Hkv, hk = h / G, past = p.past;
-    float *qs = sh.attn, *knew = qs + D, *raw = knew + D, *wm = raw + 3 * D, *wl = wm + 8, *wctx = wl + 8;
+    const float *cos_row = sh.attn, *sin_row = cos_row + half;
+    float *qs = sh.attn + D, *knew = qs + D, *raw = knew + D, *wm = raw + 3 * D, *wl = wm + 8, *wctx = wl + 8;
     float *ws = wctx + kConsumerWarps * D + warp * kKvTileRows;
+    const float *gain = warp == 0 ? l.qn : l.kn;  // of what this warp norms; requested before the wait
+    float g[VE];
+#pragma unroll
+    for (int t = 0; t < VE; ++t) {
+        const int j = lane + 32 * (t / 2);
+        g[t] = gain && j < half ? __ldg(gain + j + (t & 1) * half) : 1.f;
+    }
     stage_qkv(p, sh.abort, raw, h, hk, tid, phase_tag(p, ph - 1));
-    const float *cos_row = p.cos_t + (size_t)past * half, *sin_row = p.sin_t + (size_t)past * half;
     const int total = past + 1, chunk = (total + p.nsplit - 1) / p.nsplit;
     const bool owns_new = past >= split * chunk && past < min(total, (split + 1) * chunk);
-    if (warp == 0) load_norm_rope<true>(qs, raw, D, l.qn, p.eps, cos_row, sin_row, lane);
+    if (warp == 0) norm_rotate<VE>(qs, raw, half, g, gain != nullptr, p.eps, cos_row, sin_row, lane);
     if (owns_new && warp == kConsumerWarps - 1) {
-        load_norm_rope<true>(knew, raw + D, D, l.kn, p.eps, cos_row, sin_row, lane);
+        norm_rotate<VE>(knew, raw + D, half, g, gain != nullptr, p.eps, cos_row, sin_row, lane);
         if (h % G == 0) {  // the first head of a KV head's group stores the row
             float *k_row = l.k_cache + ((size_t)hk * p.max_seq + past) * D, *v_row = l.v_cache + ((size_t)hk * p.max_seq + past) * D;
             for (int i = lane; i < D; i += 32) {
@@ -1290,12 +1325,12 @@ __device__ __forceinline__ void attention_item(const MegaParams &p, Shared &sh, 
         for (int i = 0; i < VE; ++i) wctx[warp * D + e0 + i] = ctx[i];
     consumer_bar();
     const TaggedPartOut out{p.partT, 2 + D, p.nsplit, tag};
+    const int busy = min(kConsumerWarps, kv.pairs + (owns_new ? 1 : 0));  // the first warps had rows
     for (int e = tid; e < D; e += kConsumers) {
         float M = -INFINITY, L = 0.f, c = 0.f;
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) M = fmaxf(M, wm[w]);
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) {
+        for (int w = 0; w < busy; ++w) M = fmaxf(M, wm[w]);
+#pragma unroll 1
+        for (int w = 0; w < busy; ++w) {
             const float f = wm[w] == -INFINITY ? 0.f : expf(wm[w] - M);
             L = fmaf(wl[w], f, L);
             c = fmaf(wctx[w * D + e], f, c);
@@ -1341,6 +1376,8 @@ __device__ __forceinline__ void consumer_loop(const MegaParams &p, Shared &sh, i
         const long r0 = (long)p.H * cta / nctas, r1 = (long)p.H * (cta + 1) / nctas;
         if (r0 + tid < r1) xres = embed_elem(p, id, (int)(r0 + tid));
     }
+    for (int i = tid; i < p.D; i += kConsumers)  // (a barrier lies between this and the first attention)
+        sh.attn[i] = i < p.D / 2 ? p.cos_t[(size_t)p.past * (p.D / 2) + i] : p.sin_t[(size_t)p.past * (p.D / 2) + i - p.D / 2];
     const int nphases = 5 * p.L + 1;
     RingPos rp{0};
     int bk = 0;
