@@ -164,6 +164,47 @@ __global__ void __launch_bounds__(kThreads, 4) gemv_vec_kernel(const float *x, c
     }
 }
 
+// The same for more bf16 rows than there are warps: two adjacent rows per warp at a time, so that the 32 bytes of x that go with 16 bytes of
+// weights are read from shared memory once for both (the way to the registers, not HBM, bound it), and half as many CTAs stage x.  Rows
+// shorter than a warp's batch (2 KB) lose by it, f32 rows (16 bytes of x for 16) gain nothing.
+// bf16 [8448,2048] 8.9 -> 7.4 us, [11008,4096] 21.0 -> 16.8, [12288,12288] 54.6 -> 46.3 (6.5 TB/s); [20000,512] 6.9 -> 7.5, f32 [32000,4096] 76.1 -> 76.6.
+__global__ void __launch_bounds__(kThreads, 2) gemv_vec_pair_kernel(const float *x, const __nv_bfloat16 *w, float *y, int K, size_t N) {
+    using WT = __nv_bfloat16;
+    extern __shared__ __align__(16) float smem[];
+    constexpr int VEC = 16 / sizeof(WT);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nv = K / VEC;
+    const size_t pairs = (N + 1) / 2, p0 = (size_t)blockIdx.x * kWarps + warp, step = (size_t)gridDim.x * kWarps;
+    auto at = [&](size_t p, int r) { return reinterpret_cast<const uint4 *>(w + min(2 * p + r, N - 1) * K); };
+    pdl_launch();
+    if (p0 < pairs)
+        for (int i = lane * 8; i < min(2 * p0 + 1 < N ? 2 * nv : nv, 512); i += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(at(p0, 0) + i));
+    pdl_wait();
+    uint4 cur[2][kAhead];
+    if (p0 < pairs) {
+        batch_load<true>(at(p0, 0), 0, nv, lane, cur[0]);
+        batch_load<true>(at(p0, 1), 0, nv, lane, cur[1]);
+    }
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+#pragma unroll 4
+        for (int k = tid; k < K / 4; k += kThreads) reinterpret_cast<float4 *>(smem)[k] = reinterpret_cast<const float4 *>(x)[k];
+    } else {
+        for (int k = tid; k < K; k += kThreads) smem[k] = x[k];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (size_t p = p0; p < pairs; p += step) {
+        float v[2];
+        const bool more = p + step < pairs;
+        pair_dot_ahead<WT, true>(at(p, 0), at(p, 1), smem, nv, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            v[1] += __shfl_xor_sync(0xffffffffu, v[1], o);
+        }
+        if (lane < 2 && 2 * p + lane < N) y[2 * p + lane] = lane ? v[1] : v[0];
+    }
+}
+
 // gate/up pair: out[m,i] = silu(gate_i . x_m) * (up_i . x_m)  (src/models/llama.rs:59-63,
 // src/layers/activation.rs:143-146: sig = 1/(1+exp(-g)); g*sig).
 template <typename WT, int MB>
@@ -225,44 +266,11 @@ __host__ __device__ inline size_t step_gains(const GemvStepArgs &a) {
     const bool fits = a.K % 4 == 0 && a.K <= (size_t)4 * kHeld * kThreads && ((reinterpret_cast<uintptr_t>(a.gain) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15) == 0;
     return fits ? a.K * ((a.y ? 1 : 0) + (a.norm_w ? 1 : 0)) : 0;
 }
-// One row whose input may still owe the norm of a sublayer's output (post-norm models): x = res + RMSNorm(y) * gain is
-// formed by every CTA while it stages x, so that the norm, the residual sum and the product are one launch.  WPR warps share a
-// weight row (a slice of K each) where there are too few rows to keep enough loads in flight.
-// GATED: N gate rows and the N up rows that go with them (in blocks, see kGateBlock) are walked as pairs; out = gelu_tanh(gate) * up.
-template <typename WT, int WPR, bool GATED>
-__global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const GemvStepArgs a) {
-    extern __shared__ __align__(16) float smem[];
-    __shared__ float red[kWarps], red2[kWarps];
-    float *xs = smem;
+// The input of a one-row product in shared memory: res, or res + RMSNorm(y) * gain (stored to x_out by the first CTA), then optionally
+// RMSNorm * norm_w.  held: the gains are on their way to shared memory.
+__device__ __forceinline__ void step_stage(const GemvStepArgs &a, float *xs, const float *gains, const float *norms, bool held, float *red, float *red2) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int VEC = 16 / sizeof(WT), kRows = kWarps / WPR;
-    const int part = warp % WPR;
-    const size_t K = a.K, n_rows = GATED ? 2 * a.N : a.N, row0 = (size_t)blockIdx.x * kRows + warp / WPR;
-    const WT *w = static_cast<const WT *>(a.w);
-    // where row r of the walk is stored (GATED: r = 2 * i for gate row i, 2 * i + 1 for up row i)
-    auto stored = [&](size_t r) {
-        if (!GATED) return r;
-        const size_t i = r >> 1;
-        return i / kGateBlock * (2 * kGateBlock) + i % kGateBlock + (r & 1) * kGateBlock;
-    };
-    const bool vec_ok = (K % VEC == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    // this warp's slice of K, in whole vectors
-    const int nv = (int)(K / VEC), per = (nv + WPR - 1) / WPR, v0 = min(nv, part * per), vn = min(nv - v0, per);
-    uint4 pre[kAhead];
-    if (vec_ok && row0 < n_rows) row_ahead(reinterpret_cast<const uint4 *>(w + stored(row0) * K) + v0, vn, lane, pre);
-    // Rows of up to 2048 numbers with norms: the gains are in shared memory before the wait ends, and what there is to read behind it
-    // (y and the residual) is one batch of loads held in registers, with one barrier per sum.  A step of six Fekorax layers 183 -> 173 us, of eight
-    // Fegetar layers 428 -> 417 (with the end of the step in its last product).
-    const bool held = step_gains(a) > 0;
-    float *gains = smem + K, *norms = gains + (a.y ? K : 0);
-    if (held) {
-        for (int k = tid; k < (int)K / 4; k += kThreads) {
-            if (a.y) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(gains + 4 * k)), "l"(a.gain + 4 * k) : "memory");
-            if (a.norm_w) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(norms + 4 * k)), "l"(a.norm_w + 4 * k) : "memory");
-        }
-    }
-    pdl_launch();
-    pdl_wait();
+    const size_t K = a.K;
     auto inv_rms = [&](float ss) {
         ss = warp_sum(ss);
         if (lane == 0) red[warp] = ss;
@@ -409,6 +417,65 @@ __global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const Ge
         }
     }
     __syncthreads();
+}
+// Requests the gains (before pdl_wait); returns whether there are any to keep.
+__device__ __forceinline__ bool step_request_gains(const GemvStepArgs &a, float *gains, float *norms) {
+    if (step_gains(a) == 0) return false;
+    for (int k = threadIdx.x; k < (int)a.K / 4; k += kThreads) {
+        if (a.y) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(gains + 4 * k)), "l"(a.gain + 4 * k) : "memory");
+        if (a.norm_w) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(norms + 4 * k)), "l"(a.norm_w + 4 * k) : "memory");
+    }
+    return true;
+}
+// What the last product of a step does besides (see GemvStepArgs).
+__device__ __forceinline__ void step_end(const GemvStepArgs &a) {
+    if (!a.d_lens || blockIdx.x != gridDim.x - 1) return;
+    for (int l = threadIdx.x; l < a.layers; l += kThreads) a.d_lens[l] += 1;
+    if (threadIdx.x == 0) *a.last_tok = (int)id_to_index(a.ids[0]);
+}
+template <typename WT>
+__device__ __forceinline__ float step_act(const GemvStepArgs &a, float v, size_t row) {
+    if (a.act != StepFinish::kStore) v = gelu_tanh(v);
+    if (a.act == StepFinish::kSideGate) {
+        const unsigned long long tok = id_to_index(a.ids[0]);
+        v *= tok < a.table_rows ? to_f32(static_cast<const WT *>(a.table)[tok * a.table_ld + row]) : 0.f;
+    }
+    return v;
+}
+
+// One row whose input may still owe the norm of a sublayer's output (post-norm models): x = res + RMSNorm(y) * gain is
+// formed by every CTA while it stages x, so that the norm, the residual sum and the product are one launch.  WPR warps share a
+// weight row (a slice of K each) where there are too few rows to keep enough loads in flight.
+// GATED: N gate rows and the N up rows that go with them (in blocks, see kGateBlock) are walked as pairs; out = gelu_tanh(gate) * up.
+template <typename WT, int WPR, bool GATED>
+__global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const GemvStepArgs a) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float red[kWarps], red2[kWarps];
+    float *xs = smem;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int VEC = 16 / sizeof(WT), kRows = kWarps / WPR;
+    const int part = warp % WPR;
+    const size_t K = a.K, n_rows = GATED ? 2 * a.N : a.N, row0 = (size_t)blockIdx.x * kRows + warp / WPR;
+    const WT *w = static_cast<const WT *>(a.w);
+    // where row r of the walk is stored (GATED: r = 2 * i for gate row i, 2 * i + 1 for up row i)
+    auto stored = [&](size_t r) {
+        if (!GATED) return r;
+        const size_t i = r >> 1;
+        return i / kGateBlock * (2 * kGateBlock) + i % kGateBlock + (r & 1) * kGateBlock;
+    };
+    const bool vec_ok = (K % VEC == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+    // this warp's slice of K, in whole vectors
+    const int nv = (int)(K / VEC), per = (nv + WPR - 1) / WPR, v0 = min(nv, part * per), vn = min(nv - v0, per);
+    uint4 pre[kAhead];
+    if (vec_ok && row0 < n_rows) row_ahead(reinterpret_cast<const uint4 *>(w + stored(row0) * K) + v0, vn, lane, pre);
+    // Rows of up to 2048 numbers with norms: the gains are in shared memory before the wait ends, and what there is to read behind it
+    // (y and the residual) is one batch of loads held in registers, with one barrier per sum.  A step of six Fekorax layers 183 -> 173 us, of eight
+    // Fegetar layers 428 -> 417 (with the end of the step in its last product).
+    float *gains = smem + K, *norms = gains + (a.y ? K : 0);
+    const bool held = step_request_gains(a, gains, norms);
+    pdl_launch();
+    pdl_wait();
+    step_stage(a, xs, gains, norms, held, red, red2);
 #pragma unroll 1
     for (size_t base = (size_t)blockIdx.x * kRows; base < n_rows; base += (size_t)gridDim.x * kRows) {
         const size_t row = base + warp / WPR;
@@ -448,18 +515,72 @@ __global__ void __launch_bounds__(kThreads, kStepCtas) gemv_step_kernel(const Ge
             __syncthreads();
         }
         if (lane == 0 && part == 0 && row < n_rows) {
-            if (a.act != StepFinish::kStore) v = gelu_tanh(v);
-            if (a.act == StepFinish::kSideGate) {
-                const unsigned long long tok = id_to_index(a.ids[0]);
-                v *= tok < a.table_rows ? to_f32(static_cast<const WT *>(a.table)[tok * a.table_ld + row]) : 0.f;
-            }
-            a.out[row] = v;
+            a.out[row] = step_act<WT>(a, v, row);
         }
     }
-    if (a.d_lens && blockIdx.x == gridDim.x - 1) {
-        for (int l = tid; l < a.layers; l += kThreads) a.d_lens[l] += 1;
-        if (tid == 0) *a.last_tok = (int)id_to_index(a.ids[0]);
+    step_end(a);
+}
+
+// The same for many rows of bf16 weights: a warp (or WPR warps, a slice of K each) takes two rows at a time, as in gemv_vec_pair_kernel.
+// GATED: a gate row and the up row that goes with it, so that nothing but the slices has to meet in shared memory.
+// What bounds it: HBM for the matrices of a few MB, and the way of x through shared memory, which two rows share.  A step of eight Fegetar
+// layers 416 -> 381 us at 96 positions (442 -> 406 at 1900), of six Fekorax layers 165 -> 149.
+template <int WPR, bool GATED>
+__global__ void __launch_bounds__(kThreads, 2) gemv_step_pair_kernel(const GemvStepArgs a) {
+    using WT = __nv_bfloat16;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float red[kWarps], red2[kWarps];
+    __shared__ float2 part_s[kWarps];
+    constexpr int VEC = 16 / sizeof(WT), kPairs = kWarps / WPR;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = warp % WPR;
+    const size_t K = a.K, N = a.N, pairs = GATED ? N : (N + 1) / 2, p0 = (size_t)blockIdx.x * kPairs + warp / WPR, step = (size_t)gridDim.x * kPairs;
+    const int nv = (int)(K / VEC), per = (nv + WPR - 1) / WPR, v0 = min(nv, part * per), vn = min(nv - v0, per);
+    const WT *w = static_cast<const WT *>(a.w);
+    auto at = [&](size_t p, int r) {
+        const size_t row = GATED ? p / kGateBlock * (2 * kGateBlock) + p % kGateBlock + r * kGateBlock : min(2 * p + r, N - 1);
+        return reinterpret_cast<const uint4 *>(w + row * K) + v0;
+    };
+    uint4 cur[2][kAhead];
+    if (p0 < pairs)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) row_ahead(at(p0, r), vn, lane, cur[r]);
+    float *xs = smem, *gains = smem + K, *norms = gains + (a.y ? K : 0);
+    const bool held = step_request_gains(a, gains, norms);
+    pdl_launch();
+    pdl_wait();
+    step_stage(a, xs, gains, norms, held, red, red2);
+#pragma unroll 1
+    for (size_t base = (size_t)blockIdx.x * kPairs; base < pairs; base += step) {
+        const size_t p = base + warp / WPR;
+        float v[2] = {0.f, 0.f};
+        if (p < pairs) {
+            const bool more = p + step < pairs;
+            pair_dot_ahead<WT>(at(p, 0), at(p, 1), xs + v0 * VEC, vn, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            v[1] += __shfl_xor_sync(0xffffffffu, v[1], o);
+        }
+        if (WPR > 1) {  // the rows' slices meet in their first warp
+            if (lane == 0) part_s[warp] = make_float2(v[0], v[1]);
+            __syncthreads();
+            v[0] = v[1] = 0.f;
+#pragma unroll
+            for (int i = 0; i < WPR; ++i) {
+                v[0] += part_s[warp / WPR * WPR + i].x;
+                v[1] += part_s[warp / WPR * WPR + i].y;
+            }
+            __syncthreads();
+        }
+        if (part != 0 || p >= pairs) continue;
+        if (GATED) {
+            if (lane == 0) a.out[p] = gelu_tanh(v[0]) * v[1];
+        } else if (lane < 2 && 2 * p + lane < N) {
+            a.out[2 * p + lane] = step_act<WT>(a, lane ? v[1] : v[0], 2 * p + lane);
+        }
     }
+    step_end(a);
 }
 
 // ---- [K,N] row-major layout ---------------------------------------------------------------------
@@ -659,6 +780,13 @@ int launch_gemv_vec(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype w
     const bool pdl = ctx->pdl;
     ctx->pdl = true;
     int rc;
+    if (wpr == 1 && wdt == LUMEN_BF16 && row_bytes >= 2048) {
+        const int pairs = (int)std::min<size_t>(((N + 1) / 2 + kWarps - 1) / kWarps, (size_t)ctx->num_sms * 2);
+        rc = set_smem(ctx, gemv_vec_pair_kernel, smem);
+        if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_pair_kernel, pairs, kThreads, smem, s, x, static_cast<const __nv_bfloat16 *>(w), y, (int)K, N);
+        ctx->pdl = pdl;
+        return rc;
+    }
 #define LUMEN_VEC(T_, W_) rc = set_smem(ctx, gemv_vec_kernel<T_, W_>, smem); if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_kernel<T_, W_>, grid, kThreads, smem, s, x, static_cast<const T_ *>(w), y, (int)K, N)
 #define LUMEN_VEC_T(T_) do { if (wpr == 8) { LUMEN_VEC(T_, 8); } else if (wpr == 4) { LUMEN_VEC(T_, 4); } else if (wpr == 2) { LUMEN_VEC(T_, 2); } else { LUMEN_VEC(T_, 1); } } while (0)
     if (wdt == LUMEN_F32) LUMEN_VEC_T(float);
@@ -692,6 +820,24 @@ int launch_gemv_step(lumen_ctx *ctx, const GemvStepArgs &a, cudaStream_t s) {
     const size_t row_bytes = a.K * (a.wdt == LUMEN_F32 ? 4 : 2), want = (size_t)ctx->num_sms * 3 * kWarps;
     const bool gated = a.act == StepFinish::kGated;
     const size_t rows = gated ? 2 * a.N : a.N;
+    // Two rows per warp where there are more pairs than half of its warps, or where their long rows make up for it
+    const size_t pair_warps = (size_t)ctx->num_sms * 2 * kWarps, pairs = gated ? a.N : (a.N + 1) / 2;
+    const bool split = pairs * 2 <= pair_warps && row_bytes >= 8192;
+    if (a.wdt == LUMEN_BF16 && a.K % 8 == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0 && row_bytes >= 2048 && (split || pairs * 2 > pair_warps)) {
+        const int g2 = (int)std::min((pairs * (split ? 2 : 1) + kWarps - 1) / kWarps, pair_warps / kWarps);
+#define LUMEN_PAIR(W_, G_)                                                                            \
+    do {                                                                                              \
+        LUMEN_TRY(set_smem(ctx, gemv_step_pair_kernel<W_, G_>, smem));                                \
+        return launch_pdl(ctx, gemv_step_pair_kernel<W_, G_>, g2, kThreads, smem, s, a);              \
+    } while (0)
+        if (gated) {
+            if (split) LUMEN_PAIR(2, true);
+            LUMEN_PAIR(1, true);
+        }
+        if (split) LUMEN_PAIR(2, false);
+        LUMEN_PAIR(1, false);
+#undef LUMEN_PAIR
+    }
     const int wpr = rows * 4 <= want && row_bytes >= 4096 ? 4 : rows * 2 <= want && row_bytes >= 2048 ? 2 : row_bytes >= 8192 && rows * 2 <= 2 * want ? 2 : 1;
     // as many CTAs as the device holds: each stages its input once
     const int grid = std::min(pick_grid(ctx, rows * wpr, smem), ctx->num_sms * kStepCtas);

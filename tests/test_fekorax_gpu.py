@@ -121,6 +121,14 @@ def test_attention_alone(L, dtype, a):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,ff,vocab", [(1088, 4104, 2501), (4096, 72, 101)])
+def test_products_of_two_rows_per_warp(L, dtype, width, ff, vocab):
+    """One-row products over many bf16 rows, or over long ones that two warps share, gated and plain, and a last row without a partner."""
+    cfg = K.config([(K.attn(heads=2, kv_heads=1, dim=16, vdim=16, chunk=100, rot_dims=8, scaling=None, scale=0.3), ff)], width=width, vocab=vocab)
+    _check(L, cfg, K.weights(L, cfg, 17), _ids(8, 17, vocab), ([1], [3, 1]), dtype, mistakes=("which is gated",))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [2048, 2052])
 def test_widest_rows_with_gains_in_shared_memory(L, dtype, width):
     """One-row products keep the gains of both norms in shared memory up to 2048 numbers and read them when they need them beyond."""

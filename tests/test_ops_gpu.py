@@ -142,7 +142,8 @@ def test_gemv_kn_layout_raw_pointers(L, oracle, ctx, k, n, bf16):
     assert np.all(y[:pad] == 12345.0) and np.all(y[-pad:] == 12345.0)
     assert rel_err(y[pad:-pad], oracle.matmul(x[None], w_nk, "f64")[0]) < 2e-6
 
-@pytest.mark.parametrize("k,n", [(4, 1), (8, 9), (2052, 5), (512, 2368), (512, 2369), (1024, 1184), (1032, 1185), (4096, 592), (4096, 593), (8200, 3), (8192, 297)])
+@pytest.mark.parametrize("k,n", [(4, 1), (8, 9), (2052, 5), (512, 2368), (512, 2369), (1024, 1184), (1032, 1185), (4096, 592), (4096, 593), (8200, 3), (8192, 297),
+                                 (1016, 2400), (1024, 2369), (1032, 2370), (2056, 4737)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_gemv_warps_per_row(L, oracle, ctx, k, n, bf16):
     """[N,K] products on raw pointers on both sides of every change of the warps that share a row, and rows that end inside a warp's step.
