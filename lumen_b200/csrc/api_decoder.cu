@@ -298,8 +298,8 @@ int lumen_decoder::rotation_tables(size_t l, float *cos_t, float *sin_t) {
             sh[p * half + i] = (float)std::sin((double)p * freq);
         }
     }
-    LUMEN_CUDA(ctx, cudaMemcpy(cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice));
-    LUMEN_CUDA(ctx, cudaMemcpy(sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice));
+    LUMEN_CUDA(ctx, cudaMemcpyAsync(cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    LUMEN_CUDA(ctx, cudaMemcpyAsync(sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
     return LUMEN_OK;
 }
 

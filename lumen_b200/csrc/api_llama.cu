@@ -461,18 +461,20 @@ int run_mega(lumen_llama *m, lumen_kv_cache **caches) {
         decode_mega_build_schedule(p, host.data(), ctx->num_sms, entries, counts, stride, tmaps);
         if (!m->d_mega_layers) LUMEN_CUDA(ctx, cudaMalloc(&m->d_mega_layers, table_bytes));
         if (!m->d_sched_count) LUMEN_CUDA(ctx, cudaMalloc(&m->d_sched_count, counts.size() * sizeof(int)));
-        LUMEN_CUDA(ctx, cudaMemcpy(m->d_sched_count, counts.data(), counts.size() * sizeof(int), cudaMemcpyHostToDevice));
+        // (In stream order: a plain copy from pageable memory may return before its last part is on the device, and this stream does not
+        // wait for the default one.  The step behind it then streams by a schedule that is not there yet.)
+        LUMEN_CUDA(ctx, cudaMemcpyAsync(m->d_sched_count, counts.data(), counts.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         if (!tmaps.empty()) {
             if (!m->d_tmaps) LUMEN_CUDA(ctx, cudaMalloc(&m->d_tmaps, tmaps.size() * sizeof(CUtensorMap)));
-            LUMEN_CUDA(ctx, cudaMemcpy(m->d_tmaps, tmaps.data(), tmaps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+            LUMEN_CUDA(ctx, cudaMemcpyAsync(m->d_tmaps, tmaps.data(), tmaps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, ctx->stream));
         }
         m->sched_stride = stride;
         uint4 *sched = nullptr;
         LUMEN_CUDA(ctx, cudaMalloc(&sched, entries.size() * sizeof(uint4)));
-        const cudaError_t e = cudaMemcpy(sched, entries.data(), entries.size() * sizeof(uint4), cudaMemcpyHostToDevice);
+        const cudaError_t e = cudaMemcpyAsync(sched, entries.data(), entries.size() * sizeof(uint4), cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) {
             cudaFree(sched);
-            return cuda_fail(ctx, e, "cudaMemcpy(copy schedule)");
+            return cuda_fail(ctx, e, "cudaMemcpyAsync(copy schedule)");
         }
         m->d_sched = sched;  // (last: what is there is complete)
     }
@@ -745,8 +747,8 @@ int lumen_llama_new(lumen_ctx *ctx, const lumen_llama_config *cfg, lumen_llama *
     std::vector<float> ch, sh;
     rope_tables_host(m->D, cfg->max_seq_len, cfg->rope_theta, ch, sh);
     if (!ch.empty()) {
-        cudaMemcpy(m->cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice);
-        cudaMemcpy(m->sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice);
+        cudaMemcpyAsync(m->cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice, ctx->stream);  // (in stream order, as the schedule)
+        cudaMemcpyAsync(m->sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
     }
     m->n_expected = 3 + m->L * (cfg->qk_norm ? 11 : 9);
     // Weights one decode step reads on this rank (the embedding contributes one row per token).

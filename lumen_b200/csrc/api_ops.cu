@@ -272,8 +272,8 @@ int lumen_rope_new(lumen_ctx *ctx, size_t dim, size_t max_seq_len, float theta, 
         return cuda_fail(ctx, e, "cudaMalloc(rope tables)");
     }
     if (!ch.empty()) {
-        LUMEN_CUDA(ctx, cudaMemcpy(r->cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice));
-        LUMEN_CUDA(ctx, cudaMemcpy(r->sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice));
+        LUMEN_CUDA(ctx, cudaMemcpyAsync(r->cos_t, ch.data(), ch.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+        LUMEN_CUDA(ctx, cudaMemcpyAsync(r->sin_t, sh.data(), sh.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
     }
     *out = r;
     return LUMEN_OK;

@@ -402,6 +402,11 @@ __device__ __forceinline__ void producer_loop(const MegaParams &p, Shared &sh, i
         const uint32_t tile_n = tiles + ntiles_batch + (uint32_t)__popc(firsts_n & (0xffffffffu >> (31 - lane))) - 1u;
         bool prefetched_n = !valid_n;
         for (uint32_t t0 = tiles; __any_sync(0xffffffffu, pending) && ok; t0 += S) {
+            if (t0 - tiles > 32u) {  // 32 entries have at most 32 tiles: this is no schedule (the waits below would not be reached, nor their limit)
+                if (lane == 0) raise_abort(p, sh.abort, 101, (int)tiles);
+                ok = false;
+                break;
+            }
             const bool mine = pending && tile < t0 + S;  // this pass: tiles [t0, t0 + S)
             const long long c0 = clock64();
             int spins = 0;

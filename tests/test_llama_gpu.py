@@ -306,6 +306,23 @@ def test_caches_in_turn(L):
         assert np.array_equal(got[:, 0], want[0][:, 2])
 
 
+def test_first_step_of_a_model_just_loaded(L):
+    """The step that builds the copy schedule runs behind its way to the device: models loaded one after another give what the first gave.
+    (A schedule of more than 64 KB; one that is not there yet ends in a time-out or in other logits.)"""
+    cfg = {**small_cfg(), "vocab_size": 40000}
+    params = make_params(L, cfg, 71, std=0.08)
+    ids = np.random.default_rng(72).integers(0, cfg["vocab_size"], size=(1, 4)).astype(np.float32)
+    want, model, caches = _gpu_run(L, cfg, params, ids, 3)
+    model.reset_kv_caches(caches)
+    with L.no_grad():
+        model.forward(ids[:, :3], caches, 0)
+        again = model.forward(ids[:, 3:], caches, 0)
+    assert np.array_equal(again[:, 0], want[:, 3])  # (the schedule has been there for a while)
+    for _ in range(6):
+        got, model, caches = _gpu_run(L, cfg, params, ids, 3)
+        assert np.array_equal(got[:, 3], want[:, 3])
+
+
 @pytest.mark.parametrize("batch", [8, 9])
 def test_parameters_set_between_steps(L, batch):
     """Wide f32 models send eight rows through the products of the kept bf16 weight split, in captured steps: after set_param
