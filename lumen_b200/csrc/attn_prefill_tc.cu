@@ -101,9 +101,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     __shared__ float xch[2][kBQ];
     volatile int *failed = &failed_s;
     const int tid = threadIdx.x, warp = tid >> 5;
-    // the last tiles of a causal prompt walk the most rows: they go first
-    const int qt = (int)(gridDim.x - 1 - blockIdx.x);
-    const int h = blockIdx.y, b = blockIdx.z;
+    // The last tiles of a causal prompt walk the most rows: those of all heads go first, so that what is left at the end is short (one head after
+    // another, the SMs worked 70 % of the time on a prompt of 1777 positions and 32 heads).
+    const int lin = (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)), rows_all = (int)(gridDim.y * gridDim.z);
+    const int qt = (int)gridDim.x - 1 - lin / rows_all, h = lin % rows_all % (int)gridDim.y, b = lin % rows_all / (int)gridDim.y;
     const int hk = h / (p.Hq / p.Hkv);
     const int i0 = qt * kBQ;
     // cached rows this tile can see: up to the diagonal of its last query row
