@@ -97,6 +97,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
                  const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_blo, const PairParams p) {
     using G = PairGeom<NA, NB, BN>;
     constexpr int kStages = G::kStages, kCols = SWIGLU ? BN / 2 : BN;
+    static_assert(BN % 32 == 0 && BN <= 256, "columns of an MMA of two SMs; half of the weight rows end on a 1024-byte pattern");
     extern __shared__ unsigned char smem_raw[];
     unsigned char *ring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], quiet;
@@ -223,7 +224,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
                         const size_t at = (size_t)row * width + t.n0 + c0;  // width is a multiple of 8
 #pragma unroll
                         for (int j = 0; j < 32; j += 8) {
-                            if (t.n0 + c0 + j >= width) break;
+                            if (t.n0 + c0 + j >= width || c0 + j >= kCols) break;  // (kCols is a multiple of 16)
                             uint2 h[2], l[2];
 #pragma unroll
                             for (int q = 0; q < 2; ++q) {
@@ -315,12 +316,14 @@ int launch_gemm_pair(lumen_ctx *ctx, const GemmPairArgs &g, const GemmPairPlan &
     p.status = ctx->d_status;
     const bool two = g.w_lo != nullptr, glu = g.out_hi != nullptr;
 #define LUMEN_PAIR(NB_, BN_, GLU_) launch_pair_t<2, NB_, BN_, GLU_>(ctx, g, p, s)
-    if (plan.bn == 256) {
-        if (glu) return two ? LUMEN_PAIR(2, 256, true) : LUMEN_PAIR(1, 256, true);
-        return two ? LUMEN_PAIR(2, 256, false) : LUMEN_PAIR(1, 256, false);
+#define LUMEN_PAIR_BN(BN_) (glu ? (two ? LUMEN_PAIR(2, BN_, true) : LUMEN_PAIR(1, BN_, true)) : (two ? LUMEN_PAIR(2, BN_, false) : LUMEN_PAIR(1, BN_, false)))
+    switch (plan.bn) {
+        case 256: return LUMEN_PAIR_BN(256);
+        case 224: return LUMEN_PAIR_BN(224);
+        case 192: return LUMEN_PAIR_BN(192);
+        default: return LUMEN_PAIR_BN(128);
     }
-    if (glu) return two ? LUMEN_PAIR(2, 128, true) : LUMEN_PAIR(1, 128, true);
-    return two ? LUMEN_PAIR(2, 128, false) : LUMEN_PAIR(1, 128, false);
+#undef LUMEN_PAIR_BN
 #undef LUMEN_PAIR
 }
 

@@ -400,9 +400,10 @@ int launch_gemm_tc(lumen_ctx *ctx, const float *a, const void *w, lumen_dtype wd
     const bool many = M > (size_t)kBM && N >= 128;
     const bool glu = many && fuse && fuse->post == GemmFuse::kPostSwiglu && !tp && N % 16 == 0 && fuse->next_hi != hi && fuse->next_lo != lo;
     const bool may_split = tp || (fuse && fuse->post == GemmFuse::kPostNorm);  // (slices of K are added by the kernel that reads the product anyway)
-    const GemmPairPlan plan = !many ? GemmPairPlan()
-                              : glu || may_split ? plan_gemm_pair(M, K, N, wsplit ? 3 : 2, glu, may_split, ctx->num_sms)
-                                                 : plan_gemm_plain(M, K, N, !wsplit, ctx->num_sms);
+    GemmPairPlan plan = !many ? GemmPairPlan()
+                        : glu || may_split ? plan_gemm_pair(M, K, N, wsplit ? 3 : 2, glu, may_split, ctx->num_sms)
+                                           : plan_gemm_plain(M, K, N, !wsplit, ctx->num_sms);
+    if (plan.bn == 256) plan.bn = pair_width(M, N, glu, plan.splits, ctx->num_sms);
     const bool pair = plan.bn != 0;
     CUtensorMap map_hi, map_lo, map_b, map_blo;  // 128-row side (hi, lo), BN-row side (hi, lo)
     const int bn = swap ? 64 : pick_bn(M, N, ctx->num_sms);

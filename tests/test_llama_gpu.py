@@ -123,6 +123,14 @@ def test_prefill_of_more_than_one_row_tile(L, oracle, hidden, inter, prompt, wdt
     assert rel_err(got, want) < TOL_F32
 
 
+@pytest.mark.parametrize("inter", [2600, 2696])
+@pytest.mark.parametrize("wdt", ["f32", "bf16"])
+def test_prefill_with_swiglu_tiles_of_other_widths(L, oracle, inter, wdt):
+    """Gate and up products of 513 rows in tiles of 224 columns (112 of each: no whole number of the epilogue's steps of 32) and of 256, with a
+    remainder of 24 and of 8 columns (2008 columns, in the test above, take tiles of 192)."""
+    test_prefill_of_more_than_one_row_tile(L, oracle, 128, inter, 513, wdt)
+
+
 @pytest.mark.parametrize("heads,kv,dim,hidden,inter,batch,prompt", [
     (8, 1, 64, 512, 200, 16, 40), (4, 2, 64, 136, 136, 33, 5), (2, 2, 128, 264, 72, 64, 1), (4, 1, 128, 1032, 1352, 9, 300), (8, 1, 128, 256, 4104, 17, 2),
     (2, 1, 64, 128, 64, 32, 130), (4, 4, 64, 256, 392, 48, 17), (4, 1, 64, 128, 136, 10, 33), (4, 2, 128, 256, 200, 21, 9), (8, 1, 64, 256, 136, 9, 384)])

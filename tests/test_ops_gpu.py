@@ -101,6 +101,13 @@ def test_paired_tile_edges(L, m, k, n, bf16):
     assert rel_err(got, a.astype(np.float64) @ wt.data().astype(np.float64).T) < 2e-5
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("m,k,n", [(513, 1096, 3721), (513, 1096, 4617), (1281, 1160, 2825)])
+def test_paired_tile_widths(L, m, k, n, bf16):
+    """Plain products in tiles of 192, 224 and 256 columns (the widths that leave the fewest pairs of SMs idle), one column and more beyond a tile."""
+    test_paired_tile_edges(L, m, k, n, bf16)
+
+
 def test_matmul_batched_leading_dims_and_errors(L, oracle):
     rng = np.random.default_rng(0)
     a = rng.standard_normal((2, 3, 16), dtype=np.float32)
