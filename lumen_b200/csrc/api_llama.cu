@@ -288,7 +288,10 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     };
 
     LUMEN_TRY(launch_embedding(ctx, w.ids, m->embed, wdt, w.x, M, m->V, H, s));
-    ctx->pdl = rows_attn;  // (the embedding has waited for everything before the step)
+    // (The embedding has waited for everything before the step.)  Long prompts too: their kernels wait before they touch anything but tables, so that
+    // launches and prologues overlap (four TinyLlama layers, f32, 1777 positions 2045 -> 1933 us, 400 positions 940 -> 860; four of Llama-2-7B, bf16, 512
+    // positions 1717 -> 1626).  Not the chain of few rows: two of its CTAs share an SM and its tensor memory with a next kernel that waits.
+    ctx->pdl = rows_attn || (fuse && !few && !tp && !p.decode);
     bool nx_ready = false;  // w.nx (or, fused, the pair) already holds Norm(x) of the block about to run
     for (size_t l = 0; l < m->L; ++l) {
         const LayerW &lw = m->layers[l];
@@ -363,6 +366,7 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
         if (nx_ready) { sum_d.norm_w = m->layers[l + 1].norm1; sum_d.normed = w.nx; sum_d.eps = eps; }
         LUMEN_TRY(matmul_dispatch(ctx, w.act, lw.wdown, wdt, w.x, M, m->inter_l, H, res_x, s, tp ? &sum_d : nullptr));
     }
+    if (!p.decode) ctx->pdl = false;
     // Final norm + lm_head                                             llama.rs:202-205
     const float *xin = w.x;
     size_t rows = M;

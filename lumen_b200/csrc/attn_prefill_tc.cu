@@ -115,6 +115,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     const int jt0 = CHUNK ? chunk_lo(i0) / kBKV : 0;
     const int nt = (visible + kBKV - 1) / kBKV - jt0;
 
+    pdl_launch();
     if (tid == 0) {
         bar_init(&q_bar, 1);
         for (int s = 0; s < G::kStages; ++s) {
@@ -140,6 +141,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // tensor memory: scores of even tiles | scores of odd tiles | O of even tiles | O of odd tiles
     const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 2 * kBKV;
+    pdl_wait();
 
     float ctx[kDH];
     float l = 0.f;
@@ -447,6 +449,7 @@ __global__ void __launch_bounds__(256) fa_pack_kernel(const AttnPrefillArgs a, _
     const int S = (int)a.S, Hq = (int)a.Hq, Hkv = (int)a.Hkv;
     const size_t row = (size_t)b * S + s, pos = a.past + s;
     const bool live = s < S;
+    pdl_launch();
     float co[E], sn[E], gq[E], gk[E];
     const bool rot = a.cos_t != nullptr && live;
 #pragma unroll
@@ -457,6 +460,7 @@ __global__ void __launch_bounds__(256) fa_pack_kernel(const AttnPrefillArgs a, _
         gq[i] = a.q_norm ? a.q_norm[e0 + i] : 1.f;
         gk[i] = a.k_norm ? a.k_norm[e0 + i] : 1.f;
     }
+    pdl_wait();  // (tables and gains are no kernel's result)
     auto pair_out = [&](__nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t at, const float (&v)[E]) {
         uint32_t h[E / 2], l[E / 2];
 #pragma unroll
@@ -517,9 +521,11 @@ __global__ void __launch_bounds__(256) fa_pack_kernel(const AttnPrefillArgs a, _
 }
 
 // K cache [B*Hkv, max_seq, D] f32 -> hi / lo [B*Hkv, l_pad, D] bf16, rows >= total zero.  One thread per four elements (D is a multiple of 64).
-__global__ void __launch_bounds__(256) fa_split_k_kernel(const float *__restrict__ k_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
+__global__ void __launch_bounds__(256) fa_split_k_kernel(const float *k_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
                                                          int total, int max_seq, int D, int l_pad, size_t n4) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch();
+    pdl_wait();
     if (i >= n4) return;
     const int per = D / 4, e = (int)(i % per) * 4;
     const size_t row = i / per;
@@ -536,11 +542,13 @@ __global__ void __launch_bounds__(256) fa_split_k_kernel(const float *__restrict
 // grid (l_pad / 64, B*Hkv); a CTA transposes 64 cached rows through shared memory.
 template <int D>
 __global__ void __launch_bounds__(256)
-fa_split_vt_kernel(const float *__restrict__ v_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int total,
+fa_split_vt_kernel(const float *v_cache, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int total,
                    int max_seq, int l_pad) {
     __shared__ float tile[64][D + 1];
     const int j0 = blockIdx.x * 64;
     const size_t bh = blockIdx.y;
+    pdl_launch();
+    pdl_wait();
     for (int i = threadIdx.x; i < 64 * D; i += 256) {
         const int jr = i / D, e = i % D;
         tile[jr][e] = j0 + jr < total ? v_cache[(bh * max_seq + j0 + jr) * D + e] : 0.f;
@@ -598,9 +606,7 @@ int launch_fa(lumen_ctx *ctx, const CUtensorMap *maps, const FaParams &p, dim3 g
         LUMEN_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_tc_kernel<KB, DV, PAIR, CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem));
         attr_set[dev] = true;
     }
-    attn_prefill_tc_kernel<KB, DV, PAIR, CHUNK><<<grid, kFaThreads, G::kSmem, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
-    LUMEN_LAUNCHED(ctx);
-    return LUMEN_OK;
+    return launch_pdl(ctx, attn_prefill_tc_kernel<KB, DV, PAIR, CHUNK>, grid, kFaThreads, G::kSmem, s, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
 }
 
 }  // namespace
@@ -626,29 +632,19 @@ int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_
     LUMEN_TRY(dev_alloc(ctx, (2 * nq + 4 * nkv) * sizeof(__nv_bfloat16), &ws));  // every count is a multiple of 64 * 64
     __nv_bfloat16 *qhi = static_cast<__nv_bfloat16 *>(ws), *qlo = qhi + nq;
     __nv_bfloat16 *khi = qlo + nq, *klo = khi + nkv, *vhi = klo + nkv, *vlo = vhi + nkv;
-    int rc = LUMEN_OK;
-    auto launched = [&](const char *what) {
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_fail(ctx, e, what);
-        else ctx->launches += 1;
-    };
     const bool fresh = a.past == 0;
     const bool vec = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0 &&
                      a.q_stride % 4 == 0 && a.kv_stride % 4 == 0;
     const dim3 pack_grid((unsigned)s_pad, (unsigned)a.B);
     __nv_bfloat16 *kh = fresh ? khi : nullptr, *kl = fresh ? klo : nullptr;
-    if (a.D == 64) fa_pack_kernel<64><<<pack_grid, 256, 0, s>>>(a, qhi, qlo, kh, kl, (int)s_pad, (int)l_pad, vec);
-    else fa_pack_kernel<128><<<pack_grid, 256, 0, s>>>(a, qhi, qlo, kh, kl, (int)s_pad, (int)l_pad, vec);
-    launched("fa_pack_kernel launch");
-    if (rc == LUMEN_OK && !fresh) {
-        fa_split_k_kernel<<<(unsigned)((nkv / 4 + 255) / 256), 256, 0, s>>>(a.k_cache, khi, klo, (int)total, (int)a.max_seq, (int)a.D, (int)l_pad, nkv / 4);
-        launched("fa_split_k_kernel launch");
-    }
+    int rc = launch_pdl(ctx, a.D == 64 ? fa_pack_kernel<64> : fa_pack_kernel<128>, pack_grid, 256, 0, s, a, qhi, qlo, kh, kl, (int)s_pad, (int)l_pad, vec);
+    if (rc == LUMEN_OK && !fresh)
+        rc = launch_pdl(ctx, fa_split_k_kernel, (unsigned)((nkv / 4 + 255) / 256), 256, 0, s, (const float *)a.k_cache, khi, klo, (int)total, (int)a.max_seq,
+                        (int)a.D, (int)l_pad, nkv / 4);
     if (rc == LUMEN_OK) {
         const dim3 g((unsigned)(l_pad / 64), (unsigned)(a.B * a.Hkv));
-        if (a.D == 64) fa_split_vt_kernel<64><<<g, 256, 0, s>>>(a.v_cache, vhi, vlo, (int)total, (int)a.max_seq, (int)l_pad);
-        else fa_split_vt_kernel<128><<<g, 256, 0, s>>>(a.v_cache, vhi, vlo, (int)total, (int)a.max_seq, (int)l_pad);
-        launched("fa_split_vt_kernel launch");
+        rc = launch_pdl(ctx, a.D == 64 ? fa_split_vt_kernel<64> : fa_split_vt_kernel<128>, g, 256, 0, s, (const float *)a.v_cache, vhi, vlo, (int)total,
+                        (int)a.max_seq, (int)l_pad);
     }
     CUtensorMap maps[6];
     if (rc == LUMEN_OK) rc = make_map(ctx, &maps[0], qhi, a.B * a.Hq * s_pad, a.D, kBQ);

@@ -156,7 +156,11 @@ __global__ void kv_slab_copy_kernel(const float *__restrict__ src, float *__rest
     else dst[i] = src[slab_idx];
 }
 
-__global__ void bump_len_kernel(int *len, int delta) { *len += delta; }
+__global__ void bump_len_kernel(int *len, int delta) {
+    pdl_launch();
+    pdl_wait();
+    *len += delta;
+}
 
 inline unsigned blocks(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -233,9 +237,7 @@ int launch_kv_slab_copy(lumen_ctx *ctx, const float *src, float *dst, size_t hea
 }
 
 int launch_bump_len(lumen_ctx *ctx, int *d_len, int delta, cudaStream_t s) {
-    bump_len_kernel<<<1, 1, 0, s>>>(d_len, delta);
-    LUMEN_LAUNCHED(ctx);
-    return LUMEN_OK;
+    return launch_pdl(ctx, bump_len_kernel, 1, 1, 0, s, d_len, delta);
 }
 
 }  // namespace lumen

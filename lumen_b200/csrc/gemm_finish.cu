@@ -16,11 +16,13 @@ namespace {
 // Bound by HBM: the registers of a row (NV float4 per thread) decide how many rows an SM has under way.  8192 rows of 4096 numbers: 49 us (5.5
 // TB/s), 116 us with room for 8192 numbers a row.
 template <int NV>
-__global__ void __launch_bounds__(256) sum_norm_split_kernel(const float *__restrict__ part, int splits, const float *residual, int rows,
+__global__ void __launch_bounds__(256) sum_norm_split_kernel(const float *part, int splits, const float *residual, int rows,
                                                              int dim, RowFinish f) {
     __shared__ float red[8];
     const int tid = threadIdx.x, nvec = dim >> 2;
     const size_t mn = (size_t)rows * dim;
+    pdl_launch();
+    pdl_wait();
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * dim;
         float4 v[NV];
@@ -204,12 +206,9 @@ int launch_sum_norm_split(lumen_ctx *ctx, const float *part, int splits, const f
     if (!row_finish_usable(dim)) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "row finisher: row length %zu", dim);
     RowFinish f{out, norm_w, eps, nullptr, hi, lo};
     const unsigned grid = (unsigned)std::min<size_t>(rows, (size_t)ctx->num_sms * 8);
-    if (dim <= 1024) sum_norm_split_kernel<1><<<grid, 256, 0, s>>>(part, splits, residual, (int)rows, (int)dim, f);
-    else if (dim <= 2048) sum_norm_split_kernel<2><<<grid, 256, 0, s>>>(part, splits, residual, (int)rows, (int)dim, f);
-    else if (dim <= 4096) sum_norm_split_kernel<4><<<grid, 256, 0, s>>>(part, splits, residual, (int)rows, (int)dim, f);
-    else sum_norm_split_kernel<kRowVecs><<<grid, 256, 0, s>>>(part, splits, residual, (int)rows, (int)dim, f);
-    LUMEN_LAUNCHED(ctx);
-    return LUMEN_OK;
+    const auto kernel = dim <= 1024 ? sum_norm_split_kernel<1> : dim <= 2048 ? sum_norm_split_kernel<2> : dim <= 4096 ? sum_norm_split_kernel<4>
+                                                                                                           : sum_norm_split_kernel<kRowVecs>;
+    return launch_pdl(ctx, kernel, grid, 256, 0, s, part, splits, residual, (int)rows, (int)dim, f);
 }
 
 int launch_sum_swiglu_split(lumen_ctx *ctx, const float *part, int splits, size_t rows, size_t inter, __nv_bfloat16 *hi,

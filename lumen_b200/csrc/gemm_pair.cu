@@ -114,6 +114,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
         return min(kb_all, kb0 + p.kb_per_split) - kb0;
     };
 
+    pdl_launch();  // (the next kernel's CTAs find no shared memory beside this one's, or wait in it)
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             bar_init(&full[s], 1);
@@ -136,6 +137,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     cluster_sync();  // both CTAs' barriers exist before anything signals across
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -301,9 +303,7 @@ int launch_pair_t(lumen_ctx *ctx, const GemmPairArgs &g, const PairParams &p, cu
     const size_t width = SWIGLU ? g.N / 2 : g.N, cols = SWIGLU ? BN / 2 : BN;
     const size_t items = (g.M + kPairRows - 1) / kPairRows * ((width + cols - 1) / cols) * p.splits;
     const unsigned pairs = (unsigned)std::min<size_t>(items, std::max(1, ctx->num_sms / 2));
-    kernel<<<2 * pairs, kPairThreads, smem, s>>>(ma, ma2, mb, mb2, p);
-    LUMEN_LAUNCHED(ctx);
-    return LUMEN_OK;
+    return launch_pdl(ctx, kernel, 2 * pairs, kPairThreads, smem, s, ma, ma2, mb, mb2, p);
 }
 
 }  // namespace
