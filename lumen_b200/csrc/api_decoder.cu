@@ -843,10 +843,10 @@ int lumen_decoder::run_forward(size_t b, size_t s, lumen_kv_cache **caches, bool
     if (s == 1) {
         // every launch of the step reads the position from the device; only the pieces of the context are baked in
         // (a context picks the same piece counts for all layers of one geometry, so their combination grows with the context)
-        unsigned key = 0;
-        for (size_t l = 0; l < L; ++l) key = key * 7 + (unsigned)pick_splits(l, caches[l], b, 1);
+        std::vector<size_t> pieces(L);
+        for (size_t l = 0; l < L; ++l) pieces[l] = (size_t)pick_splits(l, caches[l], b, 1);
         const bool one = b == 1 && W * 4 <= 200 * 1024;
-        rc = run_graphed(std::make_tuple(b, (int)key, (const void *)caches[0]->k),
+        rc = run_graphed(graph_key(b, pieces, caches),
                          [&] {
                              ctx->pdl = one;
                              const int r = one ? step_row(caches) : step_rows(b, 1, caches, last_only);

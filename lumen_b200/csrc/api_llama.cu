@@ -577,7 +577,7 @@ int run_forward(lumen_llama *m, size_t b, size_t s, lumen_kv_cache **caches, boo
     if (p.M > 8) LUMEN_TRY(ensure_weight_split(m));  // (outside any stream capture; the streaming kernels of <= 8 rows read f32)
     if (p.decode) p.nsplit = pick_decode_splits(m, b, caches[0]->len + 1);
     if (p.decode) p.parts = attn_rows_splits(b, m->hq_l, m->hkv_l, m->D, caches[0]->len + 1, ctx->num_sms);
-    const int rc = p.decode ? m->run_graphed(std::make_tuple(b, p.nsplit * 16 + p.parts, (const void *)caches[0]->k),
+    const int rc = p.decode ? m->run_graphed(m->graph_key(b, {(size_t)p.nsplit, (size_t)p.parts}, caches),
                                              [&] { return enqueue_forward(m, p, caches, last_only); })
                             : enqueue_forward(m, p, caches, last_only);
     if (rc == LUMEN_OK)

@@ -88,6 +88,19 @@ void lumen_model::drop_graphs() {
     graphs_.clear();
 }
 
+lumen_model::GraphKey lumen_model::graph_key(size_t batch, const std::vector<size_t> &plan, lumen_kv_cache *const *caches) const {
+    GraphKey key;
+    key.reserve(1 + plan.size() + 5 * L);
+    key.push_back(batch);
+    key.insert(key.end(), plan.begin(), plan.end());
+    for (size_t l = 0; l < L; ++l) {
+        const lumen_kv_cache &c = *caches[l];
+        for (const void *at : {(const void *)c.k, (const void *)c.v, (const void *)c.d_len, (const void *)c.last_tok}) key.push_back(reinterpret_cast<size_t>(at));
+        key.push_back(c.max_seq);
+    }
+    return key;
+}
+
 int lumen_model::run_graphed(const GraphKey &key, const std::function<int()> &enqueue) {
     if (!use_graph) return enqueue();
     Captured &c = graphs_[key];

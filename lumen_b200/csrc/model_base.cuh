@@ -6,7 +6,7 @@
 
 #include <functional>
 #include <map>
-#include <tuple>
+#include <vector>
 
 #include "common.cuh"
 
@@ -57,8 +57,10 @@ struct lumen_model {
     int forward_device(const float *ids_dev, size_t b, size_t s, lumen_kv_cache **caches, size_t n_caches, float *logits_dev);
 
     // Decode steps: the first call with a key runs `enqueue` eagerly, the second captures it, later ones replay the graph.
-    // The key names everything that is baked into the launches (batch, split count, cache address).
-    using GraphKey = std::tuple<size_t, int, const void *>;
+    // The key holds everything that is baked into the launches: the batch, the plan (piece counts), and of every layer's cache the
+    // addresses and the row count (the first layer's address alone is shared by sets of caches that differ behind it).
+    using GraphKey = std::vector<size_t>;
+    GraphKey graph_key(size_t batch, const std::vector<size_t> &plan, lumen_kv_cache *const *caches) const;
     bool use_graph = true;
     int run_graphed(const GraphKey &key, const std::function<int()> &enqueue);
     void drop_graphs();

@@ -368,6 +368,9 @@ def test_errors_come_back_as_status_codes(L):
         for c in caches[:3]:
             with pytest.raises(L.LumenError):
                 c.read()  # a state, or rows of two sizes
+        with pytest.raises(L.LumenError) as e:
+            model.forward(np.zeros((1, 1)), list(caches[:1]) + list(model.init_kv_caches(1)[1:]))  # layers of two sets
+        assert e.value.code == L._lib.ERR_INVALID
     for layers in ([(K.attn(kv_from=0), None)], [(K.matrix(), None), (K.attn(kv_from=0), None)], [(K.attn(), None), (K.attn(kv_from=0), None), (K.attn(kv_from=1), None)],
                    [(K.attn(), None), (K.attn(dim=16, rot_dims=8, kv_from=0), None)], [(K.attn(heads=3, kv_heads=2), None)], [(K.attn(rot_dims=40), None)]):
         with pytest.raises(L.LumenError):

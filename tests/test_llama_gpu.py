@@ -284,34 +284,32 @@ def test_persistent_kernel_equals_per_op_path(L, oracle, monkeypatch, over, wdt)
         assert rel_err(k, oc[l].k) < 1e-5 and rel_err(v, oc[l].v) < 1e-5
 
 
-def test_caches_in_turn(L):
-    """The persistent kernel follows the caches of each call: two conversations of one model in turn, and caches whose first layer alone is shared."""
+@pytest.mark.parametrize("batch", [1, 2, 9])
+def test_caches_in_turn(L, batch):
+    """The persistent kernel and the captured steps of batches (products of few and of more than eight rows) follow the caches of each call: two
+    conversations of one model in turn, and sets of caches whose first layer alone is new, or alone is shared."""
     cfg = small_cfg()
     params = make_params(L, cfg, 66, std=0.08)
-    ids = np.random.default_rng(67).integers(0, cfg["vocab_size"], size=(2, 14)).astype(np.float32)
-    want = [_gpu_run(L, cfg, params, ids[i:i + 1], 3)[0][:, 3:] for i in range(2)]
+    ids = np.random.default_rng(67).integers(0, cfg["vocab_size"], size=(2, batch, 14)).astype(np.float32)
+    want = [_gpu_run(L, cfg, params, ids[i], 3)[0][:, 3:] for i in range(2)]
     model = L.LlamaModel(cfg_obj(L, cfg))
     model.load_state(params)
-    caches = [model.init_kv_caches(1) for _ in range(2)]
+    caches = [model.init_kv_caches(batch) for _ in range(2)]
     with L.no_grad():
         for i in range(2):
-            model.forward(ids[i:i + 1, :3], caches[i], 0)
+            model.forward(ids[i, :, :3], caches[i], 0)
         for t in range(3, 14):
             for i in range(2):
-                got = model.forward(ids[i:i + 1, t:t + 1], caches[i], 0)
+                got = model.forward(ids[i, :, t:t + 1], caches[i], 0)
                 assert np.array_equal(got[:, 0], want[i][:, t - 3]), (t, i)
-        third = model.init_kv_caches(1)
-        mixed = [third[0]] + list(caches[1][1:])  # (the first layer's memory is another one, the others' are not)
-        model.reset_kv_caches(mixed)
-        for part in (ids[1:2, :3], *(ids[1:2, t:t + 1] for t in range(3, 6))):
-            got = model.forward(part, mixed, 0)
-        assert np.array_equal(got[:, 0], want[1][:, 2])
-        model.reset_kv_caches(caches[0])
-        swapped = [third[0]] + list(caches[0][1:])  # the same first layer, other layers behind it
-        model.reset_kv_caches(swapped)
-        for part in (ids[0:1, :3], *(ids[0:1, t:t + 1] for t in range(3, 6))):
-            got = model.forward(part, swapped, 0)
-        assert np.array_equal(got[:, 0], want[0][:, 2])
+        third = model.init_kv_caches(batch)
+        for i in (1, 0):  # first the memory of the first layer is another one, the others' are not; then the same first layer has other layers behind it
+            mixed = [third[0]] + list(caches[i][1:])
+            model.reset_kv_caches(mixed)
+            model.forward(ids[i, :, :3], mixed, 0)
+            for t in range(3, 8):  # (steps of a batch are captured at the second and replayed from the third on)
+                got = model.forward(ids[i, :, t:t + 1], mixed, 0)
+                assert np.array_equal(got[:, 0], want[i][:, t - 3]), (t, i)
 
 
 def test_first_step_of_a_model_just_loaded(L):
