@@ -551,8 +551,11 @@ int run_mega(lumen_llama *m, lumen_kv_cache **caches) {
     return LUMEN_OK;
 }
 
-bool mega_usable(lumen_llama *m, size_t b, size_t s) {
+bool mega_usable(lumen_llama *m, size_t b, size_t s, lumen_kv_cache **caches) {
     if (!m->use_mega || b != 1 || s != 1 || m->L == 0) return false;
+    // one row count serves all layers of the kernel; caches made one by one may differ in it
+    for (size_t l = 1; l < m->L; ++l)
+        if (caches[l]->max_seq != caches[0]->max_seq) return false;
     // the kernel's fused all-reduce has forms for 2, 4 and 8 ranks; other rank counts take the per-operator path + NCCL
     const int T = m->ctx->tp_size;
     if (T != 1 && T != 2 && T != 4 && T != 8) return false;
@@ -568,7 +571,7 @@ bool mega_usable(lumen_llama *m, size_t b, size_t s) {
 // through a captured graph after the first call.
 int run_forward(lumen_llama *m, size_t b, size_t s, lumen_kv_cache **caches, bool last_only) {
     lumen_ctx *ctx = m->ctx;
-    if (mega_usable(m, b, s)) {
+    if (mega_usable(m, b, s, caches)) {
         LUMEN_TRY(run_mega(m, caches));
         for (size_t l = 0; l < m->L; ++l) caches[l]->len += 1;
         return LUMEN_OK;

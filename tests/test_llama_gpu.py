@@ -312,6 +312,23 @@ def test_caches_in_turn(L, batch):
                 assert np.array_equal(got[:, 0], want[i][:, t - 3]), (t, i)
 
 
+def test_caches_of_different_lengths(L):
+    """Caches made one by one may hold different numbers of rows: such a set decodes as a set of equal ones does, and writes to its own rows alone."""
+    cfg = small_cfg()
+    params = make_params(L, cfg, 68, std=0.08)
+    ids = np.random.default_rng(69).integers(0, cfg["vocab_size"], size=(1, 14)).astype(np.float32)
+    want, model, equal = _gpu_run(L, cfg, params, ids, 3)
+    shape = equal[0].shape  # [1, heads, rows, size]
+    caches = [L.KVCache(1, shape[1], rows, shape[3]) for rows in (20, shape[2])]
+    with L.no_grad():
+        model.forward(ids[:, :3], caches, 0)
+        for t in range(3, 14):
+            assert rel_err(model.forward(ids[:, t:t + 1], caches, 0)[:, 0], want[:, t]) < TOL_F32, t
+    for c, e in zip(caches, equal):
+        for got, ref in zip(c.read(), e.read()):
+            assert rel_err(got[:, :, :14], ref[:, :, :14]) < TOL_F32 and not got[:, :, 14:].any()
+
+
 def test_first_step_of_a_model_just_loaded(L):
     """The step that builds the copy schedule runs behind its way to the device: models loaded one after another give what the first gave.
     (A schedule of more than 64 KB; one that is not there yet ends in a time-out or in other logits.)"""
