@@ -290,7 +290,8 @@ int enqueue_forward(lumen_llama *m, const StepPlan &p, lumen_kv_cache **caches, 
     LUMEN_TRY(launch_embedding(ctx, w.ids, m->embed, wdt, w.x, M, m->V, H, s));
     // (The embedding has waited for everything before the step.)  Long prompts too: their kernels wait before they touch anything but tables, so that
     // launches and prologues overlap (four TinyLlama layers, f32, 1777 positions 2045 -> 1933 us, 400 positions 940 -> 860; four of Llama-2-7B, bf16, 512
-    // positions 1717 -> 1626).  Not the chain of few rows: two of its CTAs share an SM and its tensor memory with a next kernel that waits.
+    // positions 1717 -> 1626).  Not the chain of few rows in prompts: its CTAs
+    // share an SM and its tensor memory with the next kernel's, which would wait there; that was not measured.
     ctx->pdl = rows_attn || (fuse && !few && !tp && !p.decode);
     bool nx_ready = false;  // w.nx (or, fused, the pair) already holds Norm(x) of the block about to run
     for (size_t l = 0; l < m->L; ++l) {

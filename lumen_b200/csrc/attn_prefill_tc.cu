@@ -115,7 +115,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     const int jt0 = CHUNK ? chunk_lo(i0) / kBKV : 0;
     const int nt = (visible + kBKV - 1) / kBKV - jt0;
 
-    pdl_launch();
     if (tid == 0) {
         bar_init(&q_bar, 1);
         for (int s = 0; s < G::kStages; ++s) {
@@ -141,6 +140,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // tensor memory: scores of even tiles | scores of odd tiles | O of even tiles | O of odd tiles
     const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 2 * kBKV;
+    pdl_launch();  // (behind the allocation, as in gemm_pair_kernel: the next kernel may take tensor memory before it waits)
     pdl_wait();
 
     float ctx[kDH];

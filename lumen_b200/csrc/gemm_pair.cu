@@ -114,7 +114,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
         return min(kb_all, kb0 + p.kb_per_split) - kb0;
     };
 
-    pdl_launch();  // (the next kernel's CTAs find no shared memory beside this one's, or wait in it)
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             bar_init(&full[s], 1);
@@ -137,6 +136,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_const
     cluster_sync();  // both CTAs' barriers exist before anything signals across
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
+    // The next kernel may start now, not earlier: its CTAs may take tensor memory before they wait for this kernel, so every CTA of this one must have its own.
+    pdl_launch();
     pdl_wait();
 
     if (warp == 0) {

@@ -104,7 +104,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     };
     const int ahead = min(nkb, kStages);
-    pdl_launch();
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             bar_init(&full[s], 1);
@@ -124,6 +123,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
+    pdl_launch();  // (behind the allocation, as in gemm_pair_kernel: the next kernel takes tensor memory before it waits)
     int issued = 0;  // steps whose copies are on their way (thread 0)
     if (tid == 0) {
         pdl_wait();

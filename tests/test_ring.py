@@ -45,6 +45,19 @@ def test_limits_start_behind_the_kernel_before():
                 assert "pdl_wait()" in b[: b.index("bar_wait(")], (name, b[:60])
 
 
+def test_dependents_start_behind_the_allocation():
+    """A kernel launched behind one that takes tensor memory may take some before it waits: every CTA of the first has its own by the time it lets
+    dependents start, or the two could wait for one another without a limit."""
+    seen = 0
+    for p in sorted(CSRC.glob("*.cu")):
+        for body in p.read_text().split("__global__")[1:]:
+            if "tcgen05.alloc" in body and "pdl_launch();" in body:
+                between = body[body.index("tcgen05.alloc"): max(body.index("tcgen05.alloc"), body.index("pdl_launch();"))]
+                assert "tcgen05.relinquish_alloc_permit" in between and "__syncthreads()" in between, p.name
+                seen += 1
+    assert seen == 3
+
+
 def test_peer_addresses_come_from_mapa():
     """Where the window of a cluster's other CTA lies is the machine's business: addresses in it come from mapa, not from masked bits."""
     for p in sorted(CSRC.glob("*.cu*")):
