@@ -23,13 +23,15 @@ constexpr int kWarps = kThreads / 32;
 
 // Stage x[M,K] into shared memory, optionally RMS-normalised: xs = (x * inv_rms) * norm_w, which is
 // the element the reference's RMSNorm produces (src/layers/norm/rms_norm.rs:49-56) before its Linear.
-// A row is normed by one warp (the CTA has as many as a pass has rows).  Every CTA does all of this, so it is paid per launch: with
-// an index division per element and block-wide sums row after row the products of eight TinyLlama rows took 47 (q, k, v), 43 (o), 65 (gate,
-// up) and 103 us (down), most of it here.
+// The CTA's warps share out the rows: one each where a pass has eight, all of them for a single one.  Every CTA does all of this, so it is
+// paid per launch: with an index division per element and block-wide sums row after row the products of eight TinyLlama rows took 47
+// (q, k, v), 43 (o), 65 (gate, up) and 103 us (down), most of it here.
 // A step of 22 TinyLlama layers, f32, at 100 positions: 2401 -> 1747 us with 2 rows, 3443 -> 1943 with 4, 4884 -> 2252 with 8.
+// (With one warp per row whatever their number, eight layers took 675 us with 2 rows, 747 with 4, now 658 and 733; a prompt of two tokens whose
+// last row alone goes through an output matrix of bf16 [32000,4096], host to host, 149 us, now 141.)
 template <int MB>
 __device__ void stage_x(float *xs, const float *__restrict__ x, int M, size_t K, const float *__restrict__ norm_w, float eps) {
-    static_assert(MB <= kWarps, "a warp per row");
+    static_assert(MB <= kWarps && kWarps % MB == 0, "whole warps per row");
     const int tid = threadIdx.x, n = (int)(M * K), all = (int)(MB * K);
     const bool vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     if (vec) {
@@ -41,30 +43,47 @@ __device__ void stage_x(float *xs, const float *__restrict__ x, int M, size_t K,
     for (int i = n + tid; i < all; i += kThreads) xs[i] = 0.f;
     __syncthreads();
     if (norm_w == nullptr) return;
-    const int lane = tid & 31, m = tid >> 5;
+    constexpr int WPR = kWarps / MB, kStep = 32 * WPR;  // warps of a row
+    __shared__ float red[kWarps];
+    const int warp = tid >> 5, m = warp / WPR, at = tid % kStep;
+    float *row = xs + (size_t)m * K;
+    const bool vec_norm = vec && (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0;
+    const int n4 = (int)(K / 4);
+    float ss = 0.f;
     if (m < M) {
-        float *row = xs + (size_t)m * K;
-        float ss = 0.f;
-        if (vec && (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0) {
-            const int n4 = (int)(K / 4);
+        if (vec_norm) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);  // (four sums: short chains)
+#pragma unroll 4
+            for (int k = at; k < n4; k += kStep) {
+                const float4 v = reinterpret_cast<const float4 *>(row)[k];
+                acc = make_float4(fmaf(v.x, v.x, acc.x), fmaf(v.y, v.y, acc.y), fmaf(v.z, v.z, acc.z), fmaf(v.w, v.w, acc.w));
+            }
+            ss = (acc.x + acc.y) + (acc.z + acc.w);
+        } else {
+            for (size_t k = at; k < K; k += kStep) ss = fmaf(row[k], row[k], ss);
+        }
+    }
+    ss = warp_sum(ss);
+    if (WPR > 1) {
+        if ((tid & 31) == 0) red[warp] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int w = 0; w < WPR; ++w) ss += red[m * WPR + w];
+    }
+    if (m < M) {
+        const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+        if (vec_norm) {
             float4 *r4 = reinterpret_cast<float4 *>(row);
             const float4 *g4 = reinterpret_cast<const float4 *>(norm_w);
 #pragma unroll 4
-            for (int k = lane; k < n4; k += 32) {
-                const float4 v = r4[k];
-                ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
-            }
-            const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(warp_sum(ss), (float)K), eps)));
-#pragma unroll 4
-            for (int k = lane; k < n4; k += 32) {
+            for (int k = at; k < n4; k += kStep) {
                 const float4 v = r4[k], g = g4[k];
                 r4[k] = make_float4(__fmul_rn(__fmul_rn(v.x, inv), g.x), __fmul_rn(__fmul_rn(v.y, inv), g.y), __fmul_rn(__fmul_rn(v.z, inv), g.z),
                                     __fmul_rn(__fmul_rn(v.w, inv), g.w));
             }
         } else {
-            for (size_t k = lane; k < K; k += 32) ss = fmaf(row[k], row[k], ss);
-            const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(warp_sum(ss), (float)K), eps)));
-            for (size_t k = lane; k < K; k += 32) row[k] = __fmul_rn(__fmul_rn(row[k], inv), norm_w[k]);
+            for (size_t k = at; k < K; k += kStep) row[k] = __fmul_rn(__fmul_rn(row[k], inv), norm_w[k]);
         }
     }
     __syncthreads();
