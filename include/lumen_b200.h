@@ -232,7 +232,10 @@ int lumen_llama_forward_device(lumen_llama *m, const float *ids_dev, size_t b, s
  * softmax, stable descending sort, nucleus cut at top_p, inverse-CDF walk with `uniform` in [0,1) (the
  * reference draws it from its thread RNG, :69-72; here the caller supplies it so that runs can be repeated).
  * recent_tokens is a HOST array of at most 256 ids.
- * lumen_sample_top_p        : logits_dev[vocab] (device) -> *token_out (host); synchronises.
+ * lumen_sample_top_p        : logits_dev[vocab] (device) -> *token_out (host).  Waits for the token, not for the
+ *                             stream: all work enqueued before the call has run when it returns, the call's own kernel
+ *                             may still be ending.  Synchronise the context before the host reads memory that work of
+ *                             your own on its stream writes.  Errors that earlier work reported are returned here.
  * lumen_llama_forward_sample: LlamaModel::forward on ids[1,S] followed by the sampler on the last position's
  *                             logits, as main.rs:334-372 does on the host; only the token id is copied back. */
 typedef struct {

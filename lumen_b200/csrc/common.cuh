@@ -364,7 +364,7 @@ int launch_attn_prefill(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s
 bool attn_prefill_tc_usable(const AttnPrefillArgs &a);
 int launch_attn_prefill_tc(lumen_ctx *ctx, const AttnPrefillArgs &a, cudaStream_t s);
 
-// Nucleus sampling of one logits vector on the device (sampler.cu); waits for the stream.
+// Nucleus sampling of one logits vector on the device (sampler.cu); waits for the token.
 int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lumen_sample_params &sp, int32_t *token, cudaStream_t s);
 
 // LlamaKVCache::update: dst[h, start+s, :] = src[h, s, :].

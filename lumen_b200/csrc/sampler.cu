@@ -11,7 +11,9 @@
 // (nuclei that reach into probabilities below 2^-24, hundreds of nearly equal probabilities, vocabularies of more than
 // kNucleusMaxVocab, NaN) takes a kernel that forms the probabilities, cub::DeviceRadixSort (a library sort: not the hot
 // path) and a kernel that walks the sorted list.
+#include <chrono>
 #include <climits>
+#include <thread>
 
 #include <cooperative_groups.h>
 
@@ -556,7 +558,9 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
 
 }  // namespace
 
-// logits_dev[vocab] -> *token (waits for the stream).
+// logits_dev[vocab] -> *token.  Waits for the token: everything enqueued before the call has run by then, the stream itself may not be idle yet (the end of
+// the sampling kernel).  The answer does not release what earlier work wrote to host memory: a fence of the system in the kernel costs 1.2 us a draw (8 draws
+// 223 -> 234 us), and who needs that can wait for the stream.
 int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lumen_sample_params &sp, int32_t *token, cudaStream_t s) {
     if (vocab == 0 || vocab > (size_t)1 << 30) return set_error(ctx, LUMEN_ERR_SHAPE, "sample: vocabulary of %zu", vocab);
     if (sp.n_recent > (size_t)kMaxRecent) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "sample: %zu recent tokens, at most %d", sp.n_recent, kMaxRecent);
@@ -597,21 +601,29 @@ int sample_top_p(lumen_ctx *ctx, const float *logits_dev, size_t vocab, const lu
         for (size_t i = 0; i < sp.n_recent; ++i) a.recent[i] = sp.recent_tokens[i];
         sample_nucleus_kernel<<<kCluster, kPrepThreads, smem, s>>>(a);
         LUMEN_LAUNCHED(ctx);
-        // The kernel stores its answer to pinned memory of the host, which watches the word; the stream is asked now and then, so that a
-        // failure ends the watch.
+        // The kernel stores its answer to pinned memory of the host, which watches the word, so that no copy and no wait for
+        // the stream follow the kernel.  It spins at first, then gives way to other threads; behind a backlog of more than 20 ms, and
+        // where a failure left no answer, it waits for the stream as everything else does (as the device's scheduling flags say).
         int got = -1;
+        const auto asked = std::chrono::steady_clock::now();
         for (unsigned int spins = 1;; ++spins) {
-            const unsigned long long v = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
+            unsigned long long v = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
+            bool last = false;
+            if ((spins & 63) == 0 && (unsigned int)(v >> 32) != a.turn) {
+                const auto waited = std::chrono::steady_clock::now() - asked;
+                if (waited > std::chrono::milliseconds(20)) {
+                    LUMEN_TRY(check_device_status(ctx));
+                    v = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
+                    last = true;
+                } else if (waited > std::chrono::microseconds(50)) {
+                    std::this_thread::yield();
+                }
+            }
             if ((unsigned int)(v >> 32) == a.turn) {
                 got = (int)(unsigned int)v;
                 break;
             }
-            if ((spins & 0xffff) == 0 && cudaStreamQuery(s) != cudaErrorNotReady) {
-                LUMEN_TRY(check_device_status(ctx));
-                const unsigned long long last = __atomic_load_n(ctx->h_answer, __ATOMIC_ACQUIRE);
-                if ((unsigned int)(last >> 32) == a.turn) got = (int)(unsigned int)last;
-                break;
-            }
+            if (last) break;
 #if defined(__x86_64__)
             __builtin_ia32_pause();
 #endif

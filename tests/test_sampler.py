@@ -1,5 +1,10 @@
 """Nucleus sampling: the oracle's restatement of `sample_top_p` (src/main.rs:74-137) on CPU, and the device
 sampler against it on a GPU (same token for the same uniform draw)."""
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -105,6 +110,59 @@ def test_lists_on_both_sides_of_the_shared_memory(L, ctx, oracle):
         for u in list(rng.random(5).astype(np.float32)) + [np.float32(0), np.float32(1)]:
             mismatches += L.sample_top_p(ctx, t.data_ptr, 9000, 1.0, 0.99, 1.0, [], float(u)) != oracle.sample_top_p(lg, 1.0, 0.99, 1.0, [], float(u))
     assert mismatches <= 2, mismatches  # (as above: draws within an ulp of a boundary)
+
+
+@pytest.mark.gpu
+def test_a_report_of_earlier_work_comes_back_from_the_draw(L, ctx, oracle):
+    """An id beyond the vocabulary in a step whose errors nothing has asked for yet: the draw behind it raises, the next one draws."""
+    cfg = small_cfg()
+    model = L.LlamaModel(L.LlamaConfig(**cfg))
+    model.load_state(make_params(L, cfg, 17))
+    caches = model.init_kv_caches(2)
+    rng = np.random.default_rng(4)
+    lg = (rng.standard_normal(500) * 2).astype(np.float32)
+    t, ids, out = (L.Tensor.from_array_no_grad(a) for a in (lg, np.array([3.0, cfg["vocab_size"]], np.float32), np.zeros((2, cfg["vocab_size"]), np.float32)))
+    with L.no_grad():
+        model.forward_device(ids.data_ptr, 2, 1, caches, out.data_ptr)
+        with pytest.raises(L.LumenError) as e:
+            L.sample_top_p(ctx, t.data_ptr, 500, 0.8, 0.9, 1.0, [], 0.4)
+    assert e.value.code == L._lib.ERR_EMBED_RANGE
+    for u in (0.1, 0.4, 0.8):
+        assert L.sample_top_p(ctx, t.data_ptr, 500, 0.8, 0.9, 1.0, [], u) == oracle.sample_top_p(lg, 0.8, 0.9, 1.0, [], u)
+
+
+WAITER = textwrap.dedent("""
+    import ctypes, sys, time
+    sys.path.insert(0, %r)
+    cuda, dev = ctypes.CDLL("libcuda.so.1"), ctypes.c_int()
+    assert cuda.cuInit(0) == 0 and cuda.cuDeviceGet(ctypes.byref(dev), 0) == 0
+    assert cuda.cuDevicePrimaryCtxSetFlags_v2(dev, 4) == 0  # of this process: threads that wait for the device sleep
+    import numpy as np
+    import lumen_b200 as L
+    ctx = L.default_context()
+    logits = L.Tensor.from_array_no_grad((np.random.default_rng(0).standard_normal(32000) * 3).astype(np.float32))
+    n = 6144
+    a = L.Tensor.from_array_no_grad(np.ones((n, n), np.float32))
+    draw = lambda: L.sample_top_p(ctx, logits.data_ptr, 32000, 0.8, 0.9, 1.0, [], 0.5)
+    first = draw()
+    with L.no_grad():
+        L.matmul(a, a)
+        ctx.synchronize()
+        for _ in range(300):
+            L.matmul(a, a)
+    wall, cpu = time.perf_counter(), time.thread_time()
+    same = draw() == first
+    print("WAITED", round(time.perf_counter() - wall, 3), round(time.thread_time() - cpu, 3), same)
+""")
+
+
+@pytest.mark.gpu
+def test_a_draw_behind_a_long_backlog_waits_as_the_device_is_told():
+    """A tenth of a second and more of work ahead of the draw, in a process whose waits for the device sleep: the call does not keep a core busy all that time."""
+    r = subprocess.run([sys.executable, "-c", WAITER % str(Path(__file__).resolve().parents[1])], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+    wall, cpu, same = r.stdout.split("WAITED")[1].split()
+    assert same == "True" and float(wall) > 0.1 and float(cpu) < 0.02 + 0.4 * float(wall), r.stdout
 
 
 @pytest.mark.gpu
