@@ -3,6 +3,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "common.cuh"
 
@@ -78,6 +81,17 @@ bool pdl_enabled() {
         return !(e && e[0] == '1');
     }();
     return on;
+}
+
+int raise_smem_limit(lumen_ctx *ctx, const void *kernel, size_t bytes) {
+    static std::mutex lock;
+    static std::map<std::pair<const void *, int>, size_t> limits;
+    std::lock_guard<std::mutex> held(lock);
+    size_t &limit = limits[{kernel, ctx->device}];
+    if (bytes <= limit) return LUMEN_OK;
+    LUMEN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    limit = bytes;
+    return LUMEN_OK;
 }
 
 int kv_resync_len(lumen_kv_cache *c) {

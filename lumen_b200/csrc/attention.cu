@@ -586,8 +586,7 @@ int launch_decode_gt(lumen_ctx *ctx, const DecodeParams &p, int ni, dim3 grid, s
 #define LD(NI_)                                                                                                       \
     do {                                                                                                              \
         auto kern = attn_decode_kernel<GT, NI_>;                                                                      \
-        if (smem > 48 * 1024)                                                                                         \
-            LUMEN_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));      \
+        LUMEN_TRY(allow_smem(ctx, kern, smem));                                                                       \
         kern<<<grid, kThreads, smem, s>>>(p);                                                                         \
     } while (0)
     switch (ni) {

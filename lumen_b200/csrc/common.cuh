@@ -261,6 +261,15 @@ int launch_gemv_gate_up(lumen_ctx *ctx, const float *x, const void *w_gate, cons
 bool gemv_vec_usable(const void *w, lumen_dtype wdt, size_t K);
 int launch_gemv_vec(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype wdt, float *y, size_t K, size_t N, cudaStream_t s);
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit of a kernel is one number for all threads, contexts and captured steps of a
+// device, so it is only ever raised: a smaller call must not lower it below what another is about to launch, or has captured.  (It counts
+// together with the kernel's static shared memory against 48 KB as long as nothing raises it.)
+int raise_smem_limit(lumen_ctx *ctx, const void *kernel, size_t bytes);
+template <typename K>
+int allow_smem(lumen_ctx *ctx, K kernel, size_t bytes) {  // for kernels with less than 16 KB of their own
+    return bytes <= 32 * 1024 ? (int)LUMEN_OK : raise_smem_limit(ctx, reinterpret_cast<const void *>(kernel), bytes);
+}
+
 // y[n] = sum_k w[k, n] * x[k]; w is [K,N] row-major.  Uses `scratch` (>= gemv_kn_scratch_bytes) for
 // split-K partial sums.
 size_t gemv_kn_scratch_bytes(size_t K, size_t N, int num_sms);                           // either weight type

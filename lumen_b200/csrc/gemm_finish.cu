@@ -188,7 +188,7 @@ int launch_step_finish(lumen_ctx *ctx, const float *part, int splits, size_t row
         const size_t smem = n * sizeof(float);
         if (smem > 200 * 1024) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "row finisher: row length %zu", n);
         const auto kernel = f.next_gain ? norm_add_kernel<true> : norm_add_kernel<false>;
-        if (smem > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        LUMEN_TRY(allow_smem(ctx, kernel, smem));
         kernel<<<(unsigned)rows, 256, smem, s>>>(part, part ? splits : 0, rows, n, f);
     } else {
         const size_t total = rows * (f.kind == StepFinish::kGated ? f.ff : n);

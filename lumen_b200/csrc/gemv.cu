@@ -737,14 +737,6 @@ KnPlan plan_kn(size_t K, size_t N, int vec, int num_sms) {
     return p;
 }
 
-template <typename K>
-int set_smem(lumen_ctx *ctx, K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        LUMEN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    }
-    return LUMEN_OK;
-}
-
 int pick_grid(lumen_ctx *ctx, size_t rows, size_t smem_bytes) {
     // Resident CTAs per SM limited by shared memory (227 KB) and by 2048 threads.
     int per_sm = (int)std::min<size_t>(8, (227 * 1024) / std::max<size_t>(smem_bytes + 1024, 1));
@@ -758,7 +750,7 @@ template <typename WT, int MB>
 int launch_nk_t(lumen_ctx *ctx, const GemvArgs &a, cudaStream_t s) {
     size_t smem = (size_t)MB * a.K * sizeof(float);
     auto kern = gemv_nk_kernel<WT, MB>;
-    LUMEN_TRY(set_smem(ctx, kern, smem));
+    LUMEN_TRY(allow_smem(ctx, kern, smem));
     int grid = pick_grid(ctx, a.N, smem);
     kern<<<grid, kThreads, smem, s>>>(a.x, static_cast<const WT *>(a.w), a.y, a.M, a.K, a.N, a.ldy, a.norm_w,
                                       a.norm_eps, a.residual);
@@ -771,7 +763,7 @@ int launch_gate_up_t(lumen_ctx *ctx, const float *x, const void *wg, const void 
                      size_t I, const float *norm_w, float eps, cudaStream_t s) {
     size_t smem = (size_t)MB * K * sizeof(float);
     auto kern = gemv_gate_up_kernel<WT, MB>;
-    LUMEN_TRY(set_smem(ctx, kern, smem));
+    LUMEN_TRY(allow_smem(ctx, kern, smem));
     int grid = pick_grid(ctx, I, smem);
     kern<<<grid, kThreads, smem, s>>>(x, static_cast<const WT *>(wg), static_cast<const WT *>(wu), out, M, K, I, norm_w,
                                       eps);
@@ -809,12 +801,12 @@ int launch_gemv_vec(lumen_ctx *ctx, const float *x, const void *w, lumen_dtype w
     int rc;
     if (wpr == 1 && wdt == LUMEN_BF16 && row_bytes >= 2048) {
         const int pairs = (int)std::min<size_t>(((N + 1) / 2 + kWarps - 1) / kWarps, (size_t)ctx->num_sms * 2);
-        rc = set_smem(ctx, gemv_vec_pair_kernel, smem);
+        rc = allow_smem(ctx, gemv_vec_pair_kernel, smem);
         if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_pair_kernel, pairs, kThreads, smem, s, x, static_cast<const __nv_bfloat16 *>(w), y, (int)K, N);
         ctx->pdl = pdl;
         return rc;
     }
-#define LUMEN_VEC(T_, W_) rc = set_smem(ctx, gemv_vec_kernel<T_, W_>, smem); if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_kernel<T_, W_>, grid, kThreads, smem, s, x, static_cast<const T_ *>(w), y, (int)K, N)
+#define LUMEN_VEC(T_, W_) rc = allow_smem(ctx, gemv_vec_kernel<T_, W_>, smem); if (rc == LUMEN_OK) rc = launch_pdl(ctx, gemv_vec_kernel<T_, W_>, grid, kThreads, smem, s, x, static_cast<const T_ *>(w), y, (int)K, N)
 #define LUMEN_VEC_T(T_) do { if (wpr == 8) { LUMEN_VEC(T_, 8); } else if (wpr == 4) { LUMEN_VEC(T_, 4); } else if (wpr == 2) { LUMEN_VEC(T_, 2); } else { LUMEN_VEC(T_, 1); } } while (0)
     if (wdt == LUMEN_F32) LUMEN_VEC_T(float);
     else LUMEN_VEC_T(__nv_bfloat16);
@@ -854,7 +846,7 @@ int launch_gemv_step(lumen_ctx *ctx, const GemvStepArgs &a, cudaStream_t s) {
         const int g2 = (int)std::min((pairs * (split ? 2 : 1) + kWarps - 1) / kWarps, pair_warps / kWarps);
 #define LUMEN_PAIR(W_, G_)                                                                            \
     do {                                                                                              \
-        LUMEN_TRY(set_smem(ctx, gemv_step_pair_kernel<W_, G_>, smem));                                \
+        LUMEN_TRY(allow_smem(ctx, gemv_step_pair_kernel<W_, G_>, smem));                                \
         return launch_pdl(ctx, gemv_step_pair_kernel<W_, G_>, g2, kThreads, smem, s, a);              \
     } while (0)
         if (gated) {
@@ -870,7 +862,7 @@ int launch_gemv_step(lumen_ctx *ctx, const GemvStepArgs &a, cudaStream_t s) {
     const int grid = std::min(pick_grid(ctx, rows * wpr, smem), ctx->num_sms * kStepCtas);
 #define LUMEN_STEP_G(T_, W_, G_)                                                               \
     do {                                                                                       \
-        LUMEN_TRY(set_smem(ctx, gemv_step_kernel<T_, W_, G_>, smem));                          \
+        LUMEN_TRY(allow_smem(ctx, gemv_step_kernel<T_, W_, G_>, smem));                          \
         return launch_pdl(ctx, gemv_step_kernel<T_, W_, G_>, grid, kThreads, smem, s, a);      \
     } while (0)
 #define LUMEN_STEP(T_, W_)                                                                     \

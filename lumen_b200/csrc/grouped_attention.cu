@@ -395,7 +395,7 @@ template <typename T, int GT, int NI, bool EVEN>
 int launch_rows(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s) {
     constexpr int NV = rows_in_flight(NI) * GT;
     const size_t smem = ((GT + 1) * a.dim + 2 * kWarps * GT + kWarps * (NV + GT) + (size_t)kWarps * GT * a.vdim) * sizeof(float);
-    if (smem > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_rows_kernel<T, GT, NI, EVEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LUMEN_TRY(allow_smem(ctx, grouped_rows_kernel<T, GT, NI, EVEN>, smem));
     const dim3 grid((unsigned)a.nsplit, (unsigned)(a.H / GT), (unsigned)std::min<size_t>(a.B * a.S, 65535));
     return launch_pdl(ctx, grouped_rows_kernel<T, GT, NI, EVEN>, grid, kThreads, smem, s, a, append ? 1 : 0);
 }

@@ -247,10 +247,10 @@ int launch(lumen_ctx *ctx, const GroupedArgs &a, bool append, cudaStream_t s) {
     size_t smem = (kWarps * a.dim + 2 * kWarps * kMmaHeads + (size_t)kWarps * kMmaHeads * a.vdim) * sizeof(float);
     if (a.nsplit == 0) {
         smem += (kMmaHeads * a.vdim + kOnePieces + 2 * kOnePieces * kMmaHeads) * sizeof(float);
-        if (smem > 40 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_mma_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        LUMEN_TRY(allow_smem(ctx, grouped_mma_kernel<KB, VB, true>, smem));
         return launch_pdl_cluster(ctx, grouped_mma_kernel<KB, VB, true>, kOnePieces, dim3(kOnePieces, (unsigned)(a.G * groups)), dim3(kThreads), smem, s, a, append ? 1 : 0);
     }
-    if (smem > 40 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(grouped_mma_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LUMEN_TRY(allow_smem(ctx, grouped_mma_kernel<KB, VB, false>, smem));
     const dim3 grid((unsigned)a.nsplit, (unsigned)(a.G * groups), (unsigned)std::min<size_t>(a.B * a.S, 65535));
     return launch_pdl(ctx, grouped_mma_kernel<KB, VB, false>, grid, kThreads, smem, s, a, append ? 1 : 0);
 }

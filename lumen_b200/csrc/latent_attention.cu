@@ -310,7 +310,7 @@ int launch_scores_t(lumen_ctx *ctx, const LatentArgs &a, cudaStream_t s) {
     const dim3 grid((unsigned)a.nsplit, (unsigned)std::min<size_t>(65535, a.B * a.S * a.H));
 #define LUMEN_SCORES(NI_)                                                                                                                \
     do {                                                                                                                                 \
-        if (smem > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(latent_scores_kernel<T, NI_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        LUMEN_TRY(allow_smem(ctx, latent_scores_kernel<T, NI_>, smem));                                                                  \
         return launch_pdl(ctx, latent_scores_kernel<T, NI_>, grid, kScoreWarps * 32, smem, s, a);                                         \
     } while (0)
     if (a.rank <= 128) LUMEN_SCORES(4);

@@ -264,12 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_attn_mma_kernel(const Late
 template <int MT, int NT>
 int launch_t(lumen_ctx *ctx, const LatentArgs &a, cudaStream_t s) {
     const size_t smem = mma_geom(MT * 16, (int)a.pitch).total;
-    static size_t set[64] = {0};
-    const int dev = ctx->device >= 0 && ctx->device < 64 ? ctx->device : 0;
-    if (smem > set[dev]) {
-        LUMEN_CUDA(ctx, cudaFuncSetAttribute(latent_attn_mma_kernel<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        set[dev] = smem;
-    }
+    LUMEN_TRY(allow_smem(ctx, latent_attn_mma_kernel<MT, NT>, smem));
     const size_t rows = a.S * a.H;
     return launch_pdl(ctx, latent_attn_mma_kernel<MT, NT>, dim3((unsigned)a.nsplit, (unsigned)((rows + MT * 16 - 1) / (MT * 16)), (unsigned)a.B), kThreads,
                       smem, s, a);

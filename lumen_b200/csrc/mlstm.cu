@@ -231,7 +231,7 @@ int launch_step(lumen_ctx *ctx, const MlstmArgs &a, int cols, unsigned slices, c
     const int nx = cols / VEC, ny = kThreads / nx;
     const size_t smem = ((size_t)T * (3 * a.dim + (size_t)ny * cols) + a.dim) * sizeof(float);
     if (smem > 200 * 1024) return set_error(ctx, LUMEN_ERR_UNSUPPORTED, "matrix memory: keys of %zu numbers", a.dim);
-    if (smem > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(mlstm_step_kernel<VEC, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LUMEN_TRY(allow_smem(ctx, mlstm_step_kernel<VEC, T>, smem));
     return launch_pdl_cluster(ctx, mlstm_step_kernel<VEC, T>, slices, dim3(slices, (unsigned)a.H, (unsigned)a.B), kThreads, smem, s, a, cols, nx, ny);
 }
 

@@ -220,8 +220,8 @@ size_t down_smem(const MoeArgs &a) { return (a.top * (((a.ff + 3) & ~(size_t)3) 
 template <typename WT>
 int launch_vec_t(lumen_ctx *ctx, const MoeArgs &a, cudaStream_t s) {
     const size_t s1 = gate_up_smem(a), s2 = down_smem(a);
-    if (s1 > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(moe_gate_up_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
-    if (s2 > 48 * 1024) LUMEN_CUDA(ctx, cudaFuncSetAttribute(moe_down_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
+    LUMEN_TRY(allow_smem(ctx, moe_gate_up_kernel<WT>, s1));
+    LUMEN_TRY(allow_smem(ctx, moe_down_kernel<WT>, s2));
     auto blocks = [&](size_t rows, size_t smem, size_t per_cta) {
         const size_t per_sm = std::max<size_t>(1, std::min<size_t>(8, 227 * 1024 / (smem + 1024)));
         return (unsigned)std::max<size_t>(1, std::min((rows + per_cta - 1) / per_cta, (size_t)ctx->num_sms * per_sm));

@@ -129,7 +129,7 @@ def test_products_of_two_rows_per_warp(L, dtype, width, ff, vocab):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("width", [2048, 2052])
+@pytest.mark.parametrize("width", [2048, 2052, 12288])
 def test_widest_rows_with_gains_in_shared_memory(L, dtype, width):
     """One-row products keep the gains of both norms in shared memory up to 2048 numbers and read them when they need them beyond."""
     cfg = K.config([(K.attn(heads=2, kv_heads=1, dim=16, vdim=16, chunk=100, rot_dims=8, scaling=None, scale=0.3), 24)], width=width)

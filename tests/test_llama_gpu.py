@@ -312,6 +312,17 @@ def test_caches_in_turn(L, batch):
                 assert np.array_equal(got[:, 0], want[i][:, t - 3]), (t, i)
 
 
+@pytest.mark.parametrize("hidden,batch", [(1536, 8), (3072, 3), (6144, 2)])
+def test_steps_whose_input_fills_the_default_shared_memory(L, oracle, hidden, batch):
+    """Normed inputs of exactly 48 KB in the products of two to eight rows."""
+    cfg = small_cfg(hidden_size=hidden, num_attention_heads=2, num_key_value_heads=1, head_dim=32, intermediate_size=48)
+    params = make_params(L, cfg, 70, std=0.02)
+    ids = np.random.default_rng(71).integers(0, cfg["vocab_size"], size=(batch, 4)).astype(np.float32)
+    got, _, _ = _gpu_run(L, cfg, params, ids, 1)
+    want, _ = _oracle_run(oracle, cfg, params, ids, 1)
+    assert rel_err(got, want) < TOL_F32
+
+
 def test_caches_of_different_lengths(L):
     """Caches made one by one may hold different numbers of rows: such a set decodes as a set of equal ones does, and writes to its own rows alone."""
     cfg = small_cfg()

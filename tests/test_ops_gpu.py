@@ -150,7 +150,7 @@ def test_gemv_kn_layout_raw_pointers(L, oracle, ctx, k, n, bf16):
     assert rel_err(y[pad:-pad], oracle.matmul(x[None], w_nk, "f64")[0]) < 2e-6
 
 @pytest.mark.parametrize("k,n", [(4, 1), (8, 9), (2052, 5), (512, 2368), (512, 2369), (1024, 1184), (1032, 1185), (4096, 592), (4096, 593), (8200, 3), (8192, 297),
-                                 (1016, 2400), (1024, 2369), (1032, 2370), (2056, 4737)])
+                                 (1016, 2400), (1024, 2369), (1032, 2370), (2056, 4737), (12288, 5), (12288, 2400)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_gemv_warps_per_row(L, oracle, ctx, k, n, bf16):
     """[N,K] products on raw pointers on both sides of every change of the warps that share a row, and rows that end inside a warp's step.
@@ -167,6 +167,40 @@ def test_gemv_warps_per_row(L, oracle, ctx, k, n, bf16):
     assert np.all(got[:32] == 777.0) and np.all(got[-32:] == 777.0)
     want = w.astype(np.float64) @ x
     assert np.abs(got[32:-32] - want).max() < 4 * 2.0 ** -24 * np.sqrt(k) * np.sqrt((w.astype(np.float64) ** 2 @ x.astype(np.float64) ** 2).max())
+
+
+@pytest.mark.parametrize("m,k,bf16", [(1, 12288, False), (1, 12288, True), (2, 6144, False), (4, 3072, False), (7, 1536, False), (8, 1536, False)])
+def test_products_whose_input_fills_the_default_shared_memory(L, m, k, bf16):
+    """Staged inputs of exactly 48 KB (a kernel that has some shared memory of its own needs a raised limit for them); tolerance as above."""
+    rng = np.random.default_rng(k + m)
+    a, w = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((333, k), dtype=np.float32)
+    wt = L.Tensor.from_bf16(w) if bf16 else L.Tensor.from_array_no_grad(w)
+    got, wd = L.matmul(L.Tensor.from_array_no_grad(a), wt).data(), wt.data().astype(np.float64)
+    assert np.abs(got - a @ wd.T).max() < 4 * 2.0 ** -24 * np.sqrt(k) * np.sqrt((a.astype(np.float64) ** 2 @ (wd ** 2).T).max())
+
+
+def test_threads_with_products_of_different_sizes(L):
+    """The shared-memory limit of a kernel is one number for all threads: calls of one size do not lower it below what a call of another is about to launch."""
+    import threading
+    errors = []
+
+    def work(k):
+        try:
+            ctx = L.Context()
+            x, w, y = (L.Tensor.from_array_no_grad(np.ones(s, np.float32), ctx) for s in ((k,), (16, k), (16,)))
+            for i in range(4000):
+                L.gemv(ctx, x.data_ptr, w.data_ptr, L.F32, False, k, 16, y.data_ptr)
+            if not np.array_equal(y.data(), np.full(16, k, np.float32)):
+                errors.append(k)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (24000, 13000, 16000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
 
 
 @pytest.mark.parametrize("kn", [False, True])
