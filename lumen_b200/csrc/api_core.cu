@@ -22,6 +22,7 @@ int set_error(lumen_ctx *ctx, int code, const char *fmt, ...) {
 }
 
 int cuda_fail(lumen_ctx *ctx, cudaError_t e, const char *what) {
+    cudaGetLastError();  // reported here: the check behind the next launch must not find it again
     return set_error(ctx, LUMEN_ERR_CUDA, "CUDA error %d (%s) in %s", (int)e, cudaGetErrorString(e), what);
 }
 

@@ -123,6 +123,15 @@ def test_matmul_batched_leading_dims_and_errors(L, oracle):
     assert e.value.code == L._lib.ERR_SHAPE
 
 
+def test_a_refused_call_is_reported_once(L, ctx):
+    """An allocation of 2 TB is refused by the call that asks for it; the calls behind it run."""
+    import ctypes
+    with pytest.raises(L.LumenError) as e:
+        ctx.check(ctx._lib.lumen_tensor_empty(ctx.h, (ctypes.c_size_t * 2)(1 << 20, 1 << 19), 2, L.F32, ctypes.byref(ctypes.c_void_p())))
+    assert e.value.code == L._lib.ERR_CUDA
+    assert np.array_equal(L.matmul(L.Tensor.from_array_no_grad(np.ones((2, 8))), L.Tensor.from_array_no_grad(np.ones((3, 8)))).data(), np.full((2, 3), 8.0, np.float32))
+
+
 @pytest.mark.parametrize("k,n", [(2048, 2048), (2048, 256), (5632, 2048), (2048, 32000), (100, 37), (33, 5)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_gemv_kn_layout_raw_pointers(L, oracle, ctx, k, n, bf16):
