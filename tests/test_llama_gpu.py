@@ -3,6 +3,8 @@ and the committed fixtures.  Tolerances are the north star's: per-step logits wi
 f32 weights, 1e-2 for bf16 weights (rel = max|a-b| / max|b| over one logits vector), and identical
 argmax token ids under teacher forcing."""
 import os
+import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -11,6 +13,7 @@ import pytest
 from helpers import PAIRED_PROMPTS, TOL_BF16, TOL_F32, cfg_obj, make_params, rel_err, small_cfg
 
 pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
 GOLD = Path(__file__).resolve().parent / "golden"
 
 
@@ -321,6 +324,43 @@ def test_steps_whose_input_fills_the_default_shared_memory(L, oracle, hidden, ba
     got, _, _ = _gpu_run(L, cfg, params, ids, 1)
     want, _ = _oracle_run(oracle, cfg, params, ids, 1)
     assert rel_err(got, want) < TOL_F32
+
+
+PROMPTS = """
+import sys
+sys.path[:0] = [%r, %r]
+import numpy as np
+import lumen_b200 as L
+from helpers import cfg_obj, make_params, small_cfg
+cfg = small_cfg(hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=64, intermediate_size=520, num_hidden_layers=4, max_seq_len=1100)
+wide = {**cfg, "head_dim": 128, "num_attention_heads": 2, "qk_norm": True}
+out = []
+for c, wdt, batch, parts in ((cfg, "f32", 1, (1000,)), (cfg, "bf16", 3, (300, 200)), (wide, "bf16", 1, (513, 90, 400)), (wide, "f32", 2, (130, 700))):
+    model = L.LlamaModel(cfg_obj(L, c, wdt))
+    model.load_state(make_params(L, c, 73, std=0.05, round_bf16=wdt == "bf16"))
+    caches, at = model.init_kv_caches(batch), 0
+    ids = np.random.default_rng(74).integers(0, c["vocab_size"], size=(batch, sum(parts))).astype(np.float32)
+    with L.no_grad():
+        for n in parts:
+            out.append(model.forward(ids[:, at:at + n], caches, 0))
+            at += n
+np.savez(sys.argv[1], *out)
+"""
+
+
+def test_prompts_with_and_without_dependent_launch(tmp_path):
+    """The kernels of a long prompt start while the ones before them run, or one behind the other: the logits are the same bit for bit."""
+    got = []
+    for plain in ("0", "1"):
+        path = tmp_path / f"{plain}.npz"
+        r = subprocess.run([sys.executable, "-c", PROMPTS % (str(ROOT), str(ROOT / "tests")), str(path)], capture_output=True, text=True, timeout=300,
+                           env={**os.environ, "LUMEN_NO_PDL": plain})
+        assert r.returncode == 0, r.stderr[-2000:]
+        with np.load(path) as z:
+            got.append([z[n] for n in z.files])
+    assert len(got[0]) == 8
+    for a, b in zip(*got):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
 
 
 def test_caches_of_different_lengths(L):

@@ -239,6 +239,32 @@ def test_gemv_calls_that_feed_each_other(L, ctx, kn):
         assert np.array_equal(chain(False), want)
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("layouts", [(False,), (True,), (False, True), (False, False, True)])
+@pytest.mark.parametrize("k,n", [(1032, 2401), (1024, 2369), (2048, 2370), (264, 2400)])
+def test_gemv_chains_of_other_sizes_and_layouts(L, ctx, bf16, layouts, k, n):
+    """The same with more rows than warps (bf16 rows of 2 KB and more go in pairs), and with the two layouts in turn, which let the next call start at
+    different points: every product reads the first numbers of the one before."""
+    rng = np.random.default_rng(k + n)
+    x = rng.standard_normal(n, dtype=np.float32)
+    w = [rng.standard_normal((k, n) if kn else (n, k), dtype=np.float32) / np.float32(k ** 0.5) for kn in layouts]
+
+    def chain(wait):
+        ws = [L.Tensor.from_bf16(a) if bf16 else L.Tensor.from_array_no_grad(a) for a in w]
+        v = [L.Tensor.from_array_no_grad(x), L.Tensor.from_array_no_grad(np.zeros(n, np.float32))]
+        for i in range(24):
+            j = i % len(layouts)
+            L.gemv(ctx, v[i % 2].data_ptr, ws[j].data_ptr, L.BF16 if bf16 else L.F32, layouts[j], k, n, v[(i + 1) % 2].data_ptr)
+            if wait:
+                ctx.synchronize()
+        return v[0].data()
+
+    want = chain(True)
+    assert np.isfinite(want).all() and np.abs(want).max() > 0
+    for _ in range(6):
+        assert np.array_equal(chain(False), want)
+
+
 
 @pytest.mark.parametrize("k,n", [(1, 1), (7, 9), (64, 8), (65, 130), (256, 127), (300, 33), (511, 2049), (2049, 1031), (4097, 257), (1000, 40000), (70, 99001), (12288, 128)])
 @pytest.mark.parametrize("offset", [0, 1])
