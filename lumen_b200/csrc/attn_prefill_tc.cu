@@ -102,7 +102,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_qhi, const __grid
     volatile int *failed = &failed_s;
     const int tid = threadIdx.x, warp = tid >> 5;
     // The last tiles of a causal prompt walk the most rows: those of all heads go first, so that what is left at the end is short (one head after
-    // another, the SMs worked 70 % of the time on a prompt of 1777 positions and 32 heads).
+    // another, the SMs worked 70 % of the time on a prompt of 1777 positions and 32 heads).  That neighbours then share no keys costs nothing, also where K and V of all
+    // heads exceed the L2: four layers of the 7B shape, 4 x 2048 positions, 21.3 ms this way, 21.4 head by head, 21.2 to 21.3 in groups of 16 to 64 heads; 2 x 2048 11.0, 11.1, 11.0;
+    // 1 x 700 2172 us, 2213, 2174; of TinyLlama f32, 1777 positions, 2009 us, 2096, 2013.
     const int lin = (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)), rows_all = (int)(gridDim.y * gridDim.z);
     const int qt = (int)gridDim.x - 1 - lin / rows_all, h = lin % rows_all % (int)gridDim.y, b = lin % rows_all / (int)gridDim.y;
     const int hk = h / (p.Hq / p.Hkv);

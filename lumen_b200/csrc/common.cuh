@@ -40,7 +40,7 @@ struct lumen_ctx {
     unsigned long long *h_answer = nullptr;   // pinned: the device sampler's answer, turn << 32 | token
     unsigned int answer_turn = 0;
     char err[512] = {0};
-    bool pdl = false;  // launch_pdl may overlap kernels now (set by steps that consist of such launches alone)
+    bool pdl = false;  // launch_pdl may overlap kernels now (set where every kernel launched so waits for its predecessor; plain launches may stand between)
     unsigned long long launches = 0;  // kernels enqueued so far (graph replays add their node count)
     // Persistent decode kernel: 16 device bytes whose second word is the cross-CTA abort flag, and the
     // epoch from which the next launch derives the tags of its exchanged activations.
@@ -141,7 +141,8 @@ int cuda_fail(lumen_ctx *ctx, cudaError_t e, const char *what);
 // Launches a kernel that may start while its predecessor on the stream still runs (programmatic dependent launch; captured
 // into graphs as such).  The kernel calls pdl_wait() before it touches anything a predecessor writes - until then it may
 // read weights - and pdl_launch() once its own successor may start the same way.  Every kernel launched so waits, so the end of a
-// kernel implies the end of all before it.  Plain launches unless ctx->pdl is set; LUMEN_NO_PDL=1: always plain.
+// kernel implies the end of all before it.  Plain launches unless ctx->pdl is set (the public
+// vector products set it for their own launch); LUMEN_NO_PDL=1: always plain.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

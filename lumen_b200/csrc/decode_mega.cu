@@ -25,7 +25,7 @@
 // per phase at some four cycles an instruction (time stamps of a phase, in cycles: 900 to 2400 from the input to the first tile,
 // 1600 to 2300 for that tile, 560 to 1200 for the epilogue).  So what does not depend on the input is settled before the wait for it, words that
 // have arrived are not polled again, and the epilogue is kept short: TinyLlama f32 884 -> 839 us a token, bf16 667 -> 630,
-// Llama-2-7B bf16 2613 -> 2537.  And the kernel is kept free of register spills: with the L1 squeezed by
+// Llama-2-7B bf16 2613 -> 2537 (831, 625 and 2518 with the attention kept off the L2).  And the kernel is kept free of register spills: with the L1 squeezed by
 // ~220 KB of shared memory a spill reload inside the tile loop is a round trip through L2.
 //
 // Activations cross CTAs through global memory (L2) as tagged words {f32 bits, tag}: a consumer polls
@@ -61,7 +61,9 @@ constexpr int kPartCols = kMaxSeg;         // columns of the table of partial ro
 constexpr int kMaxSplit = 4;               // attention splits merged in the o_proj prologue
 constexpr int kKvTileRows = 64;            // cached rows of a K or V tile at most (two scores per lane)
 constexpr long long kWaitCycles = 400000000LL;  // ~0.2 s at 1.9 GHz
-constexpr long long kPrefetchGrace = 300;       // a ring that has been full for this long is a stall, not back-pressure (1000: TinyLlama f32 835 us instead of 831)
+// A ring that has been full for this long is a stall, not back-pressure.  300 / 600 / 1000 cycles, us a token in turn: TinyLlama f32 823 / 825 / 827, bf16 677 in
+// all three at 1023 positions; Llama-2-7B bf16 2506 / 2518 / 2509, its first 8 layers 643 / 642 / 641; 9 layers of Qwen3-8B 858 / 857 / 855 at 300 positions, 895 / 906 / 905 at 1500.
+constexpr long long kPrefetchGrace = 300;
 constexpr long long kPrefetchPace = 600;        // cycles between the L2 prefetches of consecutive 16 KB tiles (~54 KB/us)
 
 // Floats of the staged input vector of a phase (up to kmax elements, zero-padded to four whole steps of a

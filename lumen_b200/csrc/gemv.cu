@@ -150,8 +150,8 @@ gemv_nk_kernel(const float *__restrict__ x, const WT *__restrict__ w, float *__r
 // the first of them requested before x is staged and the next row's while a row is summed up.  WPR warps share a row where rows
 // are fewer than warps would be.
 // What bounds it: launch, first bytes and staging for matrices of a few MB, HBM for large ones.  Calls behind one another, other weights every time:
-// f32 [256,2048] 6.7 -> 2.65 us (three quarters of it the overlap), [4096,4096] 15.7 -> 12.3, [32000,4096] 79.9 -> 75.9 (6.9 TB/s);
-// bf16 [4096,4096] 11.7 -> 8.8, [12288,12288] 62.3 -> 54.9 (5.5 TB/s).
+// f32 [256,2048] 6.7 -> 2.65 us (three quarters of it the overlap), [4096,4096] 15.7 -> 12.1, [32000,4096] 79.9 -> 76.1 (6.9 TB/s);
+// bf16 (fewer rows than warps, or rows below 2 KB; others go to the kernel behind this one) [256,2048] 4.6 -> 2.45, [2048,2048] 6.2 -> 4.0, [512,8192] 8.8 -> 4.8.
 template <typename WT, int WPR>
 __global__ void __launch_bounds__(kThreads, 4) gemv_vec_kernel(const float *x, const WT *w, float *y, int K, size_t N) {
     extern __shared__ __align__(16) float smem[];
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_vec_pair_kernel(const float 
     for (size_t p = p0; p < pairs; p += step) {
         float v[2];
         const bool more = p + step < pairs;
-        pair_dot_ahead<WT, true>(at(p, 0), at(p, 1), smem, nv, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
+        pair_dot_ahead<true>(at(p, 0), at(p, 1), smem, nv, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_step_pair_kernel(const GemvS
         float v[2] = {0.f, 0.f};
         if (p < pairs) {
             const bool more = p + step < pairs;
-            pair_dot_ahead<WT>(at(p, 0), at(p, 1), xs + v0 * VEC, vn, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
+            pair_dot_ahead(at(p, 0), at(p, 1), xs + v0 * VEC, vn, lane, cur, more ? at(p + step, 0) : nullptr, more ? at(p + step, 1) : nullptr, v);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {

@@ -162,11 +162,11 @@ __device__ __forceinline__ float row_dot_ahead(const uint4 *row, const float *xs
     }
     return acc;
 }
-// Two rows at once: every read of x from shared memory serves both.
-template <typename WT, bool LIVE = false>
+// Two bf16 rows at once: every read of x from shared memory serves both.
+template <bool LIVE = false>
 __device__ __forceinline__ void pair_dot_ahead(const uint4 *row0, const uint4 *row1, const float *xs, int n, int lane, uint4 (&cur)[2][kAhead],
                                                const uint4 *next0, const uint4 *next1, float (&acc)[2]) {
-    constexpr int VEC = 16 / sizeof(WT);
+    constexpr int VEC = 8;
     acc[0] = acc[1] = 0.f;
 #pragma unroll 1
     for (int base = 0; base < n; base += kAhead * 32) {
@@ -179,27 +179,17 @@ __device__ __forceinline__ void pair_dot_ahead(const uint4 *row0, const uint4 *r
             const int i = base + u * 32 + lane;
             if (i >= n) continue;
             const float4 x0 = *reinterpret_cast<const float4 *>(xs + i * VEC);
-            if constexpr (sizeof(WT) == 4) {
+            const float4 x1 = *reinterpret_cast<const float4 *>(xs + i * VEC + 4);
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    acc[r] = fmaf(__uint_as_float(cur[r][u].x), x0.x, acc[r]);
-                    acc[r] = fmaf(__uint_as_float(cur[r][u].y), x0.y, acc[r]);
-                    acc[r] = fmaf(__uint_as_float(cur[r][u].z), x0.z, acc[r]);
-                    acc[r] = fmaf(__uint_as_float(cur[r][u].w), x0.w, acc[r]);
-                }
-            } else {
-                const float4 x1 = *reinterpret_cast<const float4 *>(xs + i * VEC + 4);
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    acc[r] = fmaf(bf16_lo(cur[r][u].x), x0.x, acc[r]);
-                    acc[r] = fmaf(bf16_hi(cur[r][u].x), x0.y, acc[r]);
-                    acc[r] = fmaf(bf16_lo(cur[r][u].y), x0.z, acc[r]);
-                    acc[r] = fmaf(bf16_hi(cur[r][u].y), x0.w, acc[r]);
-                    acc[r] = fmaf(bf16_lo(cur[r][u].z), x1.x, acc[r]);
-                    acc[r] = fmaf(bf16_hi(cur[r][u].z), x1.y, acc[r]);
-                    acc[r] = fmaf(bf16_lo(cur[r][u].w), x1.z, acc[r]);
-                    acc[r] = fmaf(bf16_hi(cur[r][u].w), x1.w, acc[r]);
-                }
+            for (int r = 0; r < 2; ++r) {
+                acc[r] = fmaf(bf16_lo(cur[r][u].x), x0.x, acc[r]);
+                acc[r] = fmaf(bf16_hi(cur[r][u].x), x0.y, acc[r]);
+                acc[r] = fmaf(bf16_lo(cur[r][u].y), x0.z, acc[r]);
+                acc[r] = fmaf(bf16_hi(cur[r][u].y), x0.w, acc[r]);
+                acc[r] = fmaf(bf16_lo(cur[r][u].z), x1.x, acc[r]);
+                acc[r] = fmaf(bf16_hi(cur[r][u].z), x1.y, acc[r]);
+                acc[r] = fmaf(bf16_lo(cur[r][u].w), x1.z, acc[r]);
+                acc[r] = fmaf(bf16_hi(cur[r][u].w), x1.w, acc[r]);
             }
         }
 #pragma unroll

@@ -1,6 +1,7 @@
 // Prints the plans of products and of decode attention, one per line of its input:
 //   plain M K N bf16   ->  bn splits kb_per_split          (bn 0: 128 x 128 tiles of single SMs)
 //   pair M K N products swiglu may_split   ->  the same
+//   width M N swiglu splits   ->  columns of a tile where the plan has 256
 //   attn B Hq Hkv D len   ->  parts of a batched decode step's context (0: the general kernel)
 #include <cstdio>
 #include <cstring>
@@ -13,6 +14,11 @@ int main() {
     size_t m, k, n;
     while (std::scanf("%15s %zu %zu %zu", kind, &m, &k, &n) == 4) {
         int a = 0, b = 0, c = 0;
+        if (!std::strcmp(kind, "width")) {
+            if (std::scanf("%d", &a) != 1) return 1;
+            std::printf("%d\n", lumen::pair_width(m, k, n != 0, a, 148));
+            continue;
+        }
         if (!std::strcmp(kind, "attn")) {
             size_t d, len;
             if (std::scanf("%zu %zu", &d, &len) != 2) return 1;

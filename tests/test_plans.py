@@ -41,6 +41,21 @@ def test_plain_products_take_the_kernel_that_was_faster(plan, m, k, n, bf16, sin
     assert times[bn] <= 1.1 * min(times.values()) and splits == 1 and per * 64 >= k
 
 
+# m, k, n, bf16 weights, microseconds with tiles of 256, 224 and 192 columns
+WIDTHS = [
+    (3000, 1024, 1024, False, 38.6, 36.5, 34.8), (1536, 2048, 2560, False, 64.7, 60.7, 78.6), (4096, 2048, 2560, False, 139.3, 128.0, 134.4),
+    (1777, 2048, 5632, False, 134.6, 123.6, 113.6), (900, 4096, 24576, False, 577.7, 535.0, 540.5), (257, 1024, 32000, False, 133.8, 126.1, 131.6),
+    (4096, 4096, 6144, True, 331.5, 328.9, 331.7), (1280, 12288, 4096, True, 276.7, 249.9, 241.7), (1777, 11008, 4096, True, 266.5, 251.0, 322.4),
+    (1777, 5632, 2048, True, 83.6, 78.1, 116.7), (513, 4096, 4096, True, 57.8, 53.2, 52.4),
+]
+
+
+@pytest.mark.parametrize("m,k,n,bf16,w256,w224,w192", WIDTHS)
+def test_widths_of_tiles_that_were_faster(plan, m, k, n, bf16, w256, w224, w192):
+    (bn,) = plan("width", m, n, 0, 1)
+    assert plan("plain", m, k, n, bf16)[0] == 256 and {256: w256, 224: w224, 192: w192}[bn] <= 1.02 * min(w256, w224, w192)
+
+
 def test_sizes_of_the_gpu_tests_reach_what_they_claim(plan):
     for m, k, n in PAIRED_PRODUCTS[:-1]:
         assert plan("plain", m, k, n, True)[0] == plan("plain", m, k, n, False)[0] == 256
